@@ -6,8 +6,8 @@
 One step = one sum all-reduce of a 128 MiB fp32 message per rank (inputs larger
 than the 126 MB L2) between pre-allocated symmetric buffers.  N > 1 runs one rank
 per GPU (torchrun exports RANK / LOCAL_RANK / WORLD_SIZE / MASTER_*); N = 1 has no
-peer, so two ranks are emulated on the one GPU by a single cooperative launch of
-the same kernels (HBM-bound, no NVLink) and the line says so.  Timing: CUDA events
+peer, so two ranks are emulated on the one GPU by a single launch that exchanges
+nothing (csrc/kernels/local_group.cu: HBM-bound, no NVLink) and the line says so.  Timing: CUDA events
 per step on the launching stream after W warm-up steps, barrier + synchronize on
 both sides, max over ranks.  The line also carries p50/p99 latency of a 1 MiB
 all-reduce (1000 calls replayed from one CUDA graph, rotating over buffers that
@@ -344,7 +344,7 @@ def run_own(args) -> dict:
             "model": "sum all-reduce, 128 MiB fp32 per rank, pre-allocated symmetric buffers",
             "global_batch": MESSAGE_BYTES * ranks,
             "seq_len": elems,
-            "parallelism": ("1 GPU: 2 ranks emulated in one cooperative launch (HBM-bound, no NVLink)" if emulated
+            "parallelism": ("1 GPU: 2 ranks emulated in one launch (HBM-bound, no NVLink)" if emulated
                             else f"{ranks} ranks, one GPU per process"),
             "l2": "inputs (128 MiB per rank) larger than L2; 1 MiB latency rotates over 320 MiB of buffers",
             "metric_note": "busBw = bytes per rank x 2(N-1)/N / time: a per-link rate that ideal scaling keeps "

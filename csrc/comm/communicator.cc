@@ -8,6 +8,7 @@
 
 #include "../core/env.h"
 #include "../kernels/launch.h"
+#include "../kernels/local_group.h"
 #include "../ops/buffer_ops.h"
 #include "topology.h"
 
@@ -431,6 +432,99 @@ Result Communicator::Launch(const Plan& plan, Dtype in, Dtype out, int epilogue,
     return Result::Success;
 }
 
+// The kernels of local_group.cu need every rank's buffers in one launch, and let one thread handle an element
+// for all ranks (or, for rows, one CTA a row for some of them): an output may share memory with an input
+// only where both hold the same element.  Anything else keeps the multi-GPU kernels, whatever they make of it.
+bool Communicator::CanRunInOneLaunch(const void* const* send, void* const* recv, uint64_t send_bytes, uint64_t recv_bytes,
+                                     uint64_t shard_bytes, Dtype in, Dtype out, const OpOptions& opt,
+                                     uint32_t extra_flags) const {
+    static const bool profile = env::ProfileKernels();
+    if (!(emulated_ || world_ == 1) || opt.skip_rank >= 0 || profile) return false;
+    auto overlap = [](const void* a, uint64_t an, const void* b, uint64_t bn) {
+        const char *p = static_cast<const char*>(a), *q = static_cast<const char*>(b);
+        return p < q + bn && q < p + an;
+    };
+    const bool rows = opt.epilogue == kEpiResidualRmsNorm;
+    for (int j = 0; j < nlocal(); ++j) {
+        for (int i = 0; i < nlocal(); ++i) {
+            if (overlap(send[i], send_bytes, recv[j], recv_bytes)) {
+                const char* s = static_cast<const char*>(send[i]);
+                const char* r = static_cast<const char*>(recv[j]);
+                if (rows || in != out) return false;
+                if (extra_flags & kFlagReduceScatterOnly) s += local_[j].rank * shard_bytes;
+                if (extra_flags & kFlagAllGatherOnly) r += local_[i].rank * shard_bytes;
+                if (s != r) return false;
+            }
+            if (!rows) continue;
+            void* ro = opt.residual_out ? opt.residual_out[j] : nullptr;
+            const void* res = opt.residual ? opt.residual[i] : nullptr;
+            if (ro && overlap(send[i], send_bytes, ro, recv_bytes)) return false;
+            if (res && ro && overlap(res, send_bytes, ro, recv_bytes) && !(i == j && res == ro)) return false;
+            if (res && overlap(res, send_bytes, recv[j], recv_bytes) && !(i == j && res == recv[j])) return false;
+        }
+    }
+    return true;
+}
+
+Result Communicator::LaunchLocal(const Plan& plan, const void* const* send, void* const* recv, uint64_t count, Dtype in,
+                                 Dtype out, const OpOptions& opt, const cudaStream_t* streams) {
+    LocalArgs a;
+    std::memset(&a, 0, sizeof(a));
+    for (int i = 0; i < nlocal(); ++i) {
+        const int r = local_[i].rank;
+        a.send[r] = send[i];
+        a.recv[r] = recv[i];
+        a.ctl[r] = reinterpret_cast<uint32_t*>(heaps_->base(r) + lay_.flags_off);
+    }
+    a.count = count;
+    a.shard_elems = plan.shard_elems;
+    a.world = static_cast<uint32_t>(world_);
+    a.flags = plan.flags;
+    a.ep.scale = opt.epilogue == kEpiScaleCast ? opt.scale : 1.0f;
+    const void* fn = nullptr;
+    dim3 grid(1), block(kLocalThreads);
+    uint64_t blocks = 1;
+    if (opt.epilogue == kEpiResidualRmsNorm) {
+        a.ep.eps = opt.eps;
+        a.ep.hidden = opt.hidden;
+        for (int i = 0; i < nlocal(); ++i) {
+            const int r = local_[i].rank;
+            a.residual[r] = opt.residual ? opt.residual[i] : nullptr;
+            a.residual_out[r] = opt.residual_out ? opt.residual_out[i] : nullptr;
+            a.weight[r] = opt.weight[i];
+        }
+        const uint64_t rows = count / opt.hidden;
+        const uint32_t vec = 16 / static_cast<uint32_t>(DtypeSize(in));
+        const LocalNormShape s = LocalNormShapeFor(rows, static_cast<uint32_t>(opt.hidden) / vec, world_, sm_count_);
+        fn = LocalNormKernelFor(in, world_, s);
+        block = dim3(s.threads);
+        blocks = rows * ((world_ + s.ranks_per_cta - 1) / s.ranks_per_cta);
+    } else {
+        const bool rs = plan.flags & kFlagReduceScatterOnly, ag = plan.flags & kFlagAllGatherOnly;
+        fn = LocalKernelFor(in, out, world_, rs ? LocalKind::ReduceScatter : ag ? LocalKind::AllGather : LocalKind::Sum);
+        const uint64_t unit = 16 / std::min(DtypeSize(in), DtypeSize(out));
+        const uint64_t span = rs || ag ? std::min(plan.shard_elems, count) : count;
+        blocks = (span + unit * kLocalThreads - 1) / (unit * kLocalThreads);
+        if (rs || ag) grid.y = static_cast<unsigned>(world_);
+    }
+    if (!fn) return Fail(Result::Unsupported, "no kernel for this dtype / epilogue combination");
+    if (blocks > 0x7fffffffull) return Fail(Result::InvalidArg, "count too large");
+    grid.x = static_cast<unsigned>(blocks);
+    last_.variant = plan.variant;
+    last_.ctas = grid.x * grid.y;
+    last_.slot_bytes = last_.stages = 0;
+    last_.flags = plan.flags;
+    void* params[] = {&a};
+    cudaStream_t s = streams && streams[0] ? streams[0] : local_[0].stream;
+    cudaError_t ce = cudaLaunchKernel(fn, grid, block, params, 0, s);
+    if (ce != cudaSuccess) {
+        (void)cudaGetLastError();
+        return Fail(Result::CudaError, std::string("kernel launch failed: ") + cudaGetErrorString(ce));
+    }
+    last_.launches += 1;
+    return Result::Success;
+}
+
 Result Communicator::Collective(const void* const* send, void* const* recv, uint64_t count, Dtype in, Dtype out,
                                 const OpOptions& opt, const cudaStream_t* streams, uint32_t extra_flags) {
     if (poisoned_) return Fail(Result::Timeout, "communicator is poisoned by an earlier timeout; call Reset()");
@@ -445,10 +539,39 @@ Result Communicator::Collective(const void* const* send, void* const* recv, uint
     const uint64_t send_elems = ag_only ? shard : count, recv_elems = rs_only ? shard : count;
     const uint64_t send_bytes = send_elems * DtypeSize(in), recv_bytes = recv_elems * DtypeSize(out);
 
+    KernelMode mode = opt.mode;
+    if (mode == KernelMode::Auto) mode = env::ForcedKernelMode();
+    PlanCaps caps;
+    caps.half_collective = rs_only || ag_only;
+    caps.force_ctas = opt.ctas > 0 ? static_cast<uint32_t>(opt.ctas) : 0u;
+    caps.force_slot_bytes = opt.slot_bytes > 0 ? static_cast<uint32_t>(opt.slot_bytes) : 0u;
+    caps.vec_ok = true;
+    for (int i = 0; i < nlocal(); ++i) caps.vec_ok = caps.vec_ok && Aligned16(send[i]) && Aligned16(recv[i]);
+    bool norm_ok = true;
+    if (opt.epilogue == kEpiResidualRmsNorm) {
+        const int vec = 16 / static_cast<int>(DtypeSize(in));
+        norm_ok = in == out && opt.hidden > 0 && count % opt.hidden == 0 && opt.hidden % vec == 0 &&
+                  opt.hidden / vec <= 4 * kFlashThreads && opt.weight && caps.vec_ok;
+    }
+    Plan plan;
+    std::string why;
+    Result r;
+    if (mode == KernelMode::Auto && norm_ok &&
+        CanRunInOneLaunch(send, recv, send_bytes, recv_bytes, shard * DtypeSize(in), in, out, opt, extra_flags)) {
+        caps.one_launch = true;
+        r = MakePlan(world_, count, in, out, opt.epilogue, mode, caps, EnvTuningTable(), &plan, &why);
+        if (r != Result::Success) return Fail(r, why);
+        if (plan.flags & kFlagOneLaunch) {
+            plan.flags |= extra_flags | (trace_ ? static_cast<uint32_t>(kFlagTrace) : 0u);
+            return LaunchLocal(plan, send, recv, count, in, out, opt, streams);
+        }
+        caps.one_launch = false;
+    }
+
     CollArgs* const args = args_scratch_.data();  // reused: no allocation on the per-call path
     std::memset(args, 0, sizeof(CollArgs) * args_scratch_.size());
     bool peer_recv = false, symmetric = false;
-    Result r = ResolvePeers(send, recv, send_bytes, recv_bytes, opt.buffers_stable, args, &peer_recv, &symmetric);
+    r = ResolvePeers(send, recv, send_bytes, recv_bytes, opt.buffers_stable, args, &peer_recv, &symmetric);
     if (r != Result::Success) return r;
     bool in_place = false;
     for (int i = 0; i < nlocal(); ++i) {
@@ -457,7 +580,6 @@ Result Communicator::Collective(const void* const* send, void* const* recv, uint
         if (s0 < r0 + recv_bytes && r0 < s0 + send_bytes) in_place = true;
     }
 
-    PlanCaps caps;
     caps.flash_cap = lay_.flash_cap;
     caps.ring_bytes = lay_.ring_bytes;
     caps.nvls_cap = lay_.nvls_cap;
@@ -471,19 +593,9 @@ Result Communicator::Collective(const void* const* send, void* const* recv, uint
     // path's kernels wait for the peers' kernels, and on 2 x B200 rank 0 ran into its deadline before
     // the host got to launch rank 1.  One process per rank only.
     caps.one_gpu_per_rank = !emulated_ && nlocal() == 1;
-    caps.half_collective = rs_only || ag_only;
     caps.sm_count = sm_count_;
     caps.max_ctas = max_ctas_;
-    caps.force_ctas = opt.ctas > 0 ? static_cast<uint32_t>(opt.ctas) : 0u;
-    caps.force_slot_bytes = opt.slot_bytes > 0 ? static_cast<uint32_t>(opt.slot_bytes) : 0u;
-    caps.vec_ok = true;
-    for (int i = 0; i < nlocal(); ++i) caps.vec_ok = caps.vec_ok && Aligned16(send[i]) && Aligned16(recv[i]);
-
-    KernelMode mode = opt.mode;
-    if (mode == KernelMode::Auto) mode = env::ForcedKernelMode();
     if (rs_only || ag_only) mode = KernelMode::Stream;
-    Plan plan;
-    std::string why;
     r = MakePlan(world_, count, in, out, opt.epilogue, mode, caps, EnvTuningTable(), &plan, &why);
     if (r != Result::Success) return Fail(r, why);
     if (world_ == 1 && plan.variant != Variant::Flash)
@@ -493,9 +605,7 @@ Result Communicator::Collective(const void* const* send, void* const* recv, uint
     std::memset(&ep, 0, sizeof(ep));
     ep.scale = opt.epilogue == kEpiScaleCast ? opt.scale : 1.0f;
     if (opt.epilogue == kEpiResidualRmsNorm) {
-        const int vec = 16 / static_cast<int>(DtypeSize(in));
-        if (in != out || opt.hidden <= 0 || count % opt.hidden != 0 || opt.hidden % vec != 0 ||
-            opt.hidden / vec > 4 * kFlashThreads || !opt.weight || !caps.vec_ok)
+        if (!norm_ok)
             return Fail(Result::Unsupported,
                         "fused RMSNorm needs equal in/out dtype, count a multiple of hidden, hidden a multiple of "
                         "16 bytes and at most 4*512 vectors, 16-byte aligned buffers and a weight");

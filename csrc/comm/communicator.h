@@ -3,8 +3,8 @@
 //
 // A process drives `nlocal` ranks: 1 in multi-process mode (one GPU per process),
 // all of them in single-process mode (one host thread launches on every GPU), or
-// all of them on ONE GPU in emulated mode (one cooperative launch runs every
-// rank; used to exercise the multi-rank kernels on a single device).
+// all of them on ONE GPU in emulated mode (one launch runs every rank: the multi-rank
+// kernels in a cooperative launch when a mode is forced, else kernels that exchange nothing).
 //
 // Parity: yali::Comm (src/ops/allreduce.cuh:78-323) and yali::MPIComm
 // (src/ops/allreduce_mpi.cuh:76-298) own P2P setup, per-lane rings, streams and
@@ -164,6 +164,11 @@ class Communicator {
                       const OpOptions& opt, const cudaStream_t* streams, uint32_t extra_flags);
     Result ResolvePeers(const void* const* send, void* const* recv, uint64_t send_bytes, uint64_t recv_bytes,
                         bool stable, CollArgs* args, bool* peer_recv, bool* symmetric);
+    // Every rank in one ordinary launch on one GPU (kernels/local_group.cu).
+    bool CanRunInOneLaunch(const void* const* send, void* const* recv, uint64_t send_bytes, uint64_t recv_bytes,
+                           uint64_t shard_bytes, Dtype in, Dtype out, const OpOptions& opt, uint32_t extra_flags) const;
+    Result LaunchLocal(const Plan& plan, const void* const* send, void* const* recv, uint64_t count, Dtype in, Dtype out,
+                       const OpOptions& opt, const cudaStream_t* streams);
     Result EnsureSmemAttr(const void* fn, uint32_t smem_bytes);
     // Copy-engine all-reduce (copy_engine_path.cc): streams, events and staging per local rank, made on first use.
     struct CeState;

@@ -1,0 +1,313 @@
+// Collectives of a group whose ranks all live on ONE GPU and run in one launch (emulated ranks, or a
+// group of one).  Nothing has to be exchanged there: every rank's input is complete when the launch
+// starts (stream order) and every rank's output counts as delivered when it ends, so the barriers, flags
+// and staging copies of the multi-GPU kernels carry no information.  What is left is the arithmetic:
+// read every rank's input once, add in fp32 in rank order, apply the epilogue, write every rank's output
+// once.  No CTA waits for another one, so the launch is an ordinary one, not a cooperative one.
+//
+// The planner picks these kernels for automatically chosen calls only (PlanCaps::one_launch); a forced
+// mode, a forced geometry or a tuning table still runs the multi-GPU kernel it names.
+//
+// Bound by HBM: bytes of all inputs plus all outputs.  One 16-byte unit per thread and a grid as large as
+// the message measured best on B200: two ranks x 128 MiB fp32 80.3 us (6.69 TB/s) with 512 threads,
+// against 81-84 us with 2 or 4 units per thread and 92-94 us with a persistent grid-stride loop; the
+// pipelined two-shot kernel (TMA stages, two cross-rank barriers) takes 97 us for the same call.  Whole calls
+// from Python, multi-GPU kernel / this one: 4 ranks x 6 MB fp16 18.7 / 10.4 us, 8 ranks x 25 MiB fp32 -> bf16
+// 61.1 / 51.0 us, reduce-scatter + all-gather of 64 MiB over 4 ranks 201 / 108 us, all-reduce + residual +
+// RMSNorm of 2048 x 4096 bf16 over 2 ranks 49.3 / 25.1 us.
+//
+// Parity: none in the reference (it always drives two GPUs).
+#include "coll_common.cuh"
+#include "launch.h"
+#include "local_group.h"
+
+namespace yali {
+
+namespace {
+
+// Timeline of a traced call (kFlagTrace): one launch serves every rank, so the first CTA stamps the start
+// and the last one the end into the ring of each of them.
+__device__ __forceinline__ void local_trace_begin(const LocalArgs& a) {
+    if (!(a.flags & kFlagTrace) || blockIdx.x != 0 || blockIdx.y != 0) return;
+    if (threadIdx.x < a.world) {
+        uint32_t* ctl = a.ctl[threadIdx.x];
+        const uint32_t idx = *reinterpret_cast<volatile uint32_t*>(ctl + kCallTraceIdx);
+        reinterpret_cast<volatile uint64_t*>(ctl + kTraceOff)[(idx % kTraceCap) * 2] = ptx::globaltimer();
+    }
+}
+__device__ __forceinline__ void local_trace_end(const LocalArgs& a) {
+    if (!(a.flags & kFlagTrace)) return;
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    uint32_t* done = a.ctl[0] + kCallDoneCtas;
+    __threadfence();
+    if (atomicAdd(done, 1u) != gridDim.x * gridDim.y - 1) return;
+    *reinterpret_cast<volatile uint32_t*>(done) = 0u;
+    for (uint32_t q = 0; q < a.world; ++q) {
+        volatile uint32_t* iw = a.ctl[q] + kCallTraceIdx;
+        const uint32_t idx = *iw;
+        reinterpret_cast<volatile uint64_t*>(a.ctl[q] + kTraceOff)[(idx % kTraceCap) * 2 + 1] = ptx::globaltimer();
+        *iw = idx + 1;
+    }
+}
+
+// The E elements at element offset e of `base`, as 16-byte vectors of the input type / of the output type.
+template <typename Tin, int E>
+__device__ __forceinline__ void load_unit(uint4 (&x)[E * sizeof(Tin) / 16], const void* base, uint64_t e) {
+#pragma unroll
+    for (int i = 0; i < static_cast<int>(E * sizeof(Tin) / 16); ++i)
+        x[i] = ptx::ld_cg_v4(static_cast<const char*>(base) + e * sizeof(Tin) + i * 16);
+}
+template <typename Tout, int E>
+__device__ __forceinline__ void store_unit(void* base, uint64_t e, const float* f) {
+    constexpr int VEC = 16 / sizeof(Tout);
+#pragma unroll
+    for (int i = 0; i < E / VEC; ++i)
+        ptx::st_v4(static_cast<char*>(base) + e * sizeof(Tout) + i * 16, pack16<Tout>(f + i * VEC));
+}
+
+// KIND: what the grid covers.  Sum: units of the whole message (grid.x).  ReduceScatter / AllGather: units of
+// shard blockIdx.y (a shard is a multiple of 16 elements, so it consists of whole units up to the message's
+// end); the owner's buffer starts at the shard.
+template <typename Tin, typename Tout, int WORLD, LocalKind KIND>
+__global__ void __launch_bounds__(kLocalThreads) local_kernel(const __grid_constant__ LocalArgs a) {
+    // Elements of a unit: 16 bytes of the narrower type, so that neither side moves less than 16 bytes.
+    constexpr int E = 16 / (sizeof(Tin) < sizeof(Tout) ? sizeof(Tin) : sizeof(Tout));
+    constexpr int NIN = E * sizeof(Tin) / 16;
+    constexpr int kMaxW = WORLD ? WORLD : kMaxRanks;
+    const uint32_t W = WORLD ? WORLD : a.world;
+    local_trace_begin(a);
+    const EpiScale epi(a.ep);
+    const uint32_t owner = KIND == LocalKind::Sum ? 0u : blockIdx.y;
+    const uint64_t lo = KIND == LocalKind::Sum ? 0ull : min(a.count, static_cast<uint64_t>(owner) * a.shard_elems);
+    const uint64_t hi = KIND == LocalKind::Sum ? a.count : min(a.count, lo + a.shard_elems);
+    const uint64_t in_off = KIND == LocalKind::AllGather ? lo : 0ull;      // the owner's input starts at its shard
+    const uint64_t out_off = KIND == LocalKind::ReduceScatter ? lo : 0ull;  // the owner's output starts at its shard
+    const uint64_t u = static_cast<uint64_t>(blockIdx.x) * kLocalThreads + threadIdx.x;
+    const uint64_t e0 = lo + u * E;
+    if (a.flags & kFlagVecOk) {
+        if (e0 + E <= hi) {
+            uint4 x[kMaxW][NIN];
+            if constexpr (KIND == LocalKind::AllGather) {
+                load_unit<Tin, E>(x[0], a.send[owner], e0 - in_off);
+#pragma unroll
+                for (int q = 0; q < kMaxW; ++q)
+                    if (q < W) {
+#pragma unroll
+                        for (int i = 0; i < NIN; ++i)
+                            ptx::st_v4(static_cast<char*>(a.recv[q]) + e0 * sizeof(Tout) + i * 16, x[0][i]);
+                    }
+            } else {
+                float f[E];
+#pragma unroll
+                for (int i = 0; i < E; ++i) f[i] = 0.f;
+#pragma unroll
+                for (int q = 0; q < kMaxW; ++q)
+                    if (q < W) load_unit<Tin, E>(x[q], a.send[q], e0);
+#pragma unroll
+                for (int q = 0; q < kMaxW; ++q)
+                    if (q < W) {
+#pragma unroll
+                        for (int i = 0; i < NIN; ++i) accumulate<Tin>(f + i * (16 / sizeof(Tin)), x[q][i]);
+                    }
+#pragma unroll
+                for (int i = 0; i < E; ++i) f[i] = epi(f[i]);
+                if constexpr (KIND == LocalKind::ReduceScatter) {
+                    store_unit<Tout, E>(a.recv[owner], e0 - out_off, f);
+                } else {
+#pragma unroll
+                    for (int q = 0; q < kMaxW; ++q)
+                        if (q < W) store_unit<Tout, E>(a.recv[q], e0, f);
+                }
+            }
+        }
+    }
+    // Elements one by one: the remainder behind the last whole unit, or all of them when some buffer is
+    // aligned to its element type only.  Every element is read and written by one thread alone, after that
+    // thread has read it from every rank: buffers may be used in place.
+    uint64_t eb, ee, step;
+    if (a.flags & kFlagVecOk) {
+        eb = lo + (hi - lo) / E * E + threadIdx.x;
+        ee = blockIdx.x == 0 ? hi : 0;
+        step = kLocalThreads;
+    } else {
+        eb = lo + u;
+        ee = hi;
+        step = static_cast<uint64_t>(gridDim.x) * kLocalThreads;
+    }
+    for (uint64_t e = eb; e < ee; e += step) {
+        Tout o;
+        if constexpr (KIND == LocalKind::AllGather) {
+            o = static_cast<const Tout*>(a.send[owner])[e - in_off];
+        } else {
+            float s = 0.f;
+#pragma unroll
+            for (int q = 0; q < kMaxW; ++q)
+                if (q < W) s += to_f32<Tin>(__ldcg(static_cast<const Tin*>(a.send[q]) + e));
+            o = from_f32<Tout>(epi(s));
+        }
+        if constexpr (KIND == LocalKind::ReduceScatter) {
+            static_cast<Tout*>(a.recv[owner])[e - out_off] = o;
+        } else {
+#pragma unroll
+            for (int q = 0; q < kMaxW; ++q)
+                if (q < W) static_cast<Tout*>(a.recv[q])[e] = o;
+        }
+    }
+    local_trace_end(a);
+}
+
+// Sum + residual + RMSNorm of one row for the ranks [g * G, g * G + G) of the group; CTA b handles row
+// b / ngroups, group b % ngroups (the groups of a row are neighbours, so the second one finds the row in
+// L2).  A thread holds NV vectors of the row: it reads them from every rank once, adds in fp32, and keeps
+// the packed residuals of its G ranks until the G sums of squares are known (one block reduction for all).
+template <typename T, int WORLD, int NV, int G>
+__global__ void __launch_bounds__(kLocalThreads) local_norm_kernel(const __grid_constant__ LocalArgs a) {
+    constexpr int VEC = TypeTraits<T>::kVec;
+    constexpr int kMaxW = WORLD ? WORLD : kMaxRanks;
+    const uint32_t W = WORLD ? WORLD : a.world;
+    __shared__ float s_red[G][kLocalThreads / 32];
+    local_trace_begin(a);
+    const uint32_t ngroups = (W + G - 1) / G;
+    const uint32_t row = blockIdx.x / ngroups, q0 = (blockIdx.x % ngroups) * G;
+    const int tid = threadIdx.x, nt = blockDim.x;
+    const uint32_t vec_per_row = a.ep.hidden / VEC;
+    const uint64_t row_off = static_cast<uint64_t>(row) * vec_per_row * 16;
+
+    uint4 res[NV][G];
+    float f[NV][VEC];
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+        const uint32_t c = tid + j * nt;
+#pragma unroll
+        for (int i = 0; i < VEC; ++i) f[j][i] = 0.f;
+#pragma unroll
+        for (int g = 0; g < G; ++g) res[j][g] = make_uint4(0, 0, 0, 0);
+        if (c < vec_per_row) {
+            uint4 x[kMaxW];
+#pragma unroll
+            for (int q = 0; q < kMaxW; ++q)
+                if (q < W) x[q] = ptx::ld_cg_v4(static_cast<const char*>(a.send[q]) + row_off + c * 16ull);
+#pragma unroll
+            for (int g = 0; g < G; ++g)
+                if (q0 + g < W && a.residual[q0 + g])
+                    res[j][g] = ptx::ld_cg_v4(static_cast<const char*>(a.residual[q0 + g]) + row_off + c * 16ull);
+#pragma unroll
+            for (int q = 0; q < kMaxW; ++q)
+                if (q < W) accumulate<T>(f[j], x[q]);
+        }
+    }
+    float ss[G];
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+        ss[g] = 0.f;
+#pragma unroll
+        for (int j = 0; j < NV; ++j) {
+            const uint32_t c = tid + j * nt;
+            float p[VEC];
+#pragma unroll
+            for (int i = 0; i < VEC; ++i) p[i] = f[j][i];
+            accumulate<T>(p, res[j][g]);
+            if (c < vec_per_row && q0 + g < W && a.residual_out[q0 + g])
+                ptx::st_v4(static_cast<char*>(a.residual_out[q0 + g]) + row_off + c * 16ull, pack16<T>(p));
+#pragma unroll
+            for (int i = 0; i < VEC; ++i) ss[g] += p[i] * p[i];
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) ss[g] += __shfl_xor_sync(0xffffffffu, ss[g], o);
+        if ((tid & 31) == 0) s_red[g][tid >> 5] = ss[g];
+    }
+    __syncthreads();
+    const float inv_h = 1.f / static_cast<float>(a.ep.hidden);
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+        if (q0 + g >= W) break;
+        float t = (tid & 31) < (nt >> 5) ? s_red[g][tid & 31] : 0.f;
+#pragma unroll
+        for (int o = 8; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        t = __shfl_sync(0xffffffffu, t, 0);
+        const float inv_rms = rsqrtf(t * inv_h + a.ep.eps);
+#pragma unroll
+        for (int j = 0; j < NV; ++j) {
+            const uint32_t c = tid + j * nt;
+            if (c < vec_per_row) {
+                float p[VEC], w[VEC];
+#pragma unroll
+                for (int i = 0; i < VEC; ++i) {
+                    p[i] = f[j][i];
+                    w[i] = 0.f;
+                }
+                accumulate<T>(p, res[j][g]);
+                accumulate<T>(w, *reinterpret_cast<const uint4*>(static_cast<const char*>(a.weight[q0 + g]) + c * 16ull));
+#pragma unroll
+                for (int i = 0; i < VEC; ++i) p[i] = p[i] * inv_rms * w[i];
+                ptx::st_v4(static_cast<char*>(a.recv[q0 + g]) + row_off + c * 16ull, pack16<T>(p));
+            }
+        }
+    }
+    local_trace_end(a);
+}
+
+template <typename Tin, typename Tout, LocalKind KIND>
+const void* pick_world(int world) {
+    switch (world) {
+        case 1: return (const void*)local_kernel<Tin, Tout, 1, KIND>;
+        case 2: return (const void*)local_kernel<Tin, Tout, 2, KIND>;
+        case 4: return (const void*)local_kernel<Tin, Tout, 4, KIND>;
+        case 8: return (const void*)local_kernel<Tin, Tout, 8, KIND>;
+        default: return (const void*)local_kernel<Tin, Tout, 0, KIND>;
+    }
+}
+template <LocalKind KIND>
+const void* pick_same(Dtype dt, int world) {
+    switch (dt) {
+        case Dtype::FP32: return pick_world<float, float, KIND>(world);
+        case Dtype::FP16: return pick_world<__half, __half, KIND>(world);
+        case Dtype::BF16: return pick_world<__nv_bfloat16, __nv_bfloat16, KIND>(world);
+    }
+    return nullptr;
+}
+template <typename T, int WORLD, int NV>
+const void* pick_norm_g(int g) {
+    constexpr int kMost = WORLD && WORLD < kLocalNormHeld / NV ? WORLD : kLocalNormHeld / NV;
+    return g == 1 ? (const void*)local_norm_kernel<T, WORLD, NV, 1> : (const void*)local_norm_kernel<T, WORLD, NV, kMost>;
+}
+template <typename T, int WORLD>
+const void* pick_norm_nv(int nv, int g) {
+    return nv == 1 ? pick_norm_g<T, WORLD, 1>(g) : nv == 2 ? pick_norm_g<T, WORLD, 2>(g) : pick_norm_g<T, WORLD, 4>(g);
+}
+template <typename T>
+const void* pick_norm(int world, int nv, int g) {
+    switch (world) {
+        case 2: return pick_norm_nv<T, 2>(nv, g);
+        case 4: return pick_norm_nv<T, 4>(nv, g);
+        case 8: return pick_norm_nv<T, 8>(nv, g);
+        default: return pick_norm_nv<T, 0>(nv, g);
+    }
+}
+
+}  // namespace
+
+const void* LocalKernelFor(Dtype in, Dtype out, int world, LocalKind kind) {
+    using bf16 = __nv_bfloat16;
+    if (kind == LocalKind::ReduceScatter) return in == out ? pick_same<LocalKind::ReduceScatter>(in, world) : nullptr;
+    if (kind == LocalKind::AllGather) return in == out ? pick_same<LocalKind::AllGather>(in, world) : nullptr;
+    constexpr LocalKind S = LocalKind::Sum;
+    if (in == out) return pick_same<S>(in, world);
+    if (in == Dtype::FP32 && out == Dtype::BF16) return pick_world<float, bf16, S>(world);
+    if (in == Dtype::FP32 && out == Dtype::FP16) return pick_world<float, __half, S>(world);
+    if (in == Dtype::BF16 && out == Dtype::FP32) return pick_world<bf16, float, S>(world);
+    if (in == Dtype::FP16 && out == Dtype::FP32) return pick_world<__half, float, S>(world);
+    return nullptr;
+}
+
+const void* LocalNormKernelFor(Dtype dt, int world, const LocalNormShape& s) {
+    switch (dt) {
+        case Dtype::FP32: return pick_norm<float>(world, s.vec_per_thread, s.ranks_per_cta);
+        case Dtype::FP16: return pick_norm<__half>(world, s.vec_per_thread, s.ranks_per_cta);
+        case Dtype::BF16: return pick_norm<__nv_bfloat16>(world, s.vec_per_thread, s.ranks_per_cta);
+    }
+    return nullptr;
+}
+
+}  // namespace yali

@@ -71,12 +71,63 @@ __global__ void validate_sum_kernel(const Tout* out, uint64_t n, uint64_t index_
               static_cast<unsigned long long>(__double_as_longlong(worst)));
 }
 
-// In-place residual add + RMSNorm over rows of `hidden` elements (one CTA per row, grid-stride).
+// In-place residual add + RMSNorm over rows of `hidden` elements, one CTA per row.
 // Used when a message is too large for the one-shot kernel that fuses this step: the all-reduce
 // runs first, then this kernel normalises the local result.
+// Bound by HBM (three or four row images in and out).  A thread keeps its NV vectors of the row in registers
+// between the sum of squares and the store, so the row is read once; 16-byte accesses.
+template <typename T, int NV>
+__global__ void __launch_bounds__(512) residual_rmsnorm_kernel(T* x, const T* residual, T* residual_out, const T* weight,
+                                                               uint32_t hidden, float eps) {
+    constexpr int VEC = TypeTraits<T>::kVec;
+    __shared__ float s_part[16];
+    const int tid = threadIdx.x, nt = blockDim.x;
+    const uint32_t vec_per_row = hidden / VEC;
+    const uint64_t row_off = static_cast<uint64_t>(blockIdx.x) * hidden;
+    float f[NV][VEC];
+    float ss = 0.f;
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+        const uint32_t c = tid + j * nt;
+#pragma unroll
+        for (int i = 0; i < VEC; ++i) f[j][i] = 0.f;
+        if (c < vec_per_row) {
+            const uint64_t e = row_off + static_cast<uint64_t>(c) * VEC;
+            const uint4 xv = ptx::ld_cg_v4(x + e);
+            const uint4 rv = residual ? ptx::ld_cg_v4(residual + e) : make_uint4(0, 0, 0, 0);
+            accumulate<T>(f[j], xv);
+            if (residual) accumulate<T>(f[j], rv);
+            if (residual_out) ptx::st_v4(residual_out + e, pack16<T>(f[j]));
+        }
+#pragma unroll
+        for (int i = 0; i < VEC; ++i) ss += f[j][i] * f[j][i];
+    }
+    for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+    if ((tid & 31) == 0) s_part[tid >> 5] = ss;
+    __syncthreads();
+    float tot = 0.f;
+    for (int w = 0; w < (nt + 31) / 32; ++w) tot += s_part[w];
+    const float inv = rsqrtf(tot / static_cast<float>(hidden) + eps);
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+        const uint32_t c = tid + j * nt;
+        if (c < vec_per_row) {
+            float w[VEC];
+#pragma unroll
+            for (int i = 0; i < VEC; ++i) w[i] = 0.f;
+            accumulate<T>(w, *reinterpret_cast<const uint4*>(weight + static_cast<uint64_t>(c) * VEC));
+#pragma unroll
+            for (int i = 0; i < VEC; ++i) f[j][i] = f[j][i] * inv * w[i];
+            ptx::st_v4(x + row_off + static_cast<uint64_t>(c) * VEC, pack16<T>(f[j]));
+        }
+    }
+}
+
+// The same element by element: rows that are no whole number of 16-byte vectors, are longer than 2048 of
+// them, or start on an address that is aligned to the element only.
 template <typename T>
-__global__ void residual_rmsnorm_kernel(T* x, const T* residual, T* residual_out, const T* weight, uint64_t rows,
-                                        uint32_t hidden, float eps) {
+__global__ void residual_rmsnorm_elems_kernel(T* x, const T* residual, T* residual_out, const T* weight, uint64_t rows,
+                                              uint32_t hidden, float eps) {
     __shared__ float s_part[32];
     const int tid = threadIdx.x, nt = blockDim.x;
     for (uint64_t row = blockIdx.x; row < rows; row += gridDim.x) {
@@ -183,26 +234,40 @@ cudaError_t ValidateSumAsync(const void* out, uint64_t n, uint64_t index_offset,
     return cudaErrorInvalidValue;
 }
 
+namespace {
+template <typename T>
+void LaunchResidualRmsNorm(void* x, const void* residual, void* residual_out, const void* weight, uint64_t rows,
+                           uint32_t hidden, float eps, cudaStream_t s) {
+    constexpr uint32_t VEC = TypeTraits<T>::kVec;
+    T* xt = static_cast<T*>(x);
+    const T* rt = static_cast<const T*>(residual);
+    T* ot = static_cast<T*>(residual_out);
+    const T* wt = static_cast<const T*>(weight);
+    const uint32_t vec_per_row = hidden / VEC;
+    const bool aligned = ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(residual) |
+                           reinterpret_cast<uintptr_t>(residual_out) | reinterpret_cast<uintptr_t>(weight)) & 15u) == 0;
+    if (hidden % VEC != 0 || vec_per_row > 2048 || !aligned || rows > 0x7fffffffull) {
+        const int grid = static_cast<int>(rows < 148 * 8 ? rows : 148 * 8);
+        residual_rmsnorm_elems_kernel<<<grid, 256, 0, s>>>(xt, rt, ot, wt, rows, hidden, eps);
+        return;
+    }
+    // Two vectors per thread from 256 vectors on: enough loads in flight, and four or more rows per SM.
+    const uint32_t nv = vec_per_row <= 128 ? 1 : vec_per_row <= 1024 ? 2 : 4;
+    const uint32_t threads = ((vec_per_row + nv - 1) / nv + 31) / 32 * 32;
+    const uint32_t grid = static_cast<uint32_t>(rows);
+    if (nv == 1) residual_rmsnorm_kernel<T, 1><<<grid, threads, 0, s>>>(xt, rt, ot, wt, hidden, eps);
+    else if (nv == 2) residual_rmsnorm_kernel<T, 2><<<grid, threads, 0, s>>>(xt, rt, ot, wt, hidden, eps);
+    else residual_rmsnorm_kernel<T, 4><<<grid, threads, 0, s>>>(xt, rt, ot, wt, hidden, eps);
+}
+}  // namespace
+
 cudaError_t ResidualRmsNormInPlace(void* x, const void* residual, void* residual_out, const void* weight,
                                    uint64_t rows, uint32_t hidden, float eps, Dtype dt, cudaStream_t s) {
     if (rows == 0) return cudaSuccess;
-    const int grid = static_cast<int>(rows < 148 * 8 ? rows : 148 * 8);
     switch (dt) {
-        case Dtype::FP32:
-            residual_rmsnorm_kernel<<<grid, 256, 0, s>>>(static_cast<float*>(x), static_cast<const float*>(residual),
-                                                         static_cast<float*>(residual_out),
-                                                         static_cast<const float*>(weight), rows, hidden, eps);
-            break;
-        case Dtype::FP16:
-            residual_rmsnorm_kernel<<<grid, 256, 0, s>>>(static_cast<__half*>(x), static_cast<const __half*>(residual),
-                                                         static_cast<__half*>(residual_out),
-                                                         static_cast<const __half*>(weight), rows, hidden, eps);
-            break;
-        case Dtype::BF16:
-            residual_rmsnorm_kernel<<<grid, 256, 0, s>>>(
-                static_cast<__nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(residual),
-                static_cast<__nv_bfloat16*>(residual_out), static_cast<const __nv_bfloat16*>(weight), rows, hidden, eps);
-            break;
+        case Dtype::FP32: LaunchResidualRmsNorm<float>(x, residual, residual_out, weight, rows, hidden, eps, s); break;
+        case Dtype::FP16: LaunchResidualRmsNorm<__half>(x, residual, residual_out, weight, rows, hidden, eps, s); break;
+        case Dtype::BF16: LaunchResidualRmsNorm<__nv_bfloat16>(x, residual, residual_out, weight, rows, hidden, eps, s); break;
     }
     return cudaGetLastError();
 }

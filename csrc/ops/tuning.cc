@@ -283,6 +283,20 @@ Result MakePlan(int world, uint64_t count, Dtype in, Dtype out, int epilogue, Ke
     Plan p;
     if (caps.vec_ok) p.flags |= kFlagVecOk;
 
+    const TuningRow* row = (table && forced == KernelMode::Auto) ? table->Find(world, static_cast<int>(in_b), bytes)
+                                                                 : nullptr;
+    // All ranks in one launch on one GPU: the kernels of local_group.cu, which exchange nothing, at every
+    // size (they measured ahead from 4 KiB to 128 MiB).  A forced mode or geometry and a tuning table ask for
+    // a multi-GPU kernel by name and get it.  The variant reported is the one whose place is taken.
+    if (caps.one_launch && forced == KernelMode::Auto && !row && !caps.force_ctas && !caps.force_slot_bytes) {
+        p.variant = caps.half_collective ? Variant::Stream
+                    : world == 1 || bytes <= FlashCrossoverBytes(in, world) ? Variant::Flash : Variant::StreamDirect;
+        p.shard_elems = ShardElems(count, world);
+        p.flags |= kFlagOneLaunch;
+        *plan = p;
+        return Result::Success;
+    }
+
     // Which variants can run this call at all.
     const bool rows = epilogue == kEpiResidualRmsNorm;
     const bool flash_ok = bytes <= caps.flash_cap || world == 1;
@@ -305,8 +319,6 @@ Result MakePlan(int world, uint64_t count, Dtype in, Dtype out, int epilogue, Ke
                        static_cast<uint64_t>(world - 1) * ShardElems(count, world) < count;
 
     Variant v;
-    const TuningRow* row = (table && forced == KernelMode::Auto) ? table->Find(world, static_cast<int>(in_b), bytes)
-                                                                 : nullptr;
     if (forced == KernelMode::Flash) v = Variant::Flash;
     else if (forced == KernelMode::Stream) v = Variant::Stream;
     else if (forced == KernelMode::NVLS) v = bytes <= (128ull << 10) ? Variant::NvlsOneShot : Variant::NvlsTwoShot;

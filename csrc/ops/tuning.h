@@ -33,6 +33,7 @@ struct PlanCaps {
     bool peer_send = false;        // every rank's send is peer-addressable (the pipelined kernels can pull it)
     bool in_place = false;         // some rank's send and recv ranges overlap
     bool one_gpu_per_rank = false; // every rank is a process with a GPU of its own (the copy-engine path needs it)
+    bool one_launch = false;       // one launch on one GPU runs every rank: nothing has to be exchanged
     bool half_collective = false;  // reduce-scatter-only / all-gather-only call (ring kernel only)
     uint32_t sm_count = 148;       // SMs of the GPU (resident CTAs of the pipelined kernels)
     bool vec_ok = true;            // all pointers 16-byte aligned

@@ -1,0 +1,109 @@
+"""Automatically chosen calls of a group whose ranks share one GPU run in one launch that exchanges nothing
+(csrc/kernels/local_group.cu).  Inputs are small whole numbers, so every sum is exact in every type and results
+are compared bit by bit; sizes sit at the edges of the 16-byte units, CTAs (512 units) and shards."""
+import pytest
+import torch
+
+import yali_b200 as yali
+
+pytestmark = pytest.mark.gpu
+
+ONE_LAUNCH = 1 << 9
+F32, F16, BF16 = torch.float32, torch.float16, torch.bfloat16
+
+
+@pytest.fixture(scope="module", params=[1, 2, 3, 4, 8])
+def comm(request):
+    c = yali.Comm.emulated(request.param, device=0)
+    yield c
+    c.close()
+
+
+def whole(shape, dtype, seed, off=0):
+    """Whole numbers in [-8, 8] in a buffer that starts `off` elements behind a 16-byte boundary."""
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    x = torch.randint(-8, 9, shape, generator=g, device="cuda").to(dtype)
+    buf = torch.empty(x.numel() + off, dtype=dtype, device="cuda")[off:].view(x.shape)
+    return buf.copy_(x)
+
+
+def total(xs):
+    return torch.stack([x.double() for x in xs]).sum(0)
+
+
+@pytest.mark.parametrize("src,dst", [(F32, F32), (F16, F16), (BF16, BF16), (F32, BF16), (F32, F16), (BF16, F32), (F16, F32)])
+@pytest.mark.parametrize("n", [1, 7, 8, 9, 2047, 2048, 2049, 4095, 4097, 100003])
+def test_sum(comm, src, dst, n):
+    for off in (0, 1):
+        xs = [whole((n,), src, 10 * n + r, off if r == comm.world - 1 else 0) for r in range(comm.world)]
+        ys = comm.all_reduce(xs, scale=0.5, out_dtype=dst)
+        assert comm.last_call()["flags"] & ONE_LAUNCH
+        for y in ys:
+            assert torch.equal(y.double(), total(xs) * 0.5)
+    if src == dst:  # in place
+        want = total(xs)
+        comm.all_reduce(xs, xs)
+        assert comm.last_call()["flags"] & ONE_LAUNCH and all(torch.equal(x.double(), want) for x in xs)
+
+
+@pytest.mark.parametrize("dtype", [F32, BF16])
+@pytest.mark.parametrize("n", [1, 16, 17, 129, 8192, 65535, 65537])
+def test_halves(comm, dtype, n):
+    W, S = comm.world, comm.shard_elems(n) if comm.world > 1 else n
+    xs = [whole((n,), dtype, n + r) for r in range(W)]
+    want = total(xs)
+    shards = comm.reduce_scatter(xs)
+    assert comm.last_call()["flags"] & ONE_LAUNCH
+    for r, s in enumerate(shards):
+        part = want[min(n, r * S):min(n, (r + 1) * S)]
+        assert torch.equal(s[:part.numel()].double(), part)
+    for f in comm.all_gather(shards, n):
+        assert torch.equal(f.double(), want)
+    assert comm.last_call()["flags"] & ONE_LAUNCH
+    # Every rank's shard at its place inside the rank's own message: both halves in place.
+    if n % (16 * W) == 0:
+        views = [x[r * S:(r + 1) * S] for r, x in enumerate(xs)]
+        comm.reduce_scatter(xs, views)
+        comm.all_gather(views, n, xs)
+        assert comm.last_call()["flags"] & ONE_LAUNCH and all(torch.equal(x.double(), want) for x in xs)
+
+
+@pytest.mark.parametrize("dtype", [F32, F16, BF16])
+@pytest.mark.parametrize("rows,hidden", [(1, 8), (3, 4096), (16, 4104), (200, 1000), (300, 4096), (40, 8192), (160, 8192)])
+def test_norm(comm, dtype, rows, hidden):
+    W = comm.world
+    xs = [whole((rows, hidden), dtype, r) for r in range(W)]
+    res = [whole((rows, hidden), dtype, 50 + r) for r in range(W)]  # not alike on the ranks: each uses its own
+    ws = [whole((hidden,), dtype, 90 + r) for r in range(W)]
+    pre = [torch.empty_like(x) for x in xs]
+    ys = comm.all_reduce_rmsnorm(xs, ws, res, eps=1e-5, residual_out=pre)
+    assert comm.last_call()["flags"] & ONE_LAUNCH
+    plain = comm.all_reduce_rmsnorm(xs, ws, None, eps=1e-5)
+    # The rows are exact; what is left is the fp32 sum of squares and product (a few 2^-23) and one rounding.
+    rtol = {F32: 2e-6, F16: 2.0 ** -10, BF16: 2.0 ** -7}[dtype]
+    for r in range(W):
+        s = total(xs) + res[r].double()
+        assert torch.equal(pre[r].double(), s)
+        for got, row in ((ys[r], s), (plain[r], total(xs))):
+            ref = row * torch.rsqrt(row.pow(2).mean(-1, keepdim=True) + 1e-5) * ws[r].double()
+            torch.testing.assert_close(got.double(), ref, rtol=rtol, atol=1e-6)
+    # The multi-GPU kernel on request, and for outputs that lie on the inputs of several ranks.
+    again = comm.all_reduce_rmsnorm(xs, ws, res, eps=1e-5, mode="flash")
+    assert not comm.last_call()["flags"] & ONE_LAUNCH
+    torch.testing.assert_close(again[0].double(), ys[0].double(), rtol=2 * rtol, atol=1e-6)
+    if rows * hidden < 65536:
+        comm.all_reduce_rmsnorm(xs, ws, res, eps=1e-5, out=xs)
+        assert not comm.last_call()["flags"] & ONE_LAUNCH
+        torch.testing.assert_close(xs[0].double(), ys[0].double(), rtol=2 * rtol, atol=1e-6)
+
+
+def test_halves_of_the_multi_gpu_kernel_on_request(comm, monkeypatch):
+    if comm.world == 1:
+        pytest.skip("a group of one has no halves")
+    monkeypatch.setenv("YALI_KERNEL_MODE", "stream")
+    n = 40001
+    xs = [whole((n,), F32, r) for r in range(comm.world)]
+    full = comm.all_gather(comm.reduce_scatter(xs), n)
+    comm.sync()
+    assert comm.last_call()["variant"] == "stream" and not comm.last_call()["flags"] & ONE_LAUNCH
+    assert torch.equal(full[-1].double(), total(xs))

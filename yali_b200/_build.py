@@ -48,6 +48,7 @@ LIB_SOURCES = [
     "kernels/flash_oneshot.cu",
     "kernels/stream_twoshot.cu",
     "kernels/nvls.cu",
+    "kernels/local_group.cu",
     "kernels/direct_pipeline.cu",
     "kernels/copy_engine.cu",
     "kernels/util_kernels.cu",

@@ -65,7 +65,9 @@ class Comm:
 
     @classmethod
     def emulated(cls, world: int, device: int = 0, heap_bytes: int = 0, timeout_ms: int = -1) -> "Comm":
-        """`world` ranks on ONE GPU, run by a single cooperative launch per collective."""
+        """`world` ranks on ONE GPU, run by a single launch per collective.  A forced `mode` (or geometry) runs the
+        multi-GPU kernel with its flags and staging in a cooperative launch; automatically chosen collectives use
+        kernels that exchange nothing, because one launch sees every rank's buffers."""
         return cls(_native.ext().Comm.emulated(world, device, heap_bytes, timeout_ms))
 
     @classmethod
