@@ -31,7 +31,6 @@ constexpr uint32_t kCallGemmEpoch = 3;    // fused GEMM calls so far
 constexpr uint32_t kCallFlashEpochHi = 5;  // upper half of the one-shot call number (flag-in-data protocol)
 constexpr uint32_t kCallGemmLLEpoch = 6;   // calls of the fused GEMM's few-token form so far (lower half)
 constexpr uint32_t kCallGemmLLEpochHi = 7;  // upper half of that call number
-constexpr uint32_t kCallGemmCnt = 4;      // arrivals (per source) this rank has been promised so far
 constexpr uint32_t kCallGemmDone = 8;     // [kMaxRanks] rows each owner has been asked to deliver so far
 constexpr uint32_t kCallDoneCtas = 16;    // [4] CTAs of the running launch that have finished, per kernel kind
 constexpr uint32_t kCallTraceIdx = 20;    // traced calls so far (index into the kTraceOff ring)
@@ -53,7 +52,11 @@ constexpr uint32_t kTraceOff = kStatusCntOff + 8;              // [kTraceCap][2]
 constexpr uint32_t kCeEnterOff = kTraceOff + kTraceCap * 4;  // [kMaxRanks] call the source has entered
 constexpr uint32_t kCePulledOff = kCeEnterOff + kMaxRanks;   // [kMaxRanks] (call << 8) | chunks the source has read here
 constexpr uint32_t kCeDoneOff = kCePulledOff + kMaxRanks;    // [kMaxRanks] call the source has finished with this rank
-constexpr uint32_t kFlagWords = kCeDoneOff + kMaxRanks;
+// Fused GEMM: the call number, written by a source when its partial sums of a tile unit (a token tile x 128
+// columns x K split) have landed here.
+constexpr uint32_t kGemmTileFlags = 4096;
+constexpr uint32_t kGemmTileFlagOff = kCeDoneOff + kMaxRanks;  // [kGemmTileFlags][kMaxRanks]
+constexpr uint32_t kFlagWords = kGemmTileFlagOff + kGemmTileFlags * kMaxRanks;
 constexpr uint64_t kFlagRegionBytes = 1ull << 20;
 static_assert(kFlagWords * 4ull <= kFlagRegionBytes, "flag region too small");
 static_assert(kTraceOff % 2 == 0, "the timeline entries are 64-bit words");

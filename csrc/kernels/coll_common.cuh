@@ -107,6 +107,15 @@ __device__ __forceinline__ bool check_out_last(const CommView& cv, uint32_t kind
     *reinterpret_cast<volatile uint32_t*>(done) = 0u;
     return true;
 }
+// The same at the start of a call, for call words that every CTA has read (and `done` not written otherwise): the last CTA
+// to check in may advance them at once, because only the next launch reads them again.  Takes the
+// counter's round trip out of the end of the call, and needs no fence: no data hangs on it.
+__device__ __forceinline__ bool check_in_last(const CommView& cv, uint32_t kind, uint32_t nctas) {
+    uint32_t* done = flag_word(cv, cv.rank, kCallDoneCtas + kind);
+    if (atomicAdd(done, 1u) != nctas - 1) return false;
+    *reinterpret_cast<volatile uint32_t*>(done) = 0u;
+    return true;
+}
 __device__ __forceinline__ void advance_call_word(const CommView& cv, uint32_t word, uint32_t inc) {
     volatile uint32_t* w = flag_word(cv, cv.rank, word);
     *w = *w + inc;

@@ -10,14 +10,29 @@
 
 namespace yali {
 
+// The tile in which announcements of partial rows were first counted, and which the host-thread model of the
+// protocol and FusedLinearCounts still use.
 constexpr int kGemmTileM = 128;
 constexpr int kGemmTileN = 256;
-constexpr int kGemmThreads = 352;  // TMA warp, MMA warp, eight epilogue warps, announcer warp
-constexpr int kGemmMaxVecPerThread = 2;  // N <= 2 * 352 threads * 8 bf16 = 5632 (the host caps N at 4096)
+// Tile of the kernel: 256 columns of the output (the M side of the MMA: rows of W, 128 per CTA of a pair) x up to
+// 256 tokens (the N side: rows of x, half of them per CTA).
+constexpr uint32_t kGemmPairCols = 256;
+constexpr uint32_t kGemmUnitCols = 128;    // columns of one CTA: the unit in which partial sums are announced
+constexpr uint32_t kGemmMaxTokens = 256;   // tokens of a tile
+constexpr int kGemmThreads = 640;          // eight epilogue warps, eight row warps, TMA, MMA, announcer and row-producer warp
+constexpr uint32_t kGemmMaxRowVecs = 512;  // 16-byte vectors of a row: N <= 4096
+
+// How the T rows are cut into token tiles: `domains` runs of `span` rows (one per row owner, or one run of all
+// rows), each cut into `tiles` tiles of `tokens` rows (a multiple of 32; the last ones may be short or empty).
+// A pair of CTAs walks the items (token tile, 256 columns, K split) of its rank; `group` token tiles are
+// walked together column by column, so that they read a slice of W at about the same time.
+struct GemmTiling {
+    uint32_t span, domains, tiles, tokens, group;
+};
 
 struct alignas(64) GemmArArgs {
-    CUtensorMap tmap_a;  // x  [T, K] bf16, box 64 x 128, 128-byte swizzle
-    CUtensorMap tmap_b;  // W  [N, K] bf16, box 64 x 256 (rows beyond N read as zeros), 128-byte swizzle
+    CUtensorMap tmap_x;  // x  [T, K] bf16, box 64 x tokens / 2, 128-byte swizzle (rows beyond T read as zeros)
+    CUtensorMap tmap_w;  // W  [N, K] bf16, box 64 x 128, 128-byte swizzle (rows beyond N read as zeros)
     CommView cv;
     const void* residual;     // [T, N] bf16 or nullptr
     void* residual_out;       // [T, N] bf16 or nullptr (sum + residual), this rank's copy
@@ -25,11 +40,12 @@ struct alignas(64) GemmArArgs {
     const void* norm_weight;  // [N] bf16
     void* out[kMaxRanks];     // every rank's output [T, N] (two-shot writes all, one-shot only its own)
     uint32_t T, N, K;
+    GemmTiling tl;
     uint32_t rows_per_owner;  // two-shot: rows normalised by each rank
     uint32_t oneshot;         // 1: every rank receives all partial rows and normalises all of them
-    uint32_t ksplit;          // one-shot, few tiles: CTAs that share the K extent of a tile (1, 2 or 4; world x ksplit <= 8)
+    uint32_t ksplit;          // one-shot, few tiles: pairs that share the K extent of a tile (1, 2 or 4; world x ksplit <= 8)
     uint32_t kper;            // k-blocks (of 64) per split
-    uint32_t cnt_inc;         // arrivals per source that complete this rank's partial rows in this call
+    uint32_t one_gpu;         // all ranks' heaps are this GPU's memory: announcements need GPU scope only
     uint32_t done_inc[kMaxRanks];  // per owner: rows it delivers to every rank's output in this call
     float eps;
     // NVLS form of the two-shot (nvls != 0): every rank keeps its partial rows in its OWN landing

@@ -218,6 +218,39 @@ uint32_t FusedLinearTileSplit(uint32_t T, uint32_t N, uint32_t K, int world, uin
     return ks;
 }
 
+// How the rows are cut into token tiles.  Candidates: one run of tiles per row owner (two-shot; rows then complete
+// owner by owner and pushes spread over the owners) or one run over all rows, each with the fewest tiles that
+// hold 256 tokens and a few more.  The time of a k-block grows with the tile's tokens above a part that does not
+// (measured 519 cycles with 256 tokens, about 340 with 160 or fewer, where issue and operand fill set the
+// pace), taken as max(340, 2 tokens + 6); the cost of a candidate is that times the rounds its items take on
+// the resident pairs.  All inputs are alike on all ranks.
+GemmTiling FusedLinearTiling(uint32_t T, uint32_t N, int world, bool oneshot, uint32_t ksplit, uint32_t pairs) {
+    const uint32_t ncol = (N + kGemmPairCols - 1) / kGemmPairCols, Rs = oneshot ? T : (T + world - 1) / world;
+    GemmTiling best{};
+    uint64_t best_cost = ~0ull;
+    auto consider = [&](uint32_t span, uint32_t domains) {
+        const uint32_t fewest = (span + kGemmMaxTokens - 1) / kGemmMaxTokens;
+        for (uint32_t n = fewest; n < fewest + 4; ++n) {
+            GemmTiling t;
+            t.span = span;
+            t.domains = domains;
+            t.tokens = ((span + n - 1) / n + 31) / 32 * 32;
+            t.tiles = (span + t.tokens - 1) / t.tokens;
+            const uint64_t items = static_cast<uint64_t>(domains) * t.tiles * ncol * ksplit;
+            const uint64_t cost = (items + pairs - 1) / pairs * std::max<uint32_t>(340, 2 * t.tokens + 6);
+            if (cost >= best_cost) continue;
+            best_cost = cost;
+            // Column by column over all tiles (a slice of W is then read from HBM once, by neighbours) unless rows can
+            // complete early: then the owners' k-th tiles together.
+            t.group = domains > 1 && t.tiles > 1 ? domains : domains * t.tiles;
+            best = t;
+        }
+    };
+    if (!oneshot && world > 1) consider(Rs, static_cast<uint32_t>(world));
+    consider(T, 1);
+    return best;
+}
+
 // Which multicast form the two-shot takes by default (0 none, 1 in-switch reduce + multicast store,
 // 2 peer pushes + multicast store), from measurements on 2, 4 and 8 B200.
 // 8 x B200, K = 512 per rank, N = 4096, CUDA-graph timing (us, modes 0 / 1 / 2): T = 128: 31.4 / 28.9 /
@@ -337,46 +370,62 @@ Result FusedLinearAllReduceRmsNorm(Communicator& comm, const FusedLinearDesc* de
     }
     const bool nvls = mc_mode == 1;
 
-    const uint32_t ntm = (T + kGemmTileM - 1) / kGemmTileM, ntn = (N + kGemmTileN - 1) / kGemmTileN;
-    // Arrivals owner q expects from every source in this call, and rows owner q delivers.
+    // Rows every owner delivers in this call.
     uint32_t arrivals[kMaxRanks] = {}, rows_of[kMaxRanks] = {};
     FusedLinearCounts(T, N, W, oneshot, arrivals, rows_of);
     const void* fn = GemmArKernel(comm.emulated());
     const uint32_t smem = GemmArSmemBytes();
     // The dynamic shared-memory limit is a per-device property of the kernel: raise it once for every
-    // (kernel flavour, device) this process launches on.
+    // (kernel flavour, device) this process launches on, and ask once how many pairs of CTAs are resident (all
+    // GPUs of a group are alike).
     static std::mutex attr_mu;
     static std::set<std::pair<int, int>> attr_done;
+    static int cached_pairs[2] = {0, 0};
+    const int flavour = comm.emulated() ? 1 : 0;
+    uint32_t pairs = 0;
     {
         std::lock_guard<std::mutex> lock(attr_mu);
         for (int i = 0; i < nlocal; ++i) {
-            const std::pair<int, int> key(comm.emulated() ? 1 : 0, comm.device_of(i));
+            const std::pair<int, int> key(flavour, comm.device_of(i));
             if (attr_done.count(key)) continue;
             if (nlocal > 1) cudaSetDevice(comm.device_of(i));
             cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
             if (e != cudaSuccess) return fail(Result::CudaError, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
             attr_done.insert(key);
         }
+        if (cached_pairs[flavour] == 0) {
+            cudaLaunchConfig_t cfg;
+            std::memset(&cfg, 0, sizeof(cfg));
+            cfg.gridDim = dim3(2);
+            cfg.blockDim = dim3(kGemmThreads);
+            cfg.dynamicSmemBytes = smem;
+            int n = 0;
+            cudaError_t e = cudaOccupancyMaxActiveClusters(&n, fn, &cfg);
+            if (e != cudaSuccess || n < 1)
+                return fail(Result::CudaError, std::string("cudaOccupancyMaxActiveClusters: ") + cudaGetErrorString(e));
+            cached_pairs[flavour] = n;
+        }
+        pairs = static_cast<uint32_t>(cached_pairs[flavour]);
     }
-    // Resident CTAs per GPU (queried once per kernel flavour; all GPUs of a group are alike).
-    static int cached_per_sm[2] = {0, 0}, cached_sms[2] = {0, 0};
-    const int flavour = comm.emulated() ? 1 : 0;
-    if (cached_sms[flavour] == 0) {
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&cached_per_sm[flavour], fn, kGemmThreads, smem);
-        cudaDeviceGetAttribute(&cached_sms[flavour], cudaDevAttrMultiProcessorCount, comm.device_of(0));
+    if (comm.emulated()) {
+        if (pairs < static_cast<uint32_t>(W)) return fail(Result::Unsupported, "the GPU holds fewer pairs of CTAs than ranks");
+        pairs /= W;
     }
-    const int per_sm = cached_per_sm[flavour], sms = cached_sms[flavour];
-    uint32_t resident = static_cast<uint32_t>(std::max(1, per_sm) * std::max(1, sms));
-    if (comm.emulated()) resident = std::max<uint32_t>(1, resident / W);
     // One-shot calls split the K extent of their tiles while that shortens the GEMM phase (see FusedLinearTileSplit).
     static const long long forced_split = env::GetInt("YALI_GEMM_KSPLIT", 0);  // measurements only
     uint32_t ksplit = oneshot && mc_mode == 0 && W > 1
-                          ? FusedLinearTileSplit(T, N, K, W, resident, lay.gemm_cap, forced_split > 0 ? static_cast<uint32_t>(forced_split) : 0u)
+                          ? FusedLinearTileSplit(T, N, K, W, pairs, lay.gemm_cap, forced_split > 0 ? static_cast<uint32_t>(forced_split) : 0u)
                           : 1u;
     const uint32_t kper = (K / 64 + ksplit - 1) / ksplit;
-    const uint32_t work = std::max<uint32_t>(ntm * ntn * ksplit, oneshot ? T : Rs);
-    uint32_t ctas = std::min<uint32_t>(resident, work);
+    const GemmTiling tiling = FusedLinearTiling(T, N, W, oneshot, ksplit, pairs);
+    const uint32_t tiles = tiling.domains * tiling.tiles;
+    if (static_cast<uint64_t>(tiles) * (N / kGemmUnitCols) * ksplit > kGemmTileFlags)
+        return fail(Result::Unsupported, "too many tiles for the fused linear");
+    const uint32_t items = tiles * ((N + kGemmPairCols - 1) / kGemmPairCols) * ksplit;
+    const uint32_t work = std::max<uint32_t>(2 * items, oneshot ? T : Rs);
+    uint32_t ctas = std::min<uint32_t>(2 * pairs, work);
     if (opt.ctas > 0) ctas = std::min<uint32_t>(ctas, opt.ctas);
+    ctas = (ctas + 1) / 2 * 2;
 
     std::vector<GemmArArgs> args(nlocal);
     for (int i = 0; i < nlocal; ++i) {
@@ -385,8 +434,8 @@ Result FusedLinearAllReduceRmsNorm(Communicator& comm, const FusedLinearDesc* de
         const FusedLinearDesc& d = descs[i];
         const int rank = comm.rank_of(i);
         if (nlocal > 1) cudaSetDevice(comm.device_of(i));
-        if (!EncodeTileMap(drv, &a.tmap_a, d.x, T, K, kGemmTileM, &derr) ||
-            !EncodeTileMap(drv, &a.tmap_b, d.w, N, K, kGemmTileN, &derr))
+        if (!EncodeTileMap(drv, &a.tmap_x, d.x, T, K, tiling.tokens / 2, &derr) ||
+            !EncodeTileMap(drv, &a.tmap_w, d.w, N, K, kGemmUnitCols, &derr))
             return fail(Result::CudaError, derr);
         a.cv = comm.View(i);
         a.residual = d.residual;
@@ -411,11 +460,12 @@ Result FusedLinearAllReduceRmsNorm(Communicator& comm, const FusedLinearDesc* de
         a.T = T;
         a.N = N;
         a.K = K;
+        a.tl = tiling;
         a.rows_per_owner = Rs;
+        a.one_gpu = comm.emulated() || W == 1 ? 1u : 0u;
         a.oneshot = oneshot ? 1u : 0u;
         a.ksplit = ksplit;
         a.kper = kper;
-        a.cnt_inc = arrivals[rank] * ksplit;  // every (tile, split) is announced
         for (int q = 0; q < W; ++q) a.done_inc[q] = rows_of[q];
         a.eps = opt.eps;
         a.nvls = nvls ? 1u : 0u;

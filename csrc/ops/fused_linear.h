@@ -9,6 +9,7 @@
 #include <cuda_runtime.h>
 
 #include "../comm/communicator.h"
+#include "../kernels/gemm_ar_rmsnorm.h"
 
 namespace yali {
 
@@ -50,6 +51,8 @@ uint32_t FusedLinearTileSplit(uint32_t T, uint32_t N, uint32_t K, int world, uin
 uint32_t FusedLinearDecodeTile(uint32_t N, uint32_t ksplit, uint32_t resident_ctas);
 uint32_t FusedLinearDecodeSplit(uint32_t T, uint32_t N, uint32_t K, int world, uint32_t resident_ctas, uint64_t ll_cap,
                                 uint32_t want);
+// Token tiles of the tile form for `pairs` resident pairs of CTAs per rank.
+GemmTiling FusedLinearTiling(uint32_t T, uint32_t N, int world, bool oneshot, uint32_t ksplit, uint32_t pairs);
 // Rows from which the two-shot form is used when `force_oneshot` is -1.
 uint32_t FusedLinearOneShotMaxRows(int world);
 int FusedLinearAutoMulticastMode(int world, uint32_t T);

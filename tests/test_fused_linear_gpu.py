@@ -118,3 +118,28 @@ def test_fused_linear_rejects_bad_shapes(comm):
     with pytest.raises(RuntimeError, match="multiple"):
         comm.fused_linear_rmsnorm(xs, ws, [nw] * W, None)
     comm.sync()
+
+
+@pytest.mark.parametrize("world", [2, 3, 8])
+@pytest.mark.parametrize("T", [1, 31, 33, 65, 161, 256, 257, 513])
+@pytest.mark.parametrize("K,N", [(64, 128), (64, 384), (192, 1024)])
+def test_tile_form_at_the_edges_of_its_tiles(world, T, K, N):
+    """Token tiles are multiples of 32 up to 256 rows, column tiles are two units of 128 (the second may lie beyond N),
+    rows go to two groups of warps in turn.  Whole-number inputs: partial sums, their sum and the new residual are
+    exact in bf16 (below 256), so the residual is compared bit by bit; the norm adds one rounding (2^-8)."""
+    g = torch.Generator(device="cuda").manual_seed(T * N + world)
+    with yali.Comm.emulated(world, device=0) as c:
+        pick = lambda *s, p: ((torch.rand(s, generator=g, device="cuda") < p).float() * torch.randint(-1, 2, s, generator=g, device="cuda")).to(torch.bfloat16)
+        xs, ws = [pick(T, K, p=0.5) for _ in range(world)], [pick(N, K, p=0.5) for _ in range(world)]
+        nw, res = torch.full((N,), 0.5, dtype=torch.bfloat16, device="cuda"), pick(T, N, p=0.9)
+        want = sum(x.double() @ w.double().T for x, w in zip(xs, ws)) + res.double()
+        assert want.abs().max() < 256
+        y = want * torch.rsqrt(want.pow(2).mean(-1, keepdim=True) + 1e-5) * 0.5
+        for oneshot in (False, True):
+            pre = [torch.empty_like(res) for _ in range(world)]
+            outs = [c.fused_linear_rmsnorm(xs, ws, [nw] * world, [res] * world, residual_out=pre, oneshot=oneshot, decode=False) for _ in range(3)]
+            c.sync()
+            for p in pre:
+                assert torch.equal(p.double(), want)
+            for o in outs[0] + outs[2]:
+                torch.testing.assert_close(o.double(), y, rtol=2.0 ** -8, atol=1e-6)
