@@ -111,6 +111,7 @@ __device__ __forceinline__ bool check_out_last(const CommView& cv, uint32_t kind
 // to check in may advance them at once, because only the next launch reads them again.  Takes the
 // counter's round trip out of the end of the call, and needs no fence: no data hangs on it.
 __device__ __forceinline__ bool check_in_last(const CommView& cv, uint32_t kind, uint32_t nctas) {
+    if (nctas == 1) return true;
     uint32_t* done = flag_word(cv, cv.rank, kCallDoneCtas + kind);
     if (atomicAdd(done, 1u) != nctas - 1) return false;
     *reinterpret_cast<volatile uint32_t*>(done) = 0u;
@@ -152,6 +153,19 @@ __device__ __forceinline__ void finish_call(const CommView& cv, uint32_t kind, u
         advance_call_word(cv, word, inc);
         trace_end(cv, flags);
     }
+}
+
+// A call that checks its CTAs in advances its call word here, after all threads of the CTA have read it, by the last
+// thread (the first ones wait for the peers).  A traced call still checks out at its end, where the timeline
+// wants its stamp.
+__device__ __forceinline__ void check_in(const CommView& cv, uint32_t kind, uint32_t word, uint32_t inc, uint32_t nctas,
+                                         uint32_t flags) {
+    if (!(flags & kFlagTrace) && threadIdx.x == blockDim.x - 1 && check_in_last(cv, kind, nctas))
+        advance_call_word(cv, word, inc);
+}
+__device__ __forceinline__ void finish_checked_in_call(const CommView& cv, uint32_t kind, uint32_t word, uint32_t inc,
+                                                       uint32_t nctas, uint32_t flags) {
+    if (flags & kFlagTrace) finish_call(cv, kind, word, inc, nctas, flags);
 }
 
 // Bounded wait on an mbarrier phase: gives up at the deadline or when another thread of the CTA

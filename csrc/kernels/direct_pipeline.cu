@@ -84,6 +84,7 @@ __device__ __forceinline__ void direct_body(const CollArgs& a, uint32_t cta) {
     }
     const uint64_t n_chunks = (range_ve - range_vb + chunk_vec - 1) / chunk_vec;
 
+    check_in(cv, 2, kCallBarEpoch, 2, nctas, a.flags);
     // Nobody touches a peer's memory before that peer's kernel runs.  On a timeout nothing is in
     // flight yet and the CTA simply leaves.
     if (!cta_barrier_all_ranks(cv, cta, epoch + 1, deadline, &s_abort)) return;
@@ -91,7 +92,7 @@ __device__ __forceinline__ void direct_body(const CollArgs& a, uint32_t cta) {
     volatile int* abort_flag = &s_abort;
     if (warp == 0) {
         // ---------------------------------------------------------------- producer
-        if (lane == 0) {
+        if (ptx::elect_one()) {  // elect.sync: the compiler then issues the copies without a loop over active threads
             // The barrier's acquire ordered the peers' earlier (generic-proxy) writes before this
             // thread; the bulk copies below read through the async proxy.
             ptx::fence_proxy_async();
@@ -185,7 +186,7 @@ __device__ __forceinline__ void direct_body(const CollArgs& a, uint32_t cta) {
     if (s_abort) return;
     // Peers have read this rank's input and their stores into this rank's output are visible.
     if (!cta_barrier_all_ranks(cv, cta, epoch + 2, deadline, &s_abort)) return;
-    finish_call(cv, 2, kCallBarEpoch, 2, nctas, a.flags);
+    finish_checked_in_call(cv, 2, kCallBarEpoch, 2, nctas, a.flags);
 }
 
 template <typename Tin, typename Tout, int WORLD, bool ONE_SHOT>

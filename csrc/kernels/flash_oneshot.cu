@@ -114,6 +114,7 @@ __device__ __forceinline__ void flash_body(const CollArgs& a, uint32_t cta) {
     push_slice<Tin, WORLD>(a, parity, vb, ve, tb, te);
     __syncthreads();
     signal_peers(cv, kFlashFlagOff + cta * kMaxRanks, epoch);
+    check_in(cv, 0, kCallFlashEpoch, 1, a.ctas, a.flags);  // while the peers' copies are on their way
     if (!wait_peers(cv, kFlashFlagOff + cta * kMaxRanks, epoch, deadline, kSiteFlashArrive, cta, &s_abort)) return;
 
     // Sum in rank order; own contribution comes from the send buffer itself.
@@ -171,7 +172,7 @@ __device__ __forceinline__ void flash_body(const CollArgs& a, uint32_t cta) {
             if (q < W) s += to_f32<Tin>(__ldcg(reinterpret_cast<const Tin*>(in[q]) + e));
         out[e] = from_f32<Tout>(epi(s));
     }
-    finish_call(cv, 0, kCallFlashEpoch, 1, a.ctas, a.flags);
+    finish_checked_in_call(cv, 0, kCallFlashEpoch, 1, a.ctas, a.flags);
 }
 
 // One-shot all-reduce fused with residual-add + RMSNorm.  The message is
@@ -204,6 +205,7 @@ __device__ __forceinline__ void flash_rmsnorm_body(const CollArgs& a, uint32_t c
     push_slice<T, WORLD>(a, parity, rb * vec_per_row, re * vec_per_row, 0, 0);
     __syncthreads();
     signal_peers(cv, kFlashFlagOff + cta * kMaxRanks, epoch);
+    check_in(cv, 0, kCallFlashEpoch, 1, a.ctas, a.flags);  // while the peers' copies are on their way
     if (!wait_peers(cv, kFlashFlagOff + cta * kMaxRanks, epoch, deadline, kSiteFlashArrive, cta, &s_abort)) return;
 
     constexpr int kMaxW = WORLD ? WORLD : kMaxRanks;
@@ -253,7 +255,7 @@ __device__ __forceinline__ void flash_rmsnorm_body(const CollArgs& a, uint32_t c
             }
         }
     }
-    finish_call(cv, 0, kCallFlashEpoch, 1, a.ctas, a.flags);
+    finish_checked_in_call(cv, 0, kCallFlashEpoch, 1, a.ctas, a.flags);
 }
 
 // Flag-in-data form of the one-shot all-reduce for small messages.  Every 16-byte line
@@ -326,6 +328,12 @@ __device__ __forceinline__ void flash_ll_body(const CollArgs& a, uint32_t cta) {
             }
         }
     }
+    const bool traced = (a.flags & kFlagTrace) != 0;
+    auto advance_call = [&] {
+        advance_call_word(cv, kCallFlashEpoch, 1);
+        if (lo == 0u) advance_call_word(cv, kCallFlashEpochHi, 1);
+    };
+    if (!traced && tid == nt - 1 && check_in_last(cv, 0, a.ctas)) advance_call();  // while the lines are on their way
     // ---- reduce: poll the peers' lines for the same vectors
     const EpiScale epi(a.ep);
     T* out = static_cast<T*>(a.recv);
@@ -362,10 +370,10 @@ __device__ __forceinline__ void flash_ll_body(const CollArgs& a, uint32_t cta) {
         if (aligned) store_lanes<T, VEC>(out + v * VEC, f);
         else store16_elems<T>(out, v, pack16<T>(f));
     }
+    if (!traced) return;
     if (__syncthreads_or(timed_out ? 1 : 0)) return;
     if (tid == 0 && check_out_last(cv, 0, a.ctas)) {
-        advance_call_word(cv, kCallFlashEpoch, 1);
-        if (lo == 0u) advance_call_word(cv, kCallFlashEpochHi, 1);
+        advance_call();
         trace_end(cv, a.flags);
     }
 }

@@ -131,6 +131,10 @@ __device__ __forceinline__ void decode_body(const GemmDecodeArgs& a, const CUten
     const uint32_t lo = s_call[0] + 1u;                                    // this call's number
     const uint32_t hi = (s_call[1] + (lo == 0u ? 1u : 0u)) | 0x80000000u;  // never zero: fresh memory never matches
     const uint32_t parity = lo & 1u;
+    if (tid == kGemmDecodeThreads - 1 && check_in_last(cv, 3, nctas)) {  // a warp that is idle until the rows
+        advance_call_word(cv, kCallGemmLLEpoch, 1);
+        if (lo == 0u) advance_call_word(cv, kCallGemmLLEpochHi, 1);
+    }
     YALI_DSTAMP(1, 0);
 
     const uint32_t DBN = a.tile_n;             // 128 or 256
@@ -147,8 +151,10 @@ __device__ __forceinline__ void decode_body(const GemmDecodeArgs& a, const CUten
     uint8_t* const smem_b = smem + stages * a_bytes;
 
     // ------------------------------------------------------------------ phase 1: GEMM items [128 x 256 x K / ksplit]
+    // The issuing threads are picked by elect.sync: behind a lane test the compiler wraps every TMA and MMA
+    // instruction in a loop over the active threads (about 200 cycles each, measured).
     if (warp == 2) {
-        if (lane == 0) {
+        if (ptx::elect_one()) {
             uint32_t s = 0, round = 0;
             for (uint32_t item = cta; item < nitems && !*abort_flag; item += nctas) {
                 const uint32_t tile = item / ksplit, ks = item % ksplit;
@@ -167,7 +173,7 @@ __device__ __forceinline__ void decode_body(const GemmDecodeArgs& a, const CUten
             }
         }
     } else if (warp == 3) {
-        if (lane == 0) {
+        if (ptx::elect_one()) {
             uint32_t s = 0, round = 0, it = 0;
             for (uint32_t item = cta; item < nitems && !*abort_flag; item += nctas, ++it) {
                 const uint32_t ks = item % ksplit;
@@ -383,10 +389,6 @@ __device__ __forceinline__ void decode_body(const GemmDecodeArgs& a, const CUten
     if (s_abort) return;
     YALI_DSTAMP(4, 0);  // rows written
 #undef YALI_DSTAMP
-    if (tid == 0 && check_out_last(cv, 3, nctas)) {
-        advance_call_word(cv, kCallGemmLLEpoch, 1);
-        if (lo == 0u) advance_call_word(cv, kCallGemmLLEpochHi, 1);
-    }
 }
 
 }  // namespace

@@ -83,6 +83,9 @@ __device__ __forceinline__ void stream_body(const CollArgs& a, uint32_t lane) {
     const uint64_t shard = a.shard_elems;
     const uint64_t piece = a.slot_bytes / kElemBytes;
     const uint64_t n_pieces = (shard + piece - 1) / piece;
+    // The next call continues after the largest sequence number any lane can use.
+    const uint32_t seq_used = static_cast<uint32_t>((n_pieces + nlanes - 1) / nlanes);
+    check_in(cv, 1, kCallStreamSeq, seq_used, nlanes, a.flags);
     const uint32_t n_it = lane < n_pieces ? static_cast<uint32_t>((n_pieces - lane + nlanes - 1) / nlanes) : 0u;
     const uint32_t rs_word = kRsSeqOff + lane * kMaxRanks;
     const uint32_t ag_word = kAgSeqOff + lane * kMaxRanks;
@@ -232,8 +235,7 @@ __device__ __forceinline__ void stream_body(const CollArgs& a, uint32_t lane) {
     if ((rs_only || (ag_only && !direct)) && n_it > 0) {
         if (!wait_peers(cv, cr_word, seq_base + n_it, deadline, kSiteStreamDrain, lane, &s_abort)) return;
     }
-    // The next call continues after the largest sequence number any lane can have used.
-    finish_call(cv, 1, kCallStreamSeq, static_cast<uint32_t>((n_pieces + nlanes - 1) / nlanes), nlanes, a.flags);
+    finish_checked_in_call(cv, 1, kCallStreamSeq, seq_used, nlanes, a.flags);
 }
 
 template <typename Tin, typename Tout, int WORLD>
