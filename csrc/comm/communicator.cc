@@ -418,7 +418,7 @@ Result Communicator::Launch(const Plan& plan, Dtype in, Dtype out, int epilogue,
             }
             cudaEventRecord(l.prof_start, s);
         }
-        cudaError_t ce = cudaLaunchKernel(fn, dim3(plan.ctas), dim3(threads), params, smem, s);
+        cudaError_t ce = LaunchInStream(fn, dim3(plan.ctas), dim3(threads), params, smem, s);
         if (ce != cudaSuccess) {
             (void)cudaGetLastError();
             return Fail(Result::CudaError, std::string("kernel launch failed: ") + cudaGetErrorString(ce));
@@ -516,7 +516,7 @@ Result Communicator::LaunchLocal(const Plan& plan, const void* const* send, void
     last_.flags = plan.flags;
     void* params[] = {&a};
     cudaStream_t s = streams && streams[0] ? streams[0] : local_[0].stream;
-    cudaError_t ce = cudaLaunchKernel(fn, grid, block, params, 0, s);
+    cudaError_t ce = LaunchInStream(fn, grid, block, params, 0, s);
     if (ce != cudaSuccess) {
         (void)cudaGetLastError();
         return Fail(Result::CudaError, std::string("kernel launch failed: ") + cudaGetErrorString(ce));

@@ -21,6 +21,9 @@ __device__ __forceinline__ uint64_t globaltimer() {
     return t;
 }
 __device__ __forceinline__ void nanosleep(uint32_t ns) { asm volatile("nanosleep.u32 %0;" ::"r"(ns)); }
+// Launches with programmatic stream serialization (kernels/launch.h, LaunchInStream) may start before the kernel in
+// front of them has finished; this waits until it has, and its writes are visible.  Otherwise no effect.
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ uint32_t lane_id() {
     uint32_t l;
     asm volatile("mov.u32 %0, %%laneid;" : "=r"(l));

@@ -45,6 +45,7 @@ template <typename Tin, typename Tout, int WORLD, bool ONE_SHOT>
 __device__ __forceinline__ void direct_body(const CollArgs& a, uint32_t cta) {
     constexpr int VEC = TypeTraits<Tin>::kVec;
     constexpr int kMaxW = WORLD ? WORLD : kMaxRanks;
+    ptx::grid_dependency_wait();
     if (a.flags & kFlagSkipRank) return;
     const CommView& cv = a.cv;
     const int W = WORLD ? WORLD : cv.world, r = cv.rank;

@@ -78,6 +78,7 @@ __device__ __forceinline__ void push_slice(const CollArgs& a, uint32_t parity, u
 template <typename Tin, typename Tout, int WORLD>
 __device__ __forceinline__ void flash_body(const CollArgs& a, uint32_t cta) {
     constexpr int VEC = TypeTraits<Tin>::kVec;
+    ptx::grid_dependency_wait();
     if (a.flags & kFlagSkipRank) return;
     const CommView& cv = a.cv;
     const int W = world_of<WORLD>(cv), r = cv.rank;
@@ -182,6 +183,7 @@ template <typename T, int WORLD>
 __device__ __forceinline__ void flash_rmsnorm_body(const CollArgs& a, uint32_t cta) {
     constexpr int VEC = TypeTraits<T>::kVec;
     constexpr int kMaxVecPerThread = 4;
+    ptx::grid_dependency_wait();
     if (a.flags & kFlagSkipRank) return;
     const CommView& cv = a.cv;
     const int W = world_of<WORLD>(cv), r = cv.rank;
@@ -281,6 +283,7 @@ __device__ __forceinline__ void flash_ll_body(const CollArgs& a, uint32_t cta) {
     constexpr int VEC = TypeTraits<T>::kVec;
     constexpr int kMaxW = WORLD ? WORLD : kMaxRanks;
     constexpr int kMaxPeers = kMaxW - 1;
+    ptx::grid_dependency_wait();
     if (a.flags & kFlagSkipRank) return;
     const CommView& cv = a.cv;
     const int W = world_of<WORLD>(cv), r = cv.rank;

@@ -96,6 +96,7 @@ __device__ __forceinline__ void decode_body(const GemmDecodeArgs& a, const CUten
     const int W = cv.world, r = cv.rank;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     volatile int* abort_flag = &s_abort;
+    ptx::grid_dependency_wait();
     const uint64_t deadline = ptx::globaltimer() + cv.timeout_ns;
 #define YALI_DSTAMP(slot, who)                                                       \
     do {                                                                             \

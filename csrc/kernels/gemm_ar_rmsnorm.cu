@@ -351,6 +351,7 @@ __device__ __forceinline__ void gemm_ar_body(const GemmArArgs& a, uint32_t cta, 
     const int W = cv.world, r = cv.rank;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t half = ptx::cluster_cta_rank();  // which 128 of the pair's 256 columns, which half of its tokens
+    ptx::grid_dependency_wait();
     const uint64_t deadline = ptx::globaltimer() + cv.timeout_ns;
     // Optional timeline of CTA 0 (a.trace != nullptr): %globaltimer at the phase boundaries.
 #define YALI_STAMP(slot, who)                                                              \

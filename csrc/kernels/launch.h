@@ -11,6 +11,8 @@
 
 #include <cuda_runtime.h>
 
+#include <cstring>
+
 #include "../comm/layout.h"
 
 namespace yali {
@@ -20,6 +22,25 @@ constexpr int kStreamThreads = 512;
 constexpr int kNvlsThreads = 512;
 constexpr int kDirectThreads = 288;   // one producer warp + eight consumer warps
 constexpr int kDirectMaxStages = kMaxPipelineStages;
+
+// Ordinary (not cooperative) launch.  Programmatic stream serialization lets the launch overlap the end of the kernel in
+// front of it in the stream, whose results the kernel waits for with ptx::grid_dependency_wait() before anything
+// else.  Without it back-to-back launches on B200 take turns on a 2.05 us grid: a 5.2 us kernel came every 8.2 us,
+// with it every 5.9 us.
+inline cudaError_t LaunchInStream(const void* fn, dim3 grid, dim3 block, void** params, size_t smem, cudaStream_t s) {
+    cudaLaunchConfig_t cfg;
+    std::memset(&cfg, 0, sizeof(cfg));
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelExC(&cfg, fn, params);
+}
 
 // nullptr when the combination is not built.
 const void* FlashKernelFor(Dtype in, Dtype out, int epilogue, int world, bool emu);

@@ -76,6 +76,7 @@ __global__ void __launch_bounds__(kLocalThreads) local_kernel(const __grid_const
     constexpr int NIN = E * sizeof(Tin) / 16;
     constexpr int kMaxW = WORLD ? WORLD : kMaxRanks;
     const uint32_t W = WORLD ? WORLD : a.world;
+    ptx::grid_dependency_wait();
     local_trace_begin(a);
     const EpiScale epi(a.ep);
     const uint32_t owner = KIND == LocalKind::Sum ? 0u : blockIdx.y;
@@ -167,6 +168,7 @@ __global__ void __launch_bounds__(kLocalThreads) local_norm_kernel(const __grid_
     constexpr int kMaxW = WORLD ? WORLD : kMaxRanks;
     const uint32_t W = WORLD ? WORLD : a.world;
     __shared__ float s_red[G][kLocalThreads / 32];
+    ptx::grid_dependency_wait();
     local_trace_begin(a);
     const uint32_t ngroups = (W + G - 1) / G;
     const uint32_t row = blockIdx.x / ngroups, q0 = (blockIdx.x % ngroups) * G;

@@ -112,6 +112,7 @@ __device__ __forceinline__ void reduce_range(const char* mc_in, char* out, uint6
 template <typename T, bool TWO_SHOT>
 __global__ void __launch_bounds__(kNvlsThreads, 2) nvls_kernel(const __grid_constant__ CollArgs a) {
     constexpr int VEC = TypeTraits<T>::kVec;
+    ptx::grid_dependency_wait();
     if (a.flags & kFlagSkipRank) return;
     const CommView& cv = a.cv;
     const int W = cv.world, r = cv.rank;

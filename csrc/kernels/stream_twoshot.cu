@@ -63,6 +63,7 @@ __device__ __forceinline__ void stream_body(const CollArgs& a, uint32_t lane) {
     constexpr int VEC = TypeTraits<Tin>::kVec;
     constexpr uint32_t kElemBytes = sizeof(Tin) > sizeof(Tout) ? sizeof(Tin) : sizeof(Tout);
     constexpr int kMaxW = WORLD ? WORLD : kMaxRanks;
+    ptx::grid_dependency_wait();
     if (a.flags & kFlagSkipRank) return;
     const CommView& cv = a.cv;
     const int W = world_of<WORLD>(cv), r = cv.rank;

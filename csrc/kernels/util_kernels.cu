@@ -13,6 +13,7 @@
 #include <cuda_fp16.h>
 
 #include "../ops/buffer_ops.h"
+#include "launch.h"
 #include "type_ops.cuh"
 
 namespace yali {
@@ -81,6 +82,7 @@ __global__ void __launch_bounds__(512) residual_rmsnorm_kernel(T* x, const T* re
                                                                uint32_t hidden, float eps) {
     constexpr int VEC = TypeTraits<T>::kVec;
     __shared__ float s_part[16];
+    ptx::grid_dependency_wait();
     const int tid = threadIdx.x, nt = blockDim.x;
     const uint32_t vec_per_row = hidden / VEC;
     const uint64_t row_off = static_cast<uint64_t>(blockIdx.x) * hidden;
@@ -255,9 +257,11 @@ void LaunchResidualRmsNorm(void* x, const void* residual, void* residual_out, co
     const uint32_t nv = vec_per_row <= 128 ? 1 : vec_per_row <= 1024 ? 2 : 4;
     const uint32_t threads = ((vec_per_row + nv - 1) / nv + 31) / 32 * 32;
     const uint32_t grid = static_cast<uint32_t>(rows);
-    if (nv == 1) residual_rmsnorm_kernel<T, 1><<<grid, threads, 0, s>>>(xt, rt, ot, wt, hidden, eps);
-    else if (nv == 2) residual_rmsnorm_kernel<T, 2><<<grid, threads, 0, s>>>(xt, rt, ot, wt, hidden, eps);
-    else residual_rmsnorm_kernel<T, 4><<<grid, threads, 0, s>>>(xt, rt, ot, wt, hidden, eps);
+    const void* fn = nv == 1   ? (const void*)residual_rmsnorm_kernel<T, 1>
+                     : nv == 2 ? (const void*)residual_rmsnorm_kernel<T, 2>
+                               : (const void*)residual_rmsnorm_kernel<T, 4>;
+    void* params[] = {&xt, &rt, &ot, &wt, &hidden, &eps};
+    (void)LaunchInStream(fn, dim3(grid), dim3(threads), params, 0, s);
 }
 }  // namespace
 

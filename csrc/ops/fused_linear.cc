@@ -10,6 +10,7 @@
 
 #include "../comm/cuda_driver.h"
 #include "../kernels/gemm_ar_rmsnorm.h"
+#include "../kernels/launch.h"
 
 namespace yali {
 
@@ -103,7 +104,7 @@ Result LaunchDecode(Communicator& comm, const DriverApi* drv, const FusedLinearD
         if (nlocal > 1) cudaSetDevice(comm.device_of(i));
         cudaStream_t s = streams && streams[i] ? streams[i] : comm.default_stream(i);
         void* params[] = {&args[i]};
-        cudaError_t ce = cudaLaunchKernel(fn, dim3(ctas), dim3(kGemmDecodeThreads), params, smem, s);
+        cudaError_t ce = LaunchInStream(fn, dim3(ctas), dim3(kGemmDecodeThreads), params, smem, s);
         if (ce != cudaSuccess) {
             (void)cudaGetLastError();
             return fail(Result::CudaError, std::string("kernel launch failed: ") + cudaGetErrorString(ce));
@@ -494,7 +495,7 @@ Result FusedLinearAllReduceRmsNorm(Communicator& comm, const FusedLinearDesc* de
         if (nlocal > 1) cudaSetDevice(comm.device_of(i));
         cudaStream_t s = streams && streams[i] ? streams[i] : comm.default_stream(i);
         void* params[] = {&args[i]};
-        cudaError_t ce = cudaLaunchKernel(fn, dim3(ctas), dim3(kGemmThreads), params, smem, s);
+        cudaError_t ce = LaunchInStream(fn, dim3(ctas), dim3(kGemmThreads), params, smem, s);
         if (ce != cudaSuccess) {
             (void)cudaGetLastError();
             return fail(Result::CudaError, std::string("kernel launch failed: ") + cudaGetErrorString(ce));
