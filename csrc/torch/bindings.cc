@@ -7,6 +7,8 @@
 // C++ headers as the only interface); this file is an addition.
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
+#include <ATen/cuda/EmptyTensor.h>
+#include <torch/csrc/autograd/python_variable.h>
 #include <torch/extension.h>
 
 #include <memory>
@@ -202,129 +204,264 @@ class PyComm {
         Throw(res, c().last_error());
     }
 
-    void AllReduceRmsNorm(std::vector<at::Tensor> send, std::vector<at::Tensor> recv,
-                          c10::optional<std::vector<at::Tensor>> residual,
-                          c10::optional<std::vector<at::Tensor>> residual_out, std::vector<at::Tensor> weight,
-                          double eps, const std::string& mode, int ctas) {
-        at::ScalarType sd, rd, wd;
-        int64_t sn, rn, wn;
-        CheckTensors(send, "send", &sd, &sn);
-        CheckTensors(recv, "recv", &rd, &rn);
-        CheckTensors(weight, "weight", &wd, &wn);
+    // ---- the calls a program makes, straight from Python objects ----
+    // A collective argument is a tensor (one local rank) or a sequence of one tensor per local rank.  Everything from
+    // here to the launch stays in C++ and allocates nothing but the outputs: for small messages the time per
+    // call is the host's, and building lists, optionals and vectors of tensors for eight ranks took longer
+    // than the kernel ran (28 us a call for the all-reduce + RMSNorm of 16 rows over eight ranks).
+    struct Args {
+        const at::Tensor* t[kMaxRanks];
+        PyObject* obj[kMaxRanks];
+        py::object held;  // a list made of another kind of sequence
+        const at::Tensor& operator[](int i) const { return *t[i]; }
+    };
+    // False: `o` is None (where that is allowed).
+    bool Read(PyObject* o, const char* what, Args* a, bool optional = false) {
+        if (optional && o == Py_None) return false;
+        const int n = c().nlocal();
+        if (THPVariable_Check(o)) {
+            if (n != 1)
+                throw py::value_error(std::string(what) + ": this communicator drives " + std::to_string(n) +
+                                      " ranks; pass one tensor per rank");
+            a->obj[0] = o;
+            a->t[0] = &THPVariable_Unpack(o);
+            return true;
+        }
+        if (!PyList_Check(o) && !PyTuple_Check(o)) {
+            a->held = py::reinterpret_steal<py::object>(PySequence_List(o));
+            if (!a->held) throw py::error_already_set();
+            o = a->held.ptr();
+        }
+        const Py_ssize_t len = PySequence_Fast_GET_SIZE(o);
+        if (len != n)
+            throw py::value_error(std::string(what) + ": expected " + std::to_string(n) + " tensors, got " + std::to_string(len));
+        PyObject** items = PySequence_Fast_ITEMS(o);
+        for (int i = 0; i < n; ++i) {
+            TORCH_CHECK_TYPE(THPVariable_Check(items[i]), "yali: ", what, "[", i, "] is not a tensor");
+            a->obj[i] = items[i];
+            a->t[i] = &THPVariable_Unpack(items[i]);
+        }
+        return true;
+    }
+    void CheckArgs(const Args& a, const char* what, at::ScalarType* dt, int64_t* numel) {
+        const int n = c().nlocal();
+        for (int i = 0; i < n; ++i) {
+            const at::Tensor& t = a[i];
+            TORCH_CHECK(t.is_cuda(), "yali: ", what, "[", i, "] is not a CUDA tensor");
+            TORCH_CHECK(t.is_contiguous(), "yali: ", what, "[", i, "] is not contiguous");
+            TORCH_CHECK(t.get_device() == c().device_of(i), "yali: ", what, "[", i, "] lives on GPU ", t.get_device(),
+                        ", rank ", c().rank_of(i), " owns GPU ", c().device_of(i));
+            if (i == 0) {
+                *dt = t.scalar_type();
+                *numel = t.numel();
+            } else {
+                TORCH_CHECK(t.scalar_type() == *dt && t.numel() == *numel, "yali: ", what,
+                            " tensors differ in dtype or size");
+            }
+        }
+    }
+    // The outputs of a call: the caller's, or new ones of this shape per local rank.
+    struct Outputs {
+        Args a;
+        at::Tensor fresh[kMaxRanks];
+        bool given = false;
+    };
+    void Out(PyObject* o, const char* what, const Args& like, c10::IntArrayRef sizes, at::ScalarType dt, Outputs* r) {
+        r->given = Read(o, what, &r->a, true);
+        if (r->given) return;
+        for (int i = 0; i < c().nlocal(); ++i) {
+            if (like[i].is_cuda()) r->fresh[i] = at::Tensor(at::detail::empty_cuda(sizes, dt, like[i].device(), c10::nullopt));
+            else r->fresh[i] = at::empty(sizes, like[i].options().dtype(dt));  // CheckArgs says what is wrong
+            r->a.t[i] = &r->fresh[i];
+        }
+    }
+    // What the Python call returns: a tensor where one was given, else a list.
+    py::object Returned(PyObject* like, Outputs& r) {
+        auto one = [&](int i) {
+            if (r.given) return py::reinterpret_borrow<py::object>(r.a.obj[i]);
+            return py::reinterpret_steal<py::object>(THPVariable_Wrap(std::move(r.fresh[i])));
+        };
+        if (THPVariable_Check(like)) return one(0);
+        py::list l(c().nlocal());
+        for (int i = 0; i < c().nlocal(); ++i) PyList_SET_ITEM(l.ptr(), i, one(i).release().ptr());
+        return l;
+    }
+    struct StreamTable {
+        cudaStream_t s[kMaxRanks];
+    };
+    StreamTable CurrentStreams() {
+        StreamTable t;
+        for (int i = 0; i < c().nlocal(); ++i)
+            t.s[i] = i > 0 && c().device_of(i) == c().device_of(0)
+                         ? t.s[0]
+                         : at::cuda::getCurrentCUDAStream(c().device_of(i)).stream();
+        return t;
+    }
+    static KernelMode ModeOf(const py::object& mode) {
+        static PyObject* const auto_name = PyUnicode_InternFromString("auto");
+        if (mode.ptr() == auto_name) return KernelMode::Auto;
+        return ToMode(py::cast<std::string>(mode));
+    }
+    void Finish(Result r) {
+        if (r != Result::Success) Throw(r, c().last_error());
+    }
+
+    py::object CallAllReduce(const py::object& send, const py::object& recv, const py::object& mode, const py::object& scale,
+                             const py::object& out_dtype, int ctas, int slot_bytes, int skip_rank) {
+        Args s;
+        Outputs r;
+        at::ScalarType sd, rd;
+        int64_t sn, rn;
+        Read(send.ptr(), "send", &s);
+        const at::ScalarType want = out_dtype.is_none() ? s[0].scalar_type() : py::cast<at::ScalarType>(out_dtype);
+        Out(recv.ptr(), "recv", s, s[0].sizes(), want, &r);
+        CheckArgs(s, "send", &sd, &sn);
+        CheckArgs(r.a, "recv", &rd, &rn);
+        TORCH_CHECK(sn == rn, "yali: send and recv differ in size");
+        OpOptions o;
+        o.mode = ModeOf(mode);
+        o.ctas = ctas;
+        o.slot_bytes = slot_bytes;
+        o.skip_rank = skip_rank;
+        if (!scale.is_none() || sd != rd) {
+            o.epilogue = kEpiScaleCast;
+            o.scale = scale.is_none() ? 1.0f : static_cast<float>(py::cast<double>(scale));
+        }
+        const void* sp[kMaxRanks];
+        void* rp[kMaxRanks];
+        for (int i = 0; i < c().nlocal(); ++i) {
+            sp[i] = s[i].data_ptr();
+            rp[i] = r.a[i].data_ptr();
+        }
+        const StreamTable st = CurrentStreams();
+        c10::cuda::OptionalCUDAGuard guard(c().device_of(0));
+        Finish(c().AllReduce(sp, rp, sn, ToDtype(sd), ToDtype(rd), o, st.s));
+        return Returned(send.ptr(), r);
+    }
+
+    py::object CallRmsNorm(const py::object& x, const py::object& weight, const py::object& residual, double eps,
+                           const py::object& out, const py::object& residual_out, const py::object& mode, int ctas) {
+        Args s, w, res, ro;
+        Outputs r;
+        at::ScalarType sd, rd, wd, d;
+        int64_t sn, rn, wn, m;
+        Read(x.ptr(), "x", &s);
+        Read(weight.ptr(), "weight", &w);
+        Out(out.ptr(), "out", s, s[0].sizes(), s[0].scalar_type(), &r);
+        const bool has_res = Read(residual.ptr(), "residual", &res, true);
+        const bool has_ro = Read(residual_out.ptr(), "residual_out", &ro, true);
+        CheckArgs(s, "send", &sd, &sn);
+        CheckArgs(r.a, "recv", &rd, &rn);
+        CheckArgs(w, "weight", &wd, &wn);
         TORCH_CHECK(sd == rd && sd == wd && sn == rn, "yali: rmsnorm tensors must agree in dtype and size");
         TORCH_CHECK(wn > 0 && sn % wn == 0, "yali: input size is not a multiple of the hidden size");
         OpOptions o;
-        o.mode = ToMode(mode);
+        o.mode = ModeOf(mode);
         o.ctas = ctas;
         o.epilogue = kEpiResidualRmsNorm;
         o.hidden = static_cast<int>(wn);
         o.eps = static_cast<float>(eps);
-        const int n = c().nlocal();
-        std::vector<const void*> s(n), w(n), res(n, nullptr);
-        std::vector<void*> r(n), ro(n, nullptr);
-        for (int i = 0; i < n; ++i) {
-            s[i] = send[i].data_ptr();
-            r[i] = recv[i].data_ptr();
-            w[i] = weight[i].data_ptr();
-        }
-        if (residual.has_value()) {
-            at::ScalarType d;
-            int64_t m;
-            CheckTensors(*residual, "residual", &d, &m);
+        const void *sp[kMaxRanks], *wp[kMaxRanks], *resp[kMaxRanks];
+        void *rp[kMaxRanks], *rop[kMaxRanks];
+        if (has_res) {
+            CheckArgs(res, "residual", &d, &m);
             TORCH_CHECK(d == sd && m == sn, "yali: residual must match the input");
-            for (int i = 0; i < n; ++i) res[i] = (*residual)[i].data_ptr();
-            o.residual = res.data();
+            o.residual = resp;
         }
-        if (residual_out.has_value()) {
-            at::ScalarType d;
-            int64_t m;
-            CheckTensors(*residual_out, "residual_out", &d, &m);
+        if (has_ro) {
+            CheckArgs(ro, "residual_out", &d, &m);
             TORCH_CHECK(d == sd && m == sn, "yali: residual_out must match the input");
-            for (int i = 0; i < n; ++i) ro[i] = (*residual_out)[i].data_ptr();
-            o.residual_out = ro.data();
+            o.residual_out = rop;
         }
-        o.weight = w.data();
-        auto st = Streams();
+        for (int i = 0; i < c().nlocal(); ++i) {
+            sp[i] = s[i].data_ptr();
+            rp[i] = r.a[i].data_ptr();
+            wp[i] = w[i].data_ptr();
+            if (has_res) resp[i] = res[i].data_ptr();
+            if (has_ro) rop[i] = ro[i].data_ptr();
+        }
+        o.weight = wp;
+        const StreamTable st = CurrentStreams();
         c10::cuda::OptionalCUDAGuard guard(c().device_of(0));
-        Throw(c().AllReduce(s.data(), r.data(), sn, ToDtype(sd), ToDtype(rd), o, st.data()), c().last_error());
+        Finish(c().AllReduce(sp, rp, sn, ToDtype(sd), ToDtype(rd), o, st.s));
+        return Returned(x.ptr(), r);
     }
 
-    // send: full message per rank; recv: ShardElems(count, world) elements per rank.
-    void ReduceScatter(std::vector<at::Tensor> send, std::vector<at::Tensor> recv, int ctas, int slot_bytes) {
+    // Reduce-scatter (rs): send is the full message, recv ShardElems(numel, world) elements per rank; all-gather: send is a
+    // shard per rank, recv `count` elements.
+    py::object CallHalf(const py::object& send, int64_t count, const py::object& recv, int ctas, int slot_bytes, bool rs) {
+        Args s;
+        Outputs r;
         at::ScalarType sd, rd;
         int64_t sn, rn;
-        CheckTensors(send, "send", &sd, &sn);
-        CheckTensors(recv, "recv", &rd, &rn);
+        Read(send.ptr(), "send", &s);
+        const int64_t full = rs ? s[0].numel() : count;
+        const int64_t shard = c().world() > 1 ? static_cast<int64_t>(ShardElems(full, c().world())) : full;
+        const int64_t size[1] = {rs ? shard : full};
+        Out(recv.ptr(), "recv", s, c10::IntArrayRef(size, 1), s[0].scalar_type(), &r);
+        CheckArgs(s, "send", &sd, &sn);
+        CheckArgs(r.a, "recv", &rd, &rn);
         TORCH_CHECK(sd == rd, "yali: dtype mismatch");
-        TORCH_CHECK(static_cast<uint64_t>(rn) >= ShardElems(sn, c().world()) || c().world() == 1,
-                    "yali: recv needs shard_elems(count, world) elements");
-        Run(send, recv, sn, ToDtype(sd), ctas, slot_bytes, true);
-    }
-    // send: ShardElems elements per rank; recv: `count` elements.
-    void AllGather(std::vector<at::Tensor> send, std::vector<at::Tensor> recv, int ctas, int slot_bytes) {
-        at::ScalarType sd, rd;
-        int64_t sn, rn;
-        CheckTensors(send, "send", &sd, &sn);
-        CheckTensors(recv, "recv", &rd, &rn);
-        TORCH_CHECK(sd == rd, "yali: dtype mismatch");
-        TORCH_CHECK(static_cast<uint64_t>(sn) >= ShardElems(rn, c().world()) || c().world() == 1,
-                    "yali: send needs shard_elems(count, world) elements");
-        Run(send, recv, rn, ToDtype(sd), ctas, slot_bytes, false);
-    }
-    void Run(std::vector<at::Tensor>& send, std::vector<at::Tensor>& recv, int64_t count, Dtype dt, int ctas,
-             int slot_bytes, bool rs) {
+        const int64_t owned = static_cast<int64_t>(ShardElems(rs ? sn : rn, c().world()));
+        TORCH_CHECK((rs ? rn : sn) >= owned || c().world() == 1, "yali: ", rs ? "recv" : "send",
+                    " needs shard_elems(count, world) elements");
         OpOptions o;
         o.ctas = ctas;
         o.slot_bytes = slot_bytes;
-        std::vector<const void*> s(send.size());
-        std::vector<void*> r(recv.size());
-        for (size_t i = 0; i < send.size(); ++i) {
-            s[i] = send[i].data_ptr();
-            r[i] = recv[i].data_ptr();
+        const void* sp[kMaxRanks];
+        void* rp[kMaxRanks];
+        for (int i = 0; i < c().nlocal(); ++i) {
+            sp[i] = s[i].data_ptr();
+            rp[i] = r.a[i].data_ptr();
         }
-        auto st = Streams();
+        const StreamTable st = CurrentStreams();
         c10::cuda::OptionalCUDAGuard guard(c().device_of(0));
-        Result res = rs ? c().ReduceScatter(s.data(), r.data(), count, dt, o, st.data())
-                        : c().AllGather(s.data(), r.data(), count, dt, o, st.data());
-        Throw(res, c().last_error());
+        Finish(rs ? c().ReduceScatter(sp, rp, sn, ToDtype(sd), o, st.s) : c().AllGather(sp, rp, rn, ToDtype(sd), o, st.s));
+        return Returned(send.ptr(), r);
     }
 
-    // out = RMSNorm(residual + sum_r x_r @ w_r^T) * norm_weight, one kernel per rank.
-    void FusedLinear(std::vector<at::Tensor> x, std::vector<at::Tensor> w, std::vector<at::Tensor> norm_weight,
-                     std::vector<at::Tensor> out, c10::optional<std::vector<at::Tensor>> residual,
-                     c10::optional<std::vector<at::Tensor>> residual_out, double eps, int force_oneshot, int ctas,
-                     c10::optional<std::vector<at::Tensor>> trace, int nvls, int decode) {
+    // out = RMSNorm(residual + sum_r x_r @ w_r^T) * norm_weight.
+    py::object FusedLinear(const py::object& x, const py::object& w, const py::object& norm_weight, const py::object& out,
+                           const py::object& residual, const py::object& residual_out, double eps, int force_oneshot,
+                           int ctas, const py::object& trace, int nvls, int decode) {
+        Args xa, wa, na, res, ro, ta;
+        Outputs r;
         at::ScalarType d;
         int64_t n;
-        CheckTensors(x, "x", &d, &n);
-        TORCH_CHECK(d == at::kBFloat16, "yali: fused linear takes bf16 tensors");
-        CheckTensors(w, "w", &d, &n);
-        TORCH_CHECK(d == at::kBFloat16, "yali: fused linear takes bf16 tensors");
-        CheckTensors(norm_weight, "norm_weight", &d, &n);
-        TORCH_CHECK(d == at::kBFloat16, "yali: fused linear takes bf16 tensors");
-        CheckTensors(out, "out", &d, &n);
-        TORCH_CHECK(d == at::kBFloat16, "yali: fused linear takes bf16 tensors");
-        TORCH_CHECK(x[0].dim() == 2 && w[0].dim() == 2 && out[0].dim() == 2, "yali: x [T,K], w [N,K], out [T,N]");
-        const int64_t T = x[0].size(0), K = x[0].size(1), N = w[0].size(0);
-        TORCH_CHECK(w[0].size(1) == K && out[0].size(0) == T && out[0].size(1) == N && norm_weight[0].numel() == N,
+        Read(x.ptr(), "x", &xa);
+        Read(w.ptr(), "w", &wa);
+        Read(norm_weight.ptr(), "norm_weight", &na);
+        TORCH_CHECK(xa[0].dim() == 2 && wa[0].dim() == 2, "yali: x [T,K], w [N,K], out [T,N]");
+        const int64_t T = xa[0].size(0), K = xa[0].size(1), N = wa[0].size(0);
+        const int64_t sizes[2] = {T, N};
+        Out(out.ptr(), "out", xa, c10::IntArrayRef(sizes, 2), at::kBFloat16, &r);
+        const bool has_res = Read(residual.ptr(), "residual", &res, true);
+        const bool has_ro = Read(residual_out.ptr(), "residual_out", &ro, true);
+        const std::pair<const Args*, const char*> all[] = {{&xa, "x"}, {&wa, "w"}, {&na, "norm_weight"}, {&r.a, "out"}};
+        for (const auto& p : all) {
+            CheckArgs(*p.first, p.second, &d, &n);
+            TORCH_CHECK(d == at::kBFloat16, "yali: fused linear takes bf16 tensors");
+        }
+        TORCH_CHECK(r.a[0].dim() == 2, "yali: x [T,K], w [N,K], out [T,N]");
+        TORCH_CHECK(wa[0].size(1) == K && r.a[0].size(0) == T && r.a[0].size(1) == N && na[0].numel() == N,
                     "yali: fused linear shape mismatch");
         const int nl = c().nlocal();
-        std::vector<FusedLinearDesc> descs(nl);
+        FusedLinearDesc descs[kMaxRanks];
         for (int i = 0; i < nl; ++i) {
-            descs[i].x = x[i].data_ptr();
-            descs[i].w = w[i].data_ptr();
-            descs[i].norm_weight = norm_weight[i].data_ptr();
-            descs[i].out = out[i].data_ptr();
+            descs[i].x = xa[i].data_ptr();
+            descs[i].w = wa[i].data_ptr();
+            descs[i].norm_weight = na[i].data_ptr();
+            descs[i].out = r.a[i].data_ptr();
         }
-        if (residual.has_value()) {
-            CheckTensors(*residual, "residual", &d, &n);
+        if (has_res) {
+            CheckArgs(res, "residual", &d, &n);
             TORCH_CHECK(d == at::kBFloat16 && n == T * N, "yali: residual must be bf16 [T,N]");
-            for (int i = 0; i < nl; ++i) descs[i].residual = (*residual)[i].data_ptr();
+            for (int i = 0; i < nl; ++i) descs[i].residual = res[i].data_ptr();
         }
-        if (residual_out.has_value()) {
-            CheckTensors(*residual_out, "residual_out", &d, &n);
+        if (has_ro) {
+            CheckArgs(ro, "residual_out", &d, &n);
             TORCH_CHECK(d == at::kBFloat16 && n == T * N, "yali: residual_out must be bf16 [T,N]");
-            for (int i = 0; i < nl; ++i) descs[i].residual_out = (*residual_out)[i].data_ptr();
+            for (int i = 0; i < nl; ++i) descs[i].residual_out = ro[i].data_ptr();
         }
         FusedLinearOptions o;
         o.force_oneshot = force_oneshot;
@@ -332,21 +469,20 @@ class PyComm {
         o.nvls = nvls;
         o.decode = decode;
         o.eps = static_cast<float>(eps);
-        std::vector<unsigned long long*> tr(nl, nullptr);
-        if (trace.has_value()) {
-            TORCH_CHECK(static_cast<int>(trace->size()) == nl, "yali: one trace tensor per local rank");
+        unsigned long long* tr[kMaxRanks] = {};
+        if (Read(trace.ptr(), "trace", &ta, true)) {
             for (int i = 0; i < nl; ++i) {
-                TORCH_CHECK((*trace)[i].scalar_type() == at::kLong && (*trace)[i].numel() >= 8 && (*trace)[i].is_cuda(),
+                TORCH_CHECK(ta[i].scalar_type() == at::kLong && ta[i].numel() >= 8 && ta[i].is_cuda(),
                             "yali: trace tensors are int64 CUDA tensors with 8 elements");
-                tr[i] = reinterpret_cast<unsigned long long*>((*trace)[i].data_ptr());
+                tr[i] = reinterpret_cast<unsigned long long*>(ta[i].data_ptr());
             }
-            o.trace = tr.data();
+            o.trace = tr;
         }
-        auto st = Streams();
+        const StreamTable st = CurrentStreams();
         c10::cuda::OptionalCUDAGuard guard(c().device_of(0));
-        Throw(FusedLinearAllReduceRmsNorm(c(), descs.data(), static_cast<uint32_t>(T), static_cast<uint32_t>(N),
-                                          static_cast<uint32_t>(K), o, st.data()),
-              c().last_error());
+        Finish(FusedLinearAllReduceRmsNorm(c(), descs, static_cast<uint32_t>(T), static_cast<uint32_t>(N),
+                                           static_cast<uint32_t>(K), o, st.s));
+        return Returned(x.ptr(), r);
     }
 
     // One tensor per local rank, at the same offset of every rank's heap.  The tensors alias
@@ -539,17 +675,10 @@ PYBIND11_MODULE(_C, m) {
         .def("read_trace", &PyComm::ReadTrace, py::arg("local_index") = 0, py::arg("max_entries") = 4096)
         .def("all_reduce", &PyComm::AllReduce, py::arg("send"), py::arg("recv"), py::arg("mode") = "auto",
              py::arg("scale") = py::none(), py::arg("ctas") = 0, py::arg("slot_bytes") = 0, py::arg("skip_rank") = -1)
-        .def("all_reduce_rmsnorm", &PyComm::AllReduceRmsNorm, py::arg("send"), py::arg("recv"),
-             py::arg("residual") = py::none(), py::arg("residual_out") = py::none(), py::arg("weight"),
-             py::arg("eps") = 1e-5, py::arg("mode") = "auto", py::arg("ctas") = 0)
-        .def("reduce_scatter", &PyComm::ReduceScatter, py::arg("send"), py::arg("recv"), py::arg("ctas") = 0,
-             py::arg("slot_bytes") = 0)
-        .def("all_gather", &PyComm::AllGather, py::arg("send"), py::arg("recv"), py::arg("ctas") = 0,
-             py::arg("slot_bytes") = 0)
-        .def("fused_linear", &PyComm::FusedLinear, py::arg("x"), py::arg("w"), py::arg("norm_weight"), py::arg("out"),
-             py::arg("residual") = py::none(), py::arg("residual_out") = py::none(), py::arg("eps") = 1e-5,
-             py::arg("force_oneshot") = -1, py::arg("ctas") = 0, py::arg("trace") = py::none(),
-             py::arg("nvls") = -1, py::arg("decode") = -1)
+        .def("call_all_reduce", &PyComm::CallAllReduce)
+        .def("call_all_reduce_rmsnorm", &PyComm::CallRmsNorm)
+        .def("call_half", &PyComm::CallHalf)
+        .def("fused_linear", &PyComm::FusedLinear)
         .def("symm_empty", &PyComm::SymmEmpty, py::arg("shape"), py::arg("dtype"))
         .def("symm_reset", &PyComm::SymmReset)
         .def("all_reduce_host", &PyComm::AllReduceHost, py::arg("src"), py::arg("dst"), py::arg("chunk_bytes") = 0,

@@ -154,31 +154,19 @@ class Comm:
                    slot_bytes: int = 0, _skip_rank: int = -1):
         """recv = cast(scale * sum over ranks of send).  `recv=None` allocates; pass `recv=send` for in place.
         `_skip_rank` makes that rank's kernel leave at once: only for testing that the others time out."""
-        s = self._as_list(send, "send")
-        if recv is None:
-            r = [torch.empty_like(x, dtype=out_dtype or x.dtype) for x in s]
-        else:
-            r = self._as_list(recv, "recv")
         try:
-            self._impl.all_reduce(s, r, mode, scale, ctas, slot_bytes, _skip_rank)
-        except RuntimeError as e:  # noqa: PERF203
+            return self._impl.call_all_reduce(send, recv, mode, scale, out_dtype, ctas, slot_bytes, _skip_rank)
+        except RuntimeError as e:
             raise _translate(e) from None
-        return self._like_input(send, r)
 
     def all_reduce_rmsnorm(self, x: TensorOrList, weight: TensorOrList, residual: Optional[TensorOrList] = None, *,
                            eps: float = 1e-5, out: Optional[TensorOrList] = None,
                            residual_out: Optional[TensorOrList] = None, mode: str = "auto", ctas: int = 0):
         """out = RMSNorm(sum over ranks of x + residual) * weight, row length = weight.numel()."""
-        s = self._as_list(x, "x")
-        w = self._as_list(weight, "weight")
-        r = [torch.empty_like(t) for t in s] if out is None else self._as_list(out, "out")
-        res = None if residual is None else self._as_list(residual, "residual")
-        ro = None if residual_out is None else self._as_list(residual_out, "residual_out")
         try:
-            self._impl.all_reduce_rmsnorm(s, r, res, ro, w, eps, mode, ctas)
+            return self._impl.call_all_reduce_rmsnorm(x, weight, residual, eps, out, residual_out, mode, ctas)
         except RuntimeError as e:
             raise _translate(e) from None
-        return self._like_input(x, r)
 
     def fused_linear_rmsnorm(self, x: TensorOrList, w: TensorOrList, norm_weight: TensorOrList,
                              residual: Optional[TensorOrList] = None, *, eps: float = 1e-5,
@@ -196,33 +184,25 @@ class Comm:
         multicast store; 1 and 2 need the multicast object and `out` from symm_empty().  `decode`: the
         few-token form (up to 64 rows: 128 x 256 tiles whose K extent is split over CTAs, partial rows sent to every rank as
         flag-in-data lines, every rank normalises all rows): None = by size, False = never, True = required."""
-        xs, ws, nws = self._as_list(x, "x"), self._as_list(w, "w"), self._as_list(norm_weight, "norm_weight")
-        if out is None:
-            T, N = xs[0].shape[0], ws[0].shape[0]
-            if self.nlocal == 1 and self.world > 1:
-                # Symmetric memory is never freed piecemeal: keep ONE output per row width, large enough for the
-                # most rows seen so far (grown by doubling, so a program that varies its token count holds at
-                # most twice its largest output per width), and hand out its first T rows.  The tensor returned
-                # by a call is therefore overwritten by the next call of that width.
-                cache = self.__dict__.setdefault("_fused_out", {})
-                buf = cache.get(N)
-                if buf is None or buf.shape[0] < T:
-                    rows = T if buf is None else max(T, 2 * buf.shape[0])
-                    buf = cache[N] = self.symm_empty([rows, N], torch.bfloat16)
-                outs = [buf[:T]]
-            else:
-                outs = [torch.empty(T, N, dtype=torch.bfloat16, device=t.device) for t in xs]
-        else:
-            outs = self._as_list(out, "out")
-        res = None if residual is None else self._as_list(residual, "residual")
-        ro = None if residual_out is None else self._as_list(residual_out, "residual_out")
+        if out is None and self.nlocal == 1 and self.world > 1:
+            # Symmetric memory is never freed piecemeal: keep ONE output per row width, large enough for the
+            # most rows seen so far (grown by doubling, so a program that varies its token count holds at
+            # most twice its largest output per width), and hand out its first T rows.  The tensor returned
+            # by a call is therefore overwritten by the next call of that width.
+            T, N = self._as_list(x, "x")[0].shape[0], self._as_list(w, "w")[0].shape[0]
+            cache = self.__dict__.setdefault("_fused_out", {})
+            buf = cache.get(N)
+            if buf is None or buf.shape[0] < T:
+                rows = T if buf is None else max(T, 2 * buf.shape[0])
+                buf = cache[N] = self.symm_empty([rows, N], torch.bfloat16)
+            out = [buf[:T]]
         try:
-            tr = None if trace is None else self._as_list(trace, "trace")
-            self._impl.fused_linear(xs, ws, nws, outs, res, ro, eps, -1 if oneshot is None else int(oneshot), ctas, tr,
-                                    -1 if nvls is None else int(nvls), -1 if decode is None else int(decode))
+            r = self._impl.fused_linear(x, w, norm_weight, out, residual, residual_out, eps,
+                                        -1 if oneshot is None else int(oneshot), ctas, trace,
+                                        -1 if nvls is None else int(nvls), -1 if decode is None else int(decode))
         except RuntimeError as e:
             raise _translate(e) from None
-        return self._like_input(x, outs)
+        return r if out is None else self._like_input(x, self._as_list(out, "out"))
 
     def all_reduce_host(self, src: TensorOrList, dst: Optional[TensorOrList] = None, *,
                         chunk_bytes: int = 0, scale: Optional[float] = None, mode: str = "auto",
@@ -257,26 +237,18 @@ class Comm:
     def reduce_scatter(self, send: TensorOrList, recv: Optional[TensorOrList] = None, *, ctas: int = 0,
                        slot_bytes: int = 0):
         """Rank q receives elements [q*S, (q+1)*S) of the sum, S = shard_elems(count) (tail padded, not written)."""
-        s = self._as_list(send, "send")
-        n = self.shard_elems(s[0].numel()) if self.world > 1 else s[0].numel()
-        r = [torch.empty(n, dtype=x.dtype, device=x.device) for x in s] if recv is None else self._as_list(recv, "recv")
         try:
-            self._impl.reduce_scatter(s, r, ctas, slot_bytes)
+            return self._impl.call_half(send, 0, recv, ctas, slot_bytes, True)
         except RuntimeError as e:
             raise _translate(e) from None
-        return self._like_input(send, r)
 
     def all_gather(self, send: TensorOrList, count: int, recv: Optional[TensorOrList] = None, *, ctas: int = 0,
                    slot_bytes: int = 0):
         """Inverse of reduce_scatter: every rank contributes its shard, all receive `count` elements."""
-        s = self._as_list(send, "send")
-        r = [torch.empty(count, dtype=x.dtype, device=x.device) for x in s] if recv is None \
-            else self._as_list(recv, "recv")
         try:
-            self._impl.all_gather(s, r, ctas, slot_bytes)
+            return self._impl.call_half(send, count, recv, ctas, slot_bytes, False)
         except RuntimeError as e:
             raise _translate(e) from None
-        return self._like_input(send, r)
 
     # ---- symmetric memory -----------------------------------------------------------------
     def symm_empty(self, shape, dtype: torch.dtype = torch.float32):
