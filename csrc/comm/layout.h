@@ -28,6 +28,7 @@ constexpr uint32_t kCallFlashEpoch = 0;   // one-shot calls so far
 constexpr uint32_t kCallStreamSeq = 1;    // ring sequence numbers consumed so far
 constexpr uint32_t kCallBarEpoch = 2;     // per-CTA barrier epochs consumed so far
 constexpr uint32_t kCallGemmEpoch = 3;    // fused GEMM calls so far
+constexpr uint32_t kCallLocalGemm = 4;     // fused linear calls of ranks that share one GPU (rank 0's word)
 constexpr uint32_t kCallFlashEpochHi = 5;  // upper half of the one-shot call number (flag-in-data protocol)
 constexpr uint32_t kCallGemmLLEpoch = 6;   // calls of the fused GEMM's few-token form so far (lower half)
 constexpr uint32_t kCallGemmLLEpochHi = 7;  // upper half of that call number
@@ -56,7 +57,11 @@ constexpr uint32_t kCeDoneOff = kCePulledOff + kMaxRanks;    // [kMaxRanks] call
 // columns x K split) have landed here.
 constexpr uint32_t kGemmTileFlags = 4096;
 constexpr uint32_t kGemmTileFlagOff = kCeDoneOff + kMaxRanks;  // [kGemmTileFlags][kMaxRanks]
-constexpr uint32_t kFlagWords = kGemmTileFlagOff + kGemmTileFlags * kMaxRanks;
+// Fused linear of ranks that share one GPU (kernels/gemm_local.cu): the call number, written when a unit of the sum (a
+// token tile x 128 columns x K split) is in memory.
+constexpr uint32_t kLocalGemmFlags = 16384;
+constexpr uint32_t kLocalGemmFlagOff = kGemmTileFlagOff + kGemmTileFlags * kMaxRanks;  // [kLocalGemmFlags]
+constexpr uint32_t kFlagWords = kLocalGemmFlagOff + kLocalGemmFlags;
 constexpr uint64_t kFlagRegionBytes = 1ull << 20;
 static_assert(kFlagWords * 4ull <= kFlagRegionBytes, "flag region too small");
 static_assert(kTraceOff % 2 == 0, "the timeline entries are 64-bit words");

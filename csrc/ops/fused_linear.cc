@@ -5,6 +5,7 @@
 
 #include <algorithm>
 #include <cstring>
+#include <map>
 #include <mutex>
 #include <set>
 
@@ -267,6 +268,157 @@ int FusedLinearAutoMulticastMode(int world, uint32_t /*T*/) {
     return world < 8 ? 0 : 2;
 }
 
+// The cost of a candidate, in cycles of an SM: rounds of items times (their k-blocks + about 2500 for the first
+// operands, the read-out of the accumulator and the flag), plus the sums' way through L2 (write and read, at
+// about 30 bytes per SM and cycle).  A k-block takes the longest of: 350 cycles of issue (2 CTAs, four MMAs); 2 per
+// token on the tensor cores; its share of reading W once from HBM (3.6 bytes per ns and cycle of 1.8 GHz) by the pairs
+// that run together and do not share a slice.  Measured on B200.
+LocalGemmShape LocalGemmShapeFor(uint32_t T, uint32_t N, uint32_t kb_total, uint64_t room, uint32_t pairs) {
+    const uint32_t ncol = (N + kLocalGemmPairCols - 1) / kLocalGemmPairCols, units = N / kLocalGemmUnitCols;
+    const uint32_t fewest = (T + kLocalGemmMaxTokens - 1) / kLocalGemmMaxTokens;
+    LocalGemmShape best{};
+    uint64_t best_cost = ~0ull;
+    for (uint32_t split = 1; split <= std::min(kLocalGemmMaxSplit, kb_total); ++split) {
+        const uint64_t sums = static_cast<uint64_t>(T) * N * 2 * split;
+        if (split > 1 && sums > room) break;
+        for (uint32_t n = fewest; n < fewest + 4; ++n) {
+            LocalGemmShape s;
+            s.tokens = ((T + n - 1) / n + 31) / 32 * 32;
+            s.tiles = (T + s.tokens - 1) / s.tokens;
+            s.kper = (kb_total + split - 1) / split;
+            s.nsplit = (kb_total + s.kper - 1) / s.kper;
+            if (static_cast<uint64_t>(s.tiles) * units * s.nsplit > kLocalGemmFlags) continue;
+            const uint64_t items = static_cast<uint64_t>(s.tiles) * ncol * s.nsplit;
+            const uint64_t together = std::min<uint64_t>(items, pairs);
+            const uint64_t slices = std::max<uint64_t>(1, together / std::min<uint64_t>(s.tiles, std::max<uint64_t>(1, together / (ncol * s.nsplit))));
+            const uint64_t block = std::max<uint64_t>({350, 2ull * s.tokens + 8, slices * 32768 * 10 / 36000});
+            const uint64_t cost = (items + pairs - 1) / pairs * (s.kper * block + 2500) + 2 * sums / (30 * 148);
+            if (cost < best_cost) {
+                best_cost = cost;
+                best = s;
+            }
+        }
+    }
+    return best;
+}
+
+namespace {
+
+// Ranks that share this GPU: a GEMM over all ranks' K extents and a row kernel that starts under it (gemm_local.cu).
+// The second kernel runs while the first still reads x and W, so no output may lie on an input, except that a
+// rank's residual may be updated in place.
+bool CanRunLocal(Communicator& comm, const FusedLinearDesc* descs, uint32_t T, uint32_t N, uint32_t K,
+                 const FusedLinearOptions& opt) {
+    static const bool measuring = env::GetInt("YALI_GEMM_DECODE", -1) >= 0 || env::GetInt("YALI_GEMM_KSPLIT", 0) > 0 ||
+                                  env::GetInt("YALI_GEMM_DECODE_KSPLIT", 0) > 0 || env::GetInt("YALI_GEMM_DECODE_TILE", 0) > 0;
+    if (!comm.emulated() || comm.world() < 2 || opt.force_oneshot >= 0 || opt.decode >= 0 || opt.nvls > 0 || opt.ctas > 0 ||
+        opt.trace || measuring)
+        return false;
+    const uint64_t rows = static_cast<uint64_t>(T) * N * 2, xb = static_cast<uint64_t>(T) * K * 2, wb = static_cast<uint64_t>(N) * K * 2;
+    // What the multi-GPU forms take (one landing zone per source): no more, so that the two agree on what is too large.
+    const uint64_t share = static_cast<uint64_t>((T + comm.world() - 1) / comm.world()) * N * 2;
+    if (share > comm.layout().gemm_cap || rows > 2ull * comm.world() * comm.layout().gemm_cap) return false;
+    auto overlap = [](const void* a, uint64_t an, const void* b, uint64_t bn) {
+        const char *p = static_cast<const char*>(a), *q = static_cast<const char*>(b);
+        return p && q && p < q + bn && q < p + an;
+    };
+    for (int j = 0; j < comm.nlocal(); ++j) {
+        const void* const outs[2] = {descs[j].out, descs[j].residual_out};
+        for (int i = 0; i < comm.nlocal(); ++i) {
+            for (const void* o : outs)
+                if (overlap(o, rows, descs[i].x, xb) || overlap(o, rows, descs[i].w, wb) ||
+                    overlap(o, rows, descs[i].norm_weight, static_cast<uint64_t>(N) * 2) ||
+                    (overlap(o, rows, descs[i].residual, rows) && !(i == j && o == descs[i].residual)))
+                    return false;
+            // Two outputs on one another: which of them is left depends on the order of the writes.
+            if (overlap(descs[j].out, rows, descs[i].residual_out, rows) ||
+                (i != j && (overlap(descs[j].out, rows, descs[i].out, rows) || overlap(descs[j].residual_out, rows, descs[i].residual_out, rows))))
+                return false;
+        }
+    }
+    return true;
+}
+
+Result LaunchLocal(Communicator& comm, const DriverApi* drv, const FusedLinearDesc* descs, uint32_t T, uint32_t N,
+                   uint32_t K, const FusedLinearOptions& opt, const cudaStream_t* streams) {
+    auto fail = [&](Result r, const std::string& what) {
+        comm.set_error(what);
+        return r;
+    };
+    const int W = comm.world();
+    const void* fn = LocalGemmKernel();
+    const uint32_t smem = LocalGemmSmemBytes();
+    static std::mutex mu;
+    static std::map<int, uint32_t> pairs_of;  // resident pairs of CTAs per device; the shared-memory limit is raised with it
+    uint32_t pairs = 0;
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        uint32_t& p = pairs_of[comm.device_of(0)];
+        if (p == 0) {
+            cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+            cudaLaunchConfig_t cfg;
+            std::memset(&cfg, 0, sizeof(cfg));
+            cfg.gridDim = dim3(2);
+            cfg.blockDim = dim3(kLocalGemmThreads);
+            cfg.dynamicSmemBytes = smem;
+            int n = 0;
+            if (e == cudaSuccess) e = cudaOccupancyMaxActiveClusters(&n, fn, &cfg);
+            if (e != cudaSuccess || n < 1) return fail(Result::CudaError, std::string("fused linear: ") + cudaGetErrorString(e));
+            p = static_cast<uint32_t>(n);
+        }
+        pairs = p;
+    }
+    const HeapLayout& lay = comm.layout();
+    LocalGemmArgs g;
+    std::memset(&g, 0, sizeof(g));
+    g.cv = comm.View(0);
+    g.sums = g.cv.heap[0] + lay.gemm_off;
+    g.T = T;
+    g.N = N;
+    g.kb_rank = K / 64;
+    g.kb_total = g.kb_rank * W;
+    g.s = LocalGemmShapeFor(T, N, g.kb_total, 2ull * W * lay.gemm_cap, pairs);
+    LocalLinearNormArgs n;
+    std::memset(&n, 0, sizeof(n));
+    n.cv = g.cv;
+    n.sums = g.sums;
+    n.T = T;
+    n.N = N;
+    n.world = static_cast<uint32_t>(W);
+    n.s = g.s;
+    n.eps = opt.eps;
+    std::string derr;
+    for (int i = 0; i < W; ++i) {
+        const int r = comm.rank_of(i);
+        const FusedLinearDesc& d = descs[i];
+        if (!EncodeTileMap(drv, &g.tmap_x[r], d.x, T, K, g.s.tokens / 2, &derr) ||
+            !EncodeTileMap(drv, &g.tmap_w[r], d.w, N, K, kLocalGemmUnitCols, &derr))
+            return fail(Result::CudaError, derr);
+        n.residual[r] = d.residual;
+        n.residual_out[r] = d.residual_out;
+        n.weight[r] = d.norm_weight;
+        n.out[r] = d.out;
+    }
+    const uint32_t items = g.s.tiles * ((N + kLocalGemmPairCols - 1) / kLocalGemmPairCols) * g.s.nsplit;
+    // With few rows the ranks of a row are spread over CTAs (each adds the splits again, from L2); from two CTAs per SM on
+    // a CTA serves as many ranks as its registers hold.
+    const int group = static_cast<uint64_t>(T) * W <= 296 ? 1 : W >= 4 ? 4 : 2;
+    const cudaStream_t s = streams && streams[0] ? streams[0] : comm.default_stream(0);
+    void* gp[] = {&g};
+    void* np[] = {&n};
+    cudaError_t e = LaunchInStream(fn, dim3(2 * std::min(items, pairs)), dim3(kLocalGemmThreads), gp, smem, s);
+    if (e == cudaSuccess)
+        e = LaunchInStream(LocalLinearNormKernel(N, group), dim3(T * ((W + group - 1) / group)), dim3(kLocalLinearNormThreads), np, 0, s);
+    if (e != cudaSuccess) {
+        (void)cudaGetLastError();
+        return fail(Result::CudaError, std::string("kernel launch failed: ") + cudaGetErrorString(e));
+    }
+    comm.CountLaunch(2);
+    return Result::Success;
+}
+
+}  // namespace
+
 Result FusedLinearAllReduceRmsNorm(Communicator& comm, const FusedLinearDesc* descs, uint32_t T, uint32_t N,
                                    uint32_t K, const FusedLinearOptions& opt, const cudaStream_t* streams) {
     YALI_NVTX_RANGE("yali::FusedLinear");
@@ -290,6 +442,8 @@ Result FusedLinearAllReduceRmsNorm(Communicator& comm, const FusedLinearDesc* de
     std::string derr;
     const DriverApi* drv = DriverApi::Get(&derr);
     if (!drv) return fail(Result::CudaError, derr);
+
+    if (CanRunLocal(comm, descs, T, N, K, opt)) return LaunchLocal(comm, drv, descs, T, N, K, opt, streams);
 
     const HeapLayout& lay = comm.layout();
     const uint64_t row_bytes = static_cast<uint64_t>(N) * 2;

@@ -143,3 +143,45 @@ def test_tile_form_at_the_edges_of_its_tiles(world, T, K, N):
                 assert torch.equal(p.double(), want)
             for o in outs[0] + outs[2]:
                 torch.testing.assert_close(o.double(), y, rtol=2.0 ** -8, atol=1e-6)
+
+
+@pytest.mark.parametrize("world", [2, 3, 8])
+@pytest.mark.parametrize("T", [1, 31, 32, 33, 65, 255, 257, 513])
+@pytest.mark.parametrize("K,N", [(64, 128), (64, 384), (192, 2176), (512, 4096)])
+def test_ranks_on_one_gpu_add_in_the_gemm(world, T, K, N):
+    """Automatically chosen calls of emulated ranks: one GEMM over all ranks' K extents (two kernels, no exchange).  Token
+    tiles are multiples of 32 up to 256 rows, column tiles are 256 wide, K may be split; each rank has a residual and
+    norm weights of its own.  Whole-number inputs: all sums are exact in bf16 (below 256), so the residual is
+    compared bit by bit; the norm adds one rounding (2^-8)."""
+    g = torch.Generator(device="cuda").manual_seed(T * N + world)
+
+    def pick(*shape, p):
+        keep = torch.rand(shape, generator=g, device="cuda") < p
+        return (keep * torch.randint(-1, 2, shape, generator=g, device="cuda")).to(torch.bfloat16)
+
+    with yali.Comm.emulated(world, device=0) as c:
+        xs, ws = [pick(T, K, p=0.4) for _ in range(world)], [pick(N, K, p=0.4) for _ in range(world)]
+        nw = [torch.full((N,), 0.5 + r, dtype=torch.bfloat16, device="cuda") for r in range(world)]
+        res = [pick(T, N, p=0.9) for _ in range(world)]
+        total = sum(x.double() @ w.double().T for x, w in zip(xs, ws))
+        assert total.abs().max() < 255
+        for residuals in (res, None):
+            pre = [torch.empty_like(r) for r in res]
+            before = c.launches
+            results = [c.fused_linear_rmsnorm(xs, ws, nw, residuals, residual_out=pre) for _ in range(3)]
+            assert c.launches - before == 6
+            c.sync()
+            for r in range(world):
+                want = total + (res[r].double() if residuals else 0)
+                assert torch.equal(pre[r].double(), want)
+                y = want * torch.rsqrt(want.pow(2).mean(-1, keepdim=True) + 1e-5) * nw[r].double()
+                for outs in results:
+                    torch.testing.assert_close(outs[r].double(), y, rtol=2.0 ** -8, atol=1e-6)
+        # The residual stream updated in place; an output on another rank's residual takes the multi-GPU form.
+        keep = [r.clone() for r in res]
+        c.fused_linear_rmsnorm(xs, ws, nw, keep, residual_out=keep)
+        assert all(torch.equal(k.double(), total + r.double()) for k, r in zip(keep, res))
+        before = c.launches
+        c.fused_linear_rmsnorm(xs, ws, nw, res, out=res[1:] + res[:1])
+        c.sync()
+        assert c.launches - before == 1

@@ -54,6 +54,7 @@ LIB_SOURCES = [
     "kernels/util_kernels.cu",
     "kernels/gemm_ar_rmsnorm.cu",
     "kernels/gemm_ar_decode.cu",
+    "kernels/gemm_local.cu",
     "kernels/no_alloc_entry.cu",
 ]
 
