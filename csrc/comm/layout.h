@@ -36,6 +36,7 @@ constexpr uint32_t kCallGemmDone = 8;     // [kMaxRanks] rows each owner has bee
 constexpr uint32_t kCallDoneCtas = 16;    // [4] CTAs of the running launch that have finished, per kernel kind
 constexpr uint32_t kCallTraceIdx = 20;    // traced calls so far (index into the kTraceOff ring)
 constexpr uint32_t kCallPlanWord = 21;    // what this rank's running (or last) collective is: PlanWord() of its plan
+constexpr uint32_t kCallLocalRows = 23;   // units the row kernel of gemm_local.cu has handed out in the running call
 constexpr uint32_t kCallCeCalls = 22;     // copy-engine all-reduce calls so far
 constexpr uint32_t kFlashFlagOff = 32;                                       // [kMaxFlashCtas][kMaxRanks]
 constexpr uint32_t kRsSeqOff = kFlashFlagOff + kMaxFlashCtas * kMaxRanks;    // [kMaxLanes][kMaxRanks]

@@ -271,12 +271,6 @@ __device__ __forceinline__ char* ll_stage(const CommView& cv, int on_rank, int s
     return cv.heap[on_rank] + cv.lay.ll_off +
            (static_cast<uint64_t>(parity) * (cv.world - 1) + SrcSlot(src, on_rank)) * (2 * cv.lay.ll_cap);
 }
-__device__ __forceinline__ uint4 ld_volatile_v4(const void* p) {
-    uint4 v;
-    asm volatile("ld.volatile.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p)
-                 : "memory");
-    return v;
-}
 
 template <typename T, int WORLD>
 __device__ __forceinline__ void flash_ll_body(const CollArgs& a, uint32_t cta) {
@@ -355,8 +349,8 @@ __device__ __forceinline__ void flash_ll_body(const CollArgs& a, uint32_t cta) {
             uint4 l0, l1;
             uint32_t polls = 0;
             for (;;) {
-                l0 = ld_volatile_v4(in[q] + v * 32);
-                l1 = ld_volatile_v4(in[q] + v * 32 + 16);
+                l0 = ptx::ld_volatile_v4(in[q] + v * 32);
+                l1 = ptx::ld_volatile_v4(in[q] + v * 32 + 16);
                 if (l0.y == lo && l0.w == hi && l1.y == lo && l1.w == hi) break;
                 if ((++polls & 63u) == 0u && ptx::globaltimer() > deadline) {
                     report_timeout(cv, kSiteFlashArrive, q, cta, lo, l0.y);

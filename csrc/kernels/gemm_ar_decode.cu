@@ -70,13 +70,6 @@ __device__ __forceinline__ uint64_t desc_sw128(uint32_t smem_addr) {
     return d;
 }
 
-__device__ __forceinline__ uint4 ld_volatile16(const void* p) {
-    uint4 v;
-    asm volatile("ld.volatile.global.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p)
-                 : "memory");
-    return v;
-}
-
 // Flag-in-data landing zone of source (rank `src`, K split `ks`) on every rank: at offset gemm_ll_off +
 // (parity * world + src) * gemm_ll_cap + ks * (gemm_ll_cap / ksplit) of the heap, cut into 32-column tiles:
 // line ((tile * T + row) * 8 + j) (16 bytes) holds columns 32 * tile + 4j .. 4j+3 of row `row`.
@@ -339,8 +332,8 @@ __device__ __forceinline__ void decode_body(const GemmDecodeArgs& a, const CUten
                     for (int q = 0; q < 8; ++q) {
                         if (static_cast<uint32_t>(q) < n && (pending >> q & 1u)) {
                             const char* p = landing0 + static_cast<uint64_t>(s0 + q) * split_bytes + off;
-                            l0[q] = ld_volatile16(p);
-                            l1[q] = ld_volatile16(p + 16);
+                            l0[q] = ptx::ld_volatile_v4(p);
+                            l1[q] = ptx::ld_volatile_v4(p + 16);
                         }
                     }
 #pragma unroll

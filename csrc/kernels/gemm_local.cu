@@ -39,12 +39,12 @@ constexpr int kMaxStages = 12;
 constexpr uint32_t kSmemBytes = kRingBytes + 1024;  // + slack to align the base
 constexpr uint32_t kTmemCols = 2 * kLocalGemmMaxTokens;  // two accumulators: all of TMEM
 constexpr uint32_t kEpiChunk = 32;                              // tokens an epilogue group moves at a time
-constexpr uint32_t kEpiRowBytes = kLocalGemmUnitCols * 2;       // 256 bytes per token
-constexpr uint32_t kEpiBufBytes = kEpiChunk * kEpiRowBytes;     // 8 KiB per group of four warps
+constexpr uint32_t kEpiBufBytes = kEpiChunk * 64;  // 2 KiB per warp: 32 columns of a chunk
 constexpr int kEpiGroups = 2, kEpilogueWarps = 4 * kEpiGroups;
-constexpr int kTmaWarp = 8, kMmaWarp = 9, kAnnounceWarp = 10;
-static_assert(kTmemCols == 512 && kLocalGemmThreads >= 32 * (kAnnounceWarp + 1), "one CTA per SM");
-static_assert(kSmemBytes + kEpiGroups * kEpiBufBytes + 1024 <= 216 * 1024, "leaves room for CTAs of the second kernel");
+constexpr int kTmaWarp = 8, kMmaWarp = 9, kAnnounceWarp = 10, kPrefetchWarp = 11;
+constexpr uint32_t kPrefetchBlocks = 8;  // how far the prefetch warp runs ahead of the loads, in k-blocks
+static_assert(kTmemCols == 512 && kLocalGemmThreads == 32 * (kPrefetchWarp + 1), "one CTA per SM");
+static_assert(kSmemBytes + kEpilogueWarps * kEpiBufBytes + 1024 <= 216 * 1024, "leaves room for CTAs of the second kernel");
 
 // tcgen05 instruction descriptor: D = fp32, A = B = bf16, both K-major, N at bit 17 (>>3), M at bit 24 (>>4).
 __device__ __forceinline__ uint32_t pair_idesc(uint32_t n) {
@@ -64,29 +64,52 @@ __device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t smem_addr) {
 }
 
 struct Item {
-    uint32_t tile, t0, nt;       // token tile, its rows [t0, t0 + nt)
+    uint32_t tile;  // token tile
     uint32_t col_tile, split;
     uint32_t kb_begin, kb_end;
 };
-// Token tile by token tile, so that rows complete early; the items in flight together read the same stretch of K.
-__device__ __forceinline__ Item item_at(const LocalGemmArgs& a, uint32_t i, uint32_t ncol) {
-    Item it;
+// The k-th item of a pair; false: no more.  Whole items first, pair by pair, then split ones: a pair without a whole item in
+// the last round starts on them at once.  Token tile by token tile, so that rows complete early.
+__device__ __forceinline__ bool item_at(const LocalGemmArgs& a, uint32_t k, uint32_t pair, uint32_t npairs, uint32_t ncol, Item* it) {
+    const uint32_t nwhole = a.s.whole * ncol, left = nwhole % npairs;
+    const uint32_t mine = nwhole / npairs + (pair < left ? 1u : 0u);
+    if (k < mine) {
+        const uint32_t i = pair + k * npairs;
+        it->tile = i / ncol;
+        it->col_tile = i % ncol;
+        it->split = 0;
+        it->kb_begin = 0;
+        it->kb_end = a.kb_total;
+        return true;
+    }
+    k -= mine;
+    uint32_t j, early = 0;
+    if (left) {
+        early = a.s.extra * (npairs - left);
+        if (pair >= left && k < a.s.extra) {
+            j = pair - left + k * (npairs - left);
+            early = ~0u;
+        } else if (pair >= left) {
+            k -= a.s.extra;
+        }
+    }
+    if (early != ~0u) j = early + pair + k * npairs;
     const uint32_t per_tile = ncol * a.s.nsplit;
-    it.tile = i / per_tile;
-    const uint32_t in_tile = i - it.tile * per_tile;
-    it.split = in_tile / ncol;
-    it.col_tile = in_tile - it.split * ncol;
-    it.t0 = it.tile * a.s.tokens;
-    it.nt = min(a.T - it.t0, a.s.tokens);
-    it.kb_begin = it.split * a.s.kper;
-    it.kb_end = min(a.kb_total, it.kb_begin + a.s.kper);
-    return it;
+    if (j >= (a.s.tiles - a.s.whole) * per_tile) return false;
+    const uint32_t t = j / per_tile, in_tile = j - t * per_tile;
+    it->tile = a.s.whole + t;
+    it->split = in_tile / ncol;
+    it->col_tile = in_tile - it->split * ncol;
+    it->kb_begin = it->split * a.s.kper;
+    it->kb_end = min(a.kb_total, it->kb_begin + a.s.kper);
+    return true;
 }
 
 struct Shared {
     __align__(8) uint64_t full_bar[kMaxStages], empty_bar[kMaxStages], tmem_full_bar[2], tmem_empty_bar[2];
     __align__(8) uint64_t stored_bar[2], announced_bar[2];  // epilogue warps -> announcer warp and back
     uint32_t tmem;
+    volatile uint32_t loaded;  // k-blocks whose loads have been issued
     volatile int abort;
 };
 
@@ -105,7 +128,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kLocalGemmThreads, 1
     local_gemm_kernel(const __grid_constant__ LocalGemmArgs a) {
     extern __shared__ uint8_t smem_raw[];
     __shared__ Shared s;
-    __shared__ __align__(16) uint8_t s_epi[kEpiGroups][kEpiBufBytes];
+    __shared__ __align__(128) uint8_t s_epi[kEpilogueWarps][kEpiBufBytes];
 
     const CommView& cv = a.cv;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -114,6 +137,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kLocalGemmThreads, 1
     // Nothing up to the wait depends on earlier kernels: it runs under the end of the one in front.
     if (tid == 64) {
         s.abort = 0;
+        s.loaded = 0;
         for (int i = 0; i < kMaxStages; ++i) {
             ptx::mbar_init(&s.full_bar[i], 1);
             ptx::mbar_init(&s.empty_bar[i], 1);
@@ -142,8 +166,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kLocalGemmThreads, 1
     ptx::grid_launch_dependents();
     const uint64_t deadline = ptx::globaltimer() + cv.timeout_ns;
 
+    // This call's number; the second kernel advances it when all of its CTAs have read it.
+    const uint32_t epoch = *reinterpret_cast<volatile uint32_t*>(flag_word(cv, 0, kCallLocalGemm)) + 1u;
     const uint32_t ncol = (a.N + kLocalGemmPairCols - 1) / kLocalGemmPairCols;
-    const uint32_t nitems = a.s.tiles * ncol * a.s.nsplit;
     const uint32_t pair = cta >> 1, npairs = gridDim.x >> 1;
     const uint32_t xbytes = a.s.tokens / 2 * (BK * 2);  // one CTA's half of the token operand of a stage: whole KiB
     const uint32_t stage_bytes = kWBytes + xbytes;
@@ -151,11 +176,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kLocalGemmThreads, 1
 
     if (warp == kTmaWarp) {
         if (ptx::elect_one()) {
-            uint32_t st = 0, round = 0;
-            for (uint32_t i = pair; i < nitems && !s.abort; i += npairs) {
-                const Item it = item_at(a, i, ncol);
+            uint32_t st = 0, round = 0, loaded = 0;
+            Item it;
+            for (uint32_t i = 0; !s.abort && item_at(a, i, pair, npairs, ncol, &it); ++i) {
                 const int wrow = it.col_tile * kLocalGemmPairCols + half * kLocalGemmUnitCols;
-                const int xrow = it.t0 + half * (a.s.tokens / 2);
+                const int xrow = it.tile * a.s.tokens + half * (a.s.tokens / 2);
                 uint32_t rank = it.kb_begin / a.kb_rank, kb = it.kb_begin - rank * a.kb_rank;  // k-block of that rank
                 for (uint32_t g = it.kb_begin; g < it.kb_end; ++g) {
                     if (!wait_bar(&s.empty_bar[st], (round & 1u) ^ 1u, deadline, &s.abort)) {
@@ -169,10 +194,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kLocalGemmThreads, 1
                     uint8_t* stage = smem + st * stage_bytes;
                     ptx::tma_load_2d_pair(stage, &a.tmap_w[rank], kb * BK, wrow, bar);
                     ptx::tma_load_2d_pair(stage + kWBytes, &a.tmap_x[rank], kb * BK, xrow, bar);
+                    s.loaded = ++loaded;
                     if (++kb == a.kb_rank) kb = 0, ++rank;
                     if (++st == stages) st = 0, ++round;
                 }
             }
+            s.loaded = 0x7fffffffu;  // nothing left to run ahead of
             // The MMAs' releases of the last stages arrive here from the leader: none may be under way when this CTA
             // leaves.
             for (uint32_t k = 0; k < stages && !s.abort; ++k) {
@@ -184,8 +211,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kLocalGemmThreads, 1
         if (half == 0 && ptx::elect_one()) {
             const uint32_t idesc = pair_idesc(a.s.tokens);
             uint32_t st = 0, round = 0, n = 0;
-            for (uint32_t i = pair; i < nitems && !s.abort; i += npairs, ++n) {
-                const Item it = item_at(a, i, ncol);
+            Item it;
+            for (; !s.abort && item_at(a, n, pair, npairs, ncol, &it); ++n) {
                 const uint32_t b = n & 1u;
                 if (!wait_bar(&s.tmem_empty_bar[b], ((n >> 1) & 1u) ^ 1u, deadline, &s.abort)) {
                     if (!s.abort) report_timeout(cv, kSiteMbar, 0, cta, 4, n);
@@ -215,90 +242,116 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kLocalGemmThreads, 1
             }
         }
     } else if (warp == kAnnounceWarp) {
-        // When the eight epilogue warps have stored their part of a unit: publish the call number in its flag.  The release
-        // orders the stores (made visible to this warp by the mbarrier) before the flag; it waits for them to
-        // arrive, so it sits in a warp of its own.
-        const uint32_t epoch = *reinterpret_cast<volatile uint32_t*>(flag_word(cv, 0, kCallLocalGemm)) + 1u;
-        const uint32_t units = a.N / kLocalGemmUnitCols;
-        uint32_t n = 0;
-        for (uint32_t i = pair; i < nitems; i += npairs, ++n) {
-            const Item it = item_at(a, i, ncol);
-            const uint32_t b = n & 1u, unit = it.col_tile * 2 + half;
-            if (!wait_bar(&s.stored_bar[b], (n >> 1) & 1u, deadline, &s.abort)) {
-                if (lane == 0 && !s.abort) report_timeout(cv, kSiteMbar, 0, cta, 5, n);
-                s.abort = 1;
-                break;
-            }
-            if (lane == 0) {
-                if (unit < units)
+        // When the epilogue warps have stored their part of a unit: publish the call number in its flag.  The release orders
+        // the stores (made visible to this warp by the mbarrier) before the flag; it waits for them to arrive, so it
+        // sits in a warp of its own.
+        if (lane == 0) {
+            const uint32_t units = a.N / kLocalGemmUnitCols;
+            Item it;
+            for (uint32_t n = 0; item_at(a, n, pair, npairs, ncol, &it); ++n) {
+                const uint32_t b = n & 1u, unit = it.col_tile * 2 + half;
+                if (!wait_bar(&s.stored_bar[b], (n >> 1) & 1u, deadline, &s.abort)) {
+                    if (!s.abort) report_timeout(cv, kSiteMbar, 0, cta, 5, n);
+                    s.abort = 1;
+                    break;
+                }
+                if (unit < units && !a.lines)
                     ptx::st_release_gpu(flag_word(cv, 0, kLocalGemmFlagOff + (it.tile * a.s.nsplit + it.split) * units + unit), epoch);
                 ptx::mbar_arrive(&s.announced_bar[b]);
             }
-            __syncwarp();
+        }
+    } else if (warp == kPrefetchWarp) {
+        // Brings the operands into L2 ahead of the loads: what a CTA has in flight in its stages does not cover the latency of
+        // HBM.  One item of those that use a slice fetches it: of W those of the first token tile, of x those of
+        // the first columns.
+        if (ptx::elect_one()) {
+            uint32_t ahead = 0;
+            Item it;
+            for (uint32_t i = 0; item_at(a, i, pair, npairs, ncol, &it); ++i) {
+                const bool w_here = it.tile == 0, x_here = it.col_tile == 0;
+                const int wrow = it.col_tile * kLocalGemmPairCols + half * kLocalGemmUnitCols;
+                const int xrow = it.tile * a.s.tokens + half * (a.s.tokens / 2);
+                uint32_t rank = it.kb_begin / a.kb_rank, kb = it.kb_begin - rank * a.kb_rank;
+                for (uint32_t g = it.kb_begin; g < it.kb_end; ++g, ++ahead) {
+                    while (static_cast<int32_t>(ahead - s.loaded) > static_cast<int32_t>(stages + kPrefetchBlocks)) ptx::nanosleep(40);
+                    if (w_here) ptx::tma_prefetch_2d(&a.tmap_w[rank], kb * BK, wrow);
+                    if (x_here) ptx::tma_prefetch_2d(&a.tmap_x[rank], kb * BK, xrow);
+                    if (++kb == a.kb_rank) kb = 0, ++rank;
+                }
+            }
         }
     } else if (warp < kEpilogueWarps) {
         const int q = warp & 3;   // TMEM lane quarter this warp may read: columns 32q .. 32q+31 of the CTA's 128
-        const int g = warp >> 2;  // its group takes every second chunk of 32 tokens
-        const int gt = tid & 127;
-        const uint32_t c16 = gt & 15, rsub = gt >> 4;  // stores: 16-byte piece of a token's 256 bytes, token % 8
+        const int g = warp >> 2;  // takes every second chunk of 32 tokens
+        // A chunk is transposed through 2 KiB of this warp's own, [32 tokens][64 bytes] with the 16-byte pieces swizzled: no
+        // barrier with other warps.  stmatrix: this thread's row of the transposed matrices is token lane % 8 of an
+        // 8-token group; matrix lane / 8 holds 8 of the warp's 32 columns.
+        uint8_t* const stage = s_epi[warp];
+        uint8_t* const st_row = stage + (lane & 7) * 64 + (((lane >> 3) ^ ((lane >> 1) & 3)) << 4);
+        const uint32_t token = lane >> 2;  // stores: token of a group of 8, 16-byte piece lane % 4
+        const uint8_t* const ld_row = stage + token * 64 + (((lane & 3) ^ ((token >> 1) & 3)) << 4);
         const uint64_t rowbytes = static_cast<uint64_t>(a.N) * 2;
-        uint8_t* const stage = s_epi[g];
-        uint32_t n = 0;
-        for (uint32_t i = pair; i < nitems; i += npairs, ++n) {
-            const Item it = item_at(a, i, ncol);
-            const uint32_t b = n & 1u;
+        Item it;
+        for (uint32_t n = 0; item_at(a, n, pair, npairs, ncol, &it); ++n) {
+            const uint32_t b = n & 1u, t0 = it.tile * a.s.tokens, nt = min(a.T - t0, a.s.tokens);
             const uint32_t col = it.col_tile * kLocalGemmPairCols + half * kLocalGemmUnitCols;
             // The second half of the last column tile may lie beyond N.
-            const uint32_t chunks = col < a.N ? (it.nt + kEpiChunk - 1) / kEpiChunk : 0u;
-            char* const dst0 = a.sums + (static_cast<uint64_t>(it.split) * a.T + it.t0) * rowbytes +
-                               static_cast<uint64_t>(col) * 2 + c16 * 16;
-            // Every warp of a group has to take the same way through the chunks (they share a barrier).
-            const bool up = wait_bar(&s.tmem_full_bar[b], (n >> 1) & 1u, deadline, &s.abort);
-            if (!up) {
+            const uint32_t chunks = col < a.N ? (nt + kEpiChunk - 1) / kEpiChunk : 0u;
+            const uint64_t first = (static_cast<uint64_t>(it.split) * a.T + t0) * rowbytes + (col + q * 32 + (lane & 3) * 8) * 2;
+            char* const dst0 = a.sums + (a.lines ? 2 * first : first);
+            if (!wait_bar(&s.tmem_full_bar[b], (n >> 1) & 1u, deadline, &s.abort)) {
                 if (lane == 0 && !s.abort) report_timeout(cv, kSiteMbar, 0, cta, 3, n);
                 s.abort = 1;
+                break;
             }
-            if (ptx::named_barrier_or(1 + g, 128, !up)) break;
+            __syncwarp();
             ptx::tc_fence_after_sync();
-            bool released = false;
             for (uint32_t ch = g; ch < chunks; ch += kEpiGroups) {
-                uint32_t v[32];
-                ptx::tmem_ld_32x32(tmem + b * kLocalGemmMaxTokens + (static_cast<uint32_t>(q * 32) << 16) + ch * kEpiChunk, v);
+                uint32_t v[2][16];  // lanes 0..15 and 16..31 of the quarter
+                const uint32_t src = tmem + b * kLocalGemmMaxTokens + (static_cast<uint32_t>(q * 32) << 16) + ch * kEpiChunk;
+                ptx::tmem_ld_16x256b_x4(src, v[0]);
+                ptx::tmem_ld_16x256b_x4(src + (16u << 16), v[1]);
                 ptx::tmem_ld_wait();
-                if (ch + kEpiGroups >= chunks) {  // this warp's last read of the accumulator: hand it back
-                    ptx::tc_fence_before_sync();
-                    __syncwarp();
-                    if (lane == 0) ptx::mbar_arrive_cluster(ptx::mapa_u32(&s.tmem_empty_bar[b], 0));
-                    released = true;
-                }
-                // Thread = column, register = token: token t's 128 columns become 256 contiguous bytes (32 lanes
-                // write 64 of them at once: no bank conflict).
-                if (ch != static_cast<uint32_t>(g)) ptx::named_barrier(1 + g, 128);  // the chunk before has been read
 #pragma unroll
-                for (int t = 0; t < 32; ++t)
-                    *reinterpret_cast<__nv_bfloat16*>(stage + t * kEpiRowBytes + q * 64 + lane * 2) =
-                        __float2bfloat16_rn(__uint_as_float(v[t]));
-                ptx::named_barrier(1 + g, 128);
-                const uint32_t tok0 = ch * kEpiChunk + rsub;  // 16 lanes cover a token's 256 bytes
+                for (int k = 0; k < 4; ++k) {  // 8 tokens each: four matrices of 8 columns x 8 tokens
+                    uint32_t m[4];
+#pragma unroll
+                    for (int h = 0; h < 4; ++h) {  // columns 8h .. 8h+7 of the warp's 32
+                        const __nv_bfloat162 p = __floats2bfloat162_rn(__uint_as_float(v[h >> 1][4 * k + 2 * (h & 1)]),
+                                                                       __uint_as_float(v[h >> 1][4 * k + 2 * (h & 1) + 1]));
+                        m[h] = *reinterpret_cast<const uint32_t*>(&p);
+                    }
+                    ptx::stmatrix_x4_trans(st_row + k * 8 * 64, m[0], m[1], m[2], m[3]);
+                }
+                __syncwarp();
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
-                    const uint4 x = *reinterpret_cast<const uint4*>(stage + (rsub + 8 * k) * kEpiRowBytes + c16 * 16);
-                    if (tok0 + 8 * k < it.nt) ptx::st_v4(dst0 + (tok0 + 8 * k) * rowbytes, x);
+                    const uint4 x = *reinterpret_cast<const uint4*>(ld_row + k * 8 * 64);
+                    const uint32_t tok = ch * kEpiChunk + k * 8 + token;
+                    if (tok >= nt) continue;
+                    if (a.lines) {  // {2 bf16, call, 2 bf16, ~call} per four columns: the flag is in the data
+                        ptx::st_v4(dst0 + tok * 2 * rowbytes, make_uint4(x.x, epoch, x.y, ~epoch));
+                        ptx::st_v4(dst0 + tok * 2 * rowbytes + 16, make_uint4(x.z, epoch, x.w, ~epoch));
+                    } else {
+                        ptx::st_v4(dst0 + tok * rowbytes, x);
+                    }
+                }
+                __syncwarp();
+            }
+            // Out of the accumulator: hand it back.
+            ptx::tc_fence_before_sync();
+            __syncwarp();
+            if (lane == 0) {
+                ptx::mbar_arrive_cluster(ptx::mapa_u32(&s.tmem_empty_bar[b], 0));
+                // Hand the unit to the announcer, which has to be done with the one before last.
+                if (n < 2 || wait_bar(&s.announced_bar[b], ((n >> 1) - 1u) & 1u, deadline, &s.abort)) {
+                    ptx::mbar_arrive(&s.stored_bar[b]);
+                } else {
+                    if (!s.abort) report_timeout(cv, kSiteMbar, 0, cta, 6, n);
+                    s.abort = 1;
                 }
             }
-            if (!released) {  // no chunk for this group
-                ptx::tc_fence_before_sync();
-                __syncwarp();
-                if (lane == 0) ptx::mbar_arrive_cluster(ptx::mapa_u32(&s.tmem_empty_bar[b], 0));
-            }
-            // Hand the unit to the announcer warp, which has to be done with the one before last.
-            const bool free = n < 2 || wait_bar(&s.announced_bar[b], ((n >> 1) - 1u) & 1u, deadline, &s.abort);
-            if (!free) {
-                if (lane == 0 && !s.abort) report_timeout(cv, kSiteMbar, 0, cta, 6, n);
-                s.abort = 1;
-            }
-            ptx::named_barrier(1 + g, 128);  // the staging buffer may be written again, and all four warps have stored
-            if (lane == 0 && free) ptx::mbar_arrive(&s.stored_bar[b]);
+            __syncwarp();
         }
     }
     __syncwarp();
@@ -312,120 +365,230 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kLocalGemmThreads, 1
 
 namespace {
 
-// NV 16-byte vectors of a row per thread, G ranks per CTA.  CTA b: row b / ngroups, ranks from (b % ngroups) * G.
-template <int NV, int G>
-__global__ void __launch_bounds__(kLocalLinearNormThreads) local_linear_norm_kernel(const __grid_constant__ LocalLinearNormArgs a) {
+// A unit of work is a row for G ranks (unit u: row u / ngroups, ranks from (u % ngroups) * G); a thread holds NV 16-byte
+// vectors of the row.  SPLIT: more than one K split; LINES: the sums come as flag-in-data lines.
+//
+// Bound by memory: what counts is how much is in flight on an SM, so a thread keeps no more than it must (the sum packed in
+// bf16 where there is one split) and registers are capped for three to five CTAs per SM.  A grid with fewer CTAs
+// than units takes them in row order from a counter, the residuals of the next unit on their way into L2: rows
+// as CTAs of their own came in waves, each a chain of launch, residual, sums and stores (8 ranks, 300 rows: 600 CTAs
+// on 444 places took two of them).
+template <int NV, int G, bool SPLIT, bool LINES>
+__global__ void __launch_bounds__(kLocalLinearNormThreads, LocalLinearNormPlaces(G, SPLIT))
+    local_linear_norm_kernel(const __grid_constant__ LocalLinearNormArgs a) {
     constexpr int VEC = 8, kThreads = kLocalLinearNormThreads, kWarps = kThreads / 32;
     __shared__ float s_red[G][kWarps];
+    __shared__ uint32_t s_next;
     const CommView& cv = a.cv;
-    const uint32_t ngroups = (a.world + G - 1) / G;
-    const uint32_t row = blockIdx.x / ngroups, q0 = (blockIdx.x % ngroups) * G;
+    const uint32_t ngroups = (a.world + G - 1) / G, units = a.T * ngroups, flags_per_split = a.N / kLocalGemmUnitCols;
     const uint32_t tid = threadIdx.x, nvec = a.N / VEC;
-    const uint64_t row_off = static_cast<uint64_t>(row) * a.N * 2;
+    const bool taking = gridDim.x < units;  // from the counter
+    uint32_t* const counter = flag_word(cv, 0, kCallLocalRows);
     const uint32_t epoch = *reinterpret_cast<volatile uint32_t*>(flag_word(cv, 0, kCallLocalGemm)) + 1u;
-
-    // Residuals are inputs of the call: complete since before the first kernel passed its own wait.
-    uint4 res[NV][G];
+    const uint64_t deadline = ptx::globaltimer() + cv.timeout_ns;
+    bool have[NV];
 #pragma unroll
-    for (int j = 0; j < NV; ++j) {
-        const uint32_t c = min(tid + j * kThreads, nvec - 1);
-#pragma unroll
-        for (int g = 0; g < G; ++g) {
-            const char* r = q0 + g < a.world ? static_cast<const char*>(a.residual[q0 + g]) : nullptr;
-            res[j][g] = r ? ptx::ld_cg_v4(r + row_off + c * 16ull) : make_uint4(0, 0, 0, 0);
-        }
+    for (int j = 0; j < NV; ++j) have[j] = tid + j * kThreads < nvec;
+    uint32_t unit = blockIdx.x, ready = ~0u;
+    if (taking) {
+        if (tid == 0) s_next = atomicAdd(counter, 1u);
+        __syncthreads();
+        unit = s_next;
+        __syncthreads();
     }
-    // The flags of this row's token tile, a few per thread.
-    const uint32_t tile = row / a.s.tokens, per_tile = a.s.nsplit * (a.N / kLocalGemmUnitCols);
+    auto check_in = [&] {
+        if (check_in_last(cv, 3, gridDim.x)) {
+            *reinterpret_cast<volatile uint32_t*>(counter) = 0u;
+            advance_call_word(cv, kCallLocalGemm, 1);
+        }
+    };
+    if (unit >= units && tid == 0) check_in();  // nothing was left for this CTA
+    const float inv_n = 1.f / static_cast<float>(a.N);
     bool late = false;
-    if (tid < per_tile) {
-        const uint64_t deadline = ptx::globaltimer() + cv.timeout_ns;
-        for (uint32_t e = tid; e < per_tile && !late; e += kThreads) {
-            const uint32_t* flag = flag_word(cv, 0, kLocalGemmFlagOff + tile * per_tile + e);
-            uint32_t polls = 0, seen;
-            while (!ptx::seq_reached(seen = ptx::ld_acquire_gpu(flag), epoch)) {
-                ptx::nanosleep(40);  // this CTA shares the SM with the GEMM
-                if ((++polls & 63u) == 0 && ptx::globaltimer() > deadline) {
-                    report_timeout(cv, kSiteGemmPartials, 0, blockIdx.x, epoch, seen);
-                    late = true;
-                    break;
+    while (unit < units) {
+        const uint32_t row = unit / ngroups, q0 = (unit - row * ngroups) * G;
+        const uint64_t off0 = static_cast<uint64_t>(row) * a.N * 2 + tid * 16;  // this thread's first vector; the others 4 KiB apart
+        if (taking && tid == 0) s_next = atomicAdd(counter, 1u);
+        // Residuals (and the weights of a CTA that serves one rank) are inputs of the call: complete since before the first
+        // kernel passed its own wait.
+        uint4 res[NV][G], w1[NV];
+#pragma unroll
+        for (int j = 0; j < NV; ++j) {
+#pragma unroll
+            for (int g = 0; g < G; ++g) {
+                const char* r = q0 + g < a.world ? static_cast<const char*>(a.residual[q0 + g]) : nullptr;
+                res[j][g] = r && have[j] ? ptx::ld_cg_v4(r + off0 + j * (kThreads * 16)) : make_uint4(0, 0, 0, 0);
+            }
+            if (G == 1 && have[j]) w1[j] = ptx::ld_cg_v4(static_cast<const char*>(a.weight[q0]) + (tid + j * kThreads) * 16);
+        }
+        const uint32_t tile = row / a.s.tokens, nsplit = tile < a.s.whole ? 1u : a.s.nsplit;
+        if (!LINES && tile != ready) {
+            // The flags of this row's token tile, a few per thread.
+            const uint32_t first = kLocalGemmFlagOff + tile * a.s.nsplit * flags_per_split;
+            for (uint32_t e = tid; e < nsplit * flags_per_split && !late; e += kThreads) {
+                uint32_t polls = 0, seen;
+                while (!ptx::seq_reached(seen = ptx::ld_acquire_gpu(flag_word(cv, 0, first + e)), epoch)) {
+                    if (++polls > 8) ptx::nanosleep(50);  // this CTA shares the SM with the GEMM
+                    if ((polls & 63u) == 0 && ptx::globaltimer() > deadline) {
+                        report_timeout(cv, kSiteGemmPartials, 0, blockIdx.x, epoch, seen);
+                        late = true;
+                        break;
+                    }
                 }
             }
+            ready = tile;
         }
-    }
-    if (__syncthreads_or(late)) return;
-    // Everybody has read the call number; the last CTA of the call advances it.
-    if (tid == kThreads - 1 && check_in_last(cv, 3, gridDim.x)) advance_call_word(cv, kCallLocalGemm, 1);
+        if (__syncthreads_or(late)) return;
+        if (taking) {
+            unit = s_next;
+            if (unit < units) {
+                const uint32_t nrow = unit / ngroups, nq = (unit - nrow * ngroups) * G;
+#pragma unroll
+                for (int g = 0; g < G; ++g) {
+                    const char* r = nq + g < a.world ? static_cast<const char*>(a.residual[nq + g]) : nullptr;
+                    // One 128-byte line per eight vectors.
+                    if (r && (tid & 7) == 0)
+#pragma unroll
+                        for (int j = 0; j < NV; ++j)
+                            if (have[j]) ptx::prefetch_l2(r + static_cast<uint64_t>(nrow) * a.N * 2 + (tid + j * kThreads) * 16);
+                }
+            }
+        } else {
+            unit = units;
+        }
+        // Once every CTA has read the call number and taken its last unit, both counters may move on: the next call reads
+        // them, nothing in this one does.  Done here, under the work of the last unit.
+        if (unit >= units && tid == kThreads - 1) check_in();
 
-    float f[NV][VEC];
+        uint4 one[SPLIT ? 1 : NV];
+        float sum[SPLIT ? NV : 1][VEC];
+        if constexpr (!SPLIT) {
 #pragma unroll
-    for (int j = 0; j < NV; ++j)
-#pragma unroll
-        for (int i = 0; i < VEC; ++i) f[j][i] = 0.f;
-    const uint64_t split_stride = static_cast<uint64_t>(a.T) * a.N * 2;
-    const char* const src = a.sums + row_off;
-    for (uint32_t k0 = 0; k0 < a.s.nsplit; k0 += 4) {  // four splits in flight, added in order
-        uint4 x[NV][4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k)
+            for (int j = 0; j < NV; ++j) one[j] = have[j] ? ptx::ld_cg_v4(a.sums + off0 + j * (kThreads * 16)) : make_uint4(0, 0, 0, 0);
+        } else {
+            const uint64_t split_stride = static_cast<uint64_t>(a.T) * a.N * (LINES ? 4 : 2);
+            const char* const src = a.sums + (LINES ? 2 * off0 : off0);
 #pragma unroll
             for (int j = 0; j < NV; ++j)
-                if (k0 + k < a.s.nsplit && tid + j * kThreads < nvec)
-                    x[j][k] = ptx::ld_cg_v4(src + (k0 + k) * split_stride + (tid + j * kThreads) * 16ull);
 #pragma unroll
-        for (int k = 0; k < 4; ++k)
+                for (int i = 0; i < VEC; ++i) sum[j][i] = 0.f;
+            // Splits in flight together, added in order: four where few rows leave the SM's registers to few CTAs.
+            constexpr int kFly = G == 1 ? 4 : 2;
+            for (uint32_t k0 = 0; k0 < nsplit && !late; k0 += kFly) {
+                uint4 x[NV][kFly];
+                if constexpr (LINES) {
+                    uint4 y[NV][kFly];
+                    uint32_t polls = 0;
+                    bool missing;
+                    do {
+                        missing = false;
 #pragma unroll
-            for (int j = 0; j < NV; ++j)
-                if (k0 + k < a.s.nsplit && tid + j * kThreads < nvec) accumulate<__nv_bfloat16>(f[j], x[j][k]);
-    }
-    float ss[G];
+                        for (int k = 0; k < kFly; ++k)
 #pragma unroll
-    for (int g = 0; g < G; ++g) {
-        ss[g] = 0.f;
-        char* const ro = q0 + g < a.world ? static_cast<char*>(a.residual_out[q0 + g]) : nullptr;
+                            for (int j = 0; j < NV; ++j)
+                                if (k0 + k < nsplit && have[j]) {
+                                    const char* p = src + (k0 + k) * split_stride + j * (kThreads * 32);
+                                    x[j][k] = ptx::ld_volatile_v4(p);
+                                    y[j][k] = ptx::ld_volatile_v4(p + 16);
+                                }
 #pragma unroll
-        for (int j = 0; j < NV; ++j) {
-            if (tid + j * kThreads >= nvec) continue;
-            float p[VEC];
+                        for (int k = 0; k < kFly; ++k)
 #pragma unroll
-            for (int i = 0; i < VEC; ++i) p[i] = f[j][i];
-            accumulate<__nv_bfloat16>(p, res[j][g]);
-            if (ro) ptx::st_v4(ro + row_off + (tid + j * kThreads) * 16ull, pack16<__nv_bfloat16>(p));
+                            for (int j = 0; j < NV; ++j)
+                                if (k0 + k < nsplit && have[j])
+                                    missing |= x[j][k].y != epoch || x[j][k].w != ~epoch || y[j][k].y != epoch || y[j][k].w != ~epoch;
+                        if (missing && (++polls & 63u) == 0 && ptx::globaltimer() > deadline) {
+                            report_timeout(cv, kSiteGemmPartials, 0, blockIdx.x, epoch, 0u);
+                            late = true;
+                        }
+                    } while (missing && !late);
 #pragma unroll
-            for (int i = 0; i < VEC; ++i) ss[g] += p[i] * p[i];
+                    for (int k = 0; k < kFly; ++k)
+#pragma unroll
+                        for (int j = 0; j < NV; ++j) x[j][k] = make_uint4(x[j][k].x, x[j][k].z, y[j][k].x, y[j][k].z);
+                } else {
+#pragma unroll
+                    for (int k = 0; k < kFly; ++k)
+#pragma unroll
+                        for (int j = 0; j < NV; ++j)
+                            if (k0 + k < nsplit && have[j]) x[j][k] = ptx::ld_cg_v4(src + (k0 + k) * split_stride + j * (kThreads * 16));
+                }
+#pragma unroll
+                for (int k = 0; k < kFly; ++k)
+#pragma unroll
+                    for (int j = 0; j < NV; ++j)
+                        if (k0 + k < nsplit && have[j]) accumulate<__nv_bfloat16>(sum[j], x[j][k]);
+            }
         }
+        // sum + residual of rank q0 + g, vector j.
+        auto row_of = [&](int j, int g, float (&p)[VEC]) {
+            if constexpr (SPLIT) {
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) ss[g] += __shfl_xor_sync(0xffffffffu, ss[g], o);
-        if ((tid & 31) == 0) s_red[g][tid >> 5] = ss[g];
-    }
-    __syncthreads();
-    const float inv_n = 1.f / static_cast<float>(a.N);
+                for (int i = 0; i < VEC; ++i) p[i] = sum[j][i];
+            } else {
 #pragma unroll
-    for (int g = 0; g < G; ++g) {
-        if (q0 + g >= a.world) break;
-        float t = 0.f;
-#pragma unroll
-        for (int w = 0; w < kWarps; ++w) t += s_red[g][w];
-        const float inv_rms = rsqrtf(t * inv_n + a.eps);
-#pragma unroll
-        for (int j = 0; j < NV; ++j) {
-            const uint32_t c = tid + j * kThreads;
-            if (c >= nvec) continue;
-            float p[VEC], w[VEC];
-#pragma unroll
-            for (int i = 0; i < VEC; ++i) {
-                p[i] = f[j][i];
-                w[i] = 0.f;
+                for (int i = 0; i < VEC; ++i) p[i] = 0.f;
+                accumulate<__nv_bfloat16>(p, one[j]);
             }
             accumulate<__nv_bfloat16>(p, res[j][g]);
-            accumulate<__nv_bfloat16>(w, ptx::ld_cg_v4(static_cast<const char*>(a.weight[q0 + g]) + c * 16ull));
+        };
 #pragma unroll
-            for (int i = 0; i < VEC; ++i) p[i] = p[i] * inv_rms * w[i];
-            ptx::st_v4(static_cast<char*>(a.out[q0 + g]) + row_off + c * 16ull, pack16<__nv_bfloat16>(p));
+        for (int g = 0; g < G; ++g) {
+            float ss = 0.f;
+            char* const ro = q0 + g < a.world ? static_cast<char*>(a.residual_out[q0 + g]) : nullptr;
+#pragma unroll
+            for (int j = 0; j < NV; ++j) {
+                float p[VEC];
+                row_of(j, g, p);
+                if (ro && have[j]) ptx::st_v4(ro + off0 + j * (kThreads * 16), pack16<__nv_bfloat16>(p));
+#pragma unroll
+                for (int i = 0; i < VEC; ++i) ss += p[i] * p[i];
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+            if ((tid & 31) == 0) s_red[g][tid >> 5] = ss;
+        }
+        if (LINES) {
+            if (__syncthreads_or(late)) return;
+        } else {
+            __syncthreads();
+        }
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+            if (q0 + g >= a.world) break;
+            float t = 0.f;
+#pragma unroll
+            for (int w = 0; w < kWarps; ++w) t += s_red[g][w];
+            const float inv_rms = rsqrtf(t * inv_n + a.eps);
+#pragma unroll
+            for (int j = 0; j < NV; ++j) {
+                if (!have[j]) continue;
+                float p[VEC], w[VEC];
+                row_of(j, g, p);
+#pragma unroll
+                for (int i = 0; i < VEC; ++i) w[i] = 0.f;
+                // (Plain loads: the rows of an SM share them in L1.)
+                accumulate<__nv_bfloat16>(w, G == 1 ? w1[j] : *reinterpret_cast<const uint4*>(static_cast<const char*>(a.weight[q0 + g]) + (tid + j * kThreads) * 16));
+#pragma unroll
+                for (int i = 0; i < VEC; ++i) p[i] = p[i] * inv_rms * w[i];
+                ptx::st_v4(static_cast<char*>(a.out[q0 + g]) + off0 + j * (kThreads * 16), pack16<__nv_bfloat16>(p));
+            }
         }
     }
-    // The call is over when both kernels are: the CTAs of the last token tile stay for the GEMM's end.
-    if (tile + 1 == a.s.tiles) ptx::grid_dependency_wait();
+    // The call is over when both kernels are.
+    ptx::grid_dependency_wait();
+}
+
+template <int NV, int G>
+const void* pick_linear_norm(bool split, bool lines) {
+    if constexpr (G == 1) {
+        if (lines) return (const void*)local_linear_norm_kernel<NV, 1, true, true>;
+    }
+    return split ? (const void*)local_linear_norm_kernel<NV, G, true, false> : (const void*)local_linear_norm_kernel<NV, G, false, false>;
+}
+template <int NV>
+const void* pick_linear_norm_g(int g, bool split, bool lines) {
+    return g == 1 ? pick_linear_norm<NV, 1>(split, lines) : g == 2 ? pick_linear_norm<NV, 2>(split, lines) : pick_linear_norm<NV, 4>(split, lines);
 }
 
 }  // namespace
@@ -433,13 +596,9 @@ __global__ void __launch_bounds__(kLocalLinearNormThreads) local_linear_norm_ker
 const void* LocalGemmKernel() { return reinterpret_cast<const void*>(local_gemm_kernel); }
 uint32_t LocalGemmSmemBytes() { return kSmemBytes; }
 
-const void* LocalLinearNormKernel(uint32_t N, int g) {
-    const bool one = N / 8 <= static_cast<uint32_t>(kLocalLinearNormThreads);
-    switch (g) {
-        case 1: return one ? (const void*)local_linear_norm_kernel<1, 1> : (const void*)local_linear_norm_kernel<2, 1>;
-        case 2: return one ? (const void*)local_linear_norm_kernel<1, 2> : (const void*)local_linear_norm_kernel<2, 2>;
-        default: return one ? (const void*)local_linear_norm_kernel<1, 4> : (const void*)local_linear_norm_kernel<2, 4>;
-    }
+const void* LocalLinearNormKernel(uint32_t N, int ranks_per_cta, bool split, bool lines) {
+    return N / 8 <= static_cast<uint32_t>(kLocalLinearNormThreads) ? pick_linear_norm_g<1>(ranks_per_cta, split, lines)
+                                                                   : pick_linear_norm_g<2>(ranks_per_cta, split, lines);
 }
 
 }  // namespace yali

@@ -13,20 +13,23 @@ constexpr uint32_t kLocalGemmPairCols = 256;   // columns of an item: rows of W 
 constexpr uint32_t kLocalGemmUnitCols = 128;   // columns of one CTA, announced together
 constexpr uint32_t kLocalGemmMaxTokens = 256;  // rows of x on the N side
 constexpr uint32_t kLocalGemmMaxSplit = 8;
-constexpr int kLocalGemmThreads = 384;         // eight epilogue warps, TMA, MMA, announcer, one idle
+constexpr int kLocalGemmThreads = 384;         // eight epilogue warps, TMA, MMA, announcer, prefetch
 constexpr int kLocalLinearNormThreads = 256;   // one row; up to two 16-byte vectors per thread: N <= 4096
 
-// T rows in `tiles` token tiles of `tokens` (a multiple of 32, at most 256), the k-blocks of all ranks (one after the
-// other) in `nsplit` runs of `kper`.
+// T rows in `tiles` token tiles of `tokens` (a multiple of 32, at most 256).  The first `whole` tiles' items (256 columns
+// each) run over all k-blocks of all ranks (one rank after the other); the items of the other tiles are cut into
+// `nsplit` runs of `kper` k-blocks.  Pairs that have nothing to do in the last round of whole items take `extra` split
+// items each meanwhile.
 struct LocalGemmShape {
-    uint32_t tiles, tokens, nsplit, kper;
+    uint32_t tiles, tokens, whole, nsplit, kper, extra;
 };
 
 struct alignas(64) LocalGemmArgs {
     CUtensorMap tmap_x[kMaxRanks];  // x_r [T, K] bf16, box 64 x tokens / 2, 128-byte swizzle
     CUtensorMap tmap_w[kMaxRanks];  // W_r [N, K] bf16, box 64 x 128, 128-byte swizzle
     CommView cv;                    // rank 0's
-    char* sums;                     // [nsplit][T, N] bf16
+    char* sums;                     // [nsplit][T, N] bf16, or lines of twice the size
+    uint32_t lines;                 // 1: flag-in-data lines {2 bf16, call, 2 bf16, ~call} instead of plain sums and flags
     uint32_t T, N;
     uint32_t kb_rank;               // k-blocks (of 64) of one rank
     uint32_t kb_total;              // of all ranks
@@ -45,9 +48,14 @@ struct LocalLinearNormArgs {
     float eps;
 };
 
+// CTAs of the row kernel per SM (with the GEMM gone) that its register cap allows.
+constexpr int LocalLinearNormPlaces(int ranks_per_cta, bool split) {
+    return ranks_per_cta == 4 ? (split ? 2 : 3) : ranks_per_cta == 2 ? (split ? 3 : 4) : 2;
+}
+
 const void* LocalGemmKernel();
 uint32_t LocalGemmSmemBytes();
-// `ranks_per_cta`: 1, 2 or 4.
-const void* LocalLinearNormKernel(uint32_t N, int ranks_per_cta);
+// `ranks_per_cta`: 1, 2 or 4; `split`: more than one K split; `lines` (one rank per CTA, split): flag-in-data sums.
+const void* LocalLinearNormKernel(uint32_t N, int ranks_per_cta, bool split, bool lines);
 
 }  // namespace yali

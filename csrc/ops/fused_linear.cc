@@ -268,34 +268,50 @@ int FusedLinearAutoMulticastMode(int world, uint32_t /*T*/) {
     return world < 8 ? 0 : 2;
 }
 
-// The cost of a candidate, in cycles of an SM: rounds of items times (their k-blocks + about 2500 for the first
-// operands, the read-out of the accumulator and the flag), plus the sums' way through L2 (write and read, at
-// about 30 bytes per SM and cycle).  A k-block takes the longest of: 350 cycles of issue (2 CTAs, four MMAs); 2 per
-// token on the tensor cores; its share of reading W once from HBM (3.6 bytes per ns and cycle of 1.8 GHz) by the pairs
-// that run together and do not share a slice.  Measured on B200.
-LocalGemmShape LocalGemmShapeFor(uint32_t T, uint32_t N, uint32_t kb_total, uint64_t room, uint32_t pairs) {
+// Tries every cut and takes the one with the lowest estimate, in cycles of an SM:
+//   * a k-block of an item takes 2 cycles per token on the tensor cores, at least 350 for its instructions, an
+//     item 600 more; the longest run of a pair counts;
+//   * no run is shorter than reading all of W and x from HBM (3440 bytes per cycle);
+//   * rows that complete in the last step of the GEMM are written after it (2670 bytes per cycle for their sums, residuals,
+//     outputs and new residuals), the others under it.
+LocalGemmShape LocalGemmShapeFor(uint32_t T, uint32_t N, uint32_t kb_total, int world, uint64_t room, uint32_t pairs) {
     const uint32_t ncol = (N + kLocalGemmPairCols - 1) / kLocalGemmPairCols, units = N / kLocalGemmUnitCols;
     const uint32_t fewest = (T + kLocalGemmMaxTokens - 1) / kLocalGemmMaxTokens;
+    const uint64_t hbm = static_cast<uint64_t>(kb_total) * (N + T) * 128 / 3440 * 115 / 100;
     LocalGemmShape best{};
     uint64_t best_cost = ~0ull;
-    for (uint32_t split = 1; split <= std::min(kLocalGemmMaxSplit, kb_total); ++split) {
-        const uint64_t sums = static_cast<uint64_t>(T) * N * 2 * split;
-        if (split > 1 && sums > room) break;
-        for (uint32_t n = fewest; n < fewest + 4; ++n) {
-            LocalGemmShape s;
-            s.tokens = ((T + n - 1) / n + 31) / 32 * 32;
-            s.tiles = (T + s.tokens - 1) / s.tokens;
+    auto consider = [&](const LocalGemmShape& s) {
+        const uint64_t block = std::max<uint64_t>(350, 2ull * s.tokens + 8);
+        const uint64_t t_whole = kb_total * block + 600, t_split = s.kper * block + 600;
+        const uint32_t nwhole = s.whole * ncol, left = nwhole % pairs;
+        const uint32_t nsplit = (s.tiles - s.whole) * ncol * s.nsplit, early = left ? s.extra * (pairs - left) : 0;
+        const uint32_t after = nsplit > early ? nsplit - early : 0;
+        const uint64_t end = (nwhole / pairs + (left ? 1 : 0)) * t_whole + (after + pairs - 1) / pairs * t_split;
+        const uint32_t last = after ? std::min(after, pairs) : left ? left : pairs;
+        const uint32_t per_tile = after ? ncol * s.nsplit : ncol;
+        const uint64_t rows = std::min<uint64_t>(T, static_cast<uint64_t>((last + per_tile - 1) / per_tile) * s.tokens);
+        const uint64_t cost = std::max(end, hbm) + rows * N * 2 * (3 * world + s.nsplit) / 2670;
+        if (cost < best_cost) {
+            best_cost = cost;
+            best = s;
+        }
+    };
+    for (uint32_t n = fewest; n < fewest + 4; ++n) {
+        LocalGemmShape s;
+        s.tokens = ((T + n - 1) / n + 31) / 32 * 32;
+        s.tiles = (T + s.tokens - 1) / s.tokens;
+        for (uint32_t split = 1; split <= std::min(kLocalGemmMaxSplit, kb_total); ++split) {
             s.kper = (kb_total + split - 1) / split;
             s.nsplit = (kb_total + s.kper - 1) / s.kper;
-            if (static_cast<uint64_t>(s.tiles) * units * s.nsplit > kLocalGemmFlags) continue;
-            const uint64_t items = static_cast<uint64_t>(s.tiles) * ncol * s.nsplit;
-            const uint64_t together = std::min<uint64_t>(items, pairs);
-            const uint64_t slices = std::max<uint64_t>(1, together / std::min<uint64_t>(s.tiles, std::max<uint64_t>(1, together / (ncol * s.nsplit))));
-            const uint64_t block = std::max<uint64_t>({350, 2ull * s.tokens + 8, slices * 32768 * 10 / 36000});
-            const uint64_t cost = (items + pairs - 1) / pairs * (s.kper * block + 2500) + 2 * sums / (30 * 148);
-            if (cost < best_cost) {
-                best_cost = cost;
-                best = s;
+            if (s.nsplit != split) continue;
+            if (split > 1 && static_cast<uint64_t>(T) * N * 2 * split > room) break;
+            if (static_cast<uint64_t>(s.tiles) * units * s.nsplit > kLocalGemmFlags) break;
+            s.extra = s.nsplit;
+            if (split == 1) {
+                s.whole = s.tiles;
+                consider(s);
+            } else {
+                for (s.whole = 0; s.whole < s.tiles; ++s.whole) consider(s);
             }
         }
     }
@@ -368,6 +384,7 @@ Result LaunchLocal(Communicator& comm, const DriverApi* drv, const FusedLinearDe
         }
         pairs = p;
     }
+    const uint32_t sms = 2 * pairs;
     const HeapLayout& lay = comm.layout();
     LocalGemmArgs g;
     std::memset(&g, 0, sizeof(g));
@@ -377,7 +394,7 @@ Result LaunchLocal(Communicator& comm, const DriverApi* drv, const FusedLinearDe
     g.N = N;
     g.kb_rank = K / 64;
     g.kb_total = g.kb_rank * W;
-    g.s = LocalGemmShapeFor(T, N, g.kb_total, 2ull * W * lay.gemm_cap, pairs);
+    g.s = LocalGemmShapeFor(T, N, g.kb_total, W, 2ull * W * lay.gemm_cap, pairs);
     LocalLinearNormArgs n;
     std::memset(&n, 0, sizeof(n));
     n.cv = g.cv;
@@ -399,16 +416,27 @@ Result LaunchLocal(Communicator& comm, const DriverApi* drv, const FusedLinearDe
         n.weight[r] = d.norm_weight;
         n.out[r] = d.out;
     }
-    const uint32_t items = g.s.tiles * ((N + kLocalGemmPairCols - 1) / kLocalGemmPairCols) * g.s.nsplit;
-    // With few rows the ranks of a row are spread over CTAs (each adds the splits again, from L2); from two CTAs per SM on
-    // a CTA serves as many ranks as its registers hold.
-    const int group = static_cast<uint64_t>(T) * W <= 296 ? 1 : W >= 4 ? 4 : 2;
+    const uint32_t items = (g.s.whole + (g.s.tiles - g.s.whole) * g.s.nsplit) * ((N + kLocalGemmPairCols - 1) / kLocalGemmPairCols);
+    // With few rows the ranks of a row are spread over CTAs (each adds the splits again, from L2) and the sums travel as
+    // flag-in-data lines, which saves the fence and the flag (2 ranks, T = 8: 11.3 -> LINES_US us a call).  From two
+    // CTAs per SM on a CTA serves as many ranks as its registers hold, and the grid is what fits the GPU.
+    const uint64_t line_bytes = static_cast<uint64_t>(T) * N * 4 * g.s.nsplit;
+    const bool few = static_cast<uint64_t>(T) * W <= 2 * sms;
+    const bool lines = few && T <= 64 && g.s.nsplit > 1 && g.s.whole == 0 && line_bytes <= 2ull * W * lay.gemm_ll_cap;
+    if (lines) {
+        g.lines = 1;
+        n.sums = g.sums = g.cv.heap[0] + lay.gemm_ll_off;
+    }
+    const int group = few ? 1 : W >= 4 ? 4 : 2;
+    const uint32_t units = T * ((W + group - 1) / group);
+    const void* const fn2 = LocalLinearNormKernel(N, group, g.s.nsplit > 1, lines);
+    const uint32_t places = sms * LocalLinearNormPlaces(group, g.s.nsplit > 1);
     const cudaStream_t s = streams && streams[0] ? streams[0] : comm.default_stream(0);
     void* gp[] = {&g};
     void* np[] = {&n};
     cudaError_t e = LaunchInStream(fn, dim3(2 * std::min(items, pairs)), dim3(kLocalGemmThreads), gp, smem, s);
     if (e == cudaSuccess)
-        e = LaunchInStream(LocalLinearNormKernel(N, group), dim3(T * ((W + group - 1) / group)), dim3(kLocalLinearNormThreads), np, 0, s);
+        e = LaunchInStream(fn2, dim3(std::min(units, places)), dim3(kLocalLinearNormThreads), np, 0, s);
     if (e != cudaSuccess) {
         (void)cudaGetLastError();
         return fail(Result::CudaError, std::string("kernel launch failed: ") + cudaGetErrorString(e));
