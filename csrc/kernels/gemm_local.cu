@@ -20,7 +20,12 @@
 // by elect.sync (behind a lane test the compiler wraps each of these instructions in a loop over the active
 // threads: 540 instead of 390 cycles per k-block of 160 tokens).
 //
-// Bound by the tensor cores from about 200 tokens on, by reading W below.
+// Bound by the tensor cores at the clock they leave (2 ranks, T = 2048, K = 2048: the GEMM reaches 1.4 PFLOP/s while the
+// first tiles come from HBM), and by writing the rows that complete with the last tiles (4.6 - 5.3 TB/s of stores);
+// by reading W from HBM for few tokens.  Measured per call, ranks on one B200, against the exchange of bf16
+// partial rows in one cooperative launch (gemm_ar_rmsnorm.cu, gemm_ar_decode.cu), us: 2 ranks, K = 2048: T = 8 15.1 ->
+// 10.8, T = 128 26.7 -> 17.7, T = 2048 78.6 -> 65.5; 8 ranks, K = 1792, T = 300 68 -> 55; 8 ranks, K = 512, T = 2048
+// 180 -> 118.
 //
 // Parity: none in the reference (it has no GEMM, no fused op and no tensor-core code).
 #include <cuda.h>
@@ -68,36 +73,13 @@ struct Item {
     uint32_t col_tile, split;
     uint32_t kb_begin, kb_end;
 };
-// The k-th item of a pair; false: no more.  Whole items first, pair by pair, then split ones: a pair without a whole item in
-// the last round starts on them at once.  Token tile by token tile, so that rows complete early.
+// The k-th item of a pair; false: no more.  Token tile by token tile, so that rows complete early; items in flight together
+// read the same stretch of K.
 __device__ __forceinline__ bool item_at(const LocalGemmArgs& a, uint32_t k, uint32_t pair, uint32_t npairs, uint32_t ncol, Item* it) {
-    const uint32_t nwhole = a.s.whole * ncol, left = nwhole % npairs;
-    const uint32_t mine = nwhole / npairs + (pair < left ? 1u : 0u);
-    if (k < mine) {
-        const uint32_t i = pair + k * npairs;
-        it->tile = i / ncol;
-        it->col_tile = i % ncol;
-        it->split = 0;
-        it->kb_begin = 0;
-        it->kb_end = a.kb_total;
-        return true;
-    }
-    k -= mine;
-    uint32_t j, early = 0;
-    if (left) {
-        early = a.s.extra * (npairs - left);
-        if (pair >= left && k < a.s.extra) {
-            j = pair - left + k * (npairs - left);
-            early = ~0u;
-        } else if (pair >= left) {
-            k -= a.s.extra;
-        }
-    }
-    if (early != ~0u) j = early + pair + k * npairs;
-    const uint32_t per_tile = ncol * a.s.nsplit;
-    if (j >= (a.s.tiles - a.s.whole) * per_tile) return false;
-    const uint32_t t = j / per_tile, in_tile = j - t * per_tile;
-    it->tile = a.s.whole + t;
+    const uint32_t i = pair + k * npairs, per_tile = ncol * a.s.nsplit;
+    if (i >= a.s.tiles * per_tile) return false;
+    it->tile = i / per_tile;
+    const uint32_t in_tile = i - it->tile * per_tile;
     it->split = in_tile / ncol;
     it->col_tile = in_tile - it->split * ncol;
     it->kb_begin = it->split * a.s.kper;
@@ -421,7 +403,7 @@ __global__ void __launch_bounds__(kLocalLinearNormThreads, LocalLinearNormPlaces
             }
             if (G == 1 && have[j]) w1[j] = ptx::ld_cg_v4(static_cast<const char*>(a.weight[q0]) + (tid + j * kThreads) * 16);
         }
-        const uint32_t tile = row / a.s.tokens, nsplit = tile < a.s.whole ? 1u : a.s.nsplit;
+        const uint32_t tile = row / a.s.tokens, nsplit = a.s.nsplit;
         if (!LINES && tile != ready) {
             // The flags of this row's token tile, a few per thread.
             const uint32_t first = kLocalGemmFlagOff + tile * a.s.nsplit * flags_per_split;

@@ -16,12 +16,10 @@ constexpr uint32_t kLocalGemmMaxSplit = 8;
 constexpr int kLocalGemmThreads = 384;         // eight epilogue warps, TMA, MMA, announcer, prefetch
 constexpr int kLocalLinearNormThreads = 256;   // one row; up to two 16-byte vectors per thread: N <= 4096
 
-// T rows in `tiles` token tiles of `tokens` (a multiple of 32, at most 256).  The first `whole` tiles' items (256 columns
-// each) run over all k-blocks of all ranks (one rank after the other); the items of the other tiles are cut into
-// `nsplit` runs of `kper` k-blocks.  Pairs that have nothing to do in the last round of whole items take `extra` split
-// items each meanwhile.
+// T rows in `tiles` token tiles of `tokens` (a multiple of 32, at most 256), the k-blocks of all ranks (one rank after the
+// other) in `nsplit` runs of `kper`.
 struct LocalGemmShape {
-    uint32_t tiles, tokens, whole, nsplit, kper, extra;
+    uint32_t tiles, tokens, nsplit, kper;
 };
 
 struct alignas(64) LocalGemmArgs {

@@ -268,50 +268,42 @@ int FusedLinearAutoMulticastMode(int world, uint32_t /*T*/) {
     return world < 8 ? 0 : 2;
 }
 
-// Tries every cut and takes the one with the lowest estimate, in cycles of an SM:
-//   * a k-block of an item takes 2 cycles per token on the tensor cores, at least 350 for its instructions, an
-//     item 600 more; the longest run of a pair counts;
-//   * no run is shorter than reading all of W and x from HBM (3440 bytes per cycle);
-//   * rows that complete in the last step of the GEMM are written after it (2670 bytes per cycle for their sums, residuals,
-//     outputs and new residuals), the others under it.
-LocalGemmShape LocalGemmShapeFor(uint32_t T, uint32_t N, uint32_t kb_total, int world, uint64_t room, uint32_t pairs) {
+// Tries the cuts and takes the one with the lowest estimate, in cycles of an SM:
+//   * a k-block of an item takes 2 cycles per token on the tensor cores, at least 350 for its instructions, and an item
+//     1500 more; every pair has the same number of items, up to one;
+//   * no run is shorter than reading all of W and x from HBM (3440 bytes per cycle, 15 % lost), by the pairs that are busy;
+//   * the sums are written and read again (1600 bytes per cycle): why splitting K costs more than cutting the tokens finer;
+//   * the last item's read-out (10 per token), 60 per pair that has nothing to do (its SMs load nothing), and 2200 for
+//     the fence and the flag of plain sums (`lines`: more than two splits travel as flag-in-data lines).
+// Fitted to sweeps on B200 (graph, us): 2 ranks, K = 2048, N = 4096: T = 256: 2 tiles of 128 x 2 splits 20.5, 1 of 256 x 4
+// 23.2, 2 of 128 unsplit 24.8; T = 512: 4 of 128 27.5, 2 of 256 x 2 30.0; T = 2048: 8 of 256 65, 11 of 192 72; T = 8: 4
+// splits 10.6, 3 11.6.  8 ranks, K = 1792, T = 300: 2 of 160 x 2 54, unsplit 71.
+LocalGemmShape LocalGemmShapeFor(uint32_t T, uint32_t N, uint32_t kb_total, uint64_t room, uint32_t pairs, bool lines) {
     const uint32_t ncol = (N + kLocalGemmPairCols - 1) / kLocalGemmPairCols, units = N / kLocalGemmUnitCols;
     const uint32_t fewest = (T + kLocalGemmMaxTokens - 1) / kLocalGemmMaxTokens;
-    const uint64_t hbm = static_cast<uint64_t>(kb_total) * (N + T) * 128 / 3440 * 115 / 100;
+    const uint64_t hbm = static_cast<uint64_t>(kb_total) * (N + T) * 128 / 3440 * 115 / 100 + 1500;
     LocalGemmShape best{};
     uint64_t best_cost = ~0ull;
-    auto consider = [&](const LocalGemmShape& s) {
-        const uint64_t block = std::max<uint64_t>(350, 2ull * s.tokens + 8);
-        const uint64_t t_whole = kb_total * block + 600, t_split = s.kper * block + 600;
-        const uint32_t nwhole = s.whole * ncol, left = nwhole % pairs;
-        const uint32_t nsplit = (s.tiles - s.whole) * ncol * s.nsplit, early = left ? s.extra * (pairs - left) : 0;
-        const uint32_t after = nsplit > early ? nsplit - early : 0;
-        const uint64_t end = (nwhole / pairs + (left ? 1 : 0)) * t_whole + (after + pairs - 1) / pairs * t_split;
-        const uint32_t last = after ? std::min(after, pairs) : left ? left : pairs;
-        const uint32_t per_tile = after ? ncol * s.nsplit : ncol;
-        const uint64_t rows = std::min<uint64_t>(T, static_cast<uint64_t>((last + per_tile - 1) / per_tile) * s.tokens);
-        const uint64_t cost = std::max(end, hbm) + rows * N * 2 * (3 * world + s.nsplit) / 2670;
-        if (cost < best_cost) {
-            best_cost = cost;
-            best = s;
-        }
-    };
     for (uint32_t n = fewest; n < fewest + 4; ++n) {
         LocalGemmShape s;
         s.tokens = ((T + n - 1) / n + 31) / 32 * 32;
         s.tiles = (T + s.tokens - 1) / s.tokens;
+        const uint64_t block = std::max<uint64_t>(350, 2ull * s.tokens + 8);
         for (uint32_t split = 1; split <= std::min(kLocalGemmMaxSplit, kb_total); ++split) {
             s.kper = (kb_total + split - 1) / split;
             s.nsplit = (kb_total + s.kper - 1) / s.kper;
+            const uint64_t sums = static_cast<uint64_t>(T) * N * 2 * s.nsplit;
             if (s.nsplit != split) continue;
-            if (split > 1 && static_cast<uint64_t>(T) * N * 2 * split > room) break;
+            if (split > 1 && sums > room) break;
             if (static_cast<uint64_t>(s.tiles) * units * s.nsplit > kLocalGemmFlags) break;
-            s.extra = s.nsplit;
-            if (split == 1) {
-                s.whole = s.tiles;
-                consider(s);
-            } else {
-                for (s.whole = 0; s.whole < s.tiles; ++s.whole) consider(s);
+            const uint64_t items = static_cast<uint64_t>(s.tiles) * ncol * s.nsplit;
+            const uint64_t rounds = (items + pairs - 1) / pairs, used = std::min<uint64_t>(items, pairs);
+            uint64_t cost = std::max(rounds * (s.kper * block + 1500), hbm * (rounds * used) / items) + 2 * sums / 1600 +
+                            10 * s.tokens + 60 * (pairs - used);
+            if (!(lines && split > 2)) cost += 2200;
+            if (cost < best_cost) {
+                best_cost = cost;
+                best = s;
             }
         }
     }
@@ -394,7 +386,8 @@ Result LaunchLocal(Communicator& comm, const DriverApi* drv, const FusedLinearDe
     g.N = N;
     g.kb_rank = K / 64;
     g.kb_total = g.kb_rank * W;
-    g.s = LocalGemmShapeFor(T, N, g.kb_total, W, 2ull * W * lay.gemm_cap, pairs);
+    const bool few = static_cast<uint64_t>(T) * W <= 2 * sms;
+    g.s = LocalGemmShapeFor(T, N, g.kb_total, 2ull * W * lay.gemm_cap, pairs, few && T <= 64);
     LocalLinearNormArgs n;
     std::memset(&n, 0, sizeof(n));
     n.cv = g.cv;
@@ -416,13 +409,13 @@ Result LaunchLocal(Communicator& comm, const DriverApi* drv, const FusedLinearDe
         n.weight[r] = d.norm_weight;
         n.out[r] = d.out;
     }
-    const uint32_t items = (g.s.whole + (g.s.tiles - g.s.whole) * g.s.nsplit) * ((N + kLocalGemmPairCols - 1) / kLocalGemmPairCols);
+    const uint32_t items = g.s.tiles * ((N + kLocalGemmPairCols - 1) / kLocalGemmPairCols) * g.s.nsplit;
     // With few rows the ranks of a row are spread over CTAs (each adds the splits again, from L2) and the sums travel as
-    // flag-in-data lines, which saves the fence and the flag (2 ranks, T = 8: 11.3 -> LINES_US us a call).  From two
-    // CTAs per SM on a CTA serves as many ranks as its registers hold, and the grid is what fits the GPU.
+    // flag-in-data lines, which saves the fence and the flag at the price of twice the bytes (2 ranks, K = 2048: T = 16 13.1 ->
+    // 12.1 us, T = 64 16.1 -> 15.1, but T = 128 18.4 -> 21.7; two splits are level).  From two CTAs per SM on a CTA
+    // serves as many ranks as its registers hold, and the grid is what fits the GPU.
     const uint64_t line_bytes = static_cast<uint64_t>(T) * N * 4 * g.s.nsplit;
-    const bool few = static_cast<uint64_t>(T) * W <= 2 * sms;
-    const bool lines = few && T <= 64 && g.s.nsplit > 1 && g.s.whole == 0 && line_bytes <= 2ull * W * lay.gemm_ll_cap;
+    const bool lines = few && T <= 64 && g.s.nsplit > 2 && line_bytes <= 2ull * W * lay.gemm_ll_cap;
     if (lines) {
         g.lines = 1;
         n.sums = g.sums = g.cv.heap[0] + lay.gemm_ll_off;

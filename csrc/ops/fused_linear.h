@@ -55,8 +55,8 @@ uint32_t FusedLinearDecodeSplit(uint32_t T, uint32_t N, uint32_t K, int world, u
 // Token tiles of the tile form for `pairs` resident pairs of CTAs per rank.
 GemmTiling FusedLinearTiling(uint32_t T, uint32_t N, int world, bool oneshot, uint32_t ksplit, uint32_t pairs);
 // Token tiles and K splits of the form for ranks that share one GPU; `kb_total` k-blocks over all ranks, room for `room`
-// bytes of sums, `pairs` resident pairs of CTAs.
-LocalGemmShape LocalGemmShapeFor(uint32_t T, uint32_t N, uint32_t kb_total, int world, uint64_t room, uint32_t pairs);
+// bytes of sums, `pairs` resident pairs of CTAs; `lines`: sums of more than two splits travel as flag-in-data lines.
+LocalGemmShape LocalGemmShapeFor(uint32_t T, uint32_t N, uint32_t kb_total, uint64_t room, uint32_t pairs, bool lines);
 // Rows from which the two-shot form is used when `force_oneshot` is -1.
 uint32_t FusedLinearOneShotMaxRows(int world);
 int FusedLinearAutoMulticastMode(int world, uint32_t T);
