@@ -296,9 +296,9 @@ def run_own(args) -> dict:
     for h, t in zip(h_in, aslist(send)):
         h.copy_(t)
 
-    # The user's call for data that lives on the host: every step copies the whole input in from
-    # pinned memory and the whole result out; the copies of both directions and the all-reduce
-    # overlap chunk by chunk inside the call.
+    # The user's call for data that lives on the host: every step moves the whole input in from
+    # pinned memory and the whole result out, both directions and the all-reduce at the same time
+    # (chunk by chunk, or inside one kernel where one GPU holds all ranks).
     def e2e_step(_i):
         comm.all_reduce_host(h_in if n_local > 1 else h_in[0], h_out if n_local > 1 else h_out[0])
 
@@ -373,9 +373,12 @@ def run_own(args) -> dict:
                 "copies_only_ms_per_step": round(copies_ms / e2e_steps, 3),
                 "fraction_of_copies_only": round(copies_ms / e2e_ms, 3) if e2e_ms else None,
                 "gpu_launches": int(e2e_launches * (1 if emulated else ranks)),
-                "api": "Comm.all_reduce_host(pinned_in, pinned_out): H2D, all-reduce and D2H of 4 MiB chunks "
-                       "overlap on three streams; copies_only = the same copies without the collective, all "
-                       "ranks at once (the ceiling of the host link)"},
+                "api": "Comm.all_reduce_host(pinned_in, pinned_out): "
+                       + ("one kernel reads every rank's input from pinned host memory and writes the results there; "
+                          "copies_only = chunked copies in and out through the device without the collective"
+                          if n_local == ranks else
+                          "H2D, all-reduce and D2H of 4 MiB chunks overlap on three streams; copies_only = the same "
+                          "copies without the collective, all ranks at once (the ceiling of the host link)")},
         "nccl": nccl,
         "gpu_launches": int(launches),
         "clocks": clocks,

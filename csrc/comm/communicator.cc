@@ -233,12 +233,6 @@ CommView Communicator::View(int i) const {
     return v;
 }
 
-uint32_t Communicator::TakeBarrierEpochs(uint32_t n) {
-    uint32_t e = bar_epoch_;
-    bar_epoch_ += n;
-    return e;
-}
-
 bool Communicator::IsSymmetric(int i, const void* p, uint64_t bytes) const {
     const char* base = heaps_->base(local_[i].rank);
     const char* c = static_cast<const char*>(p);
@@ -499,6 +493,11 @@ Result Communicator::LaunchLocal(const Plan& plan, const void* const* send, void
         fn = LocalNormKernelFor(in, world_, s);
         block = dim3(s.threads);
         blocks = rows * ((world_ + s.ranks_per_cta - 1) / s.ranks_per_cta);
+    } else if (plan.flags & kFlagHostMemory) {
+        fn = LocalHostKernelFor(in, world_);
+        block = dim3(kLocalHostThreads);
+        const uint64_t units = (plan.flags & kFlagVecOk) ? count * DtypeSize(in) / 16 + 1 : count;
+        blocks = std::min<uint64_t>((units + kLocalHostThreads - 1) / kLocalHostThreads, kLocalHostCtas);
     } else {
         const bool rs = plan.flags & kFlagReduceScatterOnly, ag = plan.flags & kFlagAllGatherOnly;
         fn = LocalKernelFor(in, out, world_, rs ? LocalKind::ReduceScatter : ag ? LocalKind::AllGather : LocalKind::Sum);
@@ -691,6 +690,34 @@ Result Communicator::AllReduce(const void* const* send, void* const* recv, uint6
     return Collective(send, recv, count, in, out, opt, streams, 0);
 }
 
+bool Communicator::AllReduceMapped(const void* const* send, void* const* recv, uint64_t count, Dtype dt,
+                                   const OpOptions& opt, const cudaStream_t* streams, Result* r) {
+    if (!(emulated_ || world_ == 1) || poisoned_ || count == 0 || opt.mode != KernelMode::Auto ||
+        env::ForcedKernelMode() != KernelMode::Auto || opt.ctas > 0 || opt.slot_bytes > 0 ||
+        opt.epilogue == kEpiResidualRmsNorm || count > (1ull << 40))
+        return false;
+    const uint64_t bytes = count * DtypeSize(dt);
+    if (!CanRunInOneLaunch(send, recv, bytes, bytes, 0, dt, dt, opt, 0)) return false;
+    const void* s[kMaxRanks];
+    void* d[kMaxRanks];
+    Plan plan;
+    plan.variant = Variant::Flash;
+    plan.flags = kFlagOneLaunch | kFlagHostMemory | kFlagVecOk | (trace_ ? static_cast<uint32_t>(kFlagTrace) : 0u);
+    for (int i = 0; i < nlocal(); ++i) {
+        cudaPointerAttributes a, b;
+        if (cudaPointerGetAttributes(&a, send[i]) != cudaSuccess || cudaPointerGetAttributes(&b, recv[i]) != cudaSuccess ||
+            !a.devicePointer || !b.devicePointer) {
+            (void)cudaGetLastError();
+            return false;
+        }
+        s[i] = a.devicePointer;
+        d[i] = b.devicePointer;
+        if (!Aligned16(s[i]) || !Aligned16(d[i])) plan.flags &= ~static_cast<uint32_t>(kFlagVecOk);
+    }
+    *r = LaunchLocal(plan, s, d, count, dt, dt, opt, streams);
+    return true;
+}
+
 Result Communicator::ReduceScatter(const void* const* send, void* const* recv, uint64_t count, Dtype dt,
                                    const OpOptions& opt, const cudaStream_t* streams) {
     YALI_NVTX_RANGE("yali::ReduceScatter");
@@ -795,8 +822,6 @@ Result Communicator::Reset() {
             return Fail(Result::CudaError, "clearing the flag region failed");
         std::memset(l.status, 0, sizeof(DeviceStatus));
     }
-    flash_epoch_ = bar_epoch_ = stream_seq_ = gemm_epoch_ = 0;
-    gemm_ = GemmCounters();
     poisoned_ = false;
     if (bs_ && bs_->barrier() != Result::Success) return Fail(Result::BootstrapError, bs_->last_error());
     return Result::Success;

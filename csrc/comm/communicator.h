@@ -90,6 +90,10 @@ class Communicator {
     // streams may be nullptr (the communicator's own stream per local rank).
     Result AllReduce(const void* const* send, void* const* recv, uint64_t count, Dtype in, Dtype out,
                      const OpOptions& opt, const cudaStream_t* streams);
+    // The same between page-locked host buffers, read and written by one kernel where they are.  False: this call cannot be
+    // done so (several GPUs, a forced mode, memory that the GPU cannot address); otherwise *r is its result.
+    bool AllReduceMapped(const void* const* send, void* const* recv, uint64_t count, Dtype dt, const OpOptions& opt,
+                         const cudaStream_t* streams, Result* r);
     // recv (ShardElems(count, world) elements, of which the valid part is used) = this rank's shard of the sum.
     Result ReduceScatter(const void* const* send, void* const* recv, uint64_t count, Dtype dt, const OpOptions& opt,
                          const cudaStream_t* streams);
@@ -118,16 +122,6 @@ class Communicator {
     // Builds the argument block for one local rank without launching (used by the
     // fused GEMM and by the allocation-free entry point's tests).
     CommView View(int local_index) const;
-    // Reserves epochs for an externally launched kernel that uses the per-CTA barrier.
-    uint32_t TakeBarrierEpochs(uint32_t n);
-    uint32_t TakeGemmEpoch() { return ++gemm_epoch_; }
-    // Cumulative targets of the fused GEMM's arrival / delivered-rows counters, indexed by rank
-    // (identical on every rank; cleared by Reset()).
-    struct GemmCounters {
-        uint32_t cnt[kMaxRanks] = {};
-        uint32_t done[kMaxRanks] = {};
-    };
-    GemmCounters& gemm_counters() { return gemm_; }
     bool poisoned() const { return poisoned_; }
     uint32_t max_ctas() const { return max_ctas_; }
     void set_error(const std::string& e) { err_ = e; }
@@ -193,12 +187,6 @@ class Communicator {
     bool trace_ = false;
     std::vector<CollArgs> args_scratch_;  // per-call argument blocks, reused (no allocation per call)
     std::vector<std::pair<const void*, int>> smem_attr_set_;  // (kernel, device) pairs with the smem limit raised
-    // Epochs: identical on every rank because every rank performs the same calls.
-    uint32_t flash_epoch_ = 0;
-    uint32_t bar_epoch_ = 0;
-    uint32_t stream_seq_ = 0;
-    uint32_t gemm_epoch_ = 0;
-    GemmCounters gemm_;
     uint64_t user_bump_ = 0;
     bool poisoned_ = false;
     LastCallInfo last_;

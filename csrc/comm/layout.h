@@ -178,6 +178,7 @@ enum CollFlags : uint32_t {
     kFlagSkipRank = 1u << 5,    // this rank leaves at once (models a rank that never launched; tests of the timeouts)
     kFlagTrace = 1u << 7,       // stamp %globaltimer at entry and check-out into the kTraceOff ring
     kFlagPullOneShot = 1u << 8, // pipelined kernel: every rank pulls and sums the whole message (no pushes)
+    kFlagHostMemory = 1u << 10,  // with kFlagOneLaunch: the buffers are page-locked host memory
     kFlagOneLaunch = 1u << 9,   // all ranks share one GPU and one launch: no exchange (kernels/local_group.cu)
 };
 

@@ -111,6 +111,12 @@ __device__ __forceinline__ uint4 ld_volatile_v4(const void* p) {
                  : "memory");
     return v;
 }
+// Host memory: nothing that a cache may still hold of it is used.
+__device__ __forceinline__ uint4 ld_cv_v4(const void* p) {
+    uint4 v;
+    asm volatile("ld.global.cv.v4.u32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+    return v;
+}
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 __device__ __forceinline__ void st_v4(void* p, const uint4& v) {
     asm volatile("st.global.v4.u32 [%0], {%1,%2,%3,%4};" ::"l"(p), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");

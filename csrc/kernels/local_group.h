@@ -28,6 +28,9 @@ struct LocalArgs {
     uint32_t flags;                   // kFlagVecOk, kFlagTrace
 };
 
+constexpr int kLocalHostThreads = 256;
+constexpr int kLocalHostCtas = 64;
+
 // How the norm kernel cuts its work: threads of a CTA (one row), vectors per thread, and for how many ranks
 // a CTA normalises the row.
 struct LocalNormShape {
@@ -53,6 +56,8 @@ inline LocalNormShape LocalNormShapeFor(uint64_t rows, uint32_t vec_per_row, int
 
 // nullptr when the combination is not built.
 const void* LocalKernelFor(Dtype in, Dtype out, int world, LocalKind kind);
+// Sum of buffers in host memory that the GPU can address; any number of CTAs.
+const void* LocalHostKernelFor(Dtype dt, int world);
 const void* LocalNormKernelFor(Dtype dt, int world, const LocalNormShape& shape);
 
 }  // namespace yali

@@ -82,6 +82,9 @@ Result HostPipeline::AllReduce(const void* const* src, void* const* dst, uint64_
         comm_.set_error("all_reduce_host: the row epilogue needs whole rows on the device; use AllReduce");
         return Result::Unsupported;
     }
+    // One launch for all ranks: a kernel that works on the host buffers themselves, unless the caller cuts chunks.
+    Result direct = Result::Success;
+    if (chunk_bytes == 0 && !copies_only && comm_.AllReduceMapped(src, dst, count, dt, opt, user_streams, &direct)) return direct;
     // Chunks are multiples of 256 elements so that every chunk keeps the 16-byte alignment of the
     // vector paths.
     // chunk_bytes == 0: about 32 chunks per message, between 1 and 8 MiB each: the first copy in and the

@@ -28,6 +28,8 @@ class HostPipeline {
     // symmetric heap on first use: every process must make the same calls).  Work is queued
     // behind `user_streams[i]` (or the communicator's own stream), which also waits for the
     // last chunk; the call itself does not block.
+    // Where one launch on one GPU runs all ranks, chunk_bytes = 0 lets one kernel read and write the host buffers directly
+    // (Communicator::AllReduceMapped): no staging, chunks or events.
     // `copies_only` leaves the collective out (dst = src through the device): the same copies on the
     // same streams, which is the ceiling the host link sets for this call.
     Result AllReduce(const void* const* src, void* const* dst, uint64_t count, Dtype dt, const OpOptions& opt,

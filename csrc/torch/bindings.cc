@@ -506,36 +506,37 @@ class PyComm {
 
     // dst = scale * sum over ranks of src, both in pinned host memory; copies and all-reduce
     // overlap chunk by chunk (ops/host_pipeline.h).
-    void AllReduceHost(std::vector<at::Tensor> src, std::vector<at::Tensor> dst, int64_t chunk_bytes,
-                       c10::optional<double> scale, const std::string& mode, bool copies_only) {
+    void AllReduceHost(const py::object& src, const py::object& dst, int64_t chunk_bytes, const py::object& scale,
+                       const py::object& mode, bool copies_only) {
         const int nl = c().nlocal();
-        TORCH_CHECK(static_cast<int>(src.size()) == nl && static_cast<int>(dst.size()) == nl,
-                    "yali: one src and one dst tensor per local rank");
-        const at::ScalarType d = src[0].scalar_type();
-        const int64_t n = src[0].numel();
-        std::vector<const void*> s(nl);
-        std::vector<void*> r(nl);
+        Args sa, da;
+        Read(src.ptr(), "src", &sa);
+        Read(dst.ptr(), "dst", &da);
+        const at::ScalarType d = sa[0].scalar_type();
+        const int64_t n = sa[0].numel();
+        const void* s[kMaxRanks];
+        void* r[kMaxRanks];
         for (int i = 0; i < nl; ++i) {
-            for (const at::Tensor& t : {src[i], dst[i]}) {
-                TORCH_CHECK(!t.is_cuda() && t.is_pinned() && t.is_contiguous(),
-                            "yali: all_reduce_host takes contiguous tensors in pinned host memory");
-                TORCH_CHECK(t.scalar_type() == d && t.numel() == n, "yali: src and dst must agree in size and dtype");
+            for (const at::Tensor* t : {&sa[i], &da[i]}) {
+                if (t->is_cuda() || !t->is_contiguous() || !t->is_pinned())
+                    throw py::value_error("all_reduce_host takes contiguous tensors in pinned host memory");
+                TORCH_CHECK(t->scalar_type() == d && t->numel() == n, "yali: src and dst must agree in size and dtype");
             }
-            s[i] = src[i].data_ptr();
-            r[i] = dst[i].data_ptr();
+            s[i] = sa[i].data_ptr();
+            r[i] = da[i].data_ptr();
         }
         OpOptions o;
-        o.mode = ToMode(mode);
-        if (scale.has_value()) {
+        o.mode = ModeOf(mode);
+        if (!scale.is_none()) {
             o.epilogue = kEpiScaleCast;
-            o.scale = static_cast<float>(*scale);
+            o.scale = static_cast<float>(py::cast<double>(scale));
         }
         if (!host_pipe_) host_pipe_ = std::make_unique<HostPipeline>(c());
-        auto st = Streams();
+        const StreamTable st = CurrentStreams();
         c10::cuda::OptionalCUDAGuard guard(c().device_of(0));
-        Throw(host_pipe_->AllReduce(s.data(), r.data(), static_cast<uint64_t>(n), ToDtype(d), o,
-                                    static_cast<uint64_t>(chunk_bytes <= 0 ? 0 : std::max<int64_t>(chunk_bytes, 4096)), st.data(), copies_only),
-              c().last_error());
+        Finish(host_pipe_->AllReduce(s, r, static_cast<uint64_t>(n), ToDtype(d), o,
+                                     static_cast<uint64_t>(chunk_bytes <= 0 ? 0 : std::max<int64_t>(chunk_bytes, 4096)), st.s,
+                                     copies_only));
     }
 
     void Sync() {

@@ -107,3 +107,28 @@ def test_halves_of_the_multi_gpu_kernel_on_request(comm, monkeypatch):
     comm.sync()
     assert comm.last_call()["variant"] == "stream" and not comm.last_call()["flags"] & ONE_LAUNCH
     assert torch.equal(full[-1].double(), total(xs))
+
+
+@pytest.mark.parametrize("dtype", [F32, F16, BF16])
+@pytest.mark.parametrize("n", [1, 7, 8, 4097, 131072, 131075, 2000003])
+def test_host_buffers_where_they_are(comm, dtype, n):
+    """Pinned host memory, one kernel; the sizes sit around a 16-byte unit and the 64 x 256 threads of the grid.  Inputs change
+    between calls: nothing of an earlier call may be read."""
+    W = comm.world
+    for off in (0, 1):
+        src = [torch.empty(n + off, dtype=dtype, pin_memory=True)[off:] for _ in range(W)]
+        dst = [torch.empty(n + off, dtype=dtype, pin_memory=True)[off:] for _ in range(W)]
+        for step in range(3):
+            for r in range(W):
+                src[r].copy_(torch.randint(-8, 9, (n,), generator=torch.Generator().manual_seed(step * 100 + r)).to(dtype))
+            before = comm.launches
+            comm.all_reduce_host(src, dst, scale=0.5)
+            torch.cuda.synchronize()
+            assert comm.launches - before == 1 and comm.last_call()["flags"] & 1 << 10
+            want = torch.stack([s.double() for s in src]).sum(0) * 0.5
+            assert all(torch.equal(d.double(), want) for d in dst)
+    comm.all_reduce_host(src, src)  # in place
+    torch.cuda.synchronize()
+    assert all(torch.equal(s.double(), want * 2) for s in src)
+    with pytest.raises(ValueError):
+        comm.all_reduce_host([torch.zeros(8) for _ in range(W)])

@@ -215,21 +215,16 @@ class Comm:
         about one direction's copy time instead of the sum of the three phases.  Staging is a ring of
         four symmetric chunk buffers per direction, allocated on first use and reused by every later
         call that fits (every rank must make the same calls).  The call returns with the work queued;
-        the caller's current stream waits for it.  `copies_only=True` leaves the collective out
-        (dst = src through the device): the ceiling the host link sets for the same call."""
-        srcs = self._as_list(src, "src")
+        the caller's current stream waits for it.  Where one GPU holds all ranks and `chunk_bytes` is 0,
+        one kernel reads and writes the host buffers directly instead.  `copies_only=True` leaves the
+        collective out (dst = src through the device): the time that copies alone take."""
         if dst is None:
-            dsts = [torch.empty_like(t).pin_memory() for t in srcs]
-        else:
-            dsts = self._as_list(dst, "dst")
-        for t in list(srcs) + list(dsts):
-            if t.is_cuda or not t.is_pinned() or not t.is_contiguous():
-                raise ValueError("all_reduce_host takes contiguous tensors in pinned host memory")
+            dst = [torch.empty_like(t).pin_memory() for t in self._as_list(src, "src")]
         try:
-            self._impl.all_reduce_host(srcs, dsts, int(chunk_bytes), scale, mode, bool(copies_only))
+            self._impl.all_reduce_host(src, dst, int(chunk_bytes), scale, mode, bool(copies_only))
         except RuntimeError as e:
             raise _translate(e) from None
-        return self._like_input(src, dsts)
+        return self._like_input(src, self._as_list(dst, "dst"))
 
     def shard_elems(self, count: int) -> int:
         return _native.ext().shard_elems(count, self.world)
