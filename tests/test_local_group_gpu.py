@@ -132,3 +132,17 @@ def test_host_buffers_where_they_are(comm, dtype, n):
     assert all(torch.equal(s.double(), want * 2) for s in src)
     with pytest.raises(ValueError):
         comm.all_reduce_host([torch.zeros(8) for _ in range(W)])
+
+
+@pytest.mark.parametrize("n", [1, 255, 256, 257, 524288, 524289])
+def test_new_outputs_of_one_call_are_apart(comm, n):
+    """Outputs that the call makes (one allocation up to 4 MiB, else one per rank; 524288 elements of 2 bytes x 4 ranks is the
+    line): contiguous, aligned, and writing one leaves the others and a later call's alone."""
+    W = comm.world
+    x = [torch.full((n,), r + 1.0, dtype=BF16, device="cuda") for r in range(W)]
+    want = float(W * (W + 1) // 2)
+    first, second = comm.all_reduce(x), comm.all_reduce(x, scale=2.0)
+    first[0].fill_(-7.0)
+    assert all(torch.equal(t, torch.full_like(t, want)) for t in first[1:])
+    assert all(torch.equal(t, torch.full_like(t, 2 * want)) for t in second)
+    assert all(t.shape == x[0].shape and t.is_contiguous() and t.data_ptr() % 16 == 0 for t in first + second)
