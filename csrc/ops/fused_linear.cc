@@ -413,15 +413,25 @@ Result LaunchLocal(Communicator& comm, const DriverApi* drv, const FusedLinearDe
     // With few rows the ranks of a row are spread over CTAs (each adds the splits again, from L2) and the sums travel as
     // flag-in-data lines, which saves the fence and the flag at the price of twice the bytes (2 ranks, K = 2048: T = 16 13.1 ->
     // 12.1 us, T = 64 16.1 -> 15.1, but T = 128 18.4 -> 21.7; two splits are level).  From two CTAs per SM on a CTA
-    // serves as many ranks as its registers hold, and the grid is what fits the GPU.
+    // serves two or four ranks, and the grid is what fits the GPU: with two more CTAs fit, with four the sums are read
+    // less often.  A round of four takes about 3/2 of a round of two (5/4 for rows of one vector per thread), so the rounds decide (8 ranks,
+    // two against four, us: T = 64 19.0 / 20.5, T = 128 24.9 / 22.7, T = 300 52.8 / 54.7, T = 512 40.7 / 44.7, T = 2048 122.9 / 131.4; 4 ranks: T = 256
+    // 26.3 / 24.0, T = 512 32.1 / 35.3; N = 2048, T = 2048 100 / 94).
     const uint64_t line_bytes = static_cast<uint64_t>(T) * N * 4 * g.s.nsplit;
     const bool lines = few && T <= 64 && g.s.nsplit > 2 && line_bytes <= 2ull * W * lay.gemm_ll_cap;
     if (lines) {
         g.lines = 1;
         n.sums = g.sums = g.cv.heap[0] + lay.gemm_ll_off;
     }
-    const int group = few ? 1 : W >= 4 ? 4 : 2;
-    const uint32_t units = T * ((W + group - 1) / group);
+    auto units_of = [&](int gr) { return T * ((W + gr - 1) / gr); };
+    auto rounds_of = [&](int gr) {
+        const uint32_t fit = sms * LocalLinearNormPlaces(gr, g.s.nsplit > 1);
+        return (units_of(gr) + fit - 1) / fit;
+    };
+    const bool one_vector = N <= 8u * kLocalLinearNormThreads;
+    const bool four = W > 2 && rounds_of(4) * (one_vector ? 5 : 6) <= rounds_of(2) * 4;
+    const int group = few ? 1 : four ? 4 : 2;
+    const uint32_t units = units_of(group);
     const void* const fn2 = LocalLinearNormKernel(N, group, g.s.nsplit > 1, lines);
     const uint32_t places = sms * LocalLinearNormPlaces(group, g.s.nsplit > 1);
     const cudaStream_t s = streams && streams[0] ? streams[0] : comm.default_stream(0);
