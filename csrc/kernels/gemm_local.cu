@@ -347,6 +347,12 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kLocalGemmThreads, 1
 
 namespace {
 
+// Pauses between two looks at a flag and at a line.  Polling costs the GEMM more than a late look costs the row: with 50 ns
+// and all lines asked for on every look, us: 2 ranks, K = 2048: T = 8 10.0 -> 9.8, T = 64 17.3 -> 14.6, T = 128 18.3 -> 16.5
+// (flags, 3000 ns level, 600 ns 16.8); 4 ranks, K = 1792, T = 100 20.4 -> 18.5 (3000 ns 20.5, 1000 ns 19.1).  Lines: 0 to 100 ns
+// are level.
+constexpr uint32_t kFlagSleepNs = 1500, kLineSleepNs = 40;
+
 // A unit of work is a row for G ranks (unit u: row u / ngroups, ranks from (u % ngroups) * G); a thread holds NV 16-byte
 // vectors of the row.  SPLIT: more than one K split; LINES: the sums come as flag-in-data lines.
 //
@@ -410,8 +416,9 @@ __global__ void __launch_bounds__(kLocalLinearNormThreads, LocalLinearNormPlaces
             for (uint32_t e = tid; e < nsplit * flags_per_split && !late; e += kThreads) {
                 uint32_t polls = 0, seen;
                 while (!ptx::seq_reached(seen = ptx::ld_acquire_gpu(flag_word(cv, 0, first + e)), epoch)) {
-                    if (++polls > 8) ptx::nanosleep(50);  // this CTA shares the SM with the GEMM
-                    if ((polls & 63u) == 0 && ptx::globaltimer() > deadline) {
+                    // This CTA shares the SM with the GEMM, and hundreds of them poll.
+                    if (++polls > 2) ptx::nanosleep(kFlagSleepNs);
+                    if ((polls & 7u) == 0 && ptx::globaltimer() > deadline) {
                         report_timeout(cv, kSiteGemmPartials, 0, blockIdx.x, epoch, seen);
                         late = true;
                         break;
@@ -462,6 +469,16 @@ __global__ void __launch_bounds__(kLocalLinearNormThreads, LocalLinearNormPlaces
                     uint4 y[NV][kFly];
                     uint32_t polls = 0;
                     bool missing;
+                    // One lane of a warp waits for one of its lines of the last split: asking for all lines again and
+                    // again (64 KiB per CTA) holds up the GEMM that writes them.
+                    if (k0 == 0 && (tid & 31) == 0 && have[0]) {
+                        uint4 l;
+                        while ((l = ptx::ld_volatile_v4(src + (nsplit - 1) * split_stride)).y != epoch || l.w != ~epoch) {
+                            ptx::nanosleep(kLineSleepNs);
+                            if ((++polls & 63u) == 0 && ptx::globaltimer() > deadline) break;  // the loop below reports it
+                        }
+                    }
+                    __syncwarp();
                     do {
                         missing = false;
 #pragma unroll
