@@ -1,6 +1,6 @@
 // Host-side entry points of the kernel translation units.  Each returns the
 // __global__ function for a (dtype, epilogue, world) combination so that the
-// dispatcher can launch it with cudaLaunchKernel (one rank per launch) or, for
+// dispatcher can launch it with LaunchInStream below (one rank per launch) or, for
 // an emulated communicator whose ranks share one GPU, with a cooperative launch
 // of the *_emu twin (ranks = blockIdx.y), which guarantees that all CTAs that
 // wait on one another are resident together.

@@ -37,7 +37,8 @@ struct FusedLinearOptions {
     unsigned long long* const* trace = nullptr;  // per local rank: device buffer of 8 timestamps, or nullptr
 };
 
-// descs: one per local rank.  Launches one kernel per rank (one cooperative launch for emulated ranks).
+// descs: one per local rank.  Launches one kernel per rank; for emulated ranks two for all of them
+// (kernels/gemm_local.cu), or one cooperative launch where a form is forced.
 Result FusedLinearAllReduceRmsNorm(Communicator& comm, const FusedLinearDesc* descs, uint32_t T, uint32_t N,
                                    uint32_t K, const FusedLinearOptions& opt, const cudaStream_t* streams);
 
@@ -55,7 +56,7 @@ uint32_t FusedLinearDecodeSplit(uint32_t T, uint32_t N, uint32_t K, int world, u
 // Token tiles of the tile form for `pairs` resident pairs of CTAs per rank.
 GemmTiling FusedLinearTiling(uint32_t T, uint32_t N, int world, bool oneshot, uint32_t ksplit, uint32_t pairs);
 // Token tiles and K splits of the form for ranks that share one GPU; `kb_total` k-blocks over all ranks, room for `room`
-// bytes of sums, `pairs` resident pairs of CTAs; `lines`: sums of more than two splits travel as flag-in-data lines.
+// bytes of sums, `pairs` resident pairs of CTAs; `lines`: the sums of splits travel as flag-in-data lines.
 LocalGemmShape LocalGemmShapeFor(uint32_t T, uint32_t N, uint32_t kb_total, uint64_t room, uint32_t pairs, bool lines);
 // Rows from which the two-shot form is used when `force_oneshot` is -1.
 uint32_t FusedLinearOneShotMaxRows(int world);

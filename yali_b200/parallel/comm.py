@@ -173,7 +173,8 @@ class Comm:
                              out: Optional[TensorOrList] = None, residual_out: Optional[TensorOrList] = None,
                              oneshot: Optional[bool] = None, ctas: int = 0, trace: Optional[TensorOrList] = None,
                              nvls: Union[None, bool, int] = None, decode: Optional[bool] = None):
-        """out = RMSNorm(residual + sum over ranks of x @ w.T) * norm_weight in ONE kernel per rank
+        """out = RMSNorm(residual + sum over ranks of x @ w.T) * norm_weight in ONE kernel per rank, or
+        in two for all ranks where they share one GPU
         (tcgen05 GEMM whose epilogue pushes partial rows to their owner over NVLink, then reduce + norm).
         x: [T, K], w: [N, K] (this rank's slice, nn.Linear layout), bf16.  With one GPU per process the
         two-shot form (T above a few dozen rows) needs `out` from symm_empty(); without `out` the call
