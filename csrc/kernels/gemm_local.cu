@@ -12,8 +12,8 @@
 //                              out and residual_out.
 //
 // The second kernel starts while the first one runs (griddepcontrol.launch_dependents, issued by every CTA of the first
-// one when it starts: all of them are resident by then, so whoever waits for them here waits for running CTAs),
-// and its CTAs wait for the flags of their token tile: rows are finished under the GEMM of later tiles.
+// one when it has read the call's number: all of them are resident by then, so whoever waits for them here waits for
+// running CTAs), and its CTAs wait for the flags of their token tile: rows are finished under the GEMM of later tiles.
 //
 // The pair computes the transposed tile, W on the M side: a tile can then be any multiple of 32 tokens wide, and each CTA
 // loads 128 rows of W and half of the tokens per 64-deep k-block.  The threads that issue TMA and MMA are picked
@@ -47,6 +47,7 @@ constexpr uint32_t kEpiChunk = 32;                              // tokens an epi
 constexpr uint32_t kEpiBufBytes = kEpiChunk * 64;  // 2 KiB per warp: 32 columns of a chunk
 constexpr int kEpiGroups = 2, kEpilogueWarps = 4 * kEpiGroups;
 constexpr int kTmaWarp = 8, kMmaWarp = 9, kAnnounceWarp = 10, kPrefetchWarp = 11;
+constexpr uint32_t kNumberBarrier = 1;  // named barrier: the announcer has read the call number, the epilogue warps use it
 constexpr uint32_t kPrefetchBlocks = 8;  // how far the prefetch warp runs ahead of the loads, in k-blocks
 static_assert(kTmemCols == 512 && kLocalGemmThreads == 32 * (kPrefetchWarp + 1), "one CTA per SM");
 static_assert(kSmemBytes + kEpilogueWarps * kEpiBufBytes + 1024 <= 216 * 1024, "leaves room for CTAs of the second kernel");
@@ -90,7 +91,7 @@ __device__ __forceinline__ bool item_at(const LocalGemmArgs& a, uint32_t k, uint
 struct Shared {
     __align__(8) uint64_t full_bar[kMaxStages], empty_bar[kMaxStages], tmem_full_bar[2], tmem_empty_bar[2];
     __align__(8) uint64_t stored_bar[2], announced_bar[2];  // epilogue warps -> announcer warp and back
-    uint32_t tmem;
+    uint32_t tmem, epoch;      // epoch: this call's number
     volatile uint32_t loaded;  // k-blocks whose loads have been issued
     volatile int abort;
 };
@@ -145,11 +146,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kLocalGemmThreads, 1
     ptx::tc_fence_after_sync();
     const uint32_t tmem = s.tmem;
     ptx::grid_dependency_wait();
-    ptx::grid_launch_dependents();
     const uint64_t deadline = ptx::globaltimer() + cv.timeout_ns;
-
-    // This call's number; the second kernel advances it when all of its CTAs have read it.
-    const uint32_t epoch = *reinterpret_cast<volatile uint32_t*>(flag_word(cv, 0, kCallLocalGemm)) + 1u;
     const uint32_t ncol = (a.N + kLocalGemmPairCols - 1) / kLocalGemmPairCols;
     const uint32_t pair = cta >> 1, npairs = gridDim.x >> 1;
     const uint32_t xbytes = a.s.tokens / 2 * (BK * 2);  // one CTA's half of the token operand of a stage: whole KiB
@@ -227,8 +224,14 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kLocalGemmThreads, 1
         // When the epilogue warps have stored their part of a unit: publish the call number in its flag.  The release orders
         // the stores (made visible to this warp by the mbarrier) before the flag; it waits for them to arrive, so it
         // sits in a warp of its own.
+        // It also reads this call's number, for the whole CTA, and then lets the second kernel start.  In this order: that
+        // kernel advances the number when all of its CTAs have read it, and waits for no data before it does so
+        // where the sums are lines, so by then every CTA here must have its number, too.
+        if (lane == 0) s.epoch = *reinterpret_cast<volatile uint32_t*>(flag_word(cv, 0, kCallLocalGemm)) + 1u;
+        ptx::named_barrier(kNumberBarrier, 32 * (kEpilogueWarps + 1));
         if (lane == 0) {
-            const uint32_t units = a.N / kLocalGemmUnitCols;
+            ptx::grid_launch_dependents();
+            const uint32_t epoch = s.epoch, units = a.N / kLocalGemmUnitCols;
             Item it;
             for (uint32_t n = 0; item_at(a, n, pair, npairs, ncol, &it); ++n) {
                 const uint32_t b = n & 1u, unit = it.col_tile * 2 + half;
@@ -273,6 +276,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kLocalGemmThreads, 1
         const uint32_t token = lane >> 2;  // stores: token of a group of 8, 16-byte piece lane % 4
         const uint8_t* const ld_row = stage + token * 64 + (((lane & 3) ^ ((token >> 1) & 3)) << 4);
         const uint64_t rowbytes = static_cast<uint64_t>(a.N) * 2;
+        ptx::named_barrier(kNumberBarrier, 32 * (kEpilogueWarps + 1));
+        const uint32_t epoch = s.epoch;
         Item it;
         for (uint32_t n = 0; item_at(a, n, pair, npairs, ncol, &it); ++n) {
             const uint32_t b = n & 1u, t0 = it.tile * a.s.tokens, nt = min(a.T - t0, a.s.tokens);
@@ -446,7 +451,8 @@ __global__ void __launch_bounds__(kLocalLinearNormThreads, LocalLinearNormPlaces
             unit = units;
         }
         // Once every CTA has read the call number and taken its last unit, both counters may move on: the next call reads
-        // them, nothing in this one does.  Done here, under the work of the last unit.
+        // them, nothing in this one does (the GEMM's CTAs had their number before they let this kernel start).
+        // Done here, under the work of the last unit.
         if (unit >= units && tid == kThreads - 1) check_in();
 
         uint4 one[SPLIT ? 1 : NV];

@@ -185,3 +185,41 @@ def test_ranks_on_one_gpu_add_in_the_gemm(world, T, K, N):
         c.fused_linear_rmsnorm(xs, ws, nw, res, out=res[1:] + res[:1])
         c.sync()
         assert c.launches - before == 1
+
+
+@pytest.mark.parametrize("world", [2, 8])
+def test_few_rows_back_to_back_with_new_inputs(world):
+    """Sums as flag-in-data lines: 60 calls in one graph, rows and inputs changing from call to call, replayed three times.
+    Whole-number inputs, so every call's residual is exact; one call's lines in another's result would show."""
+    K, N = 512, 4096
+    g = torch.Generator(device="cuda").manual_seed(world)
+
+    def pick(*shape):
+        keep = torch.rand(shape, generator=g, device="cuda") < 0.3
+        return (keep * torch.randint(-1, 2, shape, generator=g, device="cuda")).to(torch.bfloat16)
+
+    ws, nw = [pick(N, K) for _ in range(world)], [torch.ones(N, dtype=torch.bfloat16, device="cuda")] * world
+    calls = []
+    for i in range(60):
+        T = (1, 8, 64, 3, 33)[i % 5]
+        xs = [pick(T, K) for _ in range(world)]
+        calls.append((xs, [torch.empty(T, N, dtype=torch.bfloat16, device="cuda") for _ in range(world)]))
+    with yali.Comm.emulated(world, device=0, timeout_ms=2000) as c:
+        c.fused_linear_rmsnorm(calls[0][0], ws, nw, None, residual_out=calls[0][1])
+        c.sync()
+        graph, side = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+        with torch.cuda.graph(graph, stream=side):
+            for xs, pre in calls:
+                c.fused_linear_rmsnorm(xs, ws, nw, None, residual_out=pre)
+        for _ in range(3):
+            for _xs, pre in calls:
+                for p in pre:
+                    p.zero_()
+            graph.replay()
+            torch.cuda.synchronize()
+            c.check()
+            for xs, pre in calls:
+                want = sum(x.double() @ w.double().T for x, w in zip(xs, ws))
+                assert want.abs().max() < 256
+                assert all(torch.equal(p.double(), want) for p in pre)
+        del graph

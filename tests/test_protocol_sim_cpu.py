@@ -239,3 +239,42 @@ def test_in_switch_two_shot_protocol(world):
     rc, rep = simulate(mode=3, world=world, lanes=2, calls=4, count=3000, fault=1, fault_rank=world - 1, fault_call=1,
                        timeout_ms=300)
     assert rc == 2 and rep.timeout_peer == world - 1
+
+
+# ---- ranks that share one GPU: the GEMM and the row kernel that starts under it ----
+from yali_b200._native import LocalSimConfig  # noqa: E402
+
+
+def simulate_local(**kw):
+    cfg = LocalSimConfig(pairs=3, row_ctas=4, calls=5, rows=40, col_units=3, splits=2, tile_rows=16, lines=0, slow_cta=-1,
+                         late_number=0, reset_at=0, keep_lines=0, fault=0, fault_call=0, timeout_ms=5000)
+    for k, v in kw.items():
+        setattr(cfg, k, v)
+    rep = SimReport()
+    rc = _native.lib().yali_c_simulate_local(ctypes.byref(cfg), ctypes.byref(rep))
+    return rc, rep
+
+
+@pytest.mark.parametrize("lines", [0, 1])
+@pytest.mark.parametrize("rows,row_ctas", [(1, 1), (8, 8), (40, 4), (40, 13)])
+def test_local_form_protocol_back_to_back_calls(lines, rows, row_ctas):
+    # a CTA per row, and rows from the counter; more and fewer items than GEMM threads; a GEMM thread that is late
+    for pairs, splits, slow in ((1, 1, -1), (3, 2, 0), (7, 4, 5)):
+        rc, rep = simulate_local(lines=lines, rows=rows, row_ctas=row_ctas, pairs=pairs, splits=splits, slow_cta=slow)
+        assert rc == 0 and rep.mismatches == 0 and rep.timeouts == 0, (pairs, rc, rep.mismatches, rep.timeouts)
+        assert rep.flag_writes == 5 * rows * 3 * splits
+
+
+def test_local_form_needs_its_call_number_before_the_row_kernel_starts():
+    """Lines: the row kernel advances the number before it waits for data, so a GEMM thread that reads it after the
+    release may stamp its lines with the next call's.  Flags: the number advances when all flags have been seen."""
+    assert simulate_local(lines=1, rows=8, row_ctas=8, slow_cta=1)[0] == 0
+    rc, rep = simulate_local(lines=1, rows=8, row_ctas=8, slow_cta=1, late_number=1, timeout_ms=2000)
+    assert rc == 2 and rep.timeouts >= 1
+    assert simulate_local(lines=0, rows=8, row_ctas=8, slow_cta=1, late_number=1)[0] == 0
+
+
+def test_local_form_lost_item_times_out():
+    for lines in (0, 1):
+        rc, rep = simulate_local(lines=lines, fault=1, fault_call=2, timeout_ms=300)
+        assert rc == 2 and rep.timeouts >= 1

@@ -42,6 +42,7 @@ LIB_SOURCES = [
     "ops/yali_api.cc",
     "sim/protocol_sim.cc",
     "sim/gemm_protocol_sim.cc",
+    "sim/local_gemm_sim.cc",
     "ops/fused_linear.cc",
     "ops/host_pipeline.cc",
     "capi/yali_c.cc",

@@ -42,6 +42,13 @@ class FusedSimConfig(ctypes.Structure):
                 ("in_switch", ctypes.c_int), ("ksplit", ctypes.c_int)]
 
 
+class LocalSimConfig(ctypes.Structure):
+    _fields_ = [(n, ctypes.c_int) for n in ("pairs", "row_ctas", "calls")] + \
+               [(n, ctypes.c_uint32) for n in ("rows", "col_units", "splits", "tile_rows")] + \
+               [(n, ctypes.c_int) for n in ("lines", "slow_cta", "late_number", "reset_at", "keep_lines", "fault", "fault_call",
+                                            "timeout_ms")]
+
+
 class SimReport(ctypes.Structure):
     _fields_ = [("status", ctypes.c_int), ("mismatches", ctypes.c_uint64), ("timeouts", ctypes.c_uint64),
                 ("max_outstanding_slots", ctypes.c_uint64), ("flag_writes", ctypes.c_uint64),
@@ -96,6 +103,7 @@ def _declare(lib: ctypes.CDLL) -> None:
                                               c.POINTER(c.c_size_t)]),
         "yali_c_simulate": (i32, [c.POINTER(SimConfig), c.POINTER(SimReport)]),
         "yali_c_simulate_fused": (i32, [c.POINTER(FusedSimConfig), c.POINTER(SimReport)]),
+        "yali_c_simulate_local": (i32, [c.POINTER(LocalSimConfig), c.POINTER(SimReport)]),
     }
     for name, (res, args) in sig.items():
         fn = getattr(lib, name)
