@@ -815,9 +815,15 @@ Result Communicator::Reset() {
     YALI_NVTX_RANGE("yali::Reset");
     Result r = Barrier();
     if (r != Result::Success) return r;
+    // The call numbers start again, so the flag-in-data lines of the calls so far have to go with the control words: a
+    // line counts as arrived when it carries the call's number, and the numbers are about to be handed out a second time.
+    const uint64_t w = static_cast<uint64_t>(world_);
     for (const Local& l : local_) {
         cudaSetDevice(l.device);
-        if (cudaMemset(heaps_->base(l.rank) + lay_.flags_off, 0, kFlagRegionBytes) != cudaSuccess ||
+        char* const base = heaps_->base(l.rank);
+        if (cudaMemset(base + lay_.flags_off, 0, kFlagRegionBytes) != cudaSuccess ||
+            cudaMemset(base + lay_.ll_off, 0, 2 * (w - 1) * 2 * lay_.ll_cap) != cudaSuccess ||
+            cudaMemset(base + lay_.gemm_ll_off, 0, 2 * w * lay_.gemm_ll_cap) != cudaSuccess ||
             cudaDeviceSynchronize() != cudaSuccess)
             return Fail(Result::CudaError, "clearing the flag region failed");
         std::memset(l.status, 0, sizeof(DeviceStatus));

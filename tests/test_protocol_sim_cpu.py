@@ -274,6 +274,16 @@ def test_local_form_needs_its_call_number_before_the_row_kernel_starts():
     assert simulate_local(lines=0, rows=8, row_ctas=8, slow_cta=1, late_number=1)[0] == 0
 
 
+def test_local_form_after_a_reset_of_the_call_number():
+    # The numbers start again in front of call 1: the lines of call 0 must go with them, flags are control words anyway.
+    for lines in (0, 1):
+        rc, rep = simulate_local(lines=lines, rows=8, row_ctas=8, slow_cta=1, reset_at=1)
+        assert rc == 0, (lines, rc, rep.mismatches)
+    # Negative control: the row kernel takes call 0's lines for call 1's while the GEMM is late.
+    hits = sum(simulate_local(lines=1, rows=8, row_ctas=8, slow_cta=1, reset_at=1, keep_lines=1)[0] == 1 for _ in range(3))
+    assert hits >= 1
+
+
 def test_local_form_lost_item_times_out():
     for lines in (0, 1):
         rc, rep = simulate_local(lines=lines, fault=1, fault_call=2, timeout_ms=300)
