@@ -551,6 +551,10 @@ Result Communicator::Collective(const void* const* send, void* const* recv, uint
         const int vec = 16 / static_cast<int>(DtypeSize(in));
         norm_ok = in == out && opt.hidden > 0 && count % opt.hidden == 0 && opt.hidden % vec == 0 &&
                   opt.hidden / vec <= 4 * kFlashThreads && opt.weight && caps.vec_ok;
+        // The row kernels take all of a row's tensors in 16-byte units.
+        for (int i = 0; norm_ok && i < nlocal(); ++i)
+            norm_ok = Aligned16(opt.weight[i]) && (!opt.residual || Aligned16(opt.residual[i])) &&
+                      (!opt.residual_out || Aligned16(opt.residual_out[i]));
     }
     Plan plan;
     std::string why;

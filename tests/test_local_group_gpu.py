@@ -97,6 +97,20 @@ def test_norm(comm, dtype, rows, hidden):
         torch.testing.assert_close(xs[0].double(), ys[0].double(), rtol=2 * rtol, atol=1e-6)
 
 
+@pytest.mark.parametrize("odd", ["x", "weight", "residual", "out", "residual_out"])
+@pytest.mark.parametrize("mode", ["auto", "flash"])
+def test_norm_refuses_tensors_off_a_16_byte_boundary(comm, odd, mode):
+    """One rank's tensor starts at an odd element: an error of the call, before any launch."""
+    W, rows, hidden = comm.world, 4, 1024
+    off = {r: {odd: 1} if r == W - 1 else {} for r in range(W)}
+    t = {k: [whole((rows, hidden) if k != "weight" else (hidden,), BF16, r, off[r].get(k, 0)) for r in range(W)]
+         for k in ("x", "weight", "residual", "out", "residual_out")}
+    before = comm.launches
+    with pytest.raises(RuntimeError, match="16-byte aligned"):
+        comm.all_reduce_rmsnorm(t["x"], t["weight"], t["residual"], out=t["out"], residual_out=t["residual_out"], mode=mode)
+    assert comm.launches == before
+
+
 def test_halves_of_the_multi_gpu_kernel_on_request(comm, monkeypatch):
     if comm.world == 1:
         pytest.skip("a group of one has no halves")
