@@ -118,6 +118,7 @@ __device__ __forceinline__ void direct_body(const CollArgs& a, uint32_t cta) {
                     }
                 }
             }
+            mbar_drain_ring(full_bar, stages, it);  // also when the consumers stop early
         }
     } else {
         // ---------------------------------------------------------------- consumers
@@ -181,8 +182,7 @@ __device__ __forceinline__ void direct_body(const CollArgs& a, uint32_t cta) {
             if (lane == 0) ptx::mbar_arrive(&empty_bar[s]);
         }
     }
-    // Every stage that was filled has been consumed here (a consumer only leaves its loop early
-    // after a wait that ran out), so no bulk copy is in flight past this point.
+    // The producer has waited for its copies, so none is in flight past this point.
     __syncthreads();
     if (s_abort) return;
     // Peers have read this rank's input and their stores into this rank's output are visible.

@@ -78,6 +78,7 @@ __device__ __forceinline__ void decode_body(const GemmDecodeArgs& a, const CUten
                                             const CUtensorMap* tmap_b, uint32_t cta, uint32_t nctas) {
     extern __shared__ uint8_t smem_raw[];
     __shared__ __align__(8) uint64_t full_bar[kDMaxStages], empty_bar[kDMaxStages], tmem_full_bar[2], tmem_empty_bar[2];
+    __shared__ __align__(8) uint64_t drain_bar;  // all MMAs have finished
     __shared__ __align__(16) uint4 s_lines[kDEpilogueWarps][32 * 8];  // per epilogue warp: 32 rows x 8 lines, swizzled
     __shared__ uint32_t s_tmem;
     __shared__ int s_abort;
@@ -110,6 +111,7 @@ __device__ __forceinline__ void decode_body(const GemmDecodeArgs& a, const CUten
             ptx::mbar_init(&tmem_full_bar[b], 1);
             ptx::mbar_init(&tmem_empty_bar[b], kDEpilogueWarps);
         }
+        ptx::mbar_init(&drain_bar, 1);
         ptx::mbar_fence_init();
         ptx::tma_prefetch_desc(tmap_a);
         ptx::tma_prefetch_desc(tmap_b);
@@ -165,6 +167,7 @@ __device__ __forceinline__ void decode_body(const GemmDecodeArgs& a, const CUten
                     if (++s == stages) s = 0, ++round;
                 }
             }
+            mbar_drain_ring(full_bar, stages, round * stages + s);  // also when the MMAs stop early
         }
     } else if (warp == 3) {
         if (ptx::elect_one()) {
@@ -199,6 +202,8 @@ __device__ __forceinline__ void decode_body(const GemmDecodeArgs& a, const CUten
                 if (*abort_flag) break;
                 ptx::tc_commit(&tmem_full_bar[b]);
             }
+            ptx::tc_commit(&drain_bar);
+            mbar_drain(&drain_bar, 0, ptx::globaltimer() + kDrainNs);
         }
     } else if ((warp & 3) < 2) {
         const int q = warp & 3;   // TMEM lane quarter this warp may read

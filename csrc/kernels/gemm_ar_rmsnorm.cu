@@ -136,6 +136,7 @@ __device__ __forceinline__ Item item_at(const GemmArArgs& a, uint32_t i, uint32_
 struct Shared {
     __align__(8) uint64_t full_bar[kMaxStages], empty_bar[kMaxStages], tmem_full_bar[2], tmem_empty_bar[2];
     __align__(8) uint64_t pushed_bar[2], announced_bar[2];  // epilogue warps -> announcer warp and back
+    __align__(8) uint64_t drain_bar;  // all MMAs have finished
     __align__(8) uint64_t row_full[kRowGroups][kMaxRowSlots], row_empty[kRowGroups][kMaxRowSlots];
     uint32_t tmem;
     char* heap[kMaxRanks];  // the heap bases: read with a run-time rank
@@ -213,10 +214,10 @@ __device__ __forceinline__ void row_producer(const GemmArArgs& a, Shared& s, uin
         ptx::fence_proxy_async();
         const char* const part = landing + static_cast<uint64_t>(lr) * rowbytes;
         for (uint32_t k = 0; k < max(m.chunks, 1u); ++k) {
-            const bool got = wait_bar(&empty[slot], (round & 1u) ^ 1u, deadline, &s.abort);
-            if (__any_sync(0xffffffffu, !got)) {
+            late = !wait_bar(&empty[slot], (round & 1u) ^ 1u, deadline, &s.abort);
+            if (__any_sync(0xffffffffu, late)) {
                 s.abort = 1;
-                return;
+                break;
             }
             if (ptx::elect_one()) {
                 if (m.chunks == 0) {
@@ -236,7 +237,13 @@ __device__ __forceinline__ void row_producer(const GemmArArgs& a, Shared& s, uin
         rounds[0] = group ? rounds[0] : round;
         slots[1] = group ? slot : slots[1];
         rounds[1] = group ? round : rounds[1];
+        if (__any_sync(0xffffffffu, late)) break;
     }
+    // Nothing is under way when this CTA leaves, also when the row warps stop early.
+    if (ptx::elect_one())
+        for (uint32_t g = 0; g < static_cast<uint32_t>(kRowGroups); ++g)
+            mbar_drain_ring(s.row_full[g], m.slots, g ? rounds[1] * m.slots + slots[1] : rounds[0] * m.slots + slots[0]);
+    __syncwarp();
 }
 
 // The four warps of row group `group`: every second of this CTA's rows (two groups, because a row is a chain of latencies:
@@ -380,6 +387,7 @@ __device__ __forceinline__ void gemm_ar_body(const GemmArArgs& a, uint32_t cta, 
             ptx::mbar_init(&s.pushed_bar[b], kEpilogueWarps);
             ptx::mbar_init(&s.announced_bar[b], 1);
         }
+        ptx::mbar_init(&s.drain_bar, 1);
         for (int i = 0; i < kRowGroups * kMaxRowSlots; ++i) {
             ptx::mbar_init(&s.row_full[0][0] + i, 1);
             ptx::mbar_init(&s.row_empty[0][0] + i, kRowWarps);
@@ -442,10 +450,21 @@ __device__ __forceinline__ void gemm_ar_body(const GemmArArgs& a, uint32_t cta, 
             }
             // The MMAs' releases of the last stages arrive here from the leader: none may be under way when this CTA
             // leaves.
-            for (uint32_t k = 0; k < stages && !s.abort; ++k) {
-                if (!wait_bar(&s.empty_bar[st], (round & 1u) ^ 1u, deadline, &s.abort)) s.abort = 1;
+            bool up = !s.abort;
+            const uint32_t loaded = round * stages + st;
+            for (uint32_t k = 0; k < stages && up; ++k) {
+                up = wait_bar(&s.empty_bar[st], (round & 1u) ^ 1u, deadline, &s.abort);
                 if (++st == stages) st = 0, ++round;
             }
+            if (!up) {
+                // The time ran out in mid-work.  The leader's barriers count the loads of both CTAs; what this one
+                // has issued beyond the leader, nobody counts.
+                s.abort = 1;
+                if (half == 0) mbar_drain_ring(s.full_bar, stages, loaded);
+                else
+                    for (const uint64_t until = ptx::globaltimer() + kDrainNs; ptx::globaltimer() < until;) ptx::nanosleep(1000);
+            }
+            mbar_drain(&s.drain_bar, 0, ptx::globaltimer() + kDrainNs);
         }
     } else if (warp == kMmaWarp) {
         if (half == 0 && ptx::elect_one()) {
@@ -483,6 +502,8 @@ __device__ __forceinline__ void gemm_ar_body(const GemmArArgs& a, uint32_t cta, 
                 ptx::tc_commit_pair(&s.tmem_full_bar[b]);  // accumulator complete
                 ++n;
             }
+            ptx::tc_commit_pair(&s.drain_bar);
+            mbar_drain(&s.drain_bar, 0, ptx::globaltimer() + kDrainNs);
         }
     } else if (warp == kAnnounceWarp) {
         // When the eight epilogue warps have issued the pushes of a tile unit, tell every owner of rows of it.

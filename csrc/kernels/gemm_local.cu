@@ -91,6 +91,7 @@ __device__ __forceinline__ bool item_at(const LocalGemmArgs& a, uint32_t k, uint
 struct Shared {
     __align__(8) uint64_t full_bar[kMaxStages], empty_bar[kMaxStages], tmem_full_bar[2], tmem_empty_bar[2];
     __align__(8) uint64_t stored_bar[2], announced_bar[2];  // epilogue warps -> announcer warp and back
+    __align__(8) uint64_t drain_bar;  // all MMAs have finished
     uint32_t tmem, epoch;      // epoch: this call's number
     volatile uint32_t loaded;  // k-blocks whose loads have been issued
     volatile int abort;
@@ -131,6 +132,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kLocalGemmThreads, 1
             ptx::mbar_init(&s.stored_bar[b], kEpilogueWarps);
             ptx::mbar_init(&s.announced_bar[b], 1);
         }
+        ptx::mbar_init(&s.drain_bar, 1);
         ptx::mbar_fence_init();
         ptx::tma_prefetch_desc(&a.tmap_w[0]);
         ptx::tma_prefetch_desc(&a.tmap_x[0]);
@@ -181,10 +183,20 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kLocalGemmThreads, 1
             s.loaded = 0x7fffffffu;  // nothing left to run ahead of
             // The MMAs' releases of the last stages arrive here from the leader: none may be under way when this CTA
             // leaves.
-            for (uint32_t k = 0; k < stages && !s.abort; ++k) {
-                if (!wait_bar(&s.empty_bar[st], (round & 1u) ^ 1u, deadline, &s.abort)) s.abort = 1;
+            bool up = !s.abort;
+            for (uint32_t k = 0; k < stages && up; ++k) {
+                up = wait_bar(&s.empty_bar[st], (round & 1u) ^ 1u, deadline, &s.abort);
                 if (++st == stages) st = 0, ++round;
             }
+            if (!up) {
+                // The time ran out in mid-work.  The leader's barriers count the loads of both CTAs; what this one
+                // has issued beyond the leader, nobody counts.
+                s.abort = 1;
+                if (half == 0) mbar_drain_ring(s.full_bar, stages, loaded);
+                else
+                    for (const uint64_t until = ptx::globaltimer() + kDrainNs; ptx::globaltimer() < until;) ptx::nanosleep(1000);
+            }
+            mbar_drain(&s.drain_bar, 0, ptx::globaltimer() + kDrainNs);
         }
     } else if (warp == kMmaWarp) {
         if (half == 0 && ptx::elect_one()) {
@@ -219,6 +231,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kLocalGemmThreads, 1
                 if (s.abort) break;
                 ptx::tc_commit_pair(&s.tmem_full_bar[b]);  // accumulator complete
             }
+            ptx::tc_commit_pair(&s.drain_bar);
+            mbar_drain(&s.drain_bar, 0, ptx::globaltimer() + kDrainNs);
         }
     } else if (warp == kAnnounceWarp) {
         // When the epilogue warps have stored their part of a unit: publish the call number in its flag.  The release orders
@@ -432,7 +446,7 @@ __global__ void __launch_bounds__(kLocalLinearNormThreads, LocalLinearNormPlaces
             }
             ready = tile;
         }
-        if (__syncthreads_or(late)) return;
+        if (__syncthreads_or(late)) break;
         if (taking) {
             unit = s_next;
             if (unit < units) {
@@ -554,7 +568,7 @@ __global__ void __launch_bounds__(kLocalLinearNormThreads, LocalLinearNormPlaces
             if ((tid & 31) == 0) s_red[g][tid >> 5] = ss;
         }
         if (LINES) {
-            if (__syncthreads_or(late)) return;
+            if (__syncthreads_or(late)) break;
         } else {
             __syncthreads();
         }
@@ -580,7 +594,7 @@ __global__ void __launch_bounds__(kLocalLinearNormThreads, LocalLinearNormPlaces
             }
         }
     }
-    // The call is over when both kernels are.
+    // The call is over when both kernels are, also when a wait ran out here.
     ptx::grid_dependency_wait();
 }
 

@@ -81,3 +81,42 @@ def test_fused_layer_of_few_rows_after_reset(world, form):
                 want = sum(x[:, :1].double() for x in xs).expand(T, N)
                 assert all(torch.equal(p.double(), want) for p in pre)
                 comm.reset()
+
+
+@pytest.mark.parametrize("form", [{}, {"oneshot": False}])
+def test_time_limit_in_the_middle_of_a_fused_layer(form):
+    """A call that takes longer than the limit: the GEMM's waits run out while its copies and MMAs are under way.  The call
+    ends with an error, and what runs on the same SMs afterwards is right."""
+    world = 8
+    T, K, N = 4096, 16384, 4096  # 2.7 ms at the tensor cores' rate
+    big_x, big_w = (torch.ones(n, K, dtype=torch.bfloat16, device="cuda:0") for n in (T, N))
+    with yali.Comm.emulated(world, device=0, timeout_ms=1) as comm:
+        for turn in range(3):
+            nw = [torch.ones(N, dtype=torch.bfloat16, device="cuda:0")] * world
+            comm.fused_linear_rmsnorm([big_x] * world, [big_w] * world, nw, None, **form)
+            with pytest.raises(YaliTimeout):
+                comm.sync()
+            comm.reset()
+            for k in (64, 1024):
+                x = [torch.randint(-1, 2, (8, k), device="cuda:0").to(torch.bfloat16) for _ in range(world)]
+                w = [torch.eye(N, k, dtype=torch.bfloat16, device="cuda:0")] * world
+                pre = [torch.empty(8, N, dtype=torch.bfloat16, device="cuda:0") for _ in range(world)]
+                comm.fused_linear_rmsnorm(x, w, nw, None, residual_out=pre, **form)
+                comm.sync()
+                want = torch.nn.functional.pad(sum(t.double() for t in x), (0, N - k))
+                assert all(torch.equal(p.double(), want) for p in pre)
+
+
+def test_time_limit_in_the_middle_of_a_pipelined_all_reduce():
+    n = 1 << 29  # 8.6 GB in and out: 1.3 ms at least
+    with yali.Comm.emulated(2, device=0, timeout_ms=1) as comm:
+        xs = [torch.ones(n, device="cuda:0") for _ in range(2)]
+        ys = [torch.empty_like(x) for x in xs]
+        for turn in range(3):
+            comm.all_reduce(xs, ys, mode="stream_direct")
+            with pytest.raises(YaliTimeout):
+                comm.sync()
+            comm.reset()
+            small = comm.all_reduce([x[:300000] for x in xs], mode="stream_direct")
+            comm.sync()
+            assert all(torch.equal(t, torch.full_like(t, 2.0)) for t in small)
