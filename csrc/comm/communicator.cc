@@ -700,6 +700,9 @@ bool Communicator::AllReduceMapped(const void* const* send, void* const* recv, u
         env::ForcedKernelMode() != KernelMode::Auto || opt.ctas > 0 || opt.slot_bytes > 0 ||
         opt.epilogue == kEpiResidualRmsNorm || count > (1ull << 40))
         return false;
+    // A tuning table with anything for this group and type names the kernel that reduces the chunks.
+    const TuningTable* const table = EnvTuningTable();
+    if (table && table->Find(world_, static_cast<int>(DtypeSize(dt)), 1)) return false;
     const uint64_t bytes = count * DtypeSize(dt);
     if (!CanRunInOneLaunch(send, recv, bytes, bytes, 0, dt, dt, opt, 0)) return false;
     const void* s[kMaxRanks];

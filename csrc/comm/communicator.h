@@ -91,7 +91,8 @@ class Communicator {
     Result AllReduce(const void* const* send, void* const* recv, uint64_t count, Dtype in, Dtype out,
                      const OpOptions& opt, const cudaStream_t* streams);
     // The same between page-locked host buffers, read and written by one kernel where they are.  False: this call cannot be
-    // done so (several GPUs, a forced mode, memory that the GPU cannot address); otherwise *r is its result.
+    // done so (several GPUs, a forced mode, a tuning table for the group, memory that the GPU cannot address); otherwise
+    // *r is its result.
     bool AllReduceMapped(const void* const* send, void* const* recv, uint64_t count, Dtype dt, const OpOptions& opt,
                          const cudaStream_t* streams, Result* r);
     // recv (ShardElems(count, world) elements, of which the valid part is used) = this rank's shard of the sum.

@@ -1,6 +1,11 @@
 """Automatically chosen calls of a group whose ranks share one GPU run in one launch that exchanges nothing
 (csrc/kernels/local_group.cu).  Inputs are small whole numbers, so every sum is exact in every type and results
 are compared bit by bit; sizes sit at the edges of the 16-byte units, CTAs (512 units) and shards."""
+import json
+import os
+import subprocess
+import sys
+
 import pytest
 import torch
 
@@ -146,6 +151,25 @@ def test_host_buffers_where_they_are(comm, dtype, n):
     assert all(torch.equal(s.double(), want * 2) for s in src)
     with pytest.raises(ValueError):
         comm.all_reduce_host([torch.zeros(8) for _ in range(W)])
+
+
+@pytest.mark.parametrize("row_world", [2, 4])
+def test_host_buffers_with_a_tuning_table(tmp_path, row_world):
+    """A table for the group names the kernel, for pinned host memory as well; one for another group changes nothing."""
+    table = tmp_path / "table.json"
+    table.write_text(json.dumps({"rows": [{"world": row_world, "elem_bytes": 4, "max_bytes": 1 << 40, "variant": "stream",
+                                           "ctas": 8, "slot_bytes": 4096}]}))
+    code = ("import torch, yali_b200 as yali\n"
+            "c = yali.Comm.emulated(2, device=0)\n"
+            "s = [torch.full((5000,), r + 1.0).pin_memory() for r in range(2)]\n"
+            "d = c.all_reduce_host(s)\n"
+            "torch.cuda.synchronize(); c.check()\n"
+            "assert all(torch.equal(t, torch.full_like(t, 3.0)) for t in d)\n"
+            "l = c.last_call(); print(l['variant'], bool(l['flags'] & 1 << 9))\n")
+    p = subprocess.run([sys.executable, "-c", code], env=dict(os.environ, YALI_TUNING_FILE=str(table)), capture_output=True,
+                       text=True, timeout=300)
+    assert p.returncode == 0, p.stderr
+    assert p.stdout.split() == (["stream", "False"] if row_world == 2 else ["flash", "True"])
 
 
 @pytest.mark.parametrize("n", [1, 255, 256, 257, 524288, 524289])
