@@ -562,12 +562,13 @@ Result Communicator::Collective(const void* const* send, void* const* recv, uint
     if (mode == KernelMode::Auto && norm_ok &&
         CanRunInOneLaunch(send, recv, send_bytes, recv_bytes, shard * DtypeSize(in), in, out, opt, extra_flags)) {
         caps.one_launch = true;
-        r = MakePlan(world_, count, in, out, opt.epilogue, mode, caps, EnvTuningTable(), &plan, &why);
-        if (r != Result::Success) return Fail(r, why);
-        if (plan.flags & kFlagOneLaunch) {
+        if (MakePlan(world_, count, in, out, opt.epilogue, mode, caps, EnvTuningTable(), &plan, &why) == Result::Success &&
+            (plan.flags & kFlagOneLaunch)) {
             plan.flags |= extra_flags | (trace_ ? static_cast<uint32_t>(kFlagTrace) : 0u);
             return LaunchLocal(plan, send, recv, count, in, out, opt, streams);
         }
+        // A geometry of the caller's or a row of the tuning table asks for a multi-GPU kernel.  What those can do with
+        // this call is not known yet: it is planned again below.
         caps.one_launch = false;
     }
 

@@ -153,9 +153,33 @@ def test_host_buffers_where_they_are(comm, dtype, n):
         comm.all_reduce_host([torch.zeros(8) for _ in range(W)])
 
 
+@pytest.mark.parametrize("n", [8, 40001, 1 << 20])
+def test_a_geometry_of_the_caller_runs_the_multi_gpu_kernels(comm, n):
+    """`ctas` and `slot_bytes` without a mode: accepted by every collective, and nothing of them is dropped."""
+    W = comm.world
+    if W == 1:
+        pytest.skip("a group of one has the one-shot kernel only")
+    xs = [whole((n,), F32, n + r) for r in range(W)]
+    for kw in ({"ctas": 4}, {"slot_bytes": 2048}, {"ctas": 3, "slot_bytes": 4096}):
+        ys = comm.all_reduce(xs, **kw)
+        assert not comm.last_call()["flags"] & ONE_LAUNCH
+        full = comm.all_gather(comm.reduce_scatter(xs, **kw), n, **kw)
+        last = comm.last_call()
+        assert last["variant"] == "stream" and last["ctas"] <= kw.get("ctas", 1 << 30)
+        assert last["slot_bytes"] == kw.get("slot_bytes", last["slot_bytes"])
+        comm.sync()
+        assert all(torch.equal(t.double(), total(xs)) for t in ys + full)
+    x, w = [t[:8].view(1, 8) for t in xs], [torch.ones(8, device="cuda")] * W
+    y = comm.all_reduce_rmsnorm(x, w, ctas=1)
+    assert not comm.last_call()["flags"] & ONE_LAUNCH
+    comm.sync()
+    row = total(x)
+    torch.testing.assert_close(y[0].double(), row * torch.rsqrt(row.pow(2).mean(-1, keepdim=True) + 1e-5), rtol=4e-6, atol=1e-6)
+
+
 @pytest.mark.parametrize("row_world", [2, 4])
-def test_host_buffers_with_a_tuning_table(tmp_path, row_world):
-    """A table for the group names the kernel, for pinned host memory as well; one for another group changes nothing."""
+def test_calls_with_a_tuning_table(tmp_path, row_world):
+    """A table for the group names the kernel, on the device and for pinned host memory; one for another group changes nothing."""
     table = tmp_path / "table.json"
     table.write_text(json.dumps({"rows": [{"world": row_world, "elem_bytes": 4, "max_bytes": 1 << 40, "variant": "stream",
                                            "ctas": 8, "slot_bytes": 4096}]}))
@@ -165,11 +189,14 @@ def test_host_buffers_with_a_tuning_table(tmp_path, row_world):
             "d = c.all_reduce_host(s)\n"
             "torch.cuda.synchronize(); c.check()\n"
             "assert all(torch.equal(t, torch.full_like(t, 3.0)) for t in d)\n"
+            "l = c.last_call(); print(l['variant'], bool(l['flags'] & 1 << 9))\n"
+            "d = c.all_reduce([t.cuda() for t in s])\n"
+            "c.sync(); assert all(torch.equal(t, torch.full_like(t, 3.0)) for t in d)\n"
             "l = c.last_call(); print(l['variant'], bool(l['flags'] & 1 << 9))\n")
     p = subprocess.run([sys.executable, "-c", code], env=dict(os.environ, YALI_TUNING_FILE=str(table)), capture_output=True,
                        text=True, timeout=300)
     assert p.returncode == 0, p.stderr
-    assert p.stdout.split() == (["stream", "False"] if row_world == 2 else ["flash", "True"])
+    assert p.stdout.split() == 2 * (["stream", "False"] if row_world == 2 else ["flash", "True"])
 
 
 @pytest.mark.parametrize("n", [1, 255, 256, 257, 524288, 524289])
