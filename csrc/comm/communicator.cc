@@ -711,15 +711,22 @@ bool Communicator::AllReduceMapped(const void* const* send, void* const* recv, u
     Plan plan;
     plan.variant = Variant::Flash;
     plan.flags = kFlagOneLaunch | kFlagHostMemory | kFlagVecOk | (trace_ ? static_cast<uint32_t>(kFlagTrace) : 0u);
-    for (int i = 0; i < nlocal(); ++i) {
-        cudaPointerAttributes a, b;
-        if (cudaPointerGetAttributes(&a, send[i]) != cudaSuccess || cudaPointerGetAttributes(&b, recv[i]) != cudaSuccess ||
-            !a.devicePointer || !b.devicePointer) {
+    // Where the GPU sees a buffer.  Its last byte counts, too: a buffer that is registered in part is no error for a copy,
+    // which the driver checks, but would be one for a kernel.
+    auto mapped = [&](const void* p) -> void* {
+        cudaPointerAttributes first, last;
+        if (cudaPointerGetAttributes(&first, p) != cudaSuccess ||
+            cudaPointerGetAttributes(&last, static_cast<const char*>(p) + bytes - 1) != cudaSuccess) {
             (void)cudaGetLastError();
-            return false;
+            return nullptr;
         }
-        s[i] = a.devicePointer;
-        d[i] = b.devicePointer;
+        return first.devicePointer && last.devicePointer == static_cast<char*>(first.devicePointer) + bytes - 1 ? first.devicePointer
+                                                                                                                : nullptr;
+    };
+    for (int i = 0; i < nlocal(); ++i) {
+        s[i] = mapped(send[i]);
+        d[i] = mapped(recv[i]);
+        if (!s[i] || !d[i]) return false;
         if (!Aligned16(s[i]) || !Aligned16(d[i])) plan.flags &= ~static_cast<uint32_t>(kFlagVecOk);
     }
     *r = LaunchLocal(plan, s, d, count, dt, dt, opt, streams);

@@ -2,6 +2,7 @@
 (csrc/kernels/local_group.cu).  Inputs are small whole numbers, so every sum is exact in every type and results
 are compared bit by bit; sizes sit at the edges of the 16-byte units, CTAs (512 units) and shards."""
 import json
+import mmap
 import os
 import subprocess
 import sys
@@ -151,6 +152,29 @@ def test_host_buffers_where_they_are(comm, dtype, n):
     assert all(torch.equal(s.double(), want * 2) for s in src)
     with pytest.raises(ValueError):
         comm.all_reduce_host([torch.zeros(8) for _ in range(W)])
+
+
+@pytest.mark.parametrize("which", ["src", "dst"])
+def test_host_buffers_that_are_registered_in_part(which):
+    """The first half of one buffer is registered, so it passes for pinned memory: the kernel must not be given it."""
+    cudart, n = torch.cuda.cudart(), 1 << 20
+    with yali.Comm.emulated(2, device=0) as c:
+        part = torch.frombuffer(mmap.mmap(-1, n * 4), dtype=torch.float32).fill_(1)
+        bufs = {k: [torch.ones(n).pin_memory() for _ in range(2)] for k in ("src", "dst")}
+        bufs[which][1] = part
+        assert int(cudart.cudaHostRegister(part.data_ptr(), n * 2, 0)) == 0
+        try:
+            assert part.is_pinned()
+            try:
+                c.all_reduce_host(bufs["src"], bufs["dst"])
+            except RuntimeError:
+                pass  # the copies may refuse it
+            torch.cuda.synchronize()
+            assert not c.last_call()["flags"] & 1 << 10
+        finally:
+            assert int(cudart.cudaHostUnregister(part.data_ptr())) == 0
+        ok = [torch.ones(n).pin_memory() for _ in range(2)]
+        assert torch.equal((c.all_reduce_host(ok), torch.cuda.synchronize())[0][1], torch.full((n,), 2.0))
 
 
 @pytest.mark.parametrize("n", [8, 40001, 1 << 20])
