@@ -154,6 +154,34 @@ def test_host_buffers_where_they_are(comm, dtype, n):
         comm.all_reduce_host([torch.zeros(8) for _ in range(W)])
 
 
+def test_any_iterable_of_tensors_will_do(comm):
+    """One tensor per rank from a generator, a tuple or a dict's values, for every argument of every call."""
+    W = comm.world
+    it = lambda ts: (t for t in ts)  # noqa: E731
+    x, y = [whole((4, 128), BF16, r) for r in range(W)], [torch.empty(4, 128, dtype=BF16, device="cuda") for _ in range(W)]
+    w, res = [torch.ones(128, dtype=BF16, device="cuda") for _ in range(W)], [whole((4, 128), BF16, 9) for _ in range(W)]
+    for out in (None, y):
+        got = comm.all_reduce(it(x), None if out is None else it(out))
+        assert all(torch.equal(t.double(), total(x)) for t in got)
+        assert out is None or all(t is o for t, o in zip(got, out))
+        pre = [torch.empty_like(t) for t in x]
+        got = comm.all_reduce_rmsnorm(it(x), tuple(w), it(res), out=out and it(out), residual_out=it(pre))
+        assert len(got) == W and all(torch.equal(p.double(), total(x) + r.double()) for p, r in zip(pre, res))
+        full = comm.all_gather(it(comm.reduce_scatter(it(x))), 512, None if out is None else it(out))
+        assert all(torch.equal(t.double().view(4, 128), total(x)) for t in full)
+        if W > 1:
+            k = [torch.eye(128, dtype=BF16, device="cuda") for _ in range(W)]
+            got = comm.fused_linear_rmsnorm(it(x), dict(enumerate(k)).values(), it(w), it(res), out=out and it(out), residual_out=it(pre))
+            assert len(got) == W and all(torch.equal(p.double(), total(x) + r.double()) for p, r in zip(pre, res))
+            assert out is None or all(t is o for t, o in zip(got, out))
+    src, dst = [t.cpu().pin_memory() for t in x], [t.cpu().pin_memory() for t in y]
+    for out in (None, dst):
+        got = comm.all_reduce_host(it(src), out and it(out))
+        torch.cuda.synchronize()
+        assert len(got) == W and all(torch.equal(t.double(), total(src)) for t in got)
+    comm.sync()
+
+
 @pytest.mark.parametrize("which", ["src", "dst"])
 def test_host_buffers_that_are_registered_in_part(which):
     """The first half of one buffer is registered, so it passes for pinned memory: the kernel must not be given it."""

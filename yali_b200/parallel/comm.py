@@ -145,6 +145,11 @@ class Comm:
         return ts
 
     @staticmethod
+    def _once(t):
+        """An argument that is looked at more than once: an iterator becomes a list."""
+        return t if t is None or isinstance(t, (torch.Tensor, list, tuple)) else list(t)
+
+    @staticmethod
     def _like_input(t: TensorOrList, out: List[torch.Tensor]):
         return out[0] if isinstance(t, torch.Tensor) else out
 
@@ -185,6 +190,7 @@ class Comm:
         multicast store; 1 and 2 need the multicast object and `out` from symm_empty().  `decode`: the
         few-token form (up to 64 rows: 128 x 256 tiles whose K extent is split over CTAs, partial rows sent to every rank as
         flag-in-data lines, every rank normalises all rows): None = by size, False = never, True = required."""
+        x, w, out = self._once(x), self._once(w), self._once(out)
         if out is None and self.nlocal == 1 and self.world > 1:
             # Symmetric memory is never freed piecemeal: keep ONE output per row width, large enough for the
             # most rows seen so far (grown by doubling, so a program that varies its token count holds at
@@ -219,6 +225,7 @@ class Comm:
         the caller's current stream waits for it.  Where one GPU holds all ranks and `chunk_bytes` is 0,
         one kernel reads and writes the host buffers directly instead.  `copies_only=True` leaves the
         collective out (dst = src through the device): the time that copies alone take."""
+        src, dst = self._once(src), self._once(dst)
         if dst is None:
             dst = [torch.empty_like(t).pin_memory() for t in self._as_list(src, "src")]
         try:
