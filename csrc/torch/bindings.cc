@@ -319,10 +319,19 @@ class PyComm {
                          : at::cuda::getCurrentCUDAStream(c().device_of(i)).stream();
         return t;
     }
+    // An argument that is no tensor; what does not convert is a TypeError, as for arguments that pybind11 converts.
+    template <typename T>
+    static T Cast(const py::object& o, const char* what) {
+        try {
+            return py::cast<T>(o);
+        } catch (const py::cast_error&) {
+            throw py::type_error(std::string(what) + ": cannot use an object of type " + Py_TYPE(o.ptr())->tp_name);
+        }
+    }
     static KernelMode ModeOf(const py::object& mode) {
         static PyObject* const auto_name = PyUnicode_InternFromString("auto");
         if (mode.ptr() == auto_name) return KernelMode::Auto;
-        return ToMode(py::cast<std::string>(mode));
+        return ToMode(Cast<std::string>(mode, "mode"));
     }
     void Finish(Result r) {
         if (r != Result::Success) Throw(r, c().last_error());
@@ -335,7 +344,8 @@ class PyComm {
         at::ScalarType sd, rd;
         int64_t sn, rn;
         Read(send.ptr(), "send", &s);
-        const at::ScalarType want = out_dtype.is_none() ? s[0].scalar_type() : py::cast<at::ScalarType>(out_dtype);
+        // (Outputs of the caller's have a type already.)
+        const at::ScalarType want = out_dtype.is_none() || !recv.is_none() ? s[0].scalar_type() : Cast<at::ScalarType>(out_dtype, "out_dtype");
         Out(recv.ptr(), "recv", s, s[0].sizes(), want, &r);
         CheckArgs(s, "send", &sd, &sn);
         CheckArgs(r.a, "recv", &rd, &rn);
@@ -347,7 +357,7 @@ class PyComm {
         o.skip_rank = skip_rank;
         if (!scale.is_none() || sd != rd) {
             o.epilogue = kEpiScaleCast;
-            o.scale = scale.is_none() ? 1.0f : static_cast<float>(py::cast<double>(scale));
+            o.scale = scale.is_none() ? 1.0f : static_cast<float>(Cast<double>(scale, "scale"));
         }
         const void* sp[kMaxRanks];
         void* rp[kMaxRanks];
@@ -418,6 +428,7 @@ class PyComm {
         int64_t sn, rn;
         Read(send.ptr(), "send", &s);
         const int64_t full = rs ? s[0].numel() : count;
+        TORCH_CHECK(full >= 0, "yali: count must not be negative, got ", full);
         const int64_t shard = c().world() > 1 ? static_cast<int64_t>(ShardElems(full, c().world())) : full;
         const int64_t size[1] = {rs ? shard : full};
         Out(recv.ptr(), "recv", s, c10::IntArrayRef(size, 1), s[0].scalar_type(), &r);
@@ -551,7 +562,7 @@ class PyComm {
         o.mode = ModeOf(mode);
         if (!scale.is_none()) {
             o.epilogue = kEpiScaleCast;
-            o.scale = static_cast<float>(py::cast<double>(scale));
+            o.scale = static_cast<float>(Cast<double>(scale, "scale"));
         }
         if (!host_pipe_) host_pipe_ = std::make_unique<HostPipeline>(c());
         const StreamTable st = CurrentStreams();

@@ -182,6 +182,25 @@ def test_any_iterable_of_tensors_will_do(comm):
     comm.sync()
 
 
+def test_arguments_of_the_wrong_type_are_type_errors(comm):
+    x, w = [whole((4, 128), BF16, r) for r in range(comm.world)], [torch.ones(128, dtype=BF16, device="cuda")] * comm.world
+    host = [t.cpu().pin_memory() for t in x]
+    before = comm.launches
+    for call in (lambda: comm.all_reduce(x, mode=None), lambda: comm.all_reduce(x, mode=3), lambda: comm.all_reduce(x, scale="2"),
+                 lambda: comm.all_reduce(x, out_dtype="fp32"), lambda: comm.all_reduce(3), lambda: comm.all_reduce(["x"] * comm.world),
+                 lambda: comm.all_reduce_rmsnorm(x, w, mode=None), lambda: comm.all_reduce_rmsnorm(x, w, eps="1"),
+                 lambda: comm.all_reduce_host(host, mode=None), lambda: comm.all_reduce_host(host, scale=x),
+                 lambda: comm.all_gather(x, "9")):
+        with pytest.raises(TypeError):
+            call()
+    with pytest.raises(RuntimeError, match="negative"):
+        comm.all_gather(x, -1)
+    assert comm.launches == before
+    y = [torch.empty_like(t) for t in x]
+    assert comm.all_reduce(x, y, out_dtype="not looked at")[0] is y[0]
+    comm.sync()
+
+
 @pytest.mark.parametrize("which", ["src", "dst"])
 def test_host_buffers_that_are_registered_in_part(which):
     """The first half of one buffer is registered, so it passes for pinned memory: the kernel must not be given it."""
