@@ -230,6 +230,12 @@ def run_own(args) -> dict:
     launches = time_steps.launches * (1 if emulated else ranks)  # every rank launches the same count
     variant = comm.last_call()
     ok = all(ext.validate_sum(t, torch.float32, 0, 1234, ranks)["mismatches"] == 0 for t in aslist(recv))
+    exchanging = None
+    if emulated:  # the kernel that several GPUs would run for this message, its ranks on the one GPU
+        ex_ms, _ = time_steps(comm, torch, lambda _i: comm.all_reduce(send, recv, mode="stream_direct"), args.steps,
+                              args.warmup, per_step_events=False)
+        exchanging = {"kernel": comm.last_call()["kernel"], "ms_per_step": round(ex_ms / args.steps, 5),
+                      "value": round(MESSAGE_BYTES * bus_factor(ranks) / (ex_ms / args.steps * 1e-3) / 1e9, 2)}
     ms_per_step = total_ms / args.steps
     busbw = MESSAGE_BYTES * bus_factor(ranks) / (ms_per_step * 1e-3) / 1e9
 
@@ -351,6 +357,7 @@ def run_own(args) -> dict:
                            "CONSTANT as N grows (the job reduces N x 128 MiB per step); the 1-GPU figure moves "
                            "no bytes over NVLink and is bound by HBM",
             "kernel": variant,
+            "exchanging_kernel_on_one_gpu": exchanging,
             "baseline": "reference README: 79.2 GB/s at 128 MB fp32 on 2x A100 NV4",
         },
         "latency_1MiB_us": {"p50": round(p50, 2), "p99": round(p99, 2),

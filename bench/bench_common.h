@@ -87,6 +87,7 @@ inline void Usage(const char* prog, const char* what) {
 
 // Kernel name of the result line ("YALI (Flash-fp32, ...)" in the reference's format).
 inline const char* KernelLabel(yali::Variant v, uint32_t flags) {
+    if (flags & yali::kFlagOneLaunch) return "OneLaunch";  // ranks on one GPU, no exchange
     switch (v) {
         case yali::Variant::Flash: return (flags & yali::kFlagLowLatency) ? "FlashLL" : "Flash";
         case yali::Variant::Stream: return "Stream";

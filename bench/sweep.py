@@ -162,7 +162,7 @@ def main() -> None:
                     raise
                 lc = comm.last_call()
                 row = {"impl": "yali_b200", "world": world, "dtype": dname, "bytes": size, "variant": var,
-                       "kernel": lc["variant"], "ctas": lc["ctas"], "slot_bytes": lc["slot_bytes"], "us": round(us, 2),
+                       "kernel": lc["kernel"], "ctas": lc["ctas"], "slot_bytes": lc["slot_bytes"], "us": round(us, 2),
                        "busbw_gbps": round(size * factor / us / 1e3, 2), "emulated": emu,
                        "timing": "graph" if size <= args.graph_max_bytes else "events"}
                 row.update(device_times(comm, iters))

@@ -476,6 +476,7 @@ Result Communicator::LaunchLocal(const Plan& plan, const void* const* send, void
     a.flags = plan.flags;
     a.ep.scale = opt.epilogue == kEpiScaleCast ? opt.scale : 1.0f;
     const void* fn = nullptr;
+    const char* name = "";
     dim3 grid(1), block(kLocalThreads);
     uint64_t blocks = 1;
     if (opt.epilogue == kEpiResidualRmsNorm) {
@@ -491,15 +492,18 @@ Result Communicator::LaunchLocal(const Plan& plan, const void* const* send, void
         const uint32_t vec = 16 / static_cast<uint32_t>(DtypeSize(in));
         const LocalNormShape s = LocalNormShapeFor(rows, static_cast<uint32_t>(opt.hidden) / vec, world_, sm_count_);
         fn = LocalNormKernelFor(in, world_, s);
+        name = "local_norm";
         block = dim3(s.threads);
         blocks = rows * ((world_ + s.ranks_per_cta - 1) / s.ranks_per_cta);
     } else if (plan.flags & kFlagHostMemory) {
         fn = LocalHostKernelFor(in, world_);
+        name = "local_host_sum";
         block = dim3(kLocalHostThreads);
         const uint64_t units = (plan.flags & kFlagVecOk) ? count * DtypeSize(in) / 16 + 1 : count;
         blocks = std::min<uint64_t>((units + kLocalHostThreads - 1) / kLocalHostThreads, kLocalHostCtas);
     } else {
         const bool rs = plan.flags & kFlagReduceScatterOnly, ag = plan.flags & kFlagAllGatherOnly;
+        name = rs ? "local_reduce_scatter" : ag ? "local_all_gather" : "local_sum";
         fn = LocalKernelFor(in, out, world_, rs ? LocalKind::ReduceScatter : ag ? LocalKind::AllGather : LocalKind::Sum);
         const uint64_t unit = 16 / std::min(DtypeSize(in), DtypeSize(out));
         const uint64_t span = rs || ag ? std::min(plan.shard_elems, count) : count;
@@ -513,6 +517,11 @@ Result Communicator::LaunchLocal(const Plan& plan, const void* const* send, void
     last_.ctas = grid.x * grid.y;
     last_.slot_bytes = last_.stages = 0;
     last_.flags = plan.flags;
+    last_.kernel = name;
+    static const int debug_level = env::DebugLevel();
+    if (debug_level > 1)
+        std::fprintf(stderr, "[yali] %s count=%llu ctas=%u flags=0x%x\n", name, static_cast<unsigned long long>(count), last_.ctas,
+                     plan.flags);
     void* params[] = {&a};
     cudaStream_t s = streams && streams[0] ? streams[0] : local_[0].stream;
     cudaError_t ce = LaunchInStream(fn, grid, block, params, 0, s);
@@ -660,6 +669,7 @@ Result Communicator::Collective(const void* const* send, void* const* recv, uint
     last_.slot_bytes = plan.slot_bytes;
     last_.stages = plan.stages;
     last_.flags = plan.flags;
+    last_.kernel = VariantName(plan.variant);
     static const int debug_level = env::DebugLevel();
     if (debug_level > 1 && local_[0].rank == 0)
         std::fprintf(stderr, "[yali] %s count=%llu ctas=%u slot=%u stages=%u flags=0x%x\n", VariantName(plan.variant),

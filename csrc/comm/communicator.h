@@ -58,6 +58,7 @@ struct LastCallInfo {
     uint32_t stages = 0;
     uint32_t flags = 0;
     uint64_t launches = 0;  // kernels launched by this process since creation
+    const char* kernel = "";  // what ran: the variant's name, or that of a kernel for ranks that share one GPU
 };
 
 class Communicator {

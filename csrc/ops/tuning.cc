@@ -287,7 +287,8 @@ Result MakePlan(int world, uint64_t count, Dtype in, Dtype out, int epilogue, Ke
                                                                  : nullptr;
     // All ranks in one launch on one GPU: the kernels of local_group.cu, which exchange nothing, at every
     // size (they measured ahead from 4 KiB to 128 MiB).  A forced mode or geometry and a tuning table ask for
-    // a multi-GPU kernel by name and get it.  The variant reported is the one whose place is taken.
+    // a multi-GPU kernel by name and get it.  The variant is the one whose place is taken;
+    // LastCallInfo::kernel says what ran.
     if (caps.one_launch && forced == KernelMode::Auto && !row && !caps.force_ctas && !caps.force_slot_bytes) {
         p.variant = caps.half_collective ? Variant::Stream
                     : world == 1 || bytes <= FlashCrossoverBytes(in, world) ? Variant::Flash : Variant::StreamDirect;

@@ -132,6 +132,7 @@ class PyComm {
         const LastCallInfo& l = c().last_call();
         py::dict d;
         d["variant"] = VariantName(l.variant);
+        d["kernel"] = l.kernel;
         d["ctas"] = l.ctas;
         d["slot_bytes"] = l.slot_bytes;
         d["stages"] = l.stages;

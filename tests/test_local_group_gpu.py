@@ -117,6 +117,25 @@ def test_norm_refuses_tensors_off_a_16_byte_boundary(comm, odd, mode):
     assert comm.launches == before
 
 
+def test_last_call_names_the_kernel_that_ran(comm):
+    W = comm.world
+    x, w = [whole((4, 1024), F32, r) for r in range(W)], [torch.ones(1024, device="cuda")] * W
+    ran = lambda: comm.last_call()["kernel"]  # noqa: E731
+    comm.all_reduce(x)
+    assert ran() == "local_sum"
+    comm.all_reduce_rmsnorm(x, w)
+    assert ran() == "local_norm"
+    shards = comm.reduce_scatter(x)
+    assert ran() == ("local_reduce_scatter" if W > 1 else "local_sum")
+    comm.all_gather(shards, 4096)
+    assert ran() == ("local_all_gather" if W > 1 else "local_sum")
+    comm.all_reduce_host([t.cpu().pin_memory() for t in x])
+    assert ran() == "local_host_sum"
+    comm.all_reduce(x, mode="flash")
+    assert ran() == comm.last_call()["variant"] == "flash"
+    comm.sync()
+
+
 def test_halves_of_the_multi_gpu_kernel_on_request(comm, monkeypatch):
     if comm.world == 1:
         pytest.skip("a group of one has no halves")

@@ -120,6 +120,8 @@ class Comm:
         return self._impl.layout()
 
     def last_call(self) -> dict:
+        """The last collective: `kernel` is what ran; `variant` the planner's choice, whose place a kernel for ranks
+        that share one GPU may have taken; its CTAs, slot and stages, flags, and the launches since creation."""
         return self._impl.last_call()
 
     # ---- device-side timeline ------------------------------------------------------------
