@@ -380,10 +380,10 @@ constexpr uint32_t kFlagSleepNs = 1500, kLineSleepNs = 40;
 // than units takes them in row order from a counter, the residuals of the next unit on their way into L2: rows
 // as CTAs of their own came in waves, each a chain of launch, residual, sums and stores (8 ranks, 300 rows: 600 CTAs
 // on 444 places took two of them).
-template <int NV, int G, bool SPLIT, bool LINES>
-__global__ void __launch_bounds__(kLocalLinearNormThreads, LocalLinearNormPlaces(G, SPLIT))
+template <int THREADS, int NV, int G, bool SPLIT, bool LINES>
+__global__ void __launch_bounds__(THREADS, LocalLinearNormPlaces(G, SPLIT, THREADS))
     local_linear_norm_kernel(const __grid_constant__ LocalLinearNormArgs a) {
-    constexpr int VEC = 8, kThreads = kLocalLinearNormThreads, kWarps = kThreads / 32;
+    constexpr int VEC = 8, kThreads = THREADS, kWarps = kThreads / 32;
     __shared__ float s_red[G][kWarps];
     __shared__ uint32_t s_next;
     const CommView& cv = a.cv;
@@ -598,16 +598,19 @@ __global__ void __launch_bounds__(kLocalLinearNormThreads, LocalLinearNormPlaces
     ptx::grid_dependency_wait();
 }
 
-template <int NV, int G>
+template <int THREADS, int NV, int G>
 const void* pick_linear_norm(bool split, bool lines) {
     if constexpr (G == 1) {
-        if (lines) return (const void*)local_linear_norm_kernel<NV, 1, true, true>;
+        if (lines) return (const void*)local_linear_norm_kernel<THREADS, NV, 1, true, true>;
     }
-    return split ? (const void*)local_linear_norm_kernel<NV, G, true, false> : (const void*)local_linear_norm_kernel<NV, G, false, false>;
+    return split ? (const void*)local_linear_norm_kernel<THREADS, NV, G, true, false>
+                 : (const void*)local_linear_norm_kernel<THREADS, NV, G, false, false>;
 }
-template <int NV>
+template <int THREADS, int NV>
 const void* pick_linear_norm_g(int g, bool split, bool lines) {
-    return g == 1 ? pick_linear_norm<NV, 1>(split, lines) : g == 2 ? pick_linear_norm<NV, 2>(split, lines) : pick_linear_norm<NV, 4>(split, lines);
+    return g == 1   ? pick_linear_norm<THREADS, NV, 1>(split, lines)
+           : g == 2 ? pick_linear_norm<THREADS, NV, 2>(split, lines)
+                    : pick_linear_norm<THREADS, NV, 4>(split, lines);
 }
 
 }  // namespace
@@ -616,8 +619,10 @@ const void* LocalGemmKernel() { return reinterpret_cast<const void*>(local_gemm_
 uint32_t LocalGemmSmemBytes() { return kSmemBytes; }
 
 const void* LocalLinearNormKernel(uint32_t N, int ranks_per_cta, bool split, bool lines) {
-    return N / 8 <= static_cast<uint32_t>(kLocalLinearNormThreads) ? pick_linear_norm_g<1>(ranks_per_cta, split, lines)
-                                                                   : pick_linear_norm_g<2>(ranks_per_cta, split, lines);
+    constexpr int kThreads = kLocalLinearNormThreads;
+    if (LocalLinearNormThreads(N) != kThreads) return pick_linear_norm_g<LocalLinearNormThreads(1), 1>(ranks_per_cta, split, lines);
+    return N / 8 <= static_cast<uint32_t>(kThreads) ? pick_linear_norm_g<kThreads, 1>(ranks_per_cta, split, lines)
+                                                    : pick_linear_norm_g<kThreads, 2>(ranks_per_cta, split, lines);
 }
 
 }  // namespace yali

@@ -15,6 +15,9 @@ constexpr uint32_t kLocalGemmMaxTokens = 256;  // rows of x on the N side
 constexpr uint32_t kLocalGemmMaxSplit = 8;
 constexpr int kLocalGemmThreads = 384;         // eight epilogue warps, TMA, MMA, announcer, prefetch
 constexpr int kLocalLinearNormThreads = 256;   // one row; up to two 16-byte vectors per thread: N <= 4096
+// A row of up to 64 vectors leaves most of 256 threads idle, and a unit of the row kernel is a chain of latencies, so
+// what counts is how many are in flight: four times as many CTAs of 64 threads.
+constexpr int LocalLinearNormThreads(uint32_t N) { return N <= 512 ? 64 : kLocalLinearNormThreads; }
 
 // T rows in `tiles` token tiles of `tokens` (a multiple of 32, at most 256), the k-blocks of all ranks (one rank after the
 // other) in `nsplit` runs of `kper`.
@@ -47,8 +50,8 @@ struct LocalLinearNormArgs {
 };
 
 // CTAs of the row kernel per SM (with the GEMM gone) that its register cap allows.
-constexpr int LocalLinearNormPlaces(int ranks_per_cta, bool split) {
-    return ranks_per_cta == 4 ? (split ? 2 : 3) : ranks_per_cta == 2 ? (split ? 3 : 4) : 2;
+constexpr int LocalLinearNormPlaces(int ranks_per_cta, bool split, int threads) {
+    return (ranks_per_cta == 4 ? (split ? 2 : 3) : ranks_per_cta == 2 ? (split ? 3 : 4) : 2) * (kLocalLinearNormThreads / threads);
 }
 
 const void* LocalGemmKernel();

@@ -423,9 +423,10 @@ Result LaunchLocal(Communicator& comm, const DriverApi* drv, const FusedLinearDe
         g.lines = 1;
         n.sums = g.sums = g.cv.heap[0] + lay.gemm_ll_off;
     }
+    const int threads = LocalLinearNormThreads(N);
     auto units_of = [&](int gr) { return T * ((W + gr - 1) / gr); };
     auto rounds_of = [&](int gr) {
-        const uint32_t fit = sms * LocalLinearNormPlaces(gr, g.s.nsplit > 1);
+        const uint32_t fit = sms * LocalLinearNormPlaces(gr, g.s.nsplit > 1, threads);
         return (units_of(gr) + fit - 1) / fit;
     };
     const bool one_vector = N <= 8u * kLocalLinearNormThreads;
@@ -433,13 +434,13 @@ Result LaunchLocal(Communicator& comm, const DriverApi* drv, const FusedLinearDe
     const int group = few ? 1 : four ? 4 : 2;
     const uint32_t units = units_of(group);
     const void* const fn2 = LocalLinearNormKernel(N, group, g.s.nsplit > 1, lines);
-    const uint32_t places = sms * LocalLinearNormPlaces(group, g.s.nsplit > 1);
+    const uint32_t places = sms * LocalLinearNormPlaces(group, g.s.nsplit > 1, threads);
     const cudaStream_t s = streams && streams[0] ? streams[0] : comm.default_stream(0);
     void* gp[] = {&g};
     void* np[] = {&n};
     cudaError_t e = LaunchInStream(fn, dim3(2 * std::min(items, pairs)), dim3(kLocalGemmThreads), gp, smem, s);
     if (e == cudaSuccess)
-        e = LaunchInStream(fn2, dim3(std::min(units, places)), dim3(kLocalLinearNormThreads), np, 0, s);
+        e = LaunchInStream(fn2, dim3(std::min(units, places)), dim3(threads), np, 0, s);
     if (e != cudaSuccess) {
         (void)cudaGetLastError();
         return fail(Result::CudaError, std::string("kernel launch failed: ") + cudaGetErrorString(e));
