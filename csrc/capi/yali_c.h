@@ -145,14 +145,14 @@ int yali_c_simulate_fused(const YaliFusedSimConfig* cfg, YaliSimReport* rep);
 /* Host-thread model of the two kernels that ranks on one GPU run for the fused layer (sim/local_gemm_sim.cc): `pairs`
  * threads of the GEMM, `row_ctas` of the row kernel (at most one per row), `calls` back-to-back calls of [rows, col_units]
  * sums in token tiles of tile_rows rows and `splits` K splits, announced by flags or sent as flag-in-data lines.
- * slow_cta (-1: none) sleeps after it has released the row kernel.  late_number = 1: the GEMM reads the call number after
- * that release (negative control for lines).  reset_at > 0: the control words are cleared in front of that call, the
+ * slow_cta (-1: none) sleeps after it has released the row kernel.  shared_number = 1: the GEMM reads the row
+ * kernel's call number instead of one of its own (negative control for lines).  reset_at > 0: the control words are cleared in front of that call, the
  * lines with them unless keep_lines (negative control).  fault 1: the first item of every GEMM thread is lost in call
  * fault_call.  Same return codes and report as yali_c_simulate. */
 typedef struct YaliLocalSimConfig {
     int pairs, row_ctas, calls;
     uint32_t rows, col_units, splits, tile_rows;
-    int lines, slow_cta, late_number, reset_at, keep_lines, fault, fault_call, timeout_ms;
+    int lines, slow_cta, shared_number, reset_at, keep_lines, fault, fault_call, timeout_ms;
 } YaliLocalSimConfig;
 int yali_c_simulate_local(const YaliLocalSimConfig* cfg, YaliSimReport* rep);
 

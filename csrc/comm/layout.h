@@ -28,7 +28,7 @@ constexpr uint32_t kCallFlashEpoch = 0;   // one-shot calls so far
 constexpr uint32_t kCallStreamSeq = 1;    // ring sequence numbers consumed so far
 constexpr uint32_t kCallBarEpoch = 2;     // per-CTA barrier epochs consumed so far
 constexpr uint32_t kCallGemmEpoch = 3;    // fused GEMM calls so far
-constexpr uint32_t kCallLocalGemm = 4;     // fused linear calls of ranks that share one GPU (rank 0's word)
+constexpr uint32_t kCallLocalGemm = 4;     // fused linear calls of ranks that share one GPU (rank 0's word), as the GEMM counts
 constexpr uint32_t kCallFlashEpochHi = 5;  // upper half of the one-shot call number (flag-in-data protocol)
 constexpr uint32_t kCallGemmLLEpoch = 6;   // calls of the fused GEMM's few-token form so far (lower half)
 constexpr uint32_t kCallGemmLLEpochHi = 7;  // upper half of that call number
@@ -37,6 +37,8 @@ constexpr uint32_t kCallDoneCtas = 16;    // [4] CTAs of the running launch that
 constexpr uint32_t kCallTraceIdx = 20;    // traced calls so far (index into the kTraceOff ring)
 constexpr uint32_t kCallPlanWord = 21;    // what this rank's running (or last) collective is: PlanWord() of its plan
 constexpr uint32_t kCallLocalRows = 23;   // units the row kernel of gemm_local.cu has handed out in the running call
+constexpr uint32_t kCallLocalRowCalls = 24;  // the same calls, as the row kernel counts
+constexpr uint32_t kCallLocalGemmIn = 25;    // CTAs of the running GEMM that have read their call's number
 constexpr uint32_t kCallCeCalls = 22;     // copy-engine all-reduce calls so far
 constexpr uint32_t kFlashFlagOff = 32;                                       // [kMaxFlashCtas][kMaxRanks]
 constexpr uint32_t kRsSeqOff = kFlashFlagOff + kMaxFlashCtas * kMaxRanks;    // [kMaxLanes][kMaxRanks]

@@ -12,8 +12,7 @@
 //                              out and residual_out.
 //
 // The second kernel starts while the first one runs (griddepcontrol.launch_dependents, issued by every CTA of the first
-// one when it has read the call's number: all of them are resident by then, so whoever waits for them here waits for
-// running CTAs), and its CTAs wait for the flags of their token tile: rows are finished under the GEMM of later tiles.
+// one when it starts: all of them are resident by then, so whoever waits for them here waits for running CTAs), and its CTAs wait for the flags of their token tile: rows are finished under the GEMM of later tiles.
 //
 // The pair computes the transposed tile, W on the M side: a tile can then be any multiple of 32 tokens wide, and each CTA
 // loads 128 rows of W and half of the tokens per 64-deep k-block.  The threads that issue TMA and MMA are picked
@@ -148,6 +147,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kLocalGemmThreads, 1
     ptx::tc_fence_after_sync();
     const uint32_t tmem = s.tmem;
     ptx::grid_dependency_wait();
+    ptx::grid_launch_dependents();
     const uint64_t deadline = ptx::globaltimer() + cv.timeout_ns;
     const uint32_t ncol = (a.N + kLocalGemmPairCols - 1) / kLocalGemmPairCols;
     const uint32_t pair = cta >> 1, npairs = gridDim.x >> 1;
@@ -238,14 +238,24 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kLocalGemmThreads, 1
         // When the epilogue warps have stored their part of a unit: publish the call number in its flag.  The release orders
         // the stores (made visible to this warp by the mbarrier) before the flag; it waits for them to arrive, so it
         // sits in a warp of its own.
-        // It also reads this call's number, for the whole CTA, and then lets the second kernel start.  In this order: that
-        // kernel advances the number when all of its CTAs have read it, and waits for no data before it does so
-        // where the sums are lines, so by then every CTA here must have its number, too.
-        if (lane == 0) s.epoch = *reinterpret_cast<volatile uint32_t*>(flag_word(cv, 0, kCallLocalGemm)) + 1u;
-        ptx::named_barrier(kNumberBarrier, 32 * (kEpilogueWarps + 1));
+        // It also reads this call's number; the epilogue warps need it where the sums are lines.
+        uint32_t epoch = 0;
+        if (lane == 0) epoch = *reinterpret_cast<volatile uint32_t*>(flag_word(cv, 0, kCallLocalGemm)) + 1u;
+        if (a.lines) {
+            if (lane == 0) s.epoch = epoch;
+            ptx::named_barrier(kNumberBarrier, 32 * (kEpilogueWarps + 1));
+        }
         if (lane == 0) {
-            ptx::grid_launch_dependents();
-            const uint32_t epoch = s.epoch, units = a.N / kLocalGemmUnitCols;
+            // The last CTA that has read the number advances it for the next call.  The row kernel keeps a count of its own:
+            // it runs at the same time and, where the sums are lines, is done with its count before any of them is here.
+            auto check_in = [&] {
+                uint32_t* const in = flag_word(cv, 0, kCallLocalGemmIn);
+                if (atomicAdd(in, 1u) != gridDim.x - 1) return;
+                *reinterpret_cast<volatile uint32_t*>(in) = 0u;
+                *reinterpret_cast<volatile uint32_t*>(flag_word(cv, 0, kCallLocalGemm)) = epoch;
+            };
+            if (a.lines) check_in();  // nothing to announce: now rather than at the end
+            const uint32_t units = a.N / kLocalGemmUnitCols;
             Item it;
             for (uint32_t n = 0; item_at(a, n, pair, npairs, ncol, &it); ++n) {
                 const uint32_t b = n & 1u, unit = it.col_tile * 2 + half;
@@ -258,6 +268,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kLocalGemmThreads, 1
                     ptx::st_release_gpu(flag_word(cv, 0, kLocalGemmFlagOff + (it.tile * a.s.nsplit + it.split) * units + unit), epoch);
                 ptx::mbar_arrive(&s.announced_bar[b]);
             }
+            if (!a.lines) check_in();  // the rows take longer
         }
     } else if (warp == kPrefetchWarp) {
         // Brings the operands into L2 ahead of the loads: what a CTA has in flight in its stages does not cover the latency of
@@ -290,8 +301,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kLocalGemmThreads, 1
         const uint32_t token = lane >> 2;  // stores: token of a group of 8, 16-byte piece lane % 4
         const uint8_t* const ld_row = stage + token * 64 + (((lane & 3) ^ ((token >> 1) & 3)) << 4);
         const uint64_t rowbytes = static_cast<uint64_t>(a.N) * 2;
-        ptx::named_barrier(kNumberBarrier, 32 * (kEpilogueWarps + 1));
-        const uint32_t epoch = s.epoch;
+        uint32_t epoch = 0;
+        if (a.lines) {
+            ptx::named_barrier(kNumberBarrier, 32 * (kEpilogueWarps + 1));
+            epoch = s.epoch;
+        }
         Item it;
         for (uint32_t n = 0; item_at(a, n, pair, npairs, ncol, &it); ++n) {
             const uint32_t b = n & 1u, t0 = it.tile * a.s.tokens, nt = min(a.T - t0, a.s.tokens);
@@ -391,7 +405,7 @@ __global__ void __launch_bounds__(THREADS, LocalLinearNormPlaces(G, SPLIT, THREA
     const uint32_t tid = threadIdx.x, nvec = a.N / VEC;
     const bool taking = gridDim.x < units;  // from the counter
     uint32_t* const counter = flag_word(cv, 0, kCallLocalRows);
-    const uint32_t epoch = *reinterpret_cast<volatile uint32_t*>(flag_word(cv, 0, kCallLocalGemm)) + 1u;
+    const uint32_t epoch = *reinterpret_cast<volatile uint32_t*>(flag_word(cv, 0, kCallLocalRowCalls)) + 1u;
     const uint64_t deadline = ptx::globaltimer() + cv.timeout_ns;
     bool have[NV];
 #pragma unroll
@@ -406,8 +420,13 @@ __global__ void __launch_bounds__(THREADS, LocalLinearNormPlaces(G, SPLIT, THREA
     auto check_in = [&] {
         if (check_in_last(cv, 3, gridDim.x)) {
             *reinterpret_cast<volatile uint32_t*>(counter) = 0u;
-            advance_call_word(cv, kCallLocalGemm, 1);
+            advance_call_word(cv, kCallLocalRowCalls, 1);
         }
+    };
+    // A wait ran out: the two counts of calls stay alike, and the call is over when both kernels are.
+    auto give_up = [&](bool before_check_in) {
+        if (before_check_in && tid == kThreads - 1) check_in();
+        ptx::grid_dependency_wait();
     };
     if (unit >= units && tid == 0) check_in();  // nothing was left for this CTA
     const float inv_n = 1.f / static_cast<float>(a.N);
@@ -446,7 +465,7 @@ __global__ void __launch_bounds__(THREADS, LocalLinearNormPlaces(G, SPLIT, THREA
             }
             ready = tile;
         }
-        if (__syncthreads_or(late)) break;
+        if (__syncthreads_or(late)) return give_up(true);
         if (taking) {
             unit = s_next;
             if (unit < units) {
@@ -465,8 +484,7 @@ __global__ void __launch_bounds__(THREADS, LocalLinearNormPlaces(G, SPLIT, THREA
             unit = units;
         }
         // Once every CTA has read the call number and taken its last unit, both counters may move on: the next call reads
-        // them, nothing in this one does (the GEMM's CTAs had their number before they let this kernel start).
-        // Done here, under the work of the last unit.
+        // them, nothing in this one does.  Done here, under the work of the last unit.
         if (unit >= units && tid == kThreads - 1) check_in();
 
         uint4 one[SPLIT ? 1 : NV];
@@ -568,7 +586,7 @@ __global__ void __launch_bounds__(THREADS, LocalLinearNormPlaces(G, SPLIT, THREA
             if ((tid & 31) == 0) s_red[g][tid >> 5] = ss;
         }
         if (LINES) {
-            if (__syncthreads_or(late)) break;
+            if (__syncthreads_or(late)) return give_up(unit < units);
         } else {
             __syncthreads();
         }
@@ -594,7 +612,7 @@ __global__ void __launch_bounds__(THREADS, LocalLinearNormPlaces(G, SPLIT, THREA
             }
         }
     }
-    // The call is over when both kernels are, also when a wait ran out here.
+    // The call is over when both kernels are.
     ptx::grid_dependency_wait();
 }
 

@@ -1,7 +1,7 @@
 // Host-thread model of the two kernels of the fused layer for ranks that share one GPU (yali_c.h,
 // yali_c_simulate_local; kernels/gemm_local.cu).  One host thread plays one pair of CTAs of the GEMM or one CTA of the
-// row kernel.  Modelled is what passes between the two and from call to call: the call number and who reads it when,
-// the release of the dependent kernel, the walk over the items, sums announced by flags or sent as flag-in-data lines,
+// row kernel.  Modelled is what passes between the two and from call to call: the call numbers and who reads and advances
+// them when, the release of the dependent kernel, the walk over the items, sums announced by flags or sent as flag-in-data lines,
 // rows taken from a counter, the check-in that clears the counter and advances the call number, and the clearing of
 // the control words between calls (Communicator::Reset).  The GEMM itself is a formula of (call, row, unit, split).
 // Calls follow one another in stream order: a call starts when both kernels of the one before it have finished.
@@ -44,7 +44,8 @@ struct Barrier {
 struct LocalShared {
     YaliLocalSimConfig cfg;
     uint32_t T, units, ks, tiles;
-    std::atomic<uint32_t> number{0}, counter{0}, checked_in{0};  // call word, unit counter, check-ins
+    std::atomic<uint32_t> gemm_number{0}, gemm_in{0};            // the GEMM's count of calls, its CTAs that have read it
+    std::atomic<uint32_t> number{0}, counter{0}, checked_in{0};  // the row kernel's count, unit counter, check-ins
     std::atomic<int> released{0};                                // GEMM CTAs that have released the row kernel
     std::unique_ptr<std::atomic<uint64_t>[]> lines;              // [split][row][unit]: {call number, value}
     std::unique_ptr<std::atomic<uint32_t>[]> flags;              // [tile][split][unit]: call number
@@ -89,17 +90,21 @@ void GemmCta(LocalShared& s, int c, int call) {
     auto doze = [&] {
         if (c == s.cfg.slow_cta) std::this_thread::sleep_for(std::chrono::milliseconds(3));
     };
+    s.released.fetch_add(1, std::memory_order_acq_rel);
     uint32_t number;
-    if (s.cfg.late_number) {
-        const uint32_t before = s.number.load();
-        s.released.fetch_add(1, std::memory_order_acq_rel);
+    if (s.cfg.shared_number) {
         // As late as it gets: after the row kernel has moved on to the next number, if it does so without this thread.
+        const uint32_t before = static_cast<uint32_t>(call) - (s.cfg.reset_at > 0 && call >= s.cfg.reset_at ? s.cfg.reset_at : 0);
         for (int ms = 0; c == s.cfg.slow_cta && ms < 200 && s.number.load() == before; ++ms)
             std::this_thread::sleep_for(std::chrono::milliseconds(1));
         number = s.number.load(std::memory_order_acquire) + 1u;
     } else {
-        number = s.number.load(std::memory_order_acquire) + 1u;
-        s.released.fetch_add(1, std::memory_order_acq_rel);
+        doze();
+        number = s.gemm_number.load(std::memory_order_acquire) + 1u;
+        if (s.gemm_in.fetch_add(1) == static_cast<uint32_t>(s.cfg.pairs) - 1) {
+            s.gemm_in.store(0);
+            s.gemm_number.store(number, std::memory_order_release);
+        }
         doze();
     }
     const uint32_t per_tile = s.units * s.ks;
@@ -178,6 +183,7 @@ void Cta(LocalShared& s, int c) {
             if (s.counter.load() != 0 || s.checked_in.load() != 0) s.violations.fetch_add(1);
             if (call + 1 == s.cfg.reset_at) {
                 s.number.store(0);
+                s.gemm_number.store(0);
                 for (uint32_t f = 0; f < s.tiles * s.ks * s.units; ++f) s.flags[f].store(0);
                 if (!s.cfg.keep_lines)
                     for (size_t i = 0; i < s.At(s.ks, 0, 0); ++i) s.lines[i].store(0);

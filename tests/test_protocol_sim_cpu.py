@@ -247,7 +247,7 @@ from yali_b200._native import LocalSimConfig  # noqa: E402
 
 def simulate_local(**kw):
     cfg = LocalSimConfig(pairs=3, row_ctas=4, calls=5, rows=40, col_units=3, splits=2, tile_rows=16, lines=0, slow_cta=-1,
-                         late_number=0, reset_at=0, keep_lines=0, fault=0, fault_call=0, timeout_ms=5000)
+                         shared_number=0, reset_at=0, keep_lines=0, fault=0, fault_call=0, timeout_ms=5000)
     for k, v in kw.items():
         setattr(cfg, k, v)
     rep = SimReport()
@@ -265,13 +265,13 @@ def test_local_form_protocol_back_to_back_calls(lines, rows, row_ctas):
         assert rep.flag_writes == 5 * rows * 3 * splits
 
 
-def test_local_form_needs_its_call_number_before_the_row_kernel_starts():
-    """Lines: the row kernel advances the number before it waits for data, so a GEMM thread that reads it after the
-    release may stamp its lines with the next call's.  Flags: the number advances when all flags have been seen."""
+def test_local_form_gemm_and_rows_count_calls_apart():
+    """Lines: the row kernel advances its number before it waits for data, so a GEMM thread that read that word might stamp its
+    lines with the next call's.  Flags: the number advances when all flags have been seen."""
     assert simulate_local(lines=1, rows=8, row_ctas=8, slow_cta=1)[0] == 0
-    rc, rep = simulate_local(lines=1, rows=8, row_ctas=8, slow_cta=1, late_number=1, timeout_ms=2000)
+    rc, rep = simulate_local(lines=1, rows=8, row_ctas=8, slow_cta=1, shared_number=1, timeout_ms=2000)
     assert rc == 2 and rep.timeouts >= 1
-    assert simulate_local(lines=0, rows=8, row_ctas=8, slow_cta=1, late_number=1)[0] == 0
+    assert simulate_local(lines=0, rows=8, row_ctas=8, slow_cta=1, shared_number=1)[0] == 0
 
 
 def test_local_form_after_a_reset_of_the_call_number():

@@ -45,7 +45,7 @@ class FusedSimConfig(ctypes.Structure):
 class LocalSimConfig(ctypes.Structure):
     _fields_ = [(n, ctypes.c_int) for n in ("pairs", "row_ctas", "calls")] + \
                [(n, ctypes.c_uint32) for n in ("rows", "col_units", "splits", "tile_rows")] + \
-               [(n, ctypes.c_int) for n in ("lines", "slow_cta", "late_number", "reset_at", "keep_lines", "fault", "fault_call",
+               [(n, ctypes.c_int) for n in ("lines", "slow_cta", "shared_number", "reset_at", "keep_lines", "fault", "fault_call",
                                             "timeout_ms")]
 
 
