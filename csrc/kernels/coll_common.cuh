@@ -183,14 +183,15 @@ __device__ __forceinline__ bool mbar_wait_deadline(uint64_t* bar, uint32_t parit
 // TMEM) has to end before the CTA does: the next one would find them in its own memory.  Bounded, too; a copy is on its
 // way for 2 us under full load.
 constexpr uint64_t kDrainNs = 200000;
-__device__ __forceinline__ void mbar_drain(uint64_t* bar, uint32_t parity, uint64_t until_ns) {
+__device__ __forceinline__ void mbar_drain(uint64_t* bar, uint32_t parity) {
+    if (ptx::mbar_try_wait_cluster(bar, parity)) return;  // as a rule, and without the timer
+    const uint64_t until_ns = ptx::globaltimer() + kDrainNs;
     while (!ptx::mbar_try_wait_cluster(bar, parity) && ptx::globaltimer() < until_ns) {
     }
 }
 // The copies on a ring of `n` barriers that have been armed in turn, `armed` times in all.
 __device__ __forceinline__ void mbar_drain_ring(uint64_t* bars, uint32_t n, uint32_t armed) {
-    const uint64_t until_ns = ptx::globaltimer() + kDrainNs;
-    for (uint32_t k = armed > n ? armed - n : 0u; k < armed; ++k) mbar_drain(&bars[k % n], (k / n) & 1u, until_ns);
+    for (uint32_t k = armed > n ? armed - n : 0u; k < armed; ++k) mbar_drain(&bars[k % n], (k / n) & 1u);
 }
 
 // Block-wide sum of one float per thread (all threads get the result).

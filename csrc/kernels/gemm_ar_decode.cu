@@ -202,8 +202,10 @@ __device__ __forceinline__ void decode_body(const GemmDecodeArgs& a, const CUten
                 if (*abort_flag) break;
                 ptx::tc_commit(&tmem_full_bar[b]);
             }
-            ptx::tc_commit(&drain_bar);
-            mbar_drain(&drain_bar, 0, ptx::globaltimer() + kDrainNs);
+            if (it > 0 || *abort_flag) {
+                ptx::tc_commit(&drain_bar);
+                mbar_drain(&drain_bar, 0);
+            }
         }
     } else if ((warp & 3) < 2) {
         const int q = warp & 3;   // TMEM lane quarter this warp may read

@@ -464,7 +464,7 @@ __device__ __forceinline__ void gemm_ar_body(const GemmArArgs& a, uint32_t cta, 
                 else
                     for (const uint64_t until = ptx::globaltimer() + kDrainNs; ptx::globaltimer() < until;) ptx::nanosleep(1000);
             }
-            mbar_drain(&s.drain_bar, 0, ptx::globaltimer() + kDrainNs);
+            if (loaded > 0) mbar_drain(&s.drain_bar, 0);
         }
     } else if (warp == kMmaWarp) {
         if (half == 0 && ptx::elect_one()) {
@@ -502,8 +502,10 @@ __device__ __forceinline__ void gemm_ar_body(const GemmArArgs& a, uint32_t cta, 
                 ptx::tc_commit_pair(&s.tmem_full_bar[b]);  // accumulator complete
                 ++n;
             }
-            ptx::tc_commit_pair(&s.drain_bar);
-            mbar_drain(&s.drain_bar, 0, ptx::globaltimer() + kDrainNs);
+            if (n > 0 || s.abort) {  // a pair without items leaves at once
+                ptx::tc_commit_pair(&s.drain_bar);
+                mbar_drain(&s.drain_bar, 0);
+            }
         }
     } else if (warp == kAnnounceWarp) {
         // When the eight epilogue warps have issued the pushes of a tile unit, tell every owner of rows of it.

@@ -12,7 +12,8 @@
 //                              out and residual_out.
 //
 // The second kernel starts while the first one runs (griddepcontrol.launch_dependents, issued by every CTA of the first
-// one when it starts: all of them are resident by then, so whoever waits for them here waits for running CTAs), and its CTAs wait for the flags of their token tile: rows are finished under the GEMM of later tiles.
+// one when it starts: all of them are resident by then, so whoever waits for them here waits for running CTAs),
+// and its CTAs wait for the flags of their token tile: rows are finished under the GEMM of later tiles.
 //
 // The pair computes the transposed tile, W on the M side: a tile can then be any multiple of 32 tokens wide, and each CTA
 // loads 128 rows of W and half of the tokens per 64-deep k-block.  The threads that issue TMA and MMA are picked
@@ -196,7 +197,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kLocalGemmThreads, 1
                 else
                     for (const uint64_t until = ptx::globaltimer() + kDrainNs; ptx::globaltimer() < until;) ptx::nanosleep(1000);
             }
-            mbar_drain(&s.drain_bar, 0, ptx::globaltimer() + kDrainNs);
+            if (loaded > 0) mbar_drain(&s.drain_bar, 0);
         }
     } else if (warp == kMmaWarp) {
         if (half == 0 && ptx::elect_one()) {
@@ -231,8 +232,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kLocalGemmThreads, 1
                 if (s.abort) break;
                 ptx::tc_commit_pair(&s.tmem_full_bar[b]);  // accumulator complete
             }
-            ptx::tc_commit_pair(&s.drain_bar);
-            mbar_drain(&s.drain_bar, 0, ptx::globaltimer() + kDrainNs);
+            if (n > 0 || s.abort) {  // a pair without items leaves at once
+                ptx::tc_commit_pair(&s.drain_bar);
+                mbar_drain(&s.drain_bar, 0);
+            }
         }
     } else if (warp == kAnnounceWarp) {
         // When the epilogue warps have stored their part of a unit: publish the call number in its flag.  The release orders
@@ -423,11 +426,6 @@ __global__ void __launch_bounds__(THREADS, LocalLinearNormPlaces(G, SPLIT, THREA
             advance_call_word(cv, kCallLocalRowCalls, 1);
         }
     };
-    // A wait ran out: the two counts of calls stay alike, and the call is over when both kernels are.
-    auto give_up = [&](bool before_check_in) {
-        if (before_check_in && tid == kThreads - 1) check_in();
-        ptx::grid_dependency_wait();
-    };
     if (unit >= units && tid == 0) check_in();  // nothing was left for this CTA
     const float inv_n = 1.f / static_cast<float>(a.N);
     bool late = false;
@@ -465,7 +463,9 @@ __global__ void __launch_bounds__(THREADS, LocalLinearNormPlaces(G, SPLIT, THREA
             }
             ready = tile;
         }
-        if (__syncthreads_or(late)) return give_up(true);
+        // After a wait that ran out the rows are not worth anything, but the CTA goes on, without waiting: every unit is taken,
+        // every CTA checks in and the two counts of calls stay alike.
+        __syncthreads();
         if (taking) {
             unit = s_next;
             if (unit < units) {
@@ -585,11 +585,7 @@ __global__ void __launch_bounds__(THREADS, LocalLinearNormPlaces(G, SPLIT, THREA
             for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
             if ((tid & 31) == 0) s_red[g][tid >> 5] = ss;
         }
-        if (LINES) {
-            if (__syncthreads_or(late)) return give_up(unit < units);
-        } else {
-            __syncthreads();
-        }
+        __syncthreads();
 #pragma unroll
         for (int g = 0; g < G; ++g) {
             if (q0 + g >= a.world) break;
