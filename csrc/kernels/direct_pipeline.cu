@@ -55,7 +55,7 @@ __device__ __forceinline__ void direct_body(const CollArgs& a, uint32_t cta) {
     extern __shared__ __align__(128) uint8_t dsmem[];  // [stages][W sources][slot_bytes]
     __shared__ __align__(8) uint64_t full_bar[kDirectMaxStages], empty_bar[kDirectMaxStages];
     __shared__ int s_abort;
-    __shared__ uint32_t s_epoch;
+    __shared__ uint32_t s_epoch, s_armed;  // s_armed: stages filled, counted from the start
 
     trace_begin(cv, a.flags, cta);
     announce_plan(cv, a.plan_word, cta);
@@ -118,7 +118,7 @@ __device__ __forceinline__ void direct_body(const CollArgs& a, uint32_t cta) {
                     }
                 }
             }
-            mbar_drain_ring(full_bar, stages, it);  // also when the consumers stop early
+            s_armed = it;
         }
     } else {
         // ---------------------------------------------------------------- consumers
@@ -182,9 +182,13 @@ __device__ __forceinline__ void direct_body(const CollArgs& a, uint32_t cta) {
             if (lane == 0) ptx::mbar_arrive(&empty_bar[s]);
         }
     }
-    // The producer has waited for its copies, so none is in flight past this point.
+    // Every stage that was filled has been consumed here, so no bulk copy is in flight past this point, unless a consumer
+    // left its loop early after a wait that ran out.
     __syncthreads();
-    if (s_abort) return;
+    if (s_abort) {
+        if (tid == 0) mbar_drain_ring(full_bar, stages, s_armed);
+        return;
+    }
     // Peers have read this rank's input and their stores into this rank's output are visible.
     if (!cta_barrier_all_ranks(cv, cta, epoch + 2, deadline, &s_abort)) return;
     finish_checked_in_call(cv, 2, kCallBarEpoch, 2, nctas, a.flags);

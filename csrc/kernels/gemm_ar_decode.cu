@@ -79,6 +79,7 @@ __device__ __forceinline__ void decode_body(const GemmDecodeArgs& a, const CUten
     extern __shared__ uint8_t smem_raw[];
     __shared__ __align__(8) uint64_t full_bar[kDMaxStages], empty_bar[kDMaxStages], tmem_full_bar[2], tmem_empty_bar[2];
     __shared__ __align__(8) uint64_t drain_bar;  // all MMAs have finished
+    __shared__ uint32_t s_armed;                  // k-blocks whose loads have been issued
     __shared__ __align__(16) uint4 s_lines[kDEpilogueWarps][32 * 8];  // per epilogue warp: 32 rows x 8 lines, swizzled
     __shared__ uint32_t s_tmem;
     __shared__ int s_abort;
@@ -167,7 +168,7 @@ __device__ __forceinline__ void decode_body(const GemmDecodeArgs& a, const CUten
                     if (++s == stages) s = 0, ++round;
                 }
             }
-            mbar_drain_ring(full_bar, stages, round * stages + s);  // also when the MMAs stop early
+            s_armed = round * stages + s;
         }
     } else if (warp == 3) {
         if (ptx::elect_one()) {
@@ -303,6 +304,7 @@ __device__ __forceinline__ void decode_body(const GemmDecodeArgs& a, const CUten
     YALI_DSTAMP(6, 0);  // this warp's pushes issued
     ptx::tc_fence_before_sync();
     __syncthreads();
+    if (s_abort && tid == 0) mbar_drain_ring(full_bar, stages, s_armed);  // the MMAs stopped early
     if (warp == 3) ptx::tmem_dealloc(tmem, kDTmemCols);
     if (s_abort) return;
     YALI_DSTAMP(3, 0);  // all items of this CTA pushed

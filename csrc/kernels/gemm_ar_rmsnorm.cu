@@ -138,7 +138,7 @@ struct Shared {
     __align__(8) uint64_t pushed_bar[2], announced_bar[2];  // epilogue warps -> announcer warp and back
     __align__(8) uint64_t drain_bar;  // all MMAs have finished
     __align__(8) uint64_t row_full[kRowGroups][kMaxRowSlots], row_empty[kRowGroups][kMaxRowSlots];
-    uint32_t tmem;
+    uint32_t tmem, row_armed[kRowGroups];  // row_armed: pieces of rows that have been asked for
     char* heap[kMaxRanks];  // the heap bases: read with a run-time rank
     volatile int abort;
     uint32_t call[1 + kMaxRanks];
@@ -239,11 +239,10 @@ __device__ __forceinline__ void row_producer(const GemmArArgs& a, Shared& s, uin
         rounds[1] = group ? round : rounds[1];
         if (__any_sync(0xffffffffu, late)) break;
     }
-    // Nothing is under way when this CTA leaves, also when the row warps stop early.
-    if (ptx::elect_one())
-        for (uint32_t g = 0; g < static_cast<uint32_t>(kRowGroups); ++g)
-            mbar_drain_ring(s.row_full[g], m.slots, g ? rounds[1] * m.slots + slots[1] : rounds[0] * m.slots + slots[0]);
-    __syncwarp();
+    if (lane == 0) {
+        s.row_armed[0] = rounds[0] * m.slots + slots[0];
+        s.row_armed[1] = rounds[1] * m.slots + slots[1];
+    }
 }
 
 // The four warps of row group `group`: every second of this CTA's rows (two groups, because a row is a chain of latencies:
@@ -654,6 +653,9 @@ __device__ __forceinline__ void gemm_ar_body(const GemmArArgs& a, uint32_t cta, 
     ptx::tc_fence_before_sync();
     __syncthreads();
     YALI_STAMP(6, 0);  // own rows reduced and written
+    // Row warps that stop early leave copies on their way into the ring.
+    if (s.abort && warp == kRowTmaWarp && lane < kRowGroups) mbar_drain_ring(s.row_full[lane], my_rows(a).slots, s.row_armed[lane]);
+    __syncwarp();
     // Nobody leaves (or gives TMEM back) while the other CTA's MMAs, loads or arrivals may still reach this one.
     ptx::cluster_arrive();
     ptx::cluster_wait();
