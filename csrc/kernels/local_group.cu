@@ -337,6 +337,7 @@ const void* pick_norm_nv(int nv, int g) {
 template <typename T>
 const void* pick_norm(int world, int nv, int g) {
     switch (world) {
+        case 1: return pick_norm_nv<T, 1>(nv, g);
         case 2: return pick_norm_nv<T, 2>(nv, g);
         case 4: return pick_norm_nv<T, 4>(nv, g);
         case 8: return pick_norm_nv<T, 8>(nv, g);
