@@ -103,6 +103,53 @@ def test_norm(comm, dtype, rows, hidden):
         torch.testing.assert_close(xs[0].double(), ys[0].double(), rtol=2 * rtol, atol=1e-6)
 
 
+@pytest.mark.parametrize("dtype", [F32, F16, BF16])
+@pytest.mark.parametrize("rows,hidden", [(1, 4096), (16, 4096), (5, 1024), (3, 8192), (128, 4096), (7, 256)])
+def test_norm_of_the_one_shot_kernel(comm, dtype, rows, hidden):
+    """The row epilogue of the multi-GPU kernel, three calls back to back: each rank with a residual and a weight of its own."""
+    if comm.world == 1:
+        pytest.skip("a group of one has nothing to send")
+    W, rtol = comm.world, {F32: 2e-6, F16: 2.0 ** -10, BF16: 2.0 ** -7}[dtype]
+    xs, res = [whole((rows, hidden), dtype, r) for r in range(W)], [whole((rows, hidden), dtype, 50 + r) for r in range(W)]
+    ws = [whole((hidden,), dtype, 90 + r) for r in range(W)]
+    pre = [[torch.empty_like(x) for x in xs] for _ in range(3)]
+    ys = [comm.all_reduce_rmsnorm(xs, ws, res, eps=1e-5, residual_out=p, mode="flash") for p in pre]
+    assert comm.last_call()["kernel"] == "flash"
+    comm.sync()
+    for r in range(W):
+        row = total(xs) + res[r].double()
+        ref = row * torch.rsqrt(row.pow(2).mean(-1, keepdim=True) + 1e-5) * ws[r].double()
+        for y, p in zip(ys, pre):
+            assert torch.equal(p[r].double(), row)
+            torch.testing.assert_close(y[r].double(), ref, rtol=rtol, atol=1e-6)
+
+
+# Row lengths by 16-byte vectors per thread of the norm kernel (128 / 129 / 1024 / 1025 / 2048 vectors), one that is no whole
+# number of vectors, and one weight off a 16-byte boundary.
+@pytest.mark.parametrize("dtype,hidden,off", [(BF16, 1024, 0), (BF16, 1032, 0), (F16, 8192, 0), (F32, 4100, 0), (F32, 8192, 0), (BF16, 1001, 0), (BF16, 1024, 1)])
+def test_norm_beyond_the_one_shot_staging(comm, dtype, hidden, off):
+    """Above the staging's size the sum comes first and a kernel per rank normalises its rows: 1 + world launches."""
+    if comm.world == 1:
+        pytest.skip("a group of one stages nothing")
+    W, rtol = comm.world, {F32: 2e-6, F16: 2.0 ** -10, BF16: 2.0 ** -7}[dtype]
+    rows = comm.layout()["flash_cap"] // (hidden * torch.empty(0, dtype=dtype).element_size()) + 3
+    xs = [whole((rows, hidden), dtype, r) for r in range(W)]
+    res, ws = [whole((rows, hidden), dtype, 50 + r) for r in range(W)], [whole((hidden,), dtype, 90 + r, off) for r in range(W)]
+    pre, before = [torch.empty_like(x) for x in xs], comm.launches
+    ys = comm.all_reduce_rmsnorm(xs, ws, res, eps=1e-5, residual_out=pre)
+    assert comm.launches - before == 1 + W
+    plain = comm.all_reduce_rmsnorm(xs, ws, None, eps=1e-5)
+    comm.sync()
+    pick = torch.tensor([0, 1, rows // 2, rows - 2, rows - 1], device="cuda")
+    s = total([x[pick] for x in xs])
+    for r in (0, W - 1):
+        for got, row in ((ys[r], s + res[r][pick].double()), (plain[r], s)):
+            ref = row * torch.rsqrt(row.pow(2).mean(-1, keepdim=True) + 1e-5) * ws[r].double()
+            torch.testing.assert_close(got[pick].double(), ref, rtol=rtol, atol=1e-6)
+        assert torch.equal(pre[r][pick].double(), s + res[r][pick].double())
+        assert torch.equal(pre[r].float(), sum(x.float() for x in xs) + res[r].float())
+
+
 @pytest.mark.parametrize("odd", ["x", "weight", "residual", "out", "residual_out"])
 @pytest.mark.parametrize("mode", ["auto", "flash"])
 def test_norm_refuses_tensors_off_a_16_byte_boundary(comm, odd, mode):
@@ -243,13 +290,14 @@ def test_host_buffers_that_are_registered_in_part(which):
         assert torch.equal((c.all_reduce_host(ok), torch.cuda.synchronize())[0][1], torch.full((n,), 2.0))
 
 
-@pytest.mark.parametrize("n", [8, 40001, 1 << 20])
-def test_a_geometry_of_the_caller_runs_the_multi_gpu_kernels(comm, n):
+@pytest.mark.parametrize("dtype", [F32, F16, BF16])
+@pytest.mark.parametrize("n", [8, 16, 4099, 40001, 500000, 1 << 20])
+def test_a_geometry_of_the_caller_runs_the_multi_gpu_kernels(comm, n, dtype):
     """`ctas` and `slot_bytes` without a mode: accepted by every collective, and nothing of them is dropped."""
     W = comm.world
     if W == 1:
         pytest.skip("a group of one has the one-shot kernel only")
-    xs = [whole((n,), F32, n + r) for r in range(W)]
+    xs = [whole((n,), dtype, n + r) for r in range(W)]
     for kw in ({"ctas": 4}, {"slot_bytes": 2048}, {"ctas": 3, "slot_bytes": 4096}):
         ys = comm.all_reduce(xs, **kw)
         assert not comm.last_call()["flags"] & ONE_LAUNCH
@@ -259,12 +307,14 @@ def test_a_geometry_of_the_caller_runs_the_multi_gpu_kernels(comm, n):
         assert last["slot_bytes"] == kw.get("slot_bytes", last["slot_bytes"])
         comm.sync()
         assert all(torch.equal(t.double(), total(xs)) for t in ys + full)
-    x, w = [t[:8].view(1, 8) for t in xs], [torch.ones(8, device="cuda")] * W
+    x, w = [t[:8].view(1, 8) for t in xs], [torch.ones(8, dtype=dtype, device="cuda")] * W
     y = comm.all_reduce_rmsnorm(x, w, ctas=1)
     assert not comm.last_call()["flags"] & ONE_LAUNCH
     comm.sync()
     row = total(x)
-    torch.testing.assert_close(y[0].double(), row * torch.rsqrt(row.pow(2).mean(-1, keepdim=True) + 1e-5), rtol=4e-6, atol=1e-6)
+    # One rounding to the output type on top of the fp32 sum of squares and product.
+    rtol = {F32: 2e-6, F16: 2.0 ** -10, BF16: 2.0 ** -7}[dtype]
+    torch.testing.assert_close(y[0].double(), row * torch.rsqrt(row.pow(2).mean(-1, keepdim=True) + 1e-5), rtol=rtol, atol=1e-6)
 
 
 @pytest.mark.parametrize("row_world", [2, 4])
