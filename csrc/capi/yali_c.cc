@@ -156,6 +156,23 @@ void yali_c_oracle_residual_rmsnorm(const double* sum, const float* residual, co
 void yali_c_fused_linear_counts(uint32_t T, uint32_t N, int world, int oneshot, uint32_t* arrivals, uint32_t* rows_of) {
     FusedLinearCounts(T, N, world, oneshot != 0, arrivals, rows_of);
 }
+void yali_c_fused_tiling(uint32_t T, uint32_t N, int world, int oneshot, uint32_t ksplit, uint32_t pairs, uint32_t* out) {
+    const GemmTiling t = FusedLinearTiling(T, N, world, oneshot != 0, ksplit, pairs);
+    const uint32_t v[5] = {t.span, t.domains, t.tiles, t.tokens, t.group};
+    std::memcpy(out, v, sizeof(v));
+}
+void yali_c_fused_item(const uint32_t* tiling, uint32_t T, uint32_t rank, uint32_t i, uint32_t col_tiles, uint32_t ks_shift,
+                       uint32_t* out) {
+    const GemmTiling t{tiling[0], tiling[1], tiling[2], tiling[3], tiling[4]};
+    const GemmItem it = GemmItemAt(t, T, rank, i, col_tiles, ks_shift);
+    const uint32_t v[5] = {it.tile, it.t0, it.nt, it.col_tile, it.split};
+    std::memcpy(out, v, sizeof(v));
+}
+void yali_c_local_gemm_shape(uint32_t T, uint32_t N, uint32_t kb_total, uint64_t room, uint32_t pairs, int lines, uint32_t* out) {
+    const LocalGemmShape s = LocalGemmShapeFor(T, N, kb_total, room, pairs, lines != 0);
+    const uint32_t v[4] = {s.tiles, s.tokens, s.nsplit, s.kper};
+    std::memcpy(out, v, sizeof(v));
+}
 uint32_t yali_c_fused_linear_oneshot_max_rows(int world) { return FusedLinearOneShotMaxRows(world); }
 uint32_t yali_c_fused_tile_split(uint32_t T, uint32_t N, uint32_t K, int world, uint32_t resident_ctas, uint64_t gemm_cap,
                                  uint32_t want) {

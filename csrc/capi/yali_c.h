@@ -78,7 +78,14 @@ float yali_c_round_fp16(float x);
 void yali_c_oracle_allreduce(const float* const* in, int world, size_t n, double scale, double* out);
 void yali_c_oracle_residual_rmsnorm(const double* sum, const float* residual, const float* weight, size_t rows,
                                     size_t hidden, double eps, double* y, double* pre_norm);
-// Fused linear layer: counter targets per owner (arrays of `world`), default one-shot limit and multicast form.
+/* Fused linear layer: rows and 128 x 256 tiles per owner (arrays of `world`), default one-shot limit and multicast form;
+ * how the tile form cuts T rows for `pairs` pairs of CTAs per rank (out: span, domains, tiles, tokens, group) and its
+ * i-th item on a rank (out: tile, first row, rows, column tile, split); token tiles and K splits of the form for ranks
+ * on one GPU (out: tiles, tokens, nsplit, kper). */
+void yali_c_fused_tiling(uint32_t T, uint32_t N, int world, int oneshot, uint32_t ksplit, uint32_t pairs, uint32_t* out);
+void yali_c_fused_item(const uint32_t* tiling, uint32_t T, uint32_t rank, uint32_t i, uint32_t col_tiles, uint32_t ks_shift,
+                       uint32_t* out);
+void yali_c_local_gemm_shape(uint32_t T, uint32_t N, uint32_t kb_total, uint64_t room, uint32_t pairs, int lines, uint32_t* out);
 /* K splits per 256-column tile of the few-token fused layer (want = 0: the measured rule). */
 uint32_t yali_c_fused_tile_split(uint32_t T, uint32_t N, uint32_t K, int world, uint32_t resident_ctas, uint64_t gemm_cap,
                                  uint32_t want);
@@ -123,13 +130,14 @@ typedef struct YaliSimReport {
 int yali_c_simulate(const YaliSimConfig* cfg, YaliSimReport* rep);
 
 /* Host-thread model of the fused GEMM layer's cross-rank protocol (sim/gemm_protocol_sim.cc):
- * `world` x `ctas` threads, `calls` back-to-back calls of a [rows, col_tiles x 128] layer, two-shot or
+ * `world` x `ctas` threads, `calls` back-to-back calls of a [rows, col_tiles x 256] layer, two-shot or
  * one-shot.  fault: 0 none, 1 rank `fault_rank` stops launching from call `fault_call`, 2 one tile
  * announcement of that rank is lost.  slow_rank (-1: none) sleeps before its reduce phase, so that the
  * other ranks run ahead.  single_parity = 1 removes the double buffering of the landing zones (a
  * negative control: the stamps must then catch the reuse in one-shot mode).  in_switch = 1 models the
  * two-shot form whose owners read every rank's own image.  Same return codes and
- * report as yali_c_simulate; flag_writes counts counter updates. */
+ * report as yali_c_simulate; flag_writes counts announcements of tile units
+ * and updates of the delivered-row counters. */
 typedef struct YaliFusedSimConfig {
     int world, ctas, calls, oneshot;
     uint32_t rows, col_tiles;

@@ -20,7 +20,6 @@ namespace yali {
 constexpr int kMaxFlashCtas = 2048;  // one flag row per CTA of the one-shot kernel
 constexpr int kMaxLanes = 256;       // lanes (CTAs) of the two-shot ring kernel
 constexpr int kBarSlots = 1024;      // per-CTA cross-rank barriers (NVLS and fused kernels)
-constexpr int kGemmRowBlocks = 256;  // arrival counters of the fused GEMM, one per 128-row block
 
 // Call counters of this rank, advanced by the kernels themselves (the last CTA of a launch
 // bumps them), so a launch carries no per-call number and can be replayed from a CUDA graph.
@@ -45,9 +44,8 @@ constexpr uint32_t kRsSeqOff = kFlashFlagOff + kMaxFlashCtas * kMaxRanks;    // 
 constexpr uint32_t kAgSeqOff = kRsSeqOff + kMaxLanes * kMaxRanks;            // [kMaxLanes][kMaxRanks]
 constexpr uint32_t kCreditOff = kAgSeqOff + kMaxLanes * kMaxRanks;           // [kMaxLanes][kMaxRanks]
 constexpr uint32_t kBarOff = kCreditOff + kMaxLanes * kMaxRanks;             // [kBarSlots][kMaxRanks]
-constexpr uint32_t kGemmCntOff = kBarOff + kBarSlots * kMaxRanks;            // [kGemmRowBlocks][kMaxRanks]
-constexpr uint32_t kGemmDoneOff = kGemmCntOff + kGemmRowBlocks * kMaxRanks;  // [kGemmRowBlocks][kMaxRanks]
-constexpr uint32_t kStatusCntOff = kGemmDoneOff + kGemmRowBlocks * kMaxRanks;  // [1] timeouts seen by this rank
+constexpr uint32_t kGemmDoneOff = kBarOff + kBarSlots * kMaxRanks;           // [kMaxRanks] rows the owner has delivered here
+constexpr uint32_t kStatusCntOff = kGemmDoneOff + kMaxRanks;                 // [1] timeouts seen by this rank
 // Device-side timeline of the collectives (kFlagTrace): call i writes %globaltimer at the entry of
 // its first CTA and at the check-out of its last CTA into entry i % kTraceCap.
 constexpr uint32_t kTraceCap = 4096;

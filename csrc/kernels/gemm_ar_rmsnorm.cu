@@ -102,34 +102,9 @@ __device__ __forceinline__ uint64_t landing_nvls_off(const GemmArArgs& a, uint32
     return a.cv.lay.gemm_off + static_cast<uint64_t>(parity) * a.cv.world * a.cv.lay.gemm_cap;
 }
 
-// One work item of a pair.
-struct Item {
-    uint32_t tile;    // token tile, numbered alike on every rank
-    uint32_t t0, nt;  // its rows [t0, t0 + nt); nt = 0: nothing to do
-    uint32_t col_tile, split;
-};
-// Items of a rank in walking order: groups of token tiles, in a group column tile by column tile, token tile by
-// token tile, split by split.  With one domain per owner the k-th tile of every owner comes before the
-// (k+1)-th, starting with the right-hand neighbour's: at any moment the ranks push to different owners, and
-// every owner's rows complete bit by bit.
+using Item = GemmItem;
 __device__ __forceinline__ Item item_at(const GemmArArgs& a, uint32_t i, uint32_t ncol, uint32_t ks_shift) {
-    const GemmTiling& t = a.tl;
-    Item it;
-    it.split = i & ((1u << ks_shift) - 1u);
-    i >>= ks_shift;
-    const uint32_t ntt = t.domains * t.tiles, per_group = t.group * ncol;
-    const uint32_t g = i / per_group, in_g = i - g * per_group;
-    const uint32_t here = min(t.group, ntt - g * t.group);  // the last group may be smaller
-    it.col_tile = in_g / here;
-    const uint32_t pos = g * t.group + in_g % here;
-    const uint32_t b = pos / t.domains;
-    uint32_t dom = pos - b * t.domains;
-    if (t.domains > 1) dom = (dom + a.cv.rank + 1) % t.domains;
-    it.tile = dom * t.tiles + b;
-    it.t0 = dom * t.span + b * t.tokens;
-    const uint32_t end = min(min(a.T, (dom + 1) * t.span), it.t0 + t.tokens);
-    it.nt = end > it.t0 ? end - it.t0 : 0u;
-    return it;
+    return GemmItemAt(a.tl, a.T, static_cast<uint32_t>(a.cv.rank), i, ncol, ks_shift);
 }
 
 // State the roles share.
@@ -191,8 +166,7 @@ __device__ __forceinline__ void row_producer(const GemmArArgs& a, Shared& s, uin
         uint8_t* const mine = ring + group * (kRowRingBytes / kRowGroups);
         uint32_t slot = group ? slots[1] : slots[0], round = group ? rounds[1] : rounds[0];
         const uint32_t grow = m.lo + lr;
-        const uint32_t dom = a.tl.domains > 1 ? grow / a.tl.span : 0u;
-        const uint32_t tile = dom * a.tl.tiles + (grow - dom * a.tl.span) / a.tl.tokens;
+        const uint32_t tile = GemmTileOfRow(a.tl, grow);
         bool late = false;
         if (tile != ready) {
             // The flags of all (128-column unit, K split, source) of the row's token tile, a few per lane.

@@ -10,8 +10,7 @@
 
 namespace yali {
 
-// The tile in which announcements of partial rows were first counted, and which the host-thread model of the
-// protocol and FusedLinearCounts still use.
+// The tile that FusedLinearTileSplit and FusedLinearCounts count in.
 constexpr int kGemmTileM = 128;
 constexpr int kGemmTileN = 256;
 // Tile of the kernel: 256 columns of the output (the M side of the MMA: rows of W, 128 per CTA of a pair) x up to
@@ -29,6 +28,43 @@ constexpr uint32_t kGemmMaxRowVecs = 512;  // 16-byte vectors of a row: N <= 409
 struct GemmTiling {
     uint32_t span, domains, tiles, tokens, group;
 };
+
+// One work item of a pair.
+struct GemmItem {
+    uint32_t tile;    // token tile, numbered alike on every rank
+    uint32_t t0, nt;  // its rows [t0, t0 + nt); nt = 0: nothing to do
+    uint32_t col_tile, split;
+};
+// Items of a rank in walking order: groups of token tiles, in a group column tile by column tile, token tile by
+// token tile, split by split.  With one domain per owner the k-th tile of every owner comes before the
+// (k+1)-th, starting with the right-hand neighbour's: at any moment the ranks push to different owners, and
+// every owner's rows complete bit by bit.  (The host-thread model walks them, too.)
+__host__ __device__ inline GemmItem GemmItemAt(const GemmTiling& t, uint32_t T, uint32_t rank, uint32_t i, uint32_t ncol,
+                                               uint32_t ks_shift) {
+    GemmItem it;
+    it.split = i & ((1u << ks_shift) - 1u);
+    i >>= ks_shift;
+    const uint32_t ntt = t.domains * t.tiles, per_group = t.group * ncol;
+    const uint32_t g = i / per_group, in_g = i - g * per_group;
+    const uint32_t left = ntt - g * t.group, here = t.group < left ? t.group : left;  // the last group may be smaller
+    it.col_tile = in_g / here;
+    const uint32_t pos = g * t.group + in_g % here;
+    const uint32_t b = pos / t.domains;
+    uint32_t dom = pos - b * t.domains;
+    if (t.domains > 1) dom = (dom + rank + 1) % t.domains;
+    it.tile = dom * t.tiles + b;
+    it.t0 = dom * t.span + b * t.tokens;
+    uint32_t end = (dom + 1) * t.span;
+    end = end < T ? end : T;
+    end = end < it.t0 + t.tokens ? end : it.t0 + t.tokens;
+    it.nt = end > it.t0 ? end - it.t0 : 0u;
+    return it;
+}
+// The token tile of a row.
+__host__ __device__ inline uint32_t GemmTileOfRow(const GemmTiling& t, uint32_t row) {
+    const uint32_t dom = t.domains > 1 ? row / t.span : 0u;
+    return dom * t.tiles + (row - dom * t.span) / t.tokens;
+}
 
 struct alignas(64) GemmArArgs {
     CUtensorMap tmap_x;  // x  [T, K] bf16, box 64 x tokens / 2, 128-byte swizzle (rows beyond T read as zeros)

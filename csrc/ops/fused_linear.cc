@@ -177,24 +177,20 @@ uint32_t FusedLinearDecodeMaxRows(const HeapLayout& lay, uint32_t N, int world) 
     return static_cast<uint32_t>(std::min<uint64_t>(rows, kGemmDecodeMaxRows));
 }
 
-// Counter targets of one call: every source announces each 128x128 tile once to every owner
-// that has rows in the tile's row block (one-shot: to everybody), and every owner reports the
-// rows it delivered.  The kernel's announcer warp applies the same rule tile by tile.
+// Rows that every owner delivers to every rank in one call: the targets of the delivered-row counters.
+void FusedLinearRows(uint32_t T, int W, bool oneshot, uint32_t* rows_of) {
+    const uint32_t Rs = (T + W - 1) / W;
+    for (int q = 0; q < W; ++q) rows_of[q] = oneshot ? 0u : std::min<uint32_t>(Rs, T - std::min<uint32_t>(T, q * Rs));
+}
+
+// The same, and how many 128 x 256 tiles of the partial sums hold rows of every owner (one-shot: all of them).  For the
+// C API: no kernel counts such tiles any more, a unit of sums is announced by the call's number.
 void FusedLinearCounts(uint32_t T, uint32_t N, int W, bool oneshot, uint32_t* arrivals, uint32_t* rows_of) {
-    const uint32_t ntm = (T + kGemmTileM - 1) / kGemmTileM, ntn = (N + kGemmTileN - 1) / kGemmTileN;
-    const uint32_t Rs = oneshot ? T : (T + W - 1) / W;
+    const uint32_t ntm = (T + kGemmTileM - 1) / kGemmTileM, ntn = (N + kGemmTileN - 1) / kGemmTileN, Rs = (T + W - 1) / W;
+    FusedLinearRows(T, W, oneshot, rows_of);
     for (int q = 0; q < W; ++q) {
-        arrivals[q] = rows_of[q] = 0;
-        if (oneshot) {
-            arrivals[q] = ntm * ntn;
-        } else {
-            const uint32_t lo = std::min<uint32_t>(T, q * Rs), hi = std::min<uint32_t>(T, lo + Rs);
-            if (hi > lo) {
-                const uint32_t first = lo / kGemmTileM, last = (hi - 1) / kGemmTileM;
-                arrivals[q] = (last - first + 1) * ntn;
-            }
-            rows_of[q] = hi - lo;
-        }
+        const uint32_t lo = q * Rs, hi = lo + rows_of[q];
+        arrivals[q] = oneshot ? ntm * ntn : rows_of[q] ? ((hi - 1) / kGemmTileM - lo / kGemmTileM + 1) * ntn : 0u;
     }
 }
 
@@ -561,8 +557,8 @@ Result FusedLinearAllReduceRmsNorm(Communicator& comm, const FusedLinearDesc* de
     const bool nvls = mc_mode == 1;
 
     // Rows every owner delivers in this call.
-    uint32_t arrivals[kMaxRanks] = {}, rows_of[kMaxRanks] = {};
-    FusedLinearCounts(T, N, W, oneshot, arrivals, rows_of);
+    uint32_t rows_of[kMaxRanks] = {};
+    FusedLinearRows(T, W, oneshot, rows_of);
     const void* fn = GemmArKernel(comm.emulated());
     const uint32_t smem = GemmArSmemBytes();
     // The dynamic shared-memory limit is a per-device property of the kernel: raise it once for every

@@ -62,6 +62,7 @@ LocalGemmShape LocalGemmShapeFor(uint32_t T, uint32_t N, uint32_t kb_total, uint
 uint32_t FusedLinearOneShotMaxRows(int world);
 int FusedLinearAutoMulticastMode(int world, uint32_t T);
 // Per owner q: tile announcements it receives from EACH source, and rows it delivers (arrays of W).
+void FusedLinearRows(uint32_t T, int W, bool oneshot, uint32_t* rows_of);
 void FusedLinearCounts(uint32_t T, uint32_t N, int W, bool oneshot, uint32_t* arrivals, uint32_t* rows_of);
 
 }  // namespace yali

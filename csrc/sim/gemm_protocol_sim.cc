@@ -1,12 +1,12 @@
 // Host-thread model of the fused GEMM layer's cross-rank protocol (yali_c.h,
-// yali_c_simulate_fused).  One host thread plays one CTA of one rank.  What it
+// yali_c_simulate_fused).  One host thread plays one pair of CTAs of one rank.  What it
 // models is everything of kernels/gemm_ar_rmsnorm.cu that involves another rank:
-// the walk over the tiles (rotated per rank), the push of partial rows into the
-// owner's landing zone of the call's parity, the arrival counters with the
-// host-computed targets (ops/fused_linear.cc, FusedLinearCounts), the reduction of
-// the owned rows, the delivery into every rank's output, the delivered-row counters
-// and the call words that the last CTA of a launch advances.  A "row segment" is one
-// float per (row, column tile); the GEMM itself is a formula of (rank, call, row,
+// the walk over the items (the kernel's own functions, rotated per rank), the push of partial rows into the
+// owner's landing zone of the call's parity, the call number that a source writes into the flag of a tile unit when
+// its part has landed, rows that are reduced tile by tile as the flags of their tile arrive, the delivery
+// into every rank's output, the delivered-row counters with their host-computed increments (ops/fused_linear.cc,
+// FusedLinearRows) and the call words, which the last CTA to have read them advances at the START of a call.
+// A "row segment" is one float per (row, column tile); the GEMM itself is a formula of (rank, call, row,
 // column tile).  Calls follow one another with no barrier between ranks; CTAs of one
 // rank meet between calls, as kernels of one stream do.
 //
@@ -63,15 +63,17 @@ struct Cell {
 struct FusedShared {
     YaliFusedSimConfig cfg;
     int W, C;
-    uint32_t T, ntn, ntm, bm, Rs;
+    uint32_t T, ntn, Rs;
+    yali::GemmTiling tl;
     // landing[on_rank]: [parity][src][row_local][nt]
     std::vector<std::unique_ptr<Cell[]>> landing;
     // out[on_rank]: [row][nt]
     std::vector<std::unique_ptr<Cell[]>> out;
-    // counters per rank: arrivals[src], delivered[owner]; call words: epoch, cnt target, done targets
+    std::vector<std::unique_ptr<std::atomic<uint32_t>[]>> flags;  // [on_rank]: [tile][nt][src], call numbers
+    // delivered rows per owner; call words: calls so far, rows each owner has been asked for, CTAs that have read them
     struct Words {
-        std::atomic<uint32_t> cnt[yali::kMaxRanks], done[yali::kMaxRanks];
-        std::atomic<uint32_t> epoch{0}, cnt_base{0}, done_base[yali::kMaxRanks], checked_out{0};
+        std::atomic<uint32_t> done[yali::kMaxRanks];
+        std::atomic<uint32_t> epoch{0}, done_base[yali::kMaxRanks], checked_in{0};
     };
     std::unique_ptr<Words[]> words;
     std::vector<std::unique_ptr<RankBarrier>> barrier;
@@ -84,6 +86,9 @@ struct FusedShared {
     }
     size_t LandingIndex(uint32_t parity, int src, uint32_t row_local, uint32_t nt) const {
         return ((static_cast<size_t>(parity) * W + src) * Rs + row_local) * ntn + nt;
+    }
+    std::atomic<uint32_t>& Flag(int on_rank, uint32_t tile, uint32_t nt, int src) {
+        return flags[on_rank][(static_cast<size_t>(tile) * ntn + nt) * W + src];
     }
 };
 
@@ -120,23 +125,30 @@ struct RankStop {
 void FusedCta(FusedShared& s, std::vector<RankStop>& stop, int r, int c) {
     const int W = s.W, C = s.C;
     const bool oneshot = s.cfg.oneshot != 0;
-    const uint32_t T = s.T, ntn = s.ntn, ntm = s.ntm, bm = s.bm, Rs = s.Rs;
-    uint32_t arrivals[yali::kMaxRanks], rows_of[yali::kMaxRanks];
-    yali::FusedLinearCounts(T, ntn * yali::kGemmTileN, W, oneshot, arrivals, rows_of);
+    const uint32_t T = s.T, ntn = s.ntn, Rs = s.Rs;
+    uint32_t rows_of[yali::kMaxRanks];
+    yali::FusedLinearRows(T, W, oneshot, rows_of);
     FusedShared::Words& mine = s.words[r];
-    const uint32_t shift = oneshot ? 0u : (((static_cast<uint32_t>(r) + 1u) % W) * Rs / bm) % ntm;
+    const uint32_t nitems = s.tl.domains * s.tl.tiles * ntn;
     for (int call = 0; call < s.cfg.calls; ++call) {
         if (s.cfg.fault == 1 && r == s.cfg.fault_rank && call >= s.cfg.fault_call) break;  // stops launching
-        // Call words as the previous launch of this rank left them.
-        const uint32_t epoch = mine.epoch.load(std::memory_order_acquire);
-        const uint32_t parity = s.cfg.single_parity ? 0u : ((epoch + 1u) & 1u);
-        const uint32_t cnt_wanted = mine.cnt_base.load() + arrivals[r];
+        // Call words as the previous launch of this rank left them; the last CTA that has read them advances them.
+        const uint32_t epoch = mine.epoch.load(std::memory_order_acquire) + 1u;
+        uint32_t done_wanted[yali::kMaxRanks];
+        for (int q = 0; q < W; ++q) done_wanted[q] = mine.done_base[q].load() + rows_of[q];
+        if (mine.checked_in.fetch_add(1) == static_cast<uint32_t>(C) - 1) {
+            mine.checked_in.store(0);
+            mine.epoch.store(epoch, std::memory_order_release);
+            for (int q = 0; q < W; ++q) mine.done_base[q].store(done_wanted[q]);
+        }
+        const uint32_t parity = s.cfg.single_parity ? 0u : (epoch & 1u);
         const uint64_t stamp = static_cast<uint64_t>(call) + 1;
         bool ok = true;
-        // ---- phase 1: tiles -> owners' landing zones, then one announcement per owner touched
-        for (uint32_t tile = c; tile < ntm * ntn; tile += C) {
-            const uint32_t mt = (tile / ntn + shift) % ntm, nt = tile % ntn;
-            const uint32_t lo = mt * bm, hi = std::min(T, lo + bm);
+        // ---- items -> owners' landing zones, then the call number into the unit's flag on every owner touched
+        for (uint32_t i = c; i < nitems; i += C) {
+            const yali::GemmItem it = yali::GemmItemAt(s.tl, T, r, i, ntn, 0);
+            const uint32_t nt = it.col_tile, lo = it.t0, hi = it.t0 + it.nt;
+            if (it.nt == 0) continue;
             for (uint32_t row = lo; row < hi; ++row) {
                 const float v = Partial(r, call, row, nt);
                 if (s.cfg.in_switch) {
@@ -158,60 +170,58 @@ void FusedCta(FusedShared& s, std::vector<RankStop>& stop, int r, int c) {
             for (int q = 0; q < W; ++q) {
                 const bool touched = oneshot || (static_cast<uint32_t>(q) * Rs < hi && (static_cast<uint32_t>(q) + 1) * Rs > lo);
                 if (!touched) continue;
-                if (s.cfg.fault == 2 && r == s.cfg.fault_rank && call == s.cfg.fault_call && tile == static_cast<uint32_t>(c))
+                if (s.cfg.fault == 2 && r == s.cfg.fault_rank && call == s.cfg.fault_call && i == static_cast<uint32_t>(c))
                     continue;  // this announcement is lost
-                s.words[q].cnt[r].fetch_add(1, std::memory_order_release);
+                s.Flag(q, it.tile, nt, r).store(epoch, std::memory_order_release);
                 s.counter_writes.fetch_add(1, std::memory_order_relaxed);
             }
         }
         if (r == s.cfg.slow_rank) std::this_thread::sleep_for(std::chrono::milliseconds(2));
-        // ---- phase 2: reduce the owned rows, deliver them
+        // ---- reduce the owned rows as the flags of their token tile arrive, deliver them
         const uint32_t row_lo = oneshot ? 0u : std::min(T, static_cast<uint32_t>(r) * Rs);
         const uint32_t row_hi = oneshot ? T : std::min(T, row_lo + Rs);
         const uint32_t my_rows = row_hi - row_lo;
-        if (my_rows > 0) {
-            for (int src = 0; src < W && ok; ++src) ok = WaitCounter(s, mine.cnt[src], cnt_wanted, r, src, 1);
-            uint32_t rows_done = 0;
-            for (uint32_t lr = c; ok && lr < my_rows; lr += C) {
-                const uint32_t grow = row_lo + lr;
-                for (uint32_t nt = 0; nt < ntn; ++nt) {
-                    float sum = 0.f;
-                    for (int src = 0; src < W; ++src) {
-                        // in-switch form: the switch reads every rank's own image at the row's offset
-                        Cell& cell = s.cfg.in_switch ? s.landing[src][s.ImageIndex(parity, grow, nt)]
-                                                     : s.landing[r][s.LandingIndex(parity, src, lr, nt)];
-                        if (cell.stamp.load(std::memory_order_acquire) != stamp) s.violations.fetch_add(1);
-                        sum += cell.value;
-                        cell.stamp.store(0, std::memory_order_release);
-                    }
-                    for (int d = 0; d < W; ++d) {
-                        if (oneshot && d != r) continue;
-                        Cell& o = s.out[d][static_cast<size_t>(grow) * ntn + nt];
-                        if (o.stamp.load(std::memory_order_acquire) != 0) s.violations.fetch_add(1);  // not consumed yet
-                        o.value = sum;
-                        o.stamp.store(stamp, std::memory_order_release);
-                    }
+        uint32_t rows_done = 0, ready = ~0u;
+        for (uint32_t lr = c; ok && lr < my_rows; lr += C) {
+            const uint32_t grow = row_lo + lr, tile = yali::GemmTileOfRow(s.tl, grow);
+            if (tile != ready)
+                for (uint32_t nt = 0; ok && nt < ntn; ++nt)
+                    for (int src = 0; src < W && ok; ++src) ok = WaitCounter(s, s.Flag(r, tile, nt, src), epoch, r, src, 1);
+            if (!ok) break;
+            ready = tile;
+            for (uint32_t nt = 0; nt < ntn; ++nt) {
+                float sum = 0.f;
+                for (int src = 0; src < W; ++src) {
+                    // in-switch form: the switch reads every rank's own image at the row's offset
+                    Cell& cell = s.cfg.in_switch ? s.landing[src][s.ImageIndex(parity, grow, nt)]
+                                                 : s.landing[r][s.LandingIndex(parity, src, lr, nt)];
+                    if (cell.stamp.load(std::memory_order_acquire) != stamp) s.violations.fetch_add(1);
+                    sum += cell.value;
+                    cell.stamp.store(0, std::memory_order_release);
                 }
-                ++rows_done;
+                for (int d = 0; d < W; ++d) {
+                    if (oneshot && d != r) continue;
+                    Cell& o = s.out[d][static_cast<size_t>(grow) * ntn + nt];
+                    if (o.stamp.load(std::memory_order_acquire) != 0) s.violations.fetch_add(1);  // not consumed yet
+                    o.value = sum;
+                    o.stamp.store(stamp, std::memory_order_release);
+                }
             }
-            if (!oneshot && rows_done > 0)
-                for (int q = 0; q < W; ++q) {
-                    s.words[q].done[r].fetch_add(rows_done, std::memory_order_release);
-                    s.counter_writes.fetch_add(1, std::memory_order_relaxed);
-                }
+            ++rows_done;
         }
+        if (!oneshot && rows_done > 0)
+            for (int q = 0; q < W; ++q) {
+                s.words[q].done[r].fetch_add(rows_done, std::memory_order_release);
+                s.counter_writes.fetch_add(1, std::memory_order_relaxed);
+            }
         if (!oneshot && c == 0)
-            for (int q = 0; q < W && ok; ++q)
-                ok = WaitCounter(s, mine.done[q], mine.done_base[q].load() + rows_of[q], r, q, 2);
-        // ---- the launch ends when all its CTAs have; the last one advances the call words, then the
-        // rank's stream consumes the output before it launches the next call.
+            for (int q = 0; q < W && ok; ++q) ok = WaitCounter(s, mine.done[q], done_wanted[q], r, q, 2);
+        // ---- the launch ends when all its CTAs have; then the rank's stream consumes the output before it launches the
+        // next call.
         s.barrier[r]->wait();
         if (c == 0) {
             const bool aborted = s.abort.load();
             if (!aborted) {
-                mine.epoch.fetch_add(1, std::memory_order_release);
-                mine.cnt_base.fetch_add(arrivals[r]);
-                for (int q = 0; q < W; ++q) mine.done_base[q].fetch_add(rows_of[q]);
                 for (uint32_t row = 0; row < T; ++row)
                     for (uint32_t nt = 0; nt < ntn; ++nt) {
                         Cell& o = s.out[r][static_cast<size_t>(row) * ntn + nt];
@@ -241,7 +251,7 @@ struct DecodeShared {
     // lines[on_rank]: [parity][src rank][split][row][tile]
     std::vector<std::unique_ptr<std::atomic<uint64_t>[]>> lines;
     std::vector<std::unique_ptr<Cell[]>> out;  // [row][tile]
-    std::unique_ptr<std::atomic<uint32_t>[]> call_word;  // per rank: calls completed
+    std::unique_ptr<std::atomic<uint32_t>[]> call_word, checked_in;  // per rank: calls so far, CTAs that have read that
     std::vector<std::unique_ptr<RankBarrier>> barrier;
     std::atomic<uint64_t> timeouts{0}, violations{0}, mismatches{0}, line_writes{0};
     std::atomic<int> t_rank{-1}, t_peer{-1}, t_site{0};
@@ -261,6 +271,10 @@ void DecodeCta(DecodeShared& s, std::vector<RankStop>& stop, int r, int c) {
     for (int call = 0; call < s.cfg.calls; ++call) {
         if (s.cfg.fault == 1 && r == s.cfg.fault_rank && call >= s.cfg.fault_call) break;  // stops launching
         const uint32_t number = s.call_word[r].load(std::memory_order_acquire) + 1u;  // this call, never 0
+        if (s.checked_in[r].fetch_add(1) == static_cast<uint32_t>(C) - 1) {  // the last CTA that has read it
+            s.checked_in[r].store(0);
+            s.call_word[r].store(number, std::memory_order_release);
+        }
         const uint32_t parity = s.cfg.single_parity ? 0u : (number & 1u);
         // ---- phase 1: every row of every item of this CTA to every rank
         for (uint32_t item = c; item < ntn * ks; item += C) {
@@ -326,12 +340,11 @@ void DecodeCta(DecodeShared& s, std::vector<RankStop>& stop, int r, int c) {
                 o.stamp.store(static_cast<uint64_t>(call) + 1, std::memory_order_release);
             }
         }
-        // ---- end of the launch: the last CTA advances the call word; the stream consumes the output
+        // ---- end of the launch: the stream consumes the output
         s.barrier[r]->wait();
         if (c == 0) {
             const bool aborted = s.abort.load();
             if (!aborted) {
-                s.call_word[r].fetch_add(1, std::memory_order_release);
                 for (uint32_t row = 0; row < T; ++row)
                     for (uint32_t tile = 0; tile < ntn; ++tile) {
                         Cell& o = s.out[r][static_cast<size_t>(row) * ntn + tile];
@@ -361,11 +374,13 @@ int SimulateDecode(const YaliFusedSimConfig* cfg, YaliSimReport* rep) {
     s.ks = static_cast<uint32_t>(cfg->ksplit);
     const size_t nlines = 2ull * s.W * s.ks * s.T * s.ntn;
     s.call_word.reset(new std::atomic<uint32_t>[s.W]);
+    s.checked_in.reset(new std::atomic<uint32_t>[s.W]);
     for (int r = 0; r < s.W; ++r) {
         s.lines.emplace_back(new std::atomic<uint64_t>[nlines]);
         for (size_t i = 0; i < nlines; ++i) s.lines[r][i].store(0);
         s.out.emplace_back(new Cell[static_cast<size_t>(s.T) * s.ntn]);
         s.call_word[r].store(0);
+        s.checked_in[r].store(0);
         s.barrier.emplace_back(new RankBarrier(s.C));
     }
     std::vector<RankStop> stop(s.W);
@@ -402,18 +417,19 @@ extern "C" int yali_c_simulate_fused(const YaliFusedSimConfig* cfg, YaliSimRepor
     s.C = cfg->ctas;
     s.T = cfg->rows;
     s.ntn = cfg->col_tiles;
-    s.bm = yali::kGemmTileM;
-    s.ntm = (s.T + s.bm - 1) / s.bm;
     s.Rs = cfg->oneshot ? s.T : (s.T + s.W - 1) / s.W;
     if (cfg->in_switch && cfg->oneshot) return -1;  // the in-switch form is a two-shot form
     const size_t nland = std::max<size_t>(2ull * s.W * s.Rs * s.ntn, 2ull * s.T * s.ntn);
     const size_t nout = static_cast<size_t>(s.T) * s.ntn;
     s.words.reset(new FusedShared::Words[s.W]);
+    s.tl = yali::FusedLinearTiling(s.T, s.ntn * yali::kGemmPairCols, s.W, cfg->oneshot != 0, 1, static_cast<uint32_t>(s.C));
+    const size_t nflags = static_cast<size_t>(s.tl.domains) * s.tl.tiles * s.ntn * s.W;
     for (int r = 0; r < s.W; ++r) {
         s.landing.emplace_back(new Cell[nland]);
         s.out.emplace_back(new Cell[nout]);
+        s.flags.emplace_back(new std::atomic<uint32_t>[nflags]);
+        for (size_t i = 0; i < nflags; ++i) s.flags[r][i].store(0);
         for (int q = 0; q < yali::kMaxRanks; ++q) {
-            s.words[r].cnt[q].store(0);
             s.words[r].done[q].store(0);
             s.words[r].done_base[q].store(0);
         }

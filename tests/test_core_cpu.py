@@ -418,3 +418,55 @@ def test_fused_linear_counter_targets_match_the_kernels_announcements(native_lib
     assert lib.yali_c_fused_linear_oneshot_max_rows(2) >= lib.yali_c_fused_linear_oneshot_max_rows(8) >= 1
     assert lib.yali_c_fused_linear_multicast_mode(2, 2048) == 0
     assert lib.yali_c_fused_linear_multicast_mode(8, 128) in (1, 2) and lib.yali_c_fused_linear_multicast_mode(8, 2048) in (1, 2)
+
+
+@pytest.mark.parametrize("world", [2, 3, 8])
+@pytest.mark.parametrize("oneshot", [0, 1])
+def test_fused_linear_items_cover_every_row_and_column_once(native_lib, world, oneshot):
+    """The kernel's walk over its tiles: on every rank each (row, 256 columns, K split) is in exactly one item, tiles are numbered
+    alike on all ranks, and the flags of the tile units fit their region."""
+    import ctypes
+    lib = native_lib
+    for T, N, ks, pairs in [(t, n, k, p) for t in [1, 31, 32, 33, 255, 256, 257, 300, 2048] for n, k, p in
+                            [(128, 1, 74), (384, 1, 9), (4096, 4 if oneshot else 1, 37)]]:
+        tl, it = (ctypes.c_uint32 * 5)(), (ctypes.c_uint32 * 5)()
+        lib.yali_c_fused_tiling(T, N, world, oneshot, ks, pairs, tl)
+        span, domains, tiles, tokens, group = tl
+        assert tokens % 32 == 0 and 32 <= tokens <= 256 and tiles * tokens >= span and domains * span >= T
+        assert domains * tiles * (N // 128) * ks <= 4096
+        ncol, shift = -(-N // 256), ks.bit_length() - 1
+        rows_of_tile = {}
+        for rank in range(world):
+            seen = set()
+            for i in range(domains * tiles * ncol * ks):
+                lib.yali_c_fused_item(tl, T, rank, i, ncol, shift, it)
+                tile, t0, nt, col, split = it
+                assert nt <= tokens and (nt == 0 or t0 + nt <= T) and col < ncol and split < ks
+                assert rows_of_tile.setdefault(tile, (t0, nt)) == (t0, nt)
+                assert (tile, col, split) not in seen
+                seen.add((tile, col, split))
+            assert len(seen) == domains * tiles * ncol * ks
+        covered = sorted(r for t0, nt in rows_of_tile.values() for r in range(t0, t0 + nt))
+        assert covered == list(range(T)), (T, N, tuple(tl))
+
+
+@pytest.mark.parametrize("world", [2, 3, 8])
+def test_shape_of_the_fused_layer_for_ranks_on_one_gpu(native_lib, world):
+    """Token tiles, K splits: every row and k-block is covered, no split is empty, sums and flags fit what the heap has."""
+    import ctypes
+    lib, out = native_lib, (ctypes.c_uint32 * 4)()
+    cap = max(4, -(-16 // world)) << 20  # bytes per (call parity, source) of the landing zone
+    room = 2 * world * cap
+    for N in (128, 384, 1024, 4096):
+        most = min(room, world * cap) // (N * 2)  # rows that the call takes at most
+        for T in [t for t in (1, 8, 31, 33, 64, 257, 300, 2048, most) if t <= most]:
+            for K in (64, 192, 2048, 8192):
+                for pairs in (1, 66, 74):
+                    for lines in (0, 1):
+                        kb = world * K // 64
+                        lib.yali_c_local_gemm_shape(T, N, kb, room, pairs, lines, out)
+                        tiles, tokens, nsplit, kper = out
+                        assert tokens % 32 == 0 and 32 <= tokens <= 256 and (tiles - 1) * tokens < T <= tiles * tokens
+                        assert 1 <= nsplit <= 8 and (nsplit - 1) * kper < kb <= nsplit * kper
+                        assert nsplit == 1 or T * N * 2 * nsplit <= room
+                        assert tiles * (N // 128) * nsplit <= 16384

@@ -93,6 +93,9 @@ def _declare(lib: ctypes.CDLL) -> None:
         "yali_c_oracle_allreduce": (None, [vp, i32, c.c_size_t, f64, vp]),
         "yali_c_oracle_residual_rmsnorm": (None, [vp, vp, vp, c.c_size_t, c.c_size_t, f64, vp, vp]),
         "yali_c_fused_linear_counts": (None, [c.c_uint32, c.c_uint32, i32, i32, vp, vp]),
+        "yali_c_fused_tiling": (None, [u32, u32, i32, i32, u32, u32, vp]),
+        "yali_c_fused_item": (None, [vp, u32, u32, u32, u32, u32, vp]),
+        "yali_c_local_gemm_shape": (None, [u32, u32, u32, u64, u32, i32, vp]),
         "yali_c_fused_decode_split": (u32, [u32, u32, u32, i32, u32, u64, u32]),
         "yali_c_fused_decode_tile": (u32, [u32, u32, u32]),
         "yali_c_fused_tile_split": (u32, [u32, u32, u32, i32, u32, u64, u32]),
