@@ -38,8 +38,8 @@
 // Parity: none in the reference (no GEMM, no fused op, no tensor-core code there).
 #include <cuda.h>
 
-#include "coll_common.cuh"
 #include "gemm_ar_rmsnorm.h"
+#include "tc_common.cuh"
 
 namespace yali {
 
@@ -54,21 +54,6 @@ constexpr uint32_t kDRingBytes = 160 * 1024;
 constexpr uint32_t kDSmemBytes = kDRingBytes + 1024;  // + slack to align the base
 constexpr uint32_t kDTmemCols = 2 * DBNMax;           // two accumulators of up to 256 fp32 columns: all of TMEM
 constexpr int kDEpilogueWarps = 8;                    // lane quarters 0 and 1, four column groups of 32 or 64 each
-
-// D = fp32, A = B = bf16, both K-major, N at bit 17 (>>3), M at bit 24 (>>4).
-__device__ __forceinline__ uint32_t decode_idesc(uint32_t n) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((n >> 3) << 17) | (static_cast<uint32_t>(DBM >> 4) << 24);
-}
-
-__device__ __forceinline__ uint64_t desc_sw128(uint32_t smem_addr) {
-    uint64_t d = 0;
-    d |= static_cast<uint64_t>((smem_addr & 0x3ffffu) >> 4);
-    d |= static_cast<uint64_t>(1) << 16;
-    d |= static_cast<uint64_t>(1024 >> 4) << 32;
-    d |= static_cast<uint64_t>(1) << 46;
-    d |= static_cast<uint64_t>(2) << 61;
-    return d;
-}
 
 // Flag-in-data landing zone of source (rank `src`, K split `ks`) on every rank: at offset gemm_ll_off +
 // (parity * world + src) * gemm_ll_cap + ks * (gemm_ll_cap / ksplit) of the heap, cut into 32-column tiles:
@@ -184,7 +169,7 @@ __device__ __forceinline__ void decode_body(const GemmDecodeArgs& a, const CUten
                 }
                 ptx::tc_fence_after_sync();
                 const uint32_t d_tmem = tmem + b * DBNMax;
-                const uint32_t idesc = decode_idesc(DBN);
+                const uint32_t idesc = mma_idesc_bf16(DBM, DBN);
                 for (uint32_t kb = kb_begin; kb < kb_end; ++kb) {
                     if (!mbar_wait_deadline(&full_bar[s], round & 1u, deadline, abort_flag)) {
                         if (!*abort_flag) report_timeout(cv, kSiteMbar, r, cta, 12, round * stages + s);
@@ -192,8 +177,8 @@ __device__ __forceinline__ void decode_body(const GemmDecodeArgs& a, const CUten
                         break;
                     }
                     ptx::tc_fence_after_sync();
-                    const uint64_t da = desc_sw128(ptx::smem_u32(smem + s * a_bytes));
-                    const uint64_t db = desc_sw128(ptx::smem_u32(smem_b + s * kDStageB));
+                    const uint64_t da = smem_desc_sw128(ptx::smem_u32(smem + s * a_bytes));
+                    const uint64_t db = smem_desc_sw128(ptx::smem_u32(smem_b + s * kDStageB));
 #pragma unroll
                     for (int k = 0; k < DBK / 16; ++k)
                         ptx::tc_mma_f16(d_tmem, da + 2 * k, db + 2 * k, idesc, (kb != kb_begin || k != 0) ? 1u : 0u);

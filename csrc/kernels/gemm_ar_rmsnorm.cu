@@ -47,8 +47,8 @@
 // GEMM, all-reduce, separate norm kernel) is kept in Python as the baseline.
 #include <cuda.h>
 
-#include "coll_common.cuh"
 #include "gemm_ar_rmsnorm.h"
+#include "tc_common.cuh"
 
 namespace yali {
 
@@ -74,23 +74,6 @@ constexpr uint32_t kRowBarrier = 1 + kEpiGroups;  // named barriers: 1.. epilogu
 static_assert(kRowGroups == 2 && kRowRingBytes / kRowGroups >= 2 * kGemmMaxRowVecs * 16, "two rows at least");
 static_assert(kTmemCols == 512 && kGemmThreads == 32 * (kRowTmaWarp + 1), "one CTA per SM");
 static_assert(kSmemBytes + kEpiGroups * kEpiBufBytes + 1024 <= 227 * 1024, "shared memory of one SM");
-
-// tcgen05 instruction descriptor: D = fp32, A = B = bf16, both K-major, N at bit 17 (>>3), M at bit 24 (>>4).
-__device__ __forceinline__ uint32_t pair_idesc(uint32_t n) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((n >> 3) << 17) | ((kGemmPairCols >> 4) << 24);
-}
-
-// Shared-memory matrix descriptor of a K-major operand tile stored by TMA with 128-byte
-// swizzle: rows of 128 bytes, groups of 8 rows 1024 bytes apart.
-__device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t smem_addr) {
-    uint64_t d = 0;
-    d |= static_cast<uint64_t>((smem_addr & 0x3ffffu) >> 4);  // start address
-    d |= static_cast<uint64_t>(1) << 16;                      // leading byte offset (unused with swizzle)
-    d |= static_cast<uint64_t>(1024 >> 4) << 32;              // stride byte offset: next 8-row group
-    d |= static_cast<uint64_t>(1) << 46;                      // descriptor version of sm_100
-    d |= static_cast<uint64_t>(2) << 61;                      // SWIZZLE_128B
-    return d;
-}
 
 // Landing zone of the partial rows of source `src` on a rank, relative to that rank's heap base.
 __device__ __forceinline__ uint64_t landing_off(const GemmArArgs& a, int src, uint32_t parity) {
@@ -119,15 +102,6 @@ struct Shared {
     uint32_t call[1 + kMaxRanks];
     float red[kRowGroups][2][kRowWarps];  // sums of squares of the row warps, two rows alternating
 };
-
-// Bounded waits: give up at the deadline or when another role of this CTA has.
-__device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity, uint64_t deadline, volatile int* abort) {
-    uint32_t tries = 0;
-    while (!ptx::mbar_try_wait_cluster(bar, parity)) {
-        if ((++tries & 15u) == 0 && (*abort || ptx::globaltimer() > deadline)) return false;
-    }
-    return true;
-}
 
 // The rows this rank normalises (CTA c takes rows c, c + nctas, ...) and how they travel through the row ring.
 struct MyRows {
@@ -441,7 +415,7 @@ __device__ __forceinline__ void gemm_ar_body(const GemmArArgs& a, uint32_t cta, 
         }
     } else if (warp == kMmaWarp) {
         if (half == 0 && ptx::elect_one()) {
-            const uint32_t idesc = pair_idesc(a.tl.tokens);
+            const uint32_t idesc = mma_idesc_bf16(kGemmPairCols, a.tl.tokens);
             uint32_t st = 0, round = 0, n = 0;
             for (uint32_t i = pair; i < nitems && !s.abort; i += npairs) {
                 const Item it = item_at(a, i, ncol, ks_shift);

@@ -30,8 +30,8 @@
 // Parity: none in the reference (it has no GEMM, no fused op and no tensor-core code).
 #include <cuda.h>
 
-#include "coll_common.cuh"
 #include "gemm_local.h"
+#include "tc_common.cuh"
 
 namespace yali {
 
@@ -51,23 +51,6 @@ constexpr uint32_t kNumberBarrier = 1;  // named barrier: the announcer has read
 constexpr uint32_t kPrefetchBlocks = 8;  // how far the prefetch warp runs ahead of the loads, in k-blocks
 static_assert(kTmemCols == 512 && kLocalGemmThreads == 32 * (kPrefetchWarp + 1), "one CTA per SM");
 static_assert(kSmemBytes + kEpilogueWarps * kEpiBufBytes + 1024 <= 216 * 1024, "leaves room for CTAs of the second kernel");
-
-// tcgen05 instruction descriptor: D = fp32, A = B = bf16, both K-major, N at bit 17 (>>3), M at bit 24 (>>4).
-__device__ __forceinline__ uint32_t pair_idesc(uint32_t n) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | ((n >> 3) << 17) | ((kLocalGemmPairCols >> 4) << 24);
-}
-
-// Shared-memory matrix descriptor of a K-major operand tile stored by TMA with 128-byte
-// swizzle: rows of 128 bytes, groups of 8 rows 1024 bytes apart.
-__device__ __forceinline__ uint64_t smem_desc_sw128(uint32_t smem_addr) {
-    uint64_t d = 0;
-    d |= static_cast<uint64_t>((smem_addr & 0x3ffffu) >> 4);  // start address
-    d |= static_cast<uint64_t>(1) << 16;                      // leading byte offset (unused with swizzle)
-    d |= static_cast<uint64_t>(1024 >> 4) << 32;              // stride byte offset: next 8-row group
-    d |= static_cast<uint64_t>(1) << 46;                      // descriptor version of sm_100
-    d |= static_cast<uint64_t>(2) << 61;                      // SWIZZLE_128B
-    return d;
-}
 
 struct Item {
     uint32_t tile;  // token tile
@@ -96,15 +79,6 @@ struct Shared {
     volatile uint32_t loaded;  // k-blocks whose loads have been issued
     volatile int abort;
 };
-
-// Bounded waits: give up at the deadline or when another role of this CTA has.
-__device__ __forceinline__ bool wait_bar(uint64_t* bar, uint32_t parity, uint64_t deadline, volatile int* abort) {
-    uint32_t tries = 0;
-    while (!ptx::mbar_try_wait_cluster(bar, parity)) {
-        if ((++tries & 15u) == 0 && (*abort || ptx::globaltimer() > deadline)) return false;
-    }
-    return true;
-}
 
 }  // namespace
 
@@ -201,7 +175,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kLocalGemmThreads, 1
         }
     } else if (warp == kMmaWarp) {
         if (half == 0 && ptx::elect_one()) {
-            const uint32_t idesc = pair_idesc(a.s.tokens);
+            const uint32_t idesc = mma_idesc_bf16(kLocalGemmPairCols, a.s.tokens);
             uint32_t st = 0, round = 0, n = 0;
             Item it;
             for (; !s.abort && item_at(a, n, pair, npairs, ncol, &it); ++n) {

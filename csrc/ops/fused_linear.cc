@@ -135,7 +135,7 @@ bool EncodeTileMap(const DriverApi* d, CUtensorMap* map, const void* base, uint6
 }  // namespace
 
 // Up to how many rows every rank receives all partial rows and normalises all of them itself (one NVLink
-// phase instead of two, (W - 1) times the bytes).  Measured with 128 x 256 tiles, us one-shot / two-shot:
+// phase instead of two, (W - 1) times the bytes).  Measured with one CTA per 128 x 256 tile, us one-shot / two-shot:
 // 2 ranks T = 128: 25.3 / 30.8, T = 512: 35.0 / 36.5; 4 ranks T = 128: 25.0 / 27.5, T = 512: 42.3 / 33.6.
 uint32_t FusedLinearOneShotMaxRows(int world) { return world <= 2 ? 256u : world <= 4 ? 128u : 32u; }
 
@@ -194,12 +194,14 @@ void FusedLinearCounts(uint32_t T, uint32_t N, int W, bool oneshot, uint32_t* ar
     }
 }
 
-// K splits per tile of a one-shot call of the tile form: powers of two while world x ksplit <= 8 (the reduction
-// holds eight partial rows in registers), every split keeps at least four k-blocks, the work items fit the
-// resident CTAs, a split's partial rows fit its share of the landing zone, and the partial rows a rank sends
-// to its peers (every split sends its own) stay within 2 MiB (4 MiB for two splits): measured on 2 x B200,
-// K = 2048, us with 1 / 2 / 4 splits: T = 128: 25.0 / 21.1 / 23.4; T = 256: - / 27.2 / 32.3 (two-shot: 30.8).
-// `want` > 0 replaces the k-block and traffic rules (measurements).
+// K splits per tile of a one-shot call of the tile form: powers of two while world x ksplit <= 8 (the flags and the row
+// producer count sources by rank and split), every split keeps at least four k-blocks, as many 128 x 256 tiles fit the
+// resident pairs (each of which now works on 256 x 256, so this errs on the side of fewer splits), a split's
+// partial rows fit its share of the landing zone, and the partial rows a rank sends to its peers (every split sends
+// its own) stay within 2 MiB (4 MiB for two splits).  The limits come from the form with one CTA per 128 x 256 tile, on 2 x
+// B200 with K = 2048, us with 1 / 2 / 4 splits: T = 128: 25.0 / 21.1 / 23.4; T = 256: - / 27.2 / 32.3 (two-shot: 30.8);
+// pairs of CTAs have not been measured on several GPUs.  `want` > 0 replaces the k-block and traffic rules
+// (measurements).
 uint32_t FusedLinearTileSplit(uint32_t T, uint32_t N, uint32_t K, int world, uint32_t resident_ctas, uint64_t gemm_cap,
                               uint32_t want) {
     const uint32_t ntiles = ((T + kGemmTileM - 1) / kGemmTileM) * ((N + kGemmTileN - 1) / kGemmTileN), kblocks = K / 64;
