@@ -20,12 +20,12 @@
 // by elect.sync (behind a lane test the compiler wraps each of these instructions in a loop over the active
 // threads: 540 instead of 390 cycles per k-block of 160 tokens).
 //
-// Bound by the tensor cores at the clock they leave (2 ranks, T = 2048, K = 2048: the GEMM reaches 1.4 PFLOP/s while the
-// first tiles come from HBM), and by writing the rows that complete with the last tiles (4.6 - 5.3 TB/s of stores);
-// by reading W from HBM for few tokens.  Measured per call, ranks on one B200, against the exchange of bf16
-// partial rows in one cooperative launch (gemm_ar_rmsnorm.cu, gemm_ar_decode.cu), us: 2 ranks, K = 2048: T = 8 15.1 ->
-// 10.8, T = 128 26.7 -> 17.7, T = 2048 78.6 -> 65.5; 8 ranks, K = 1792, T = 300 68 -> 55; 8 ranks, K = 512, T = 2048
-// 180 -> 118.
+// Bound by the tensor cores at the clock they leave (2 ranks, T = 2048, K = 2048: the GEMM takes 55 us in the profiler, 1.24
+// PFLOP/s), and by writing the rows that complete with the last tiles (4.6 - 5.3 TB/s of stores); by reading W from HBM
+// for few tokens.  Measured per call, ranks on one B200, N = 4096, inputs beyond L2, against the exchange of bf16 partial
+// rows in one cooperative launch (gemm_ar_rmsnorm.cu, gemm_ar_decode.cu), us back to back / in single bursts of 20 calls,
+// where the clock stays up: 2 ranks, K = 2048: T = 8 16.4 -> 12.0 / 15.3 -> 11.9, T = 128 26.7 -> 17.3 / 24.9 -> 17.3,
+// T = 2048 85 -> 76 / 75 -> 66; 8 ranks: K = 1792, T = 300 69 -> 57 / 67 -> 53; K = 512, T = 2048 179 -> 130 / 177 -> 112.
 //
 // Parity: none in the reference (it has no GEMM, no fused op and no tensor-core code).
 #include <cuda.h>

@@ -273,9 +273,11 @@ int FusedLinearAutoMulticastMode(int world, uint32_t /*T*/) {
 //   * the sums are written and read again (1600 bytes per cycle): why splitting K costs more than cutting the tokens finer;
 //   * the last item's read-out (10 per token), 60 per pair that has nothing to do (its SMs load nothing), and 2200 for
 //     the fence and the flag of plain sums (`lines`: the splits travel as flag-in-data lines).
-// Fitted to sweeps on B200 (graph, us): 2 ranks, K = 2048, N = 4096: T = 256: 2 tiles of 128 x 2 splits 20.5, 1 of 256 x 4
-// 23.2, 2 of 128 unsplit 24.8; T = 512: 4 of 128 27.5, 2 of 256 x 2 30.0; T = 2048: 8 of 256 65, 11 of 192 72; T = 8: 4
-// splits 10.6, 3 11.6.  8 ranks, K = 1792, T = 300: 2 of 160 x 2 54, unsplit 71.
+// Fitted to sweeps on B200 (in a graph, short bursts; back to back the long ones take 10-20 % more), us: 2 ranks, K = 2048,
+// N = 4096: T = 256: 2 tiles of 128 x 2 splits 20.5, 1 of 256 x 4 23.2, 2 of 128 unsplit 24.8; T = 512: 4 of 128 27.5, 2 of
+// 256 x 2 30.0; T = 2048: 8 of 256 65, 11 of 192 72; T = 8: 4 splits 10.6, 3 11.6.  8 ranks, K = 1792, T = 300: 2 of 160 x 2
+// 54, unsplit 71.  It ranks shapes and is no prediction: rows that become ready with the last items, and so cannot run
+// under the GEMM, have no term, and where all items fit one round it comes out far too low (T = 300: 28-33 of 53 us).
 LocalGemmShape LocalGemmShapeFor(uint32_t T, uint32_t N, uint32_t kb_total, uint64_t room, uint32_t pairs, bool lines) {
     const uint32_t ncol = (N + kLocalGemmPairCols - 1) / kLocalGemmPairCols, units = N / kLocalGemmUnitCols;
     const uint32_t fewest = (T + kLocalGemmMaxTokens - 1) / kLocalGemmMaxTokens;
@@ -409,12 +411,13 @@ Result LaunchLocal(Communicator& comm, const DriverApi* drv, const FusedLinearDe
     }
     const uint32_t items = g.s.tiles * ((N + kLocalGemmPairCols - 1) / kLocalGemmPairCols) * g.s.nsplit;
     // With few rows the ranks of a row are spread over CTAs (each adds the splits again, from L2) and the sums travel as
-    // flag-in-data lines, which saves the fence and the flag at the price of twice the bytes (2 ranks, K = 2048: T = 16 13.1 ->
-    // 12.1 us, T = 64 16.1 -> 15.1; 8 ranks, K = 1792, two splits: T = 36 34.6 -> 33.4; but 2 ranks T = 96 16.0 -> 16.9, T = 128 16.5 -> 18.4).  From two CTAs per SM on a CTA
-    // serves two or four ranks, and the grid is what fits the GPU: with two more CTAs fit, with four the sums are read
-    // less often.  A round of four takes about 3/2 of a round of two (5/4 for rows of one vector per thread), so the rounds decide (8 ranks,
-    // two against four, us: T = 64 19.0 / 20.5, T = 128 24.9 / 22.7, T = 300 52.8 / 54.7, T = 512 40.7 / 44.7, T = 2048 122.9 / 131.4; 4 ranks: T = 256
-    // 26.3 / 24.0, T = 512 32.1 / 35.3; N = 2048, T = 2048 100 / 94).
+    // flag-in-data lines, which saves the fence and the flag at the price of twice the bytes.  (All figures here: in a graph,
+    // short bursts, us.  2 ranks, K = 2048: T = 16 13.1 -> 12.1, T = 64 16.1 -> 15.1; 8 ranks, K = 1792, two splits:
+    // T = 36 34.6 -> 33.4; but 2 ranks T = 96 16.0 -> 16.9, T = 128 16.5 -> 18.4.)  From two CTAs per SM on a CTA serves two
+    // or four ranks, and the grid is what fits the GPU: with two more CTAs fit, with four the sums are read less often.  A
+    // round of four takes about 3/2 of a round of two (5/4 for rows of one vector per thread), so the rounds decide
+    // (8 ranks, two against four: T = 64 19.0 / 20.5, T = 128 24.9 / 22.7, T = 300 52.8 / 54.7, T = 512 40.7 / 44.7,
+    // T = 2048 122.9 / 131.4; 4 ranks: T = 256 26.3 / 24.0, T = 512 32.1 / 35.3; N = 2048, T = 2048 100 / 94).
     const uint64_t line_bytes = static_cast<uint64_t>(T) * N * 4 * g.s.nsplit;
     const bool lines = few && T <= 64 && g.s.nsplit > 1 && line_bytes <= 2ull * W * lay.gemm_ll_cap;
     if (lines) {
