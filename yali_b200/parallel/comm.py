@@ -192,8 +192,9 @@ class Comm:
         multicast store; 1 and 2 need the multicast object and `out` from symm_empty().  `decode`: the
         few-token form (up to 64 rows: 128 x 256 tiles whose K extent is split over CTAs, partial rows sent to every rank as
         flag-in-data lines, every rank normalises all rows): None = by size, False = never, True = required."""
-        kept = None
-        if out is None and self.nlocal == 1 and self.world > 1:
+        if out is not None:
+            out = self._once(out)
+        elif self.nlocal == 1 and self.world > 1:
             x, w = self._once(x), self._once(w)
             # Symmetric memory is never freed piecemeal: keep ONE output per row width, large enough for the
             # most rows seen so far (grown by doubling, so a program that varies its token count holds at
@@ -205,14 +206,14 @@ class Comm:
             if buf is None or buf.shape[0] < T:
                 rows = T if buf is None else max(T, 2 * buf.shape[0])
                 buf = cache[N] = self.symm_empty([rows, N], torch.bfloat16)
-            out = kept = [buf[:T]]
+            out = [buf[:T]]
         try:
             r = self._impl.fused_linear(x, w, norm_weight, out, residual, residual_out, eps,
                                         -1 if oneshot is None else int(oneshot), ctas, trace,
                                         -1 if nvls is None else int(nvls), -1 if decode is None else int(decode))
         except RuntimeError as e:
             raise _translate(e) from None
-        return r if kept is None else self._like_input(x, kept)
+        return r if out is None else self._like_input(x, self._as_list(out, "out"))
 
     def all_reduce_host(self, src: TensorOrList, dst: Optional[TensorOrList] = None, *,
                         chunk_bytes: int = 0, scale: Optional[float] = None, mode: str = "auto",
