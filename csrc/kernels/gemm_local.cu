@@ -20,6 +20,11 @@
 // by elect.sync (behind a lane test the compiler wraps each of these instructions in a loop over the active
 // threads: 540 instead of 390 cycles per k-block of 160 tokens).
 //
+// Calls that follow one another overlap: the row kernel lets the next call's GEMM start when all of its own CTAs have, and that
+// one sets up and asks L2 for its first k-blocks of W before it waits for the rows.  In a graph, weights beyond or at the
+// edge of L2, without / with, us: 2 ranks, K = 1024, N = 3072: T = 45 9.6 / 8.2; K = 2048, N = 4096: T = 8 10.1 / 9.6, T = 64
+// 14.6 / 13.2, T = 400 23.9 / 22.1.  kLocalLinearEarly says up to where.
+//
 // Bound by the tensor cores at the clock they leave (2 ranks, T = 2048, K = 2048: the GEMM takes 55 us in the profiler, 1.24
 // PFLOP/s), and by writing the rows that complete with the last tiles (4.6 - 5.3 TB/s of stores); by reading W from HBM
 // for few tokens.  Measured per call, ranks on one B200, N = 4096, inputs beyond L2, against the exchange of bf16 partial
@@ -92,7 +97,26 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kLocalGemmThreads, 1
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t cta = blockIdx.x, half = ptx::cluster_cta_rank();
     uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    const uint32_t ncol = (a.N + kLocalGemmPairCols - 1) / kLocalGemmPairCols;
+    const uint32_t pair = cta >> 1, npairs = gridDim.x >> 1;
+    const uint32_t xbytes = a.s.tokens / 2 * (BK * 2);  // one CTA's half of the token operand of a stage: whole KiB
+    const uint32_t stage_bytes = kWBytes + xbytes;
+    const uint32_t stages = min(kRingBytes / stage_bytes, static_cast<uint32_t>(kMaxStages));
     // Nothing up to the wait depends on earlier kernels: it runs under the end of the one in front.
+    uint32_t fetched = 0;  // prefetch warp: k-blocks of W that are on their way into L2 already
+    if (warp == kPrefetchWarp && ptx::elect_one()) {
+        // The rows of the call in front leave HBM time, and what this call waits for first is W.  It is no more than asked for
+        // here: should the kernel in front still be writing it, the loads behind the wait see that.
+        Item it;
+        if (a.early && item_at(a, 0, pair, npairs, ncol, &it) && it.tile == 0) {
+            const int wrow = it.col_tile * kLocalGemmPairCols + half * kLocalGemmUnitCols;
+            uint32_t rank = it.kb_begin / a.kb_rank, kb = it.kb_begin - rank * a.kb_rank;
+            for (uint32_t g = it.kb_begin; g < it.kb_end && fetched < stages + kPrefetchBlocks; ++g, ++fetched) {
+                ptx::tma_prefetch_2d(&a.tmap_w[rank], kb * BK, wrow);
+                if (++kb == a.kb_rank) kb = 0, ++rank;
+            }
+        }
+    }
     if (tid == 64) {
         s.abort = 0;
         s.loaded = 0;
@@ -124,11 +148,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kLocalGemmThreads, 1
     ptx::grid_dependency_wait();
     ptx::grid_launch_dependents();
     const uint64_t deadline = ptx::globaltimer() + cv.timeout_ns;
-    const uint32_t ncol = (a.N + kLocalGemmPairCols - 1) / kLocalGemmPairCols;
-    const uint32_t pair = cta >> 1, npairs = gridDim.x >> 1;
-    const uint32_t xbytes = a.s.tokens / 2 * (BK * 2);  // one CTA's half of the token operand of a stage: whole KiB
-    const uint32_t stage_bytes = kWBytes + xbytes;
-    const uint32_t stages = min(kRingBytes / stage_bytes, static_cast<uint32_t>(kMaxStages));
 
     if (warp == kTmaWarp) {
         if (ptx::elect_one()) {
@@ -261,7 +280,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kLocalGemmThreads, 1
                 uint32_t rank = it.kb_begin / a.kb_rank, kb = it.kb_begin - rank * a.kb_rank;
                 for (uint32_t g = it.kb_begin; g < it.kb_end; ++g, ++ahead) {
                     while (static_cast<int32_t>(ahead - s.loaded) > static_cast<int32_t>(stages + kPrefetchBlocks)) ptx::nanosleep(40);
-                    if (w_here) ptx::tma_prefetch_2d(&a.tmap_w[rank], kb * BK, wrow);
+                    if (w_here && ahead >= fetched) ptx::tma_prefetch_2d(&a.tmap_w[rank], kb * BK, wrow);
                     if (x_here) ptx::tma_prefetch_2d(&a.tmap_x[rank], kb * BK, xrow);
                     if (++kb == a.kb_rank) kb = 0, ++rank;
                 }
@@ -382,6 +401,8 @@ __global__ void __launch_bounds__(THREADS, LocalLinearNormPlaces(G, SPLIT, THREA
     const uint32_t tid = threadIdx.x, nvec = a.N / VEC;
     const bool taking = gridDim.x < units;  // from the counter
     uint32_t* const counter = flag_word(cv, 0, kCallLocalRows);
+    // The next kernel may set up, and ask for its weights, under this one.
+    if (a.early) ptx::grid_launch_dependents();
     const uint32_t epoch = *reinterpret_cast<volatile uint32_t*>(flag_word(cv, 0, kCallLocalRowCalls)) + 1u;
     const uint64_t deadline = ptx::globaltimer() + cv.timeout_ns;
     bool have[NV];

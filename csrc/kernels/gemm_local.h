@@ -14,6 +14,10 @@ constexpr uint32_t kLocalGemmUnitCols = 128;   // columns of one CTA, announced 
 constexpr uint32_t kLocalGemmMaxTokens = 256;  // rows of x on the N side
 constexpr uint32_t kLocalGemmMaxSplit = 8;
 constexpr int kLocalGemmThreads = 384;         // eight epilogue warps, TMA, MMA, announcer, prefetch
+// Elements of all ranks' outputs up to which a call's GEMM starts under the rows of the call in front.  With more, the rows keep
+// HBM busy by themselves and W on its way only delays them: 2 ranks, K = 2048, N = 4096, back to back, without / with, us: T =
+// 400 24.5 / 23.8, T = 700 37.2 / 36.6, T = 2048 77.5 / 78.8 (4 ranks, K = 1024, N = 2048, T = 1024 34.3 / 33.9).
+constexpr uint64_t kLocalLinearEarly = 12ull << 20;
 constexpr int kLocalLinearNormThreads = 256;   // one row; up to two 16-byte vectors per thread: N <= 4096
 // A row of up to 64 vectors leaves most of 256 threads idle, and a unit of the row kernel is a chain of latencies, so
 // what counts is how many are in flight: four times as many CTAs of 64 threads (K = 64, N = 128, 4096 rows: 2 ranks 33 ->
@@ -36,6 +40,7 @@ struct alignas(64) LocalGemmArgs {
     uint32_t kb_rank;               // k-blocks (of 64) of one rank
     uint32_t kb_total;              // of all ranks
     LocalGemmShape s;
+    uint32_t early;  // at most kLocalLinearEarly elements
 };
 
 struct LocalLinearNormArgs {
@@ -47,6 +52,7 @@ struct LocalLinearNormArgs {
     void* out[kMaxRanks];             // [T, N]
     uint32_t T, N, world;
     LocalGemmShape s;
+    uint32_t early;
     float eps;
 };
 
