@@ -270,18 +270,19 @@ int FusedLinearAutoMulticastMode(int world, uint32_t /*T*/) {
 //   * a k-block of an item takes 2 cycles per token on the tensor cores, at least 350 for its instructions, and an item
 //     1500 more; every pair has the same number of items, up to one;
 //   * no run is shorter than reading all of W and x from HBM (3440 bytes per cycle, 15 % lost), by the pairs that are busy;
+//   * a sixteenth of W comes from HBM once more for every further token tile of a round (not `lines`, whose fit is older);
 //   * the sums are written and read again (1600 bytes per cycle): why splitting K costs more than cutting the tokens finer;
 //   * the last item's read-out (10 per token), 60 per pair that has nothing to do (its SMs load nothing), and 2200 for
 //     the fence and the flag of plain sums (`lines`: the splits travel as flag-in-data lines).
 // Fitted to sweeps on B200 (in a graph, short bursts; back to back the long ones take 10-20 % more), us: 2 ranks, K = 2048,
 // N = 4096: T = 256: 2 tiles of 128 x 2 splits 20.5, 1 of 256 x 4 23.2, 2 of 128 unsplit 24.8; T = 512: 4 of 128 27.5, 2 of
 // 256 x 2 30.0; T = 2048: 8 of 256 65, 11 of 192 72; T = 8: 4 splits 10.6, 3 11.6.  8 ranks, K = 1792, T = 300: 2 of 160 x 2
-// 54, unsplit 71.  It ranks shapes and is no prediction: rows that become ready with the last items, and so cannot run
-// under the GEMM, have no term, and where all items fit one round it comes out far too low (T = 300: 28-33 of 53 us).
+// 54, unsplit 71.  W read again: 8 ranks, K = 1792, T = 64: 2 tiles of 32 x 2 37.0, 1 of 64 x 4 32.8.  It ranks shapes and
+// is no prediction: rows that become ready with the last items, and so cannot run under the GEMM, have no term, and where
+// all items fit one round it comes out far too low (T = 300: 28-33 of 53 us).
 LocalGemmShape LocalGemmShapeFor(uint32_t T, uint32_t N, uint32_t kb_total, uint64_t room, uint32_t pairs, bool lines) {
     const uint32_t ncol = (N + kLocalGemmPairCols - 1) / kLocalGemmPairCols, units = N / kLocalGemmUnitCols;
     const uint32_t fewest = (T + kLocalGemmMaxTokens - 1) / kLocalGemmMaxTokens;
-    const uint64_t hbm = static_cast<uint64_t>(kb_total) * (N + T) * 128 / 3440 * 115 / 100 + 1500;
     LocalGemmShape best{};
     uint64_t best_cost = ~0ull;
     for (uint32_t n = fewest; n < fewest + 4; ++n) {
@@ -298,6 +299,8 @@ LocalGemmShape LocalGemmShapeFor(uint32_t T, uint32_t N, uint32_t kb_total, uint
             if (static_cast<uint64_t>(s.tiles) * units * s.nsplit > kLocalGemmFlags) break;
             const uint64_t items = static_cast<uint64_t>(s.tiles) * ncol * s.nsplit;
             const uint64_t rounds = (items + pairs - 1) / pairs, used = std::min<uint64_t>(items, pairs);
+            const uint64_t again = lines ? 0 : (N / 16) * ((s.tiles + rounds - 1) / rounds - 1);
+            const uint64_t hbm = static_cast<uint64_t>(kb_total) * (N + again + T) * 128 / 3440 * 115 / 100 + 1500;
             uint64_t cost = std::max(rounds * (s.kper * block + 1500), hbm * (rounds * used) / items) + 2 * sums / 1600 +
                             10 * s.tokens + 60 * (pairs - used);
             if (!(lines && split > 1)) cost += 2200;
