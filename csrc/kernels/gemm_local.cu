@@ -104,45 +104,54 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kLocalGemmThreads, 1
     const uint32_t stages = min(kRingBytes / stage_bytes, static_cast<uint32_t>(kMaxStages));
     // Nothing up to the wait depends on earlier kernels: it runs under the end of the one in front.
     uint32_t fetched = 0;  // prefetch warp: k-blocks of W that are on their way into L2 already
-    if (warp == kPrefetchWarp && ptx::elect_one()) {
+    if (warp == kPrefetchWarp) {
         // The rows of the call in front leave HBM time, and what this call waits for first is W.  It is no more than asked for
-        // here: should the kernel in front still be writing it, the loads behind the wait see that.
-        Item it;
-        if (a.early && item_at(a, 0, pair, npairs, ncol, &it) && it.tile == 0) {
-            const int wrow = it.col_tile * kLocalGemmPairCols + half * kLocalGemmUnitCols;
-            uint32_t rank = it.kb_begin / a.kb_rank, kb = it.kb_begin - rank * a.kb_rank;
-            for (uint32_t g = it.kb_begin; g < it.kb_end && fetched < stages + kPrefetchBlocks; ++g, ++fetched) {
-                ptx::tma_prefetch_2d(&a.tmap_w[rank], kb * BK, wrow);
-                if (++kb == a.kb_rank) kb = 0, ++rank;
+        // here: should the kernel in front still be writing it, the loads behind the wait see that.  Beside the set-up and not
+        // in front of it: this warp has nothing to set up, arrives at once and does not hold up the others.  Graph of calls, 2
+        // ranks, T = 8, K = 2048, N = 4096, W in L2 / partly / beyond it, us: no overlap of calls 8.7 / 11.6 / 12.3, without
+        // this 7.65 / 10.1 / 10.75, in front of the set-up 8.7 / 9.7 / 9.95, behind it 7.9 / 9.8 / 10.35, here 7.7 / 9.3 /
+        // 10.1.  One call after which the host waits, in that order: 21.9, 22.0, 23.3, 22.5, 22.25.
+        ptx::cluster_arrive();
+        if (a.early && ptx::elect_one()) {
+            Item it;
+            if (item_at(a, 0, pair, npairs, ncol, &it) && it.tile == 0) {
+                const int wrow = it.col_tile * kLocalGemmPairCols + half * kLocalGemmUnitCols;
+                uint32_t rank = it.kb_begin / a.kb_rank, kb = it.kb_begin - rank * a.kb_rank;
+                for (uint32_t g = it.kb_begin; g < it.kb_end && fetched < stages + kPrefetchBlocks; ++g, ++fetched) {
+                    ptx::tma_prefetch_2d(&a.tmap_w[rank], kb * BK, wrow);
+                    if (++kb == a.kb_rank) kb = 0, ++rank;
+                }
             }
         }
-    }
-    if (tid == 64) {
-        s.abort = 0;
-        s.loaded = 0;
-        for (int i = 0; i < kMaxStages; ++i) {
-            ptx::mbar_init(&s.full_bar[i], 1);
-            ptx::mbar_init(&s.empty_bar[i], 1);
+        __syncwarp();
+    } else {
+        if (tid == 64) {
+            s.abort = 0;
+            s.loaded = 0;
+            for (int i = 0; i < kMaxStages; ++i) {
+                ptx::mbar_init(&s.full_bar[i], 1);
+                ptx::mbar_init(&s.empty_bar[i], 1);
+            }
+            for (int b = 0; b < 2; ++b) {
+                ptx::mbar_init(&s.tmem_full_bar[b], 1);
+                ptx::mbar_init(&s.tmem_empty_bar[b], 2 * kEpilogueWarps);  // the epilogue warps of both CTAs
+                ptx::mbar_init(&s.stored_bar[b], kEpilogueWarps);
+                ptx::mbar_init(&s.announced_bar[b], 1);
+            }
+            ptx::mbar_init(&s.drain_bar, 1);
+            ptx::mbar_fence_init();
+            ptx::tma_prefetch_desc(&a.tmap_w[0]);
+            ptx::tma_prefetch_desc(&a.tmap_x[0]);
         }
-        for (int b = 0; b < 2; ++b) {
-            ptx::mbar_init(&s.tmem_full_bar[b], 1);
-            ptx::mbar_init(&s.tmem_empty_bar[b], 2 * kEpilogueWarps);  // the epilogue warps of both CTAs
-            ptx::mbar_init(&s.stored_bar[b], kEpilogueWarps);
-            ptx::mbar_init(&s.announced_bar[b], 1);
+        if (warp == kMmaWarp) {
+            ptx::tmem_alloc_pair(&s.tmem, kTmemCols);
+            ptx::tmem_relinquish_pair();
         }
-        ptx::mbar_init(&s.drain_bar, 1);
-        ptx::mbar_fence_init();
-        ptx::tma_prefetch_desc(&a.tmap_w[0]);
-        ptx::tma_prefetch_desc(&a.tmap_x[0]);
+        ptx::tc_fence_before_sync();
+        __syncwarp();
+        ptx::cluster_arrive();
     }
-    if (warp == kMmaWarp) {
-        ptx::tmem_alloc_pair(&s.tmem, kTmemCols);
-        ptx::tmem_relinquish_pair();
-    }
-    ptx::tc_fence_before_sync();
-    __syncthreads();
-    ptx::cluster_arrive();  // the other CTA's barriers and TMEM are ready, too
-    ptx::cluster_wait();
+    ptx::cluster_wait();  // barriers and TMEM are ready, in both CTAs
     ptx::tc_fence_after_sync();
     const uint32_t tmem = s.tmem;
     ptx::grid_dependency_wait();
