@@ -112,7 +112,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kLocalGemmThreads, 1
         // this 7.65 / 10.1 / 10.75, in front of the set-up 8.7 / 9.7 / 9.95, behind it 7.9 / 9.8 / 10.35, here 7.7 / 9.3 /
         // 10.1.  One call after which the host waits, in that order: 21.9, 22.0, 23.3, 22.5, 22.25.
         ptx::cluster_arrive();
-        if (a.early && ptx::elect_one()) {
+        if (ptx::elect_one()) {
             Item it;
             if (item_at(a, 0, pair, npairs, ncol, &it) && it.tile == 0) {
                 const int wrow = it.col_tile * kLocalGemmPairCols + half * kLocalGemmUnitCols;

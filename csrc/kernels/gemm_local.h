@@ -14,9 +14,12 @@ constexpr uint32_t kLocalGemmUnitCols = 128;   // columns of one CTA, announced 
 constexpr uint32_t kLocalGemmMaxTokens = 256;  // rows of x on the N side
 constexpr uint32_t kLocalGemmMaxSplit = 8;
 constexpr int kLocalGemmThreads = 384;         // eight epilogue warps, TMA, MMA, announcer, prefetch
-// Elements of all ranks' outputs up to which a call's GEMM starts under the rows of the call in front.  With more, the rows keep
-// HBM busy by themselves and W on its way only delays them: 2 ranks, K = 2048, N = 4096, back to back, without / with, us: T =
-// 400 24.5 / 23.8, T = 700 37.2 / 36.6, T = 2048 77.5 / 78.8 (4 ranks, K = 1024, N = 2048, T = 1024 34.3 / 33.9).
+// Elements of all ranks' outputs up to which the rows of a call release the kernel behind it when they start.  With more, the rows keep
+// HBM busy by themselves and W on its way only delays them.  Back to back, without / with, us: 2 ranks, K = 2048, N = 4096: T =
+// 400 26.0 / 24.0, T = 1400 (11 Mi) 60.1 / 61.0, T = 2048 (16 Mi) 77.7 / 78.7; 4 ranks: K = 1024, N = 2048, T = 1024 (8 Mi)
+// 33.2 / 32.8, K = 2048, N = 4096, T = 600 (9.4 Mi) 61.4 / 60.0; 8 ranks, N = 4096: K = 512, T = 256 (8 Mi) 27.7 / 28.2, K = 1792,
+// T = 300 (9.4 Mi) 60.5 / 59.5, T = 350 (11 Mi) 67.3 / 66.2.  The kernel behind asks for its W whatever its own size: large calls
+// behind small ones 80.2 / 78.0, 68.6 / 67.9, 90.6 / 91.3 with / without such a limit, large behind large level.
 constexpr uint64_t kLocalLinearEarly = 12ull << 20;
 constexpr int kLocalLinearNormThreads = 256;   // one row; up to two 16-byte vectors per thread: N <= 4096
 // A row of up to 64 vectors leaves most of 256 threads idle, and a unit of the row kernel is a chain of latencies, so
@@ -40,7 +43,6 @@ struct alignas(64) LocalGemmArgs {
     uint32_t kb_rank;               // k-blocks (of 64) of one rank
     uint32_t kb_total;              // of all ranks
     LocalGemmShape s;
-    uint32_t early;  // at most kLocalLinearEarly elements
 };
 
 struct LocalLinearNormArgs {
@@ -52,7 +54,7 @@ struct LocalLinearNormArgs {
     void* out[kMaxRanks];             // [T, N]
     uint32_t T, N, world;
     LocalGemmShape s;
-    uint32_t early;
+    uint32_t early;  // at most kLocalLinearEarly elements: the next kernel may start under these rows
     float eps;
 };
 

@@ -391,10 +391,9 @@ Result LaunchLocal(Communicator& comm, const DriverApi* drv, const FusedLinearDe
     g.kb_total = g.kb_rank * W;
     const bool few = static_cast<uint64_t>(T) * W <= 2 * sms;
     g.s = LocalGemmShapeFor(T, N, g.kb_total, 2ull * W * lay.gemm_cap, pairs, few && T <= 64);
-    g.early = static_cast<uint64_t>(T) * N * W <= kLocalLinearEarly;
     LocalLinearNormArgs n;
     std::memset(&n, 0, sizeof(n));
-    n.early = g.early;
+    n.early = static_cast<uint64_t>(T) * N * W <= kLocalLinearEarly;
     n.cv = g.cv;
     n.sums = g.sums;
     n.T = T;
