@@ -270,19 +270,28 @@ int FusedLinearAutoMulticastMode(int world, uint32_t /*T*/) {
 //   * a k-block of an item takes 2 cycles per token on the tensor cores, at least 350 for its instructions, and an item
 //     1500 more; every pair has the same number of items, up to one;
 //   * no run is shorter than reading all of W and x from HBM (3440 bytes per cycle, 15 % lost), by the pairs that are busy;
-//   * a sixteenth of W comes from HBM once more for every further token tile of a round (not `lines`, whose fit is older);
+//   * with more than one token tile, a twelfth of reading W from HBM on top: tiles that run together ask for the same W at
+//     slightly different times, and part of it comes twice.  The same for two tiles and for eight: it decides between one tile and
+//     several (T <= 256) and never makes more tiles the cheaper cut;
 //   * the sums are written and read again (1600 bytes per cycle): why splitting K costs more than cutting the tokens finer;
 //   * the last item's read-out (10 per token), 60 per pair that has nothing to do (its SMs load nothing), and 2200 for
 //     the fence and the flag of plain sums (`lines`: the splits travel as flag-in-data lines).
 // Fitted to sweeps on B200 (in a graph, short bursts; back to back the long ones take 10-20 % more), us: 2 ranks, K = 2048,
 // N = 4096: T = 256: 2 tiles of 128 x 2 splits 20.5, 1 of 256 x 4 23.2, 2 of 128 unsplit 24.8; T = 512: 4 of 128 27.5, 2 of
 // 256 x 2 30.0; T = 2048: 8 of 256 65, 11 of 192 72; T = 8: 4 splits 10.6, 3 11.6.  8 ranks, K = 1792, T = 300: 2 of 160 x 2
-// 54, unsplit 71.  W read again: 8 ranks, K = 1792, T = 64: 2 tiles of 32 x 2 37.0, 1 of 64 x 4 32.8.  It ranks shapes and
-// is no prediction: rows that become ready with the last items, and so cannot run under the GEMM, have no term, and where
-// all items fit one round it comes out far too low (T = 300: 28-33 of 53 us).
+// 54, unsplit 71.  One tile or several, W beyond / in L2: 8 ranks: N = 4096, K = 1792: T = 64: 2 tiles of 32 x 2 34.6 / 33.6, 1 of
+// 64 x 4 32.5 / 32.5, T = 33: 32 x 2 32.9 / 32.9, 64 x 4 31.5 / 31.6; N = 2816, K = 1728, T = 57: 32 x 3 26.1 / 26.8, 64 x 6 24.2 / 18.1;
+// 4 ranks, N = 3840, K = 1600, T = 65: 64 x 2 18.6 / 17.6, 96 x 4 17.4 / 14.1; 2 ranks, N = 3584, K = 1408, T = 66: 64 x 2 12.4 / 11.5,
+// 96 x 5 10.6 / 10.5.  Of 310 sizes timed with the cuts of both the term changes 51, to 0.90 of the time in the mean; three of
+// them, with little of W per pair, lose 4 - 10 % (8 ranks, K = 256, N = 2432, T = 40: 32 x 3 12.2 / 10.5, 64 x 7 12.5 / 12.6).
+// A tenth to a sixteenth rank much alike; with an eighth eight of 83 lose.
+// The whole ranks shapes and is no prediction: rows that become ready with the last items, and so cannot run under the
+// GEMM, have no term, and where all items fit one round it comes out far too low (T = 300: 28-33 of 53 us).
 LocalGemmShape LocalGemmShapeFor(uint32_t T, uint32_t N, uint32_t kb_total, uint64_t room, uint32_t pairs, bool lines) {
     const uint32_t ncol = (N + kLocalGemmPairCols - 1) / kLocalGemmPairCols, units = N / kLocalGemmUnitCols;
     const uint32_t fewest = (T + kLocalGemmMaxTokens - 1) / kLocalGemmMaxTokens;
+    const uint64_t hbm = static_cast<uint64_t>(kb_total) * (N + T) * 128 / 3440 * 115 / 100 + 1500;
+    const uint64_t again = static_cast<uint64_t>(kb_total) * N * 128 / 3440 / 12;
     LocalGemmShape best{};
     uint64_t best_cost = ~0ull;
     for (uint32_t n = fewest; n < fewest + 4; ++n) {
@@ -299,11 +308,10 @@ LocalGemmShape LocalGemmShapeFor(uint32_t T, uint32_t N, uint32_t kb_total, uint
             if (static_cast<uint64_t>(s.tiles) * units * s.nsplit > kLocalGemmFlags) break;
             const uint64_t items = static_cast<uint64_t>(s.tiles) * ncol * s.nsplit;
             const uint64_t rounds = (items + pairs - 1) / pairs, used = std::min<uint64_t>(items, pairs);
-            const uint64_t again = lines ? 0 : (N / 16) * ((s.tiles + rounds - 1) / rounds - 1);
-            const uint64_t hbm = static_cast<uint64_t>(kb_total) * (N + again + T) * 128 / 3440 * 115 / 100 + 1500;
             uint64_t cost = std::max(rounds * (s.kper * block + 1500), hbm * (rounds * used) / items) + 2 * sums / 1600 +
                             10 * s.tokens + 60 * (pairs - used);
             if (!(lines && split > 1)) cost += 2200;
+            if (s.tiles > 1) cost += again;
             if (cost < best_cost) {
                 best_cost = cost;
                 best = s;

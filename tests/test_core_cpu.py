@@ -470,3 +470,21 @@ def test_shape_of_the_fused_layer_for_ranks_on_one_gpu(native_lib, world):
                         assert 1 <= nsplit <= 8 and (nsplit - 1) * kper < kb <= nsplit * kper
                         assert nsplit == 1 or T * N * 2 * nsplit <= room
                         assert tiles * (N // 128) * nsplit <= 16384
+
+
+@pytest.mark.parametrize("world,T,K,N,tokens,splits", [
+    # One token tile reads W once.  Two of half the size took 32.9, 33.6, 26.8 and 17.6 us, one takes 31.6, 32.5, 18.1 and 14.1.
+    (8, 33, 1792, 4096, 64, 4), (8, 64, 1792, 4096, 64, 4), (8, 57, 1728, 2816, 64, 6), (4, 65, 1600, 3840, 96, 4),
+    # That W is read again makes no cut with more tiles, or with fewer splits, the better one: three tiles of 96, three of 64 and
+    # three splits took 16.5, 14.5 and 35.9 us, these take 15.5, 14.1 and 35.0.
+    (4, 204, 1408, 2048, 128, 4), (2, 169, 1344, 2944, 96, 3), (8, 260, 1600, 2304, 160, 4),
+    # No cut of one tile: nor does it change the others.
+    (8, 386, 1792, 3584, 224, 2), (8, 300, 1792, 4096, 160, 2), (2, 2048, 2048, 4096, 256, 1),
+    # Few rows: one tile in any case.
+    (2, 8, 2048, 4096, 32, 4)])
+def test_one_token_tile_or_several(native_lib, world, T, K, N, tokens, splits):
+    import ctypes
+    out, pairs = (ctypes.c_uint32 * 4)(), 74
+    few = T * world <= 4 * pairs and T <= 64
+    native_lib.yali_c_local_gemm_shape(T, N, world * K // 64, 2 * world * (max(4, -(-16 // world)) << 20), pairs, few, out)
+    assert (out[1], out[2]) == (tokens, splits)
