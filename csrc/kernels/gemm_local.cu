@@ -20,10 +20,10 @@
 // by elect.sync (behind a lane test the compiler wraps each of these instructions in a loop over the active
 // threads: 540 instead of 390 cycles per k-block of 160 tokens).
 //
-// Calls that follow one another overlap: the row kernel lets the next call's GEMM start when all of its own CTAs have, and that
-// one sets up and asks L2 for its first k-blocks of W before it waits for the rows.  In a graph, weights beyond or at the
-// edge of L2, without / with, us: 2 ranks, K = 1024, N = 3072: T = 45 9.6 / 8.2; K = 2048, N = 4096: T = 8 10.1 / 9.6, T = 64
-// 14.6 / 13.2, T = 400 23.9 / 22.1.  kLocalLinearEarly says up to where.
+// Calls that follow one another overlap: the row kernel lets the kernel behind it start when all of its own CTAs have, and where that
+// is the next call's GEMM, it sets up and asks L2 for its first k-blocks of W before it waits for the rows.  In a graph, weights beyond
+// L2, without / with, us: 2 ranks: K = 1024, N = 3072, T = 45 10.8 / 8.3; K = 2048, N = 4096: T = 8 12.3 / 10.1, T = 64 14.7 / 12.7,
+// T = 400 26.0 / 23.4.  kLocalLinearEarly says up to where.
 //
 // Bound by the tensor cores at the clock they leave (2 ranks, T = 2048, K = 2048: the GEMM takes 55 us in the profiler, 1.24
 // PFLOP/s), and by writing the rows that complete with the last tiles (4.6 - 5.3 TB/s of stores); by reading W from HBM
@@ -154,6 +154,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kLocalGemmThreads, 1
     ptx::cluster_wait();  // barriers and TMEM are ready, in both CTAs
     ptx::tc_fence_after_sync();
     const uint32_t tmem = s.tmem;
+    // In this order: the row kernel behind does not wait for the kernels in front of this one.  It reads its call number, the unit counter
+    // and the call's inputs as soon as it starts, which is right because some thread of every CTA here has been through its wait.
     ptx::grid_dependency_wait();
     ptx::grid_launch_dependents();
     const uint64_t deadline = ptx::globaltimer() + cv.timeout_ns;
@@ -410,7 +412,8 @@ __global__ void __launch_bounds__(THREADS, LocalLinearNormPlaces(G, SPLIT, THREA
     const uint32_t tid = threadIdx.x, nvec = a.N / VEC;
     const bool taking = gridDim.x < units;  // from the counter
     uint32_t* const counter = flag_word(cv, 0, kCallLocalRows);
-    // The next kernel may set up, and ask for its weights, under this one.
+    // The next kernel may set up, and ask for its weights, under this one.  Whatever it is, it waits for the end of this kernel, and with
+    // it of the GEMM (see the last line), before it touches memory.
     if (a.early) ptx::grid_launch_dependents();
     const uint32_t epoch = *reinterpret_cast<volatile uint32_t*>(flag_word(cv, 0, kCallLocalRowCalls)) + 1u;
     const uint64_t deadline = ptx::globaltimer() + cv.timeout_ns;

@@ -24,9 +24,11 @@ constexpr int kDirectThreads = 288;   // one producer warp + eight consumer warp
 constexpr int kDirectMaxStages = kMaxPipelineStages;
 
 // Ordinary (not cooperative) launch.  Programmatic stream serialization lets the launch overlap the end of the kernel in
-// front of it in the stream, whose results the kernel waits for with ptx::grid_dependency_wait() before anything
-// else.  Without it back-to-back launches on B200 take turns on a 2.05 us grid: a 5.2 us kernel came every 8.2 us,
-// with it every 5.9 us.
+// front of it in the stream, whose end the kernel waits for with ptx::grid_dependency_wait() before it reads or writes memory
+// (prefetches into L2 aside).  Every kernel launched here has to: the row kernel of the fused layer for one GPU releases
+// the kernel behind it when it starts.  That row kernel itself is the one exception.  It waits only at its end, and may run
+// because the GEMM in front of it releases it behind its own wait.  Without the attribute back-to-back launches on B200 take
+// turns on a 2.05 us grid: a 5.2 us kernel came every 8.2 us, with it every 5.9 us.
 inline cudaError_t LaunchInStream(const void* fn, dim3 grid, dim3 block, void** params, size_t smem, cudaStream_t s) {
     cudaLaunchConfig_t cfg;
     std::memset(&cfg, 0, sizeof(cfg));

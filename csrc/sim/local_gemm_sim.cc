@@ -4,7 +4,9 @@
 // them when, the release of the dependent kernel, the walk over the items, sums announced by flags or sent as flag-in-data lines,
 // rows taken from a counter, the check-in that clears the counter and advances the call number, and the clearing of
 // the control words between calls (Communicator::Reset).  The GEMM itself is a formula of (call, row, unit, split).
-// Calls follow one another in stream order: a call starts when both kernels of the one before it have finished.
+// Calls follow one another in stream order.  A call's GEMM may start under the rows of the call in front, but all it does before they
+// have finished is to set up and to prefetch its weights, which touches none of this: here a call starts when both kernels of
+// the one before it have finished.
 //
 // Parity: the reference has neither the fused layer nor a protocol model.
 #include <atomic>
