@@ -390,26 +390,36 @@ namespace {
 // Pauses between two looks at a flag and at a line.  Polling costs the GEMM more than a late look costs the row: with 50 ns
 // and all lines asked for on every look, us: 2 ranks, K = 2048: T = 8 10.0 -> 9.8, T = 64 17.3 -> 14.6, T = 128 18.3 -> 16.5
 // (flags, 3000 ns level, 600 ns 16.8); 4 ranks, K = 1792, T = 100 20.4 -> 18.5 (3000 ns 20.5, 1000 ns 19.1).  Lines: 0 to 100 ns
-// are level.
-constexpr uint32_t kFlagSleepNs = 1500, kLineSleepNs = 40;
+// are level.  Once one flag of a tile is set, the others are not far: 8 ranks, 678 x 640 x 1664 31.0 -> 29.3 us, 688 x 1792 x 2816
+// 67.5 -> 65.5 (100 and 400 ns are level).
+constexpr uint32_t kFlagSleepNs = 1500, kFlagNearNs = 400, kLineSleepNs = 40;
 
 // A unit of work is a row for G ranks (unit u: row u / ngroups, ranks from (u % ngroups) * G); a thread holds NV 16-byte
-// vectors of the row.  SPLIT: more than one K split; LINES: the sums come as flag-in-data lines.
+// vectors of the row.  SPLIT: more than one K split; LINES: the sums come as flag-in-data lines; SLIM: of the instances that serve one
+// rank, the one that leaves room for a second CTA beside the GEMM.
 //
-// Bound by memory: what counts is how much is in flight on an SM, so a thread keeps no more than it must (the sum packed in
-// bf16 where there is one split) and registers are capped for three to five CTAs per SM.  A grid with fewer CTAs
-// than units takes them in row order from a counter, the residuals of the next unit on their way into L2: rows
-// as CTAs of their own came in waves, each a chain of launch, residual, sums and stores (8 ranks, 300 rows: 600 CTAs
-// on 444 places took two of them).
-template <int THREADS, int NV, int G, bool SPLIT, bool LINES>
-__global__ void __launch_bounds__(THREADS, LocalLinearNormPlaces(G, SPLIT, THREADS))
+// Bound by memory once enough is in flight, and before that by the chain of a unit: residuals and sums, two barriers, weights, stores.
+// So a unit waits for memory as seldom as it can (the sums of a complete tile are asked for with the residuals, the weights of all its
+// ranks at once), a CTA has no more warps than a row needs, and instructions that do no arithmetic are kept out (no division, no
+// branch or zeros for the threads beyond the row's end).  Registers are capped so that 16 to 32 warps share an SM, and none is spilled:
+// 16 bytes of it cost 1 us of 23 (8 ranks, 4 x 1728 x 4096).  A grid with fewer CTAs than units takes them in row order from a
+// counter, the residuals of the next unit on their way into L2: rows as CTAs of their own came in waves, each a chain of
+// launch, residual, sums and stores (8 ranks, 300 rows: 600 CTAs on 444 places took two of them).
+//
+// In a graph, W from HBM, before these measures / with them, us: 8 ranks: 1000 x 256 x 1024 35.1 / 22.5, 2048 x 256 x 1024 47.9 / 32.6,
+// 1500 x 512 x 2304 68.9 / 53.4, 678 x 640 x 1664 33.4 / 29.0, 688 x 1792 x 2816 72.9 / 65.4, 300 x 1792 x 4096 51.0 / 49.0, 32 x 1792 x 4096
+// 31.0 / 26.9, 21 x 384 x 3328 11.9 / 9.4; 4 ranks: 300 x 512 x 1024 14.7 / 10.4, 512 x 2048 x 4096 41.7 / 40.2, 60 x 256 x 3072 10.5 / 8.4;
+// 2 ranks: 188 x 1024 x 2944 13.5 / 11.9, 2048 x 2048 x 4096 level.  Of the 16 us that the rows of 8 x 300 x 4096 take behind the GEMM
+// for 59 MB, 2 go by before the first row is complete and 3 while the last CTAs finish.
+template <int NV, int G, bool SPLIT, bool LINES, bool SLIM>
+__global__ void __launch_bounds__(kLocalLinearNormThreads) __maxnreg__(LocalLinearNormRegs(NV, G, SPLIT, SLIM))
     local_linear_norm_kernel(const __grid_constant__ LocalLinearNormArgs a) {
-    constexpr int VEC = 8, kThreads = THREADS, kWarps = kThreads / 32;
-    __shared__ float s_red[G][kWarps];
+    constexpr int VEC = 8, kMostWarps = kLocalLinearNormThreads / 32;
+    __shared__ __align__(16) float s_red[G][kMostWarps];
     __shared__ uint32_t s_next;
     const CommView& cv = a.cv;
     const uint32_t ngroups = (a.world + G - 1) / G, units = a.T * ngroups, flags_per_split = a.N / kLocalGemmUnitCols;
-    const uint32_t tid = threadIdx.x, nvec = a.N / VEC;
+    const uint32_t tid = threadIdx.x, nthreads = blockDim.x, nvec = a.N / VEC, rowbytes = a.N * 2;
     const bool taking = gridDim.x < units;  // from the counter
     uint32_t* const counter = flag_word(cv, 0, kCallLocalRows);
     // The next kernel may set up, and ask for its weights, under this one.  Whatever it is, it waits for the end of this kernel, and with
@@ -417,10 +427,18 @@ __global__ void __launch_bounds__(THREADS, LocalLinearNormPlaces(G, SPLIT, THREA
     if (a.early) ptx::grid_launch_dependents();
     const uint32_t epoch = *reinterpret_cast<volatile uint32_t*>(flag_word(cv, 0, kCallLocalRowCalls)) + 1u;
     const uint64_t deadline = ptx::globaltimer() + cv.timeout_ns;
+    // A thread without a vector of the row (the last ones of a CTA) loads the row's last one, which costs no branch and no zeros,
+    // and keeps it out of the sum of squares and of memory.
     bool have[NV];
+    uint32_t at[NV];  // byte in the row
 #pragma unroll
-    for (int j = 0; j < NV; ++j) have[j] = tid + j * kThreads < nvec;
-    uint32_t unit = blockIdx.x, ready = ~0u;
+    for (int j = 0; j < NV; ++j) {
+        have[j] = tid + j * nthreads < nvec;
+        at[j] = min(tid + j * nthreads, nvec - 1) * 16;
+    }
+    uint32_t unit = blockIdx.x;
+    uint32_t tile = 0, tile_end = 0;  // the tile in front of row tile_end is complete (a CTA's rows only go up)
+    if (tid < G * kMostWarps) (&s_red[0][0])[tid] = 0.f;  // those of warps that a CTA of this size has not
     if (taking) {
         if (tid == 0) s_next = atomicAdd(counter, 1u);
         __syncthreads();
@@ -436,39 +454,73 @@ __global__ void __launch_bounds__(THREADS, LocalLinearNormPlaces(G, SPLIT, THREA
     if (unit >= units && tid == 0) check_in();  // nothing was left for this CTA
     const float inv_n = 1.f / static_cast<float>(a.N);
     bool late = false;
+    // When a step asks for its weights (plain loads: the rows of an SM share them in L1).  One by one behind the stores and the barrier
+    // each rank's is a latency of its own, so: 0 with the residuals, 1 ahead of the stores, 2 all at once behind the barrier, 3 one by
+    // one where registers are short and there are enough rows to hide it.
+    constexpr int kWeights = G == 1 ? 0 : NV * G == 2 ? 1 : NV == 1 || SPLIT ? 2 : 3;
+    uint4 w1[NV][G];
+    auto load_weight = [&](int g, int j, uint32_t q) { w1[j][g] = ptx::ld_v4(static_cast<const char*>(a.weight[q]) + at[j]); };
+    const uint32_t most = a.world - 1;  // a group beyond the last rank computes that one again and stores nothing
+    auto load_weights = [&](uint32_t q0) {
+#pragma unroll
+        for (int g = 0; g < G; ++g)
+#pragma unroll
+            for (int j = 0; j < NV; ++j) load_weight(g, j, min(q0 + g, most));
+    };
     while (unit < units) {
-        const uint32_t row = unit / ngroups, q0 = (unit - row * ngroups) * G;
-        const uint64_t off0 = static_cast<uint64_t>(row) * a.N * 2 + tid * 16;  // this thread's first vector; the others 4 KiB apart
+        const uint32_t row = ngroups == 1 ? unit : __umulhi(unit, a.by_groups), q0 = (unit - row * ngroups) * G;
+        const uint32_t off0 = row * rowbytes;
         if (taking && tid == 0) s_next = atomicAdd(counter, 1u);
-        // Residuals (and the weights of a CTA that serves one rank) are inputs of the call: complete since before the first
-        // kernel passed its own wait.
-        uint4 res[NV][G], w1[NV];
+        // Residuals and weights are inputs of the call: complete since before the first kernel passed its own wait.
+        uint4 res[NV][G];
+        if (kWeights == 0) load_weights(q0);
 #pragma unroll
-        for (int j = 0; j < NV; ++j) {
+        for (int g = 0; g < G; ++g) {
+            const char* const r = static_cast<const char*>(a.residual[min(q0 + g, most)]);
+            if (r) {
 #pragma unroll
-            for (int g = 0; g < G; ++g) {
-                const char* r = q0 + g < a.world ? static_cast<const char*>(a.residual[q0 + g]) : nullptr;
-                res[j][g] = r && have[j] ? ptx::ld_cg_v4(r + off0 + j * (kThreads * 16)) : make_uint4(0, 0, 0, 0);
+                for (int j = 0; j < NV; ++j) res[j][g] = ptx::ld_cg_v4(r + off0 + at[j]);
+            } else {
+#pragma unroll
+                for (int j = 0; j < NV; ++j) res[j][g] = make_uint4(0, 0, 0, 0);
             }
-            if (G == 1 && have[j]) w1[j] = ptx::ld_cg_v4(static_cast<const char*>(a.weight[q0]) + (tid + j * kThreads) * 16);
         }
-        const uint32_t tile = row / a.s.tokens, nsplit = a.s.nsplit;
-        if (!LINES && tile != ready) {
+        const uint32_t nsplit = a.s.nsplit;
+        const uint64_t split_stride = static_cast<uint64_t>(a.T) * a.N * (LINES ? 4 : 2);
+        // Splits in flight together, added in order.
+        constexpr int kFly = !SPLIT ? 1 : G > 1 ? 2 : SLIM ? (NV == 2 ? 1 : LINES ? 2 : 4) : 4;
+        uint4 x[NV][kFly];
+        auto load_sums = [&](uint32_t k0) {
+#pragma unroll
+            for (int k = 0; k < kFly; ++k)
+                if (k0 + k < nsplit) {
+#pragma unroll
+                    for (int j = 0; j < NV; ++j) x[j][k] = ptx::ld_cg_v4(a.sums + (k0 + k) * split_stride + off0 + at[j]);
+                }
+        };
+        // The first sums of a tile that is known to be complete are asked for together with the residuals.
+        const bool asked = !LINES && row < tile_end;
+        if (asked) load_sums(0);
+        if (!LINES && !asked) {
             // The flags of this row's token tile, a few per thread.
-            const uint32_t first = kLocalGemmFlagOff + tile * a.s.nsplit * flags_per_split;
-            for (uint32_t e = tid; e < nsplit * flags_per_split && !late; e += kThreads) {
-                uint32_t polls = 0, seen;
-                while (!ptx::seq_reached(seen = ptx::ld_acquire_gpu(flag_word(cv, 0, first + e)), epoch)) {
-                    // This CTA shares the SM with the GEMM, and hundreds of them poll.
-                    if (++polls > 2) ptx::nanosleep(kFlagSleepNs);
-                    if ((polls & 7u) == 0 && ptx::globaltimer() > deadline) {
-                        report_timeout(cv, kSiteGemmPartials, 0, blockIdx.x, epoch, seen);
-                        late = true;
-                        break;
-                    }
+            while (row >= tile_end) tile_end += a.s.tokens, ++tile;
+            const uint32_t first = kLocalGemmFlagOff + (tile - 1) * nsplit * flags_per_split;
+            // (There are no more flags than threads: at most eight splits of one flag per 128 columns.)
+            bool there = tid >= nsplit * flags_per_split || late;
+            for (uint32_t polls = 1;; ++polls) {
+                uint32_t seen = 0;
+                if (!there) there = ptx::seq_reached(seen = ptx::ld_acquire_gpu(flag_word(cv, 0, first + tid)), epoch);
+                const uint32_t waiting = __ballot_sync(0xffffffffu, !there);
+                if (waiting == 0) break;
+                // This CTA shares the SM with the GEMM, and hundreds of them poll; but once the first unit of the tile is there, the
+                // last one is not far.
+                if (polls > 2) ptx::nanosleep(waiting == 0xffffffffu ? kFlagSleepNs : kFlagNearNs);
+                if ((polls & 7u) == 0 && __any_sync(0xffffffffu, ptx::globaltimer() > deadline)) {
+                    if (!there) report_timeout(cv, kSiteGemmPartials, 0, blockIdx.x, epoch, seen);
+                    late = true;
+                    break;
                 }
             }
-            ready = tile;
         }
         // After a wait that ran out the rows are not worth anything, but the CTA goes on, without waiting: every unit is taken,
         // every CTA checks in and the two counts of calls stay alike.
@@ -476,15 +528,16 @@ __global__ void __launch_bounds__(THREADS, LocalLinearNormPlaces(G, SPLIT, THREA
         if (taking) {
             unit = s_next;
             if (unit < units) {
-                const uint32_t nrow = unit / ngroups, nq = (unit - nrow * ngroups) * G;
+                const uint32_t nrow = ngroups == 1 ? unit : __umulhi(unit, a.by_groups), nq = (unit - nrow * ngroups) * G;
+                // One 128-byte line per eight vectors.
+                if ((tid & 7) == 0) {
 #pragma unroll
-                for (int g = 0; g < G; ++g) {
-                    const char* r = nq + g < a.world ? static_cast<const char*>(a.residual[nq + g]) : nullptr;
-                    // One 128-byte line per eight vectors.
-                    if (r && (tid & 7) == 0)
+                    for (int g = 0; g < G; ++g) {
+                        const char* const r = static_cast<const char*>(a.residual[min(nq + g, most)]);
+                        if (r)
 #pragma unroll
-                        for (int j = 0; j < NV; ++j)
-                            if (have[j]) ptx::prefetch_l2(r + static_cast<uint64_t>(nrow) * a.N * 2 + (tid + j * kThreads) * 16);
+                            for (int j = 0; j < NV; ++j) ptx::prefetch_l2(r + nrow * rowbytes + at[j]);
+                    }
                 }
             }
         } else {
@@ -492,33 +545,23 @@ __global__ void __launch_bounds__(THREADS, LocalLinearNormPlaces(G, SPLIT, THREA
         }
         // Once every CTA has read the call number and taken its last unit, both counters may move on: the next call reads
         // them, nothing in this one does.  Done here, under the work of the last unit.
-        if (unit >= units && tid == kThreads - 1) check_in();
+        if (unit >= units && tid == nthreads - 1) check_in();
 
-        uint4 one[SPLIT ? 1 : NV];
         float sum[SPLIT ? NV : 1][VEC];
         if constexpr (!SPLIT) {
-#pragma unroll
-            for (int j = 0; j < NV; ++j) one[j] = have[j] ? ptx::ld_cg_v4(a.sums + off0 + j * (kThreads * 16)) : make_uint4(0, 0, 0, 0);
+            if (!asked) load_sums(0);
         } else {
-            const uint64_t split_stride = static_cast<uint64_t>(a.T) * a.N * (LINES ? 4 : 2);
-            const char* const src = a.sums + (LINES ? 2 * off0 : off0);
-#pragma unroll
-            for (int j = 0; j < NV; ++j)
-#pragma unroll
-                for (int i = 0; i < VEC; ++i) sum[j][i] = 0.f;
-            // Splits in flight together, added in order: four where few rows leave the SM's registers to few CTAs.
-            constexpr int kFly = G == 1 ? 4 : 2;
             for (uint32_t k0 = 0; k0 < nsplit && !late; k0 += kFly) {
-                uint4 x[NV][kFly];
                 if constexpr (LINES) {
+                    const char* const src = a.sums + 2 * static_cast<uint64_t>(off0);
                     uint4 y[NV][kFly];
                     uint32_t polls = 0;
                     bool missing;
                     // One lane of a warp waits for one of its lines of the last split: asking for all lines again and
                     // again (64 KiB per CTA) holds up the GEMM that writes them.
-                    if (k0 == 0 && (tid & 31) == 0 && have[0]) {
+                    if (k0 == 0 && (tid & 31) == 0) {
                         uint4 l;
-                        while ((l = ptx::ld_volatile_v4(src + (nsplit - 1) * split_stride)).y != epoch || l.w != ~epoch) {
+                        while ((l = ptx::ld_volatile_v4(src + 2 * at[0] + (nsplit - 1) * split_stride)).y != epoch || l.w != ~epoch) {
                             ptx::nanosleep(kLineSleepNs);
                             if ((++polls & 63u) == 0 && ptx::globaltimer() > deadline) break;  // the loop below reports it
                         }
@@ -528,18 +571,19 @@ __global__ void __launch_bounds__(THREADS, LocalLinearNormPlaces(G, SPLIT, THREA
                         missing = false;
 #pragma unroll
                         for (int k = 0; k < kFly; ++k)
+                            if (k0 + k < nsplit) {
 #pragma unroll
-                            for (int j = 0; j < NV; ++j)
-                                if (k0 + k < nsplit && have[j]) {
-                                    const char* p = src + (k0 + k) * split_stride + j * (kThreads * 32);
+                                for (int j = 0; j < NV; ++j) {
+                                    const char* p = src + (k0 + k) * split_stride + 2 * at[j];
                                     x[j][k] = ptx::ld_volatile_v4(p);
                                     y[j][k] = ptx::ld_volatile_v4(p + 16);
                                 }
+                            }
 #pragma unroll
                         for (int k = 0; k < kFly; ++k)
 #pragma unroll
                             for (int j = 0; j < NV; ++j)
-                                if (k0 + k < nsplit && have[j])
+                                if (k0 + k < nsplit)
                                     missing |= x[j][k].y != epoch || x[j][k].w != ~epoch || y[j][k].y != epoch || y[j][k].w != ~epoch;
                         if (missing && (++polls & 63u) == 0 && ptx::globaltimer() > deadline) {
                             report_timeout(cv, kSiteGemmPartials, 0, blockIdx.x, epoch, 0u);
@@ -551,67 +595,75 @@ __global__ void __launch_bounds__(THREADS, LocalLinearNormPlaces(G, SPLIT, THREA
 #pragma unroll
                         for (int j = 0; j < NV; ++j) x[j][k] = make_uint4(x[j][k].x, x[j][k].z, y[j][k].x, y[j][k].z);
                 } else {
-#pragma unroll
-                    for (int k = 0; k < kFly; ++k)
-#pragma unroll
-                        for (int j = 0; j < NV; ++j)
-                            if (k0 + k < nsplit && have[j]) x[j][k] = ptx::ld_cg_v4(src + (k0 + k) * split_stride + j * (kThreads * 16));
+                    if (k0 > 0 || !asked) load_sums(k0);
                 }
 #pragma unroll
                 for (int k = 0; k < kFly; ++k)
 #pragma unroll
-                    for (int j = 0; j < NV; ++j)
-                        if (k0 + k < nsplit && have[j]) accumulate<__nv_bfloat16>(sum[j], x[j][k]);
+                    for (int j = 0; j < NV; ++j) {
+                        if (k == 0 && k0 == 0) unpack16<__nv_bfloat16>(sum[j], x[j][0]);
+                        else if (k0 + k < nsplit) accumulate<__nv_bfloat16>(sum[j], x[j][k]);
+                    }
+            }
+            if (late) {
+#pragma unroll
+                for (int j = 0; j < NV; ++j)
+#pragma unroll
+                    for (int i = 0; i < VEC; ++i) sum[j][i] = 0.f;
             }
         }
+        if (kWeights == 1) load_weights(q0);
         // sum + residual of rank q0 + g, vector j.
         auto row_of = [&](int j, int g, float (&p)[VEC]) {
             if constexpr (SPLIT) {
 #pragma unroll
                 for (int i = 0; i < VEC; ++i) p[i] = sum[j][i];
             } else {
-#pragma unroll
-                for (int i = 0; i < VEC; ++i) p[i] = 0.f;
-                accumulate<__nv_bfloat16>(p, one[j]);
+                unpack16<__nv_bfloat16>(p, x[j][0]);
             }
             accumulate<__nv_bfloat16>(p, res[j][g]);
         };
 #pragma unroll
         for (int g = 0; g < G; ++g) {
             float ss = 0.f;
-            char* const ro = q0 + g < a.world ? static_cast<char*>(a.residual_out[q0 + g]) : nullptr;
+            char* const ro = q0 + g <= most ? static_cast<char*>(a.residual_out[q0 + g]) : nullptr;
 #pragma unroll
             for (int j = 0; j < NV; ++j) {
                 float p[VEC];
                 row_of(j, g, p);
-                if (ro && have[j]) ptx::st_v4(ro + off0 + j * (kThreads * 16), pack16<__nv_bfloat16>(p));
+                if (ro && have[j]) ptx::st_v4(ro + off0 + at[j], pack16<__nv_bfloat16>(p));
+                float sq = p[0] * p[0];
 #pragma unroll
-                for (int i = 0; i < VEC; ++i) ss += p[i] * p[i];
+                for (int i = 1; i < VEC; ++i) sq += p[i] * p[i];
+                ss += have[j] ? sq : 0.f;
             }
 #pragma unroll
             for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
             if ((tid & 31) == 0) s_red[g][tid >> 5] = ss;
         }
         __syncthreads();
+        if (kWeights == 2) load_weights(q0);
 #pragma unroll
         for (int g = 0; g < G; ++g) {
-            if (q0 + g >= a.world) break;
+            if (q0 + g > most) break;
             float t = 0.f;
 #pragma unroll
-            for (int w = 0; w < kWarps; ++w) t += s_red[g][w];
+            for (int w = 0; w < kMostWarps; w += 4) {
+                const float4 part = *reinterpret_cast<const float4*>(&s_red[g][w]);
+                t += (part.x + part.y) + (part.z + part.w);
+            }
             const float inv_rms = rsqrtf(t * inv_n + a.eps);
+            char* const out = static_cast<char*>(a.out[q0 + g]) + off0;
 #pragma unroll
             for (int j = 0; j < NV; ++j) {
                 if (!have[j]) continue;
                 float p[VEC], w[VEC];
                 row_of(j, g, p);
-#pragma unroll
-                for (int i = 0; i < VEC; ++i) w[i] = 0.f;
-                // (Plain loads: the rows of an SM share them in L1.)
-                accumulate<__nv_bfloat16>(w, G == 1 ? w1[j] : *reinterpret_cast<const uint4*>(static_cast<const char*>(a.weight[q0 + g]) + (tid + j * kThreads) * 16));
+                if (kWeights == 3) load_weight(g, j, q0 + g);
+                unpack16<__nv_bfloat16>(w, w1[j][g]);
 #pragma unroll
                 for (int i = 0; i < VEC; ++i) p[i] = p[i] * inv_rms * w[i];
-                ptx::st_v4(static_cast<char*>(a.out[q0 + g]) + off0 + j * (kThreads * 16), pack16<__nv_bfloat16>(p));
+                ptx::st_v4(out + at[j], pack16<__nv_bfloat16>(p));
             }
         }
     }
@@ -619,19 +671,10 @@ __global__ void __launch_bounds__(THREADS, LocalLinearNormPlaces(G, SPLIT, THREA
     ptx::grid_dependency_wait();
 }
 
-template <int THREADS, int NV, int G>
-const void* pick_linear_norm(bool split, bool lines) {
-    if constexpr (G == 1) {
-        if (lines) return (const void*)local_linear_norm_kernel<THREADS, NV, 1, true, true>;
-    }
-    return split ? (const void*)local_linear_norm_kernel<THREADS, NV, G, true, false>
-                 : (const void*)local_linear_norm_kernel<THREADS, NV, G, false, false>;
-}
-template <int THREADS, int NV>
-const void* pick_linear_norm_g(int g, bool split, bool lines) {
-    return g == 1   ? pick_linear_norm<THREADS, NV, 1>(split, lines)
-           : g == 2 ? pick_linear_norm<THREADS, NV, 2>(split, lines)
-                    : pick_linear_norm<THREADS, NV, 4>(split, lines);
+template <int NV, int G>
+const void* pick_linear_norm(bool split) {
+    return split ? (const void*)local_linear_norm_kernel<NV, G, true, false, true>
+                 : (const void*)local_linear_norm_kernel<NV, G, false, false, true>;
 }
 
 }  // namespace
@@ -639,11 +682,15 @@ const void* pick_linear_norm_g(int g, bool split, bool lines) {
 const void* LocalGemmKernel() { return reinterpret_cast<const void*>(local_gemm_kernel); }
 uint32_t LocalGemmSmemBytes() { return kSmemBytes; }
 
-const void* LocalLinearNormKernel(uint32_t N, int ranks_per_cta, bool split, bool lines) {
-    constexpr int kThreads = kLocalLinearNormThreads;
-    if (LocalLinearNormThreads(N) != kThreads) return pick_linear_norm_g<LocalLinearNormThreads(1), 1>(ranks_per_cta, split, lines);
-    return N / 8 <= static_cast<uint32_t>(kThreads) ? pick_linear_norm_g<kThreads, 1>(ranks_per_cta, split, lines)
-                                                    : pick_linear_norm_g<kThreads, 2>(ranks_per_cta, split, lines);
+const void* LocalLinearNormKernel(uint32_t N, int ranks_per_cta, bool split, bool lines, bool slim) {
+    const bool wide = LocalLinearNormVectors(N) == 2;
+    if (lines) {
+        if (wide) return slim ? (const void*)local_linear_norm_kernel<2, 1, true, true, true> : (const void*)local_linear_norm_kernel<2, 1, true, true, false>;
+        return slim ? (const void*)local_linear_norm_kernel<1, 1, true, true, true> : (const void*)local_linear_norm_kernel<1, 1, true, true, false>;
+    }
+    if (ranks_per_cta == 4) return pick_linear_norm<1, 4>(split);
+    if (ranks_per_cta == 2) return wide ? pick_linear_norm<2, 2>(split) : pick_linear_norm<1, 2>(split);
+    return wide ? pick_linear_norm<2, 1>(split) : pick_linear_norm<1, 1>(split);
 }
 
 }  // namespace yali

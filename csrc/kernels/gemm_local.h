@@ -21,11 +21,13 @@ constexpr int kLocalGemmThreads = 384;         // eight epilogue warps, TMA, MMA
 // T = 300 (9.4 Mi) 60.5 / 59.5, T = 350 (11 Mi) 67.3 / 66.2.  The kernel behind asks for its W whatever its own size: large calls
 // behind small ones 80.2 / 78.0, 68.6 / 67.9, 90.6 / 91.3 with / without such a limit, large behind large level.
 constexpr uint64_t kLocalLinearEarly = 12ull << 20;
-constexpr int kLocalLinearNormThreads = 256;   // one row; up to two 16-byte vectors per thread: N <= 4096
-// A row of up to 64 vectors leaves most of 256 threads idle, and a unit of the row kernel is a chain of latencies, so
-// what counts is how many are in flight: four times as many CTAs of 64 threads (K = 64, N = 128, 4096 rows: 2 ranks 33 ->
-// 19 us, 8 ranks 110 -> 39; above 512 columns 128 or 256 threads are busy).
-constexpr int LocalLinearNormThreads(uint32_t N) { return N <= 512 ? 64 : kLocalLinearNormThreads; }
+constexpr int kLocalLinearNormThreads = 256;   // at most; one row, one or two 16-byte vectors per thread: N <= 4096
+constexpr int LocalLinearNormVectors(uint32_t N) { return N <= 8u * kLocalLinearNormThreads ? 1 : 2; }
+// No more warps than a row needs.  A unit of the row kernel is a chain of latencies, so what counts is how many are in flight.
+constexpr int LocalLinearNormThreads(uint32_t N) {
+    const uint32_t per_warp = 32u * 8u * LocalLinearNormVectors(N);
+    return 32 * static_cast<int>((N + per_warp - 1) / per_warp);
+}
 
 // T rows in `tiles` token tiles of `tokens` (a multiple of 32, at most 256), the k-blocks of all ranks (one rank after the
 // other) in `nsplit` runs of `kper`.
@@ -54,18 +56,25 @@ struct LocalLinearNormArgs {
     void* out[kMaxRanks];             // [T, N]
     uint32_t T, N, world;
     LocalGemmShape s;
+    uint32_t by_groups;  // ceil(2^32 / groups of ranks): the row of a unit without a division
     uint32_t early;  // at most kLocalLinearEarly elements: the next kernel may start under these rows
     float eps;
 };
 
-// CTAs of the row kernel per SM (with the GEMM gone) that its register cap allows.
-constexpr int LocalLinearNormPlaces(int ranks_per_cta, bool split, int threads) {
-    return (ranks_per_cta == 4 ? (split ? 2 : 3) : ranks_per_cta == 2 ? (split ? 3 : 4) : 2) * (kLocalLinearNormThreads / threads);
+// Registers per thread of the row kernel.  Up to 72, two CTAs of 256 threads fit beside the GEMM's, so that up to two units per SM are there,
+// with their residuals, when the sums come; CTAs that start when the GEMM's have left are 2.5 us later (8 ranks, 32 x 1792 x 4096 31.0
+// with 128 registers, 26.9 with 72).  `slim` is about the instances that serve one rank: the other one asks for the lines of four K splits
+// at a time.  Two vectors of two ranks and several splits do not fit 72 (spills: 50 -> 55 us).
+constexpr int LocalLinearNormRegs(int vectors, int ranks_per_cta, bool split, bool slim) {
+    if (ranks_per_cta == 1) return slim ? 72 : vectors == 1 ? 104 : 144;
+    if (ranks_per_cta == 2) return !split ? 64 : vectors == 1 ? 72 : 96;
+    return !split ? 72 : 96;
 }
 
 const void* LocalGemmKernel();
 uint32_t LocalGemmSmemBytes();
-// `ranks_per_cta`: 1, 2 or 4; `split`: more than one K split; `lines` (one rank per CTA, split): flag-in-data sums.
-const void* LocalLinearNormKernel(uint32_t N, int ranks_per_cta, bool split, bool lines);
+// `ranks_per_cta`: 1, 2 or (rows of one vector per thread) 4; `split`: more than one K split; `lines` (one rank per CTA, split):
+// flag-in-data sums.
+const void* LocalLinearNormKernel(uint32_t N, int ranks_per_cta, bool split, bool lines, bool slim);
 
 }  // namespace yali

@@ -95,6 +95,37 @@ __device__ __forceinline__ void accumulate<__nv_bfloat16>(float* acc, const uint
     }
 }
 
+// f[0..kVec) = lanes of the 16-byte vector v interpreted as T.  (accumulate() onto zeros costs an addition per lane, which the
+// compiler has to keep for the sake of -0.)
+template <typename T>
+__device__ __forceinline__ void unpack16(float* f, const uint4& v);
+template <>
+__device__ __forceinline__ void unpack16<float>(float* f, const uint4& v) {
+    f[0] = __uint_as_float(v.x);
+    f[1] = __uint_as_float(v.y);
+    f[2] = __uint_as_float(v.z);
+    f[3] = __uint_as_float(v.w);
+}
+template <>
+__device__ __forceinline__ void unpack16<__half>(float* f, const uint4& v) {
+    const __half2* h = reinterpret_cast<const __half2*>(&v);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float2 p = __half22float2(h[i]);
+        f[2 * i] = p.x;
+        f[2 * i + 1] = p.y;
+    }
+}
+template <>
+__device__ __forceinline__ void unpack16<__nv_bfloat16>(float* f, const uint4& v) {
+    const uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        f[2 * i] = __uint_as_float(w[i] << 16);
+        f[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+    }
+}
+
 // Packs n = 16/sizeof(T) fp32 lanes into one 16-byte vector of T.
 template <typename T>
 __device__ __forceinline__ uint4 pack16(const float* f);

@@ -4,6 +4,7 @@
 #include "../core/nvtx.h"
 
 #include <algorithm>
+#include <atomic>
 #include <cstring>
 #include <map>
 #include <mutex>
@@ -358,6 +359,21 @@ bool CanRunLocal(Communicator& comm, const FusedLinearDesc* descs, uint32_t T, u
     return true;
 }
 
+// CTAs of the row kernel on an SM with the GEMM gone.  Asked for once: registers are shared out to the SM's four quarters by warps, which
+// no formula of threads and registers says.
+uint32_t LocalLinearNormPlaces(uint32_t N, int ranks_per_cta, bool split, bool lines, bool slim) {
+    static std::atomic<int> known[4][3][2][kLocalLinearNormThreads / 32 + 1];
+    const int threads = LocalLinearNormThreads(N);
+    std::atomic<int>& k = known[ranks_per_cta == 1 && slim ? 3 : ranks_per_cta / 2][lines ? 2 : split ? 1 : 0][LocalLinearNormVectors(N) - 1][threads / 32];
+    int n = k.load(std::memory_order_relaxed);
+    if (n == 0) {
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, LocalLinearNormKernel(N, ranks_per_cta, split, lines, slim), threads, 0) != cudaSuccess) (void)cudaGetLastError();
+        n = std::max(n, 1);
+        k.store(n, std::memory_order_relaxed);
+    }
+    return static_cast<uint32_t>(n);
+}
+
 Result LaunchLocal(Communicator& comm, const DriverApi* drv, const FusedLinearDesc* descs, uint32_t T, uint32_t N,
                    uint32_t K, const FusedLinearOptions& opt, const cudaStream_t* streams) {
     auto fail = [&](Result r, const std::string& what) {
@@ -422,32 +438,36 @@ Result LaunchLocal(Communicator& comm, const DriverApi* drv, const FusedLinearDe
         n.out[r] = d.out;
     }
     const uint32_t items = g.s.tiles * ((N + kLocalGemmPairCols - 1) / kLocalGemmPairCols) * g.s.nsplit;
-    // With few rows the ranks of a row are spread over CTAs (each adds the splits again, from L2) and the sums travel as
-    // flag-in-data lines, which saves the fence and the flag at the price of twice the bytes.  (All figures here: in a graph,
-    // short bursts, us.  2 ranks, K = 2048: T = 16 13.1 -> 12.1, T = 64 16.1 -> 15.1; 8 ranks, K = 1792, two splits:
-    // T = 36 34.6 -> 33.4; but 2 ranks T = 96 16.0 -> 16.9, T = 128 16.5 -> 18.4.)  From two CTAs per SM on a CTA serves two
-    // or four ranks, and the grid is what fits the GPU: with two more CTAs fit, with four the sums are read less often.  A
-    // round of four takes about 3/2 of a round of two (5/4 for rows of one vector per thread), so the rounds decide
-    // (8 ranks, two against four: T = 64 19.0 / 20.5, T = 128 24.9 / 22.7, T = 300 52.8 / 54.7, T = 512 40.7 / 44.7,
-    // T = 2048 122.9 / 131.4; 4 ranks: T = 256 26.3 / 24.0, T = 512 32.1 / 35.3; N = 2048, T = 2048 100 / 94).
+    // With few rows the sums travel as flag-in-data lines, which saves the fence and the flag at the price of twice the bytes.
+    // (In a graph, short bursts, us.  2 ranks, K = 2048: T = 16 13.1 -> 12.1, T = 64 16.1 -> 15.1; 8 ranks, K = 1792, two splits:
+    // T = 36 34.6 -> 33.4; but 2 ranks T = 96 16.0 -> 16.9, T = 128 16.5 -> 18.4.)
     const uint64_t line_bytes = static_cast<uint64_t>(T) * N * 4 * g.s.nsplit;
     const bool lines = few && T <= 64 && g.s.nsplit > 1 && line_bytes <= 2ull * W * lay.gemm_ll_cap;
     if (lines) {
         g.lines = 1;
         n.sums = g.sums = g.cv.heap[0] + lay.gemm_ll_off;
     }
-    const int threads = LocalLinearNormThreads(N);
-    auto units_of = [&](int gr) { return T * ((W + gr - 1) / gr); };
-    auto rounds_of = [&](int gr) {
-        const uint32_t fit = sms * LocalLinearNormPlaces(gr, g.s.nsplit > 1, threads);
-        return (units_of(gr) + fit - 1) / fit;
-    };
-    const bool one_vector = N <= 8u * kLocalLinearNormThreads;
-    const bool four = W > 2 && rounds_of(4) * (one_vector ? 5 : 6) <= rounds_of(2) * 4;
-    const int group = few ? 1 : four ? 4 : 2;
-    const uint32_t units = units_of(group);
-    const void* const fn2 = LocalLinearNormKernel(N, group, g.s.nsplit > 1, lines);
-    const uint32_t places = sms * LocalLinearNormPlaces(group, g.s.nsplit > 1, threads);
+    const uint32_t threads = LocalLinearNormThreads(N);
+    const bool split = g.s.nsplit > 1;
+    const bool narrow = LocalLinearNormVectors(N) == 1;
+    auto units_of = [&](int gr) { return static_cast<uint32_t>(T * ((W + gr - 1) / gr)); };
+    // Few CTAs have the SMs' registers to themselves, and then ask for the lines of four splits at a time (slim / not: 2 ranks, 8 x 2048 x
+    // 4096 10.2 / 9.5; 8 ranks, 8 x 1792 x 4096 24.3 / 24.9, 24 x 512 x 1024 7.2 / 6.9, 30 x 1024 x 2048 11.7 / 13.6).
+    const bool slim = narrow ? units_of(1) * threads > 256 * sms : units_of(1) > 32;
+    auto places_of = [&](int gr) { return sms * LocalLinearNormPlaces(N, gr, split, lines, slim); };
+    // Ranks that a CTA serves, each CTA adding the splits again: one while that needs no more than two CTAs of 256 threads per SM and four
+    // of any size (one / two / four ranks, us: 8 ranks, 40 x 256 x 512 7.1 / 8.4 / 8.4, 60 x 512 x 1024 9.7 / 10.2 / 10.3; 4 ranks, 76 x 1024 x
+    // 2048 10.9 / 10.5 / 12.3; 2 ranks, 1000 x 256 x 128 13.2 / 9.7).  Above, two for wide rows (four, which spill: 8 ranks, 2048 x 512 x 4096
+    // 120 / 105, 1500 x 512 x 2304 61.7 / 53.1; one, 300 x 1792 x 4096 51.6 / 50.4).  For narrow rows two while they leave half of the places
+    // free, else four, which read the sums less often (two / four: 8 ranks, 40 x 1024 x 2048 14.5 / 15.3, 133 x 448 x 1152 12.3 / 11.6, 1000 x 256
+    // x 1024 23.2 / 21.1; 4 ranks, 200 x 1024 x 2048 14.3 / 13.8), unless the last group would hold one or two ranks (6 ranks, 300 x 1024 x
+    // 2048 21.2 / 21.8).
+    int group = 1;
+    if (!few && !(narrow && units_of(1) <= 4 * sms && units_of(1) * threads <= 512 * sms))
+        group = !narrow || (W & 3) == 1 || (W & 3) == 2 || 2 * units_of(2) <= places_of(2) ? 2 : 4;
+    const uint32_t ngroups = (W + group - 1) / group, units = units_of(group), places = places_of(group);
+    n.by_groups = static_cast<uint32_t>(((1ull << 32) + ngroups - 1) / ngroups);
+    const void* const fn2 = LocalLinearNormKernel(N, group, split, lines, slim);
     const cudaStream_t s = streams && streams[0] ? streams[0] : comm.default_stream(0);
     void* gp[] = {&g};
     void* np[] = {&n};

@@ -187,6 +187,40 @@ def test_ranks_on_one_gpu_add_in_the_gemm(world, T, K, N):
         assert c.launches - before == 1
 
 
+# Every way in which the row kernel shares out rows: one rank of a row per CTA (flag-in-data lines of few and of many CTAs, flags), two and four
+# ranks, groups that the last ranks do not fill; row widths that fill their last warp and that do not, with one and with two vectors per
+# thread.
+@pytest.mark.parametrize("world,T,K,N", [(8, 3, 64, 2304), (8, 33, 128, 4096), (4, 40, 64, 640), (4, 36, 256, 384), (2, 100, 256, 3968),
+                                         (4, 75, 128, 1024), (3, 120, 64, 768), (2, 300, 64, 512), (5, 130, 64, 1280), (3, 260, 64, 2048),
+                                         (7, 200, 128, 1152), (8, 161, 64, 1664), (4, 1025, 64, 1152), (6, 100, 64, 2176), (7, 60, 512, 2176),
+                                         (8, 150, 256, 3200)])
+def test_rows_of_ranks_on_one_gpu(world, T, K, N):
+    """Whole-number inputs as above: residuals bit by bit, the norm to one rounding.  Two calls, the second with other inputs."""
+    g = torch.Generator(device="cuda").manual_seed(T * N + world)
+
+    def pick(*shape, p):
+        keep = torch.rand(shape, generator=g, device="cuda") < p
+        return (keep * torch.randint(-1, 2, shape, generator=g, device="cuda")).to(torch.bfloat16)
+
+    with yali.Comm.emulated(world, device=0) as c:
+        ws, calls = [pick(N, K, p=0.3) for _ in range(world)], []
+        nw = [(torch.rand(N, generator=g, device="cuda") + 0.5).to(torch.bfloat16) for _ in range(world)]
+        for _ in range(2):
+            xs, res = [pick(T, K, p=0.3) for _ in range(world)], [pick(T, N, p=0.9) for _ in range(world)]
+            pre, before = [torch.empty_like(r) for r in res], c.launches
+            calls.append((xs, res, pre, c.fused_linear_rmsnorm(xs, ws, nw, res, residual_out=pre)))
+            assert c.launches - before == 2
+        c.sync()
+        for xs, res, pre, outs in calls:
+            total = sum(x.double() @ w.double().T for x, w in zip(xs, ws))
+            assert total.abs().max() < 255
+            for r in range(world):
+                want = total + res[r].double()
+                assert torch.equal(pre[r].double(), want)
+                y = want * torch.rsqrt(want.pow(2).mean(-1, keepdim=True) + 1e-5) * nw[r].double()
+                torch.testing.assert_close(outs[r].double(), y, rtol=2.0 ** -8, atol=1e-6)
+
+
 @pytest.mark.parametrize("world", [2, 8])
 def test_few_rows_back_to_back_with_new_inputs(world):
     """Sums as flag-in-data lines: 60 calls in one graph, rows and inputs changing from call to call, replayed three times.
