@@ -490,7 +490,7 @@ Result Communicator::LaunchLocal(const Plan& plan, const void* const* send, void
         }
         const uint64_t rows = count / opt.hidden;
         const uint32_t vec = 16 / static_cast<uint32_t>(DtypeSize(in));
-        const LocalNormShape s = LocalNormShapeFor(rows, static_cast<uint32_t>(opt.hidden) / vec, world_, sm_count_);
+        const LocalNormShape s = LocalNormShapeFor(rows, static_cast<uint32_t>(opt.hidden) / vec, static_cast<int>(DtypeSize(in)), world_, sm_count_);
         fn = LocalNormKernelFor(in, world_, s);
         name = "local_norm";
         block = dim3(s.threads);

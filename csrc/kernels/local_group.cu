@@ -14,7 +14,7 @@
 // pipelined two-shot kernel (TMA stages, two cross-rank barriers) takes 97 us for the same call.  Whole calls
 // from Python, back to back, multi-GPU kernel / this one: 4 ranks x 6 MB fp16 18.7 / 8.7 us, 8 ranks x 25 MiB fp32 -> bf16
 // 61.1 / 48.4 us, reduce-scatter + all-gather of 64 MiB over 4 ranks 201 / 103 us, all-reduce + residual +
-// RMSNorm of 2048 x 4096 bf16 over 2 ranks 49.3 / 23.3 us.
+// RMSNorm of 2048 x 4096 bf16 over 2 ranks 49.3 / 23.1 us.
 //
 // Parity: none in the reference (it always drives two GPUs).
 #include "coll_common.cuh"
@@ -204,93 +204,122 @@ __global__ void __launch_bounds__(kLocalHostThreads) local_host_kernel(const __g
     local_trace_end(a);
 }
 
+// Registers per thread of the norm kernel.  What counts is the warps that share an SM: 2 ranks, 2048 x 4096 bf16 22.9 us with 40
+// registers, 23.4 with 64.
+constexpr int norm_regs(int world, int nv, int g, bool late, int elem_bytes) {
+    if (world == 1) return nv == 1 ? 32 : (nv == 2 ? 48 : 96) - (elem_bytes == 4 ? nv * 8 - 8 : 0);
+    if (nv == 1) return late ? 40 : 64;
+    return nv == 2 ? 64 : g == 1 && world < 5 ? 96 : 128;
+}
+
 // Sum + residual + RMSNorm of one row for the ranks [g * G, g * G + G) of the group; CTA b handles row
 // b / ngroups, group b % ngroups (the groups of a row are neighbours, so the second one finds the row in
 // L2).  A thread holds NV vectors of the row: it reads them from every rank once, adds in fp32, and keeps
 // the packed residuals of its G ranks until the G sums of squares are known (one block reduction for all).
-template <typename T, int WORLD, int NV, int G>
-__global__ void __launch_bounds__(kLocalThreads) local_norm_kernel(const __grid_constant__ LocalArgs a) {
-    constexpr int VEC = TypeTraits<T>::kVec;
-    constexpr int kMaxW = WORLD ? WORLD : kMaxRanks;
-    const uint32_t W = WORLD ? WORLD : a.world;
-    __shared__ float s_red[G][kLocalThreads / 32];
-    ptx::grid_dependency_wait();
-    local_trace_begin(a);
-    const uint32_t ngroups = (W + G - 1) / G;
-    const uint32_t row = blockIdx.x / ngroups, q0 = (blockIdx.x % ngroups) * G;
+//
+// Bound by HBM with many rows, where the phases of a CTA (loads, barrier, stores) have to run under those of others: few registers, so
+// that two or more CTAs of 512 threads share an SM, and for that two ranks at a time (LATE asks for their weights behind the barrier).
+// Bound by the chain of latencies with few, where it helps to have the weights before the barrier (one by one behind the stores each
+// rank's is a latency) and ranks spread over CTAs.  LocalNormShapeFor has the lines.  In a graph, inputs from HBM, all ranks of a row in a
+// CTA and weights one by one / now, us (floor): bf16, 8 ranks: 64 x 4096 9.5 / 4.9 (2.6), 256 x 4096 19.4 / 14.0 (10.3), 512 x 4096 33.2 / 25.5
+// (20.6), 1000 x 2944 44.7 / 34.9 (28.9), 500 x 8192 59.8 / 48.5 (40.2); 4 ranks: 256 x 1024 4.7 / 3.1, 1024 x 8192 57.3 / 46.7 (41.1);
+// 2 ranks: 64 x 8192 4.1 / 2.9, 2000 x 8192 44.6 / 41.7 (40.2), 2048 x 4096 22.9 / 22.8 (20.6); 3 ranks, 1500 x 4096 45 / 27.4 (22.6); one rank,
+// 8192 x 8192 83.6 / 82.2 (82.2); fp32, 8 ranks, 250 x 8192 71.8 / 49.6 (40.2).
+template <typename T, int WORLD, int NV, int G, bool LATE>
+__global__ void __launch_bounds__(kLocalThreads) __maxnreg__(norm_regs(WORLD, NV, G, LATE, sizeof(T))) local_norm_kernel(const __grid_constant__ LocalArgs a) {
+    constexpr int VEC = TypeTraits<T>::kVec, kMostWarps = kLocalThreads / 32;
+    constexpr uint32_t W = WORLD;
+    __shared__ __align__(16) float s_red[G][kMostWarps];
     const int tid = threadIdx.x, nt = blockDim.x;
+    if (nt < kLocalThreads)  // those of warps that a CTA of this size has not
+        for (int i = tid; i < G * kMostWarps; i += nt) (&s_red[0][0])[i] = 0.f;
+    const uint32_t ngroups = (W + G - 1) / G;
+    const uint32_t row = ngroups == 1 ? blockIdx.x : blockIdx.x / ngroups, q0 = (blockIdx.x - row * ngroups) * G;
     const uint32_t vec_per_row = a.ep.hidden / VEC;
     const uint64_t row_off = static_cast<uint64_t>(row) * vec_per_row * 16;
+    // A thread without a vector of the row (the last ones of a CTA) loads the row's last one, which costs no branch and no zeros, and
+    // keeps it out of the sum of squares and of memory.
+    bool have[NV];
+    uint32_t at[NV];  // byte in the row
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+        have[j] = tid + j * nt < vec_per_row;
+        at[j] = min(static_cast<uint32_t>(tid + j * nt), vec_per_row - 1) * 16;
+    }
+    if (nt < kLocalThreads) __syncthreads();
+    ptx::grid_dependency_wait();
+    local_trace_begin(a);
 
-    uint4 res[NV][G];
+    uint4 res[NV][G], wgt[NV][LATE ? 1 : G];
     float f[NV][VEC];
 #pragma unroll
     for (int j = 0; j < NV; ++j) {
-        const uint32_t c = tid + j * nt;
+        uint4 x[W];
 #pragma unroll
-        for (int i = 0; i < VEC; ++i) f[j][i] = 0.f;
+        for (int q = 0; q < WORLD; ++q) x[q] = ptx::ld_cg_v4(static_cast<const char*>(a.send[q]) + row_off + at[j]);
 #pragma unroll
-        for (int g = 0; g < G; ++g) res[j][g] = make_uint4(0, 0, 0, 0);
-        if (c < vec_per_row) {
-            uint4 x[kMaxW];
-#pragma unroll
-            for (int q = 0; q < kMaxW; ++q)
-                if (q < W) x[q] = ptx::ld_cg_v4(static_cast<const char*>(a.send[q]) + row_off + c * 16ull);
-#pragma unroll
-            for (int g = 0; g < G; ++g)
-                if (q0 + g < W && a.residual[q0 + g])
-                    res[j][g] = ptx::ld_cg_v4(static_cast<const char*>(a.residual[q0 + g]) + row_off + c * 16ull);
-#pragma unroll
-            for (int q = 0; q < kMaxW; ++q)
-                if (q < W) accumulate<T>(f[j], x[q]);
+        for (int g = 0; g < G; ++g) {
+            const char* const r = q0 + g < W ? static_cast<const char*>(a.residual[q0 + g]) : nullptr;
+            res[j][g] = r ? ptx::ld_cg_v4(r + row_off + at[j]) : make_uint4(0, 0, 0, 0);
         }
+        unpack16<T>(f[j], x[0]);
+#pragma unroll
+        for (int q = 1; q < WORLD; ++q) accumulate<T>(f[j], x[q]);
     }
-    float ss[G];
+    auto load_weight = [&](int j, int g) { return ptx::ld_v4(static_cast<const char*>(a.weight[min(q0 + g, W - 1)]) + at[j]); };
+    if constexpr (!LATE) {
+#pragma unroll
+        for (int g = 0; g < G; ++g)
+#pragma unroll
+            for (int j = 0; j < NV; ++j) wgt[j][g] = load_weight(j, g);
+    }
 #pragma unroll
     for (int g = 0; g < G; ++g) {
-        ss[g] = 0.f;
+        float ss = 0.f;
+        char* const ro = q0 + g < W ? static_cast<char*>(a.residual_out[q0 + g]) : nullptr;
 #pragma unroll
         for (int j = 0; j < NV; ++j) {
-            const uint32_t c = tid + j * nt;
             float p[VEC];
 #pragma unroll
             for (int i = 0; i < VEC; ++i) p[i] = f[j][i];
             accumulate<T>(p, res[j][g]);
-            if (c < vec_per_row && q0 + g < W && a.residual_out[q0 + g])
-                ptx::st_v4(static_cast<char*>(a.residual_out[q0 + g]) + row_off + c * 16ull, pack16<T>(p));
+            if (ro && have[j]) ptx::st_v4(ro + row_off + at[j], pack16<T>(p));
+            float sq = p[0] * p[0];
 #pragma unroll
-            for (int i = 0; i < VEC; ++i) ss[g] += p[i] * p[i];
+            for (int i = 1; i < VEC; ++i) sq += p[i] * p[i];
+            ss += have[j] ? sq : 0.f;
         }
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) ss[g] += __shfl_xor_sync(0xffffffffu, ss[g], o);
-        if ((tid & 31) == 0) s_red[g][tid >> 5] = ss[g];
+        for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        if ((tid & 31) == 0) s_red[g][tid >> 5] = ss;
     }
     __syncthreads();
     const float inv_h = 1.f / static_cast<float>(a.ep.hidden);
 #pragma unroll
     for (int g = 0; g < G; ++g) {
         if (q0 + g >= W) break;
-        float t = (tid & 31) < (nt >> 5) ? s_red[g][tid & 31] : 0.f;
+        if constexpr (LATE) {
 #pragma unroll
-        for (int o = 8; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-        t = __shfl_sync(0xffffffffu, t, 0);
+            for (int j = 0; j < NV; ++j) wgt[j][0] = load_weight(j, g);
+        }
+        float t = 0.f;
+#pragma unroll
+        for (int w = 0; w < kMostWarps; w += 4) {
+            const float4 part = *reinterpret_cast<const float4*>(&s_red[g][w]);
+            t += (part.x + part.y) + (part.z + part.w);
+        }
         const float inv_rms = rsqrtf(t * inv_h + a.ep.eps);
 #pragma unroll
         for (int j = 0; j < NV; ++j) {
-            const uint32_t c = tid + j * nt;
-            if (c < vec_per_row) {
-                float p[VEC], w[VEC];
+            if (!have[j]) continue;
+            float p[VEC], w[VEC];
 #pragma unroll
-                for (int i = 0; i < VEC; ++i) {
-                    p[i] = f[j][i];
-                    w[i] = 0.f;
-                }
-                accumulate<T>(p, res[j][g]);
-                accumulate<T>(w, *reinterpret_cast<const uint4*>(static_cast<const char*>(a.weight[q0 + g]) + c * 16ull));
+            for (int i = 0; i < VEC; ++i) p[i] = f[j][i];
+            accumulate<T>(p, res[j][g]);
+            unpack16<T>(w, wgt[j][LATE ? 0 : g]);
 #pragma unroll
-                for (int i = 0; i < VEC; ++i) p[i] = p[i] * inv_rms * w[i];
-                ptx::st_v4(static_cast<char*>(a.recv[q0 + g]) + row_off + c * 16ull, pack16<T>(p));
-            }
+            for (int i = 0; i < VEC; ++i) p[i] = p[i] * inv_rms * w[i];
+            ptx::st_v4(static_cast<char*>(a.recv[q0 + g]) + row_off + at[j], pack16<T>(p));
         }
     }
     local_trace_end(a);
@@ -325,24 +354,49 @@ const void* pick_same(Dtype dt, int world) {
     }
     return nullptr;
 }
+// The instances that LocalNormShapeFor asks for; nullptr for others.
+template <typename T, int WORLD, int NV, int G>
+const void* pick_norm_late(bool late) {
+    constexpr bool kEarly = NV == 1 || G == 1 || (sizeof(T) == 4 && WORLD == 2 && NV == 2);
+    constexpr bool kLate = WORLD > 1 && (NV == 1 ? G == 2 && WORLD != 4 : NV == 2 ? G == 2 : G == (WORLD == 2 ? 1 : 2));
+    if constexpr (kLate) {
+        if (late) return (const void*)local_norm_kernel<T, WORLD, NV, G, true>;
+    }
+    if constexpr (kEarly) {
+        if (!late) return (const void*)local_norm_kernel<T, WORLD, NV, G, false>;
+    }
+    return nullptr;
+}
 template <typename T, int WORLD, int NV>
-const void* pick_norm_g(int g) {
-    constexpr int kMost = WORLD && WORLD < kLocalNormHeld / NV ? WORLD : kLocalNormHeld / NV;
-    return g == 1 ? (const void*)local_norm_kernel<T, WORLD, NV, 1> : (const void*)local_norm_kernel<T, WORLD, NV, kMost>;
+const void* pick_norm_g(const LocalNormShape& s) {
+    if constexpr (NV == 1 && WORLD >= 4) {
+        if (s.ranks_per_cta == 4) return pick_norm_late<T, WORLD, NV, 4>(s.late);
+    }
+    if constexpr (WORLD >= 2) {
+        if (s.ranks_per_cta == 2) return pick_norm_late<T, WORLD, NV, 2>(s.late);
+    }
+    return pick_norm_late<T, WORLD, NV, 1>(s.late);
 }
 template <typename T, int WORLD>
-const void* pick_norm_nv(int nv, int g) {
-    return nv == 1 ? pick_norm_g<T, WORLD, 1>(g) : nv == 2 ? pick_norm_g<T, WORLD, 2>(g) : pick_norm_g<T, WORLD, 4>(g);
+const void* pick_norm_nv(const LocalNormShape& s) {
+    return s.vec_per_thread == 1   ? pick_norm_g<T, WORLD, 1>(s)
+           : s.vec_per_thread == 2 ? pick_norm_g<T, WORLD, 2>(s)
+                                   : pick_norm_g<T, WORLD, 4>(s);
 }
 template <typename T>
-const void* pick_norm(int world, int nv, int g) {
+const void* pick_norm(int world, const LocalNormShape& s) {
+    static_assert(kMaxRanks == 8, "one instance per group size");
     switch (world) {
-        case 1: return pick_norm_nv<T, 1>(nv, g);  // (8192 x 8192 bf16: 84 us, 182 with the instance for any world)
-        case 2: return pick_norm_nv<T, 2>(nv, g);
-        case 4: return pick_norm_nv<T, 4>(nv, g);
-        case 8: return pick_norm_nv<T, 8>(nv, g);
-        default: return pick_norm_nv<T, 0>(nv, g);
+        case 1: return pick_norm_nv<T, 1>(s);
+        case 2: return pick_norm_nv<T, 2>(s);
+        case 3: return pick_norm_nv<T, 3>(s);
+        case 4: return pick_norm_nv<T, 4>(s);
+        case 5: return pick_norm_nv<T, 5>(s);
+        case 6: return pick_norm_nv<T, 6>(s);
+        case 7: return pick_norm_nv<T, 7>(s);
+        case 8: return pick_norm_nv<T, 8>(s);
     }
+    return nullptr;
 }
 
 }  // namespace
@@ -371,9 +425,9 @@ const void* LocalHostKernelFor(Dtype dt, int world) {
 
 const void* LocalNormKernelFor(Dtype dt, int world, const LocalNormShape& s) {
     switch (dt) {
-        case Dtype::FP32: return pick_norm<float>(world, s.vec_per_thread, s.ranks_per_cta);
-        case Dtype::FP16: return pick_norm<__half>(world, s.vec_per_thread, s.ranks_per_cta);
-        case Dtype::BF16: return pick_norm<__nv_bfloat16>(world, s.vec_per_thread, s.ranks_per_cta);
+        case Dtype::FP32: return pick_norm<float>(world, s);
+        case Dtype::FP16: return pick_norm<__half>(world, s);
+        case Dtype::BF16: return pick_norm<__nv_bfloat16>(world, s);
     }
     return nullptr;
 }

@@ -103,6 +103,37 @@ def test_norm(comm, dtype, rows, hidden):
         torch.testing.assert_close(xs[0].double(), ys[0].double(), rtol=2 * rtol, atol=1e-6)
 
 
+# The cuts of the norm kernel: one, two or four ranks per CTA, weights ahead of the barrier and behind it, one to four vectors per thread, rows
+# that do not fill their last warp.  Groups of 2, 4 and 8 change the cut at different rows, so every group runs all of them.
+@pytest.mark.parametrize("dtype,hidden,rows", [(BF16, 2944, (40, 90, 300, 900)), (F16, 24, (5, 2000, 20000)), (BF16, 8192, (3, 30, 400)),
+                                               (F32, 4096, (20, 130, 400)), (F32, 8192, (9, 250)), (BF16, 12296, (9, 300)), (F32, 1000, (37, 1300))])
+def test_cuts_of_the_norm(comm, dtype, hidden, rows):
+    W, rtol = comm.world, {F32: 2e-6, F16: 2.0 ** -10, BF16: 2.0 ** -7}[dtype]
+    ws = [whole((hidden,), dtype, 90 + r) for r in range(W)]
+    for n in rows:
+        xs, res = [whole((n, hidden), dtype, r) for r in range(W)], [whole((n, hidden), dtype, 50 + r) for r in range(W)]
+        pre = [torch.empty_like(x) for x in xs]
+        ys = comm.all_reduce_rmsnorm(xs, ws, res, eps=1e-5, residual_out=pre)
+        assert comm.last_call()["kernel"] == "local_norm"
+        s = total(xs)
+        for r in range(W):
+            row = s + res[r].double()
+            assert torch.equal(pre[r].double(), row)
+            ref = row * torch.rsqrt(row.pow(2).mean(-1, keepdim=True) + 1e-5) * ws[r].double()
+            torch.testing.assert_close(ys[r].double(), ref, rtol=rtol, atol=1e-6)
+        # In place: the residual stream is its own output.
+        keep = [t.clone() for t in res]
+        comm.all_reduce_rmsnorm(xs, ws, keep, eps=1e-5, residual_out=keep)
+        assert all(torch.equal(k, p) for k, p in zip(keep, pre))
+
+
+@pytest.mark.parametrize("world", [5, 6, 7])
+@pytest.mark.parametrize("dtype,hidden,rows", [(BF16, 2944, (40, 200, 800)), (F16, 8192, (10, 300)), (F32, 8192, (9, 150)), (F32, 1000, (37, 1300))])
+def test_norm_of_odd_groups(world, dtype, hidden, rows):
+    with yali.Comm.emulated(world, device=0) as c:
+        test_cuts_of_the_norm(c, dtype, hidden, rows)
+
+
 @pytest.mark.parametrize("dtype", [F32, F16, BF16])
 @pytest.mark.parametrize("rows,hidden", [(1, 4096), (16, 4096), (5, 1024), (3, 8192), (128, 4096), (7, 256)])
 def test_norm_of_the_one_shot_kernel(comm, dtype, rows, hidden):
