@@ -504,7 +504,10 @@ Result Communicator::LaunchLocal(const Plan& plan, const void* const* send, void
     } else {
         const bool rs = plan.flags & kFlagReduceScatterOnly, ag = plan.flags & kFlagAllGatherOnly;
         name = rs ? "local_reduce_scatter" : ag ? "local_all_gather" : "local_sum";
-        fn = LocalKernelFor(in, out, world_, rs ? LocalKind::ReduceScatter : ag ? LocalKind::AllGather : LocalKind::Sum);
+        bool wide = DtypeSize(out) > DtypeSize(in);
+        for (int i = 0; i < nlocal() && wide; ++i)
+            wide = ((reinterpret_cast<uintptr_t>(send[i]) | reinterpret_cast<uintptr_t>(recv[i])) & 31u) == 0;
+        fn = LocalKernelFor(in, out, world_, rs ? LocalKind::ReduceScatter : ag ? LocalKind::AllGather : LocalKind::Sum, wide);
         const uint64_t unit = 16 / std::min(DtypeSize(in), DtypeSize(out));
         const uint64_t span = rs || ag ? std::min(plan.shard_elems, count) : count;
         blocks = (span + unit * kLocalThreads - 1) / (unit * kLocalThreads);

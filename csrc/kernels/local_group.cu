@@ -51,29 +51,37 @@ __device__ __forceinline__ void local_trace_end(const LocalArgs& a) {
     }
 }
 
-// The E elements at element offset e of `base`, as 16-byte vectors of the input type / of the output type.
+// The E elements at element offset e of `base`, as 16-byte vectors.
 template <typename Tin, int E>
 __device__ __forceinline__ void load_unit(uint4 (&x)[E * sizeof(Tin) / 16], const void* base, uint64_t e) {
 #pragma unroll
     for (int i = 0; i < static_cast<int>(E * sizeof(Tin) / 16); ++i)
         x[i] = ptx::ld_cg_v4(static_cast<const char*>(base) + e * sizeof(Tin) + i * 16);
 }
-template <typename Tout, int E>
-__device__ __forceinline__ void store_unit(void* base, uint64_t e, const float* f) {
-    constexpr int VEC = 16 / sizeof(Tout);
+// WIDE: a unit of two vectors in one access, on a 32-byte boundary.  Sums to a type of twice the width: a warp that stores 16 bytes at a
+// 32-byte stride leaves every sector half written.  In a graph, us, 16 / 32 bytes: bf16 -> fp32: 2 ranks x 1000003 3.9 / 3.4, 6000017 14.8 /
+// 12.4; 4 ranks x 1000003 7.0 / 5.2, 6000017 30.2 / 23.2; 8 ranks x 6000017 59.6 / 46.0 (floor 44.1).  Loads of 32 bytes (fp32 ->
+// bf16) gain where the inputs are in L2 and lose where they are not: 8 ranks x 250000 3.6 / 3.4 and 5.6 / 6.2, x 6553600 47.2 / 47.8; units
+// of 32 bytes for equal types lose (8 ranks x 1000003 bf16 6.5 / 7.1).
+template <bool WIDE, int N>
+__device__ __forceinline__ void store_vectors(void* base, uint64_t byte, const uint4 (&y)[N]) {
+    char* const p = static_cast<char*>(base) + byte;
+    if constexpr (N == 2 && WIDE) {
+        ptx::st_v8(p, y[0], y[1]);
+    } else {
 #pragma unroll
-    for (int i = 0; i < E / VEC; ++i)
-        ptx::st_v4(static_cast<char*>(base) + e * sizeof(Tout) + i * 16, pack16<Tout>(f + i * VEC));
+        for (int i = 0; i < N; ++i) ptx::st_v4(p + i * 16, y[i]);
+    }
 }
 
 // KIND: what the grid covers.  Sum: units of the whole message (grid.x).  ReduceScatter / AllGather: units of
 // shard blockIdx.y (a shard is a multiple of 16 elements, so it consists of whole units up to the message's
 // end); the owner's buffer starts at the shard.
-template <typename Tin, typename Tout, int WORLD, LocalKind KIND>
+template <typename Tin, typename Tout, int WORLD, LocalKind KIND, bool WIDE>
 __global__ void __launch_bounds__(kLocalThreads) local_kernel(const __grid_constant__ LocalArgs a) {
     // Elements of a unit: 16 bytes of the narrower type, so that neither side moves less than 16 bytes.
     constexpr int E = 16 / (sizeof(Tin) < sizeof(Tout) ? sizeof(Tin) : sizeof(Tout));
-    constexpr int NIN = E * sizeof(Tin) / 16;
+    constexpr int NIN = E * sizeof(Tin) / 16, NOUT = E * sizeof(Tout) / 16, VOUT = 16 / sizeof(Tout);
     constexpr int kMaxW = WORLD ? WORLD : kMaxRanks;
     const uint32_t W = WORLD ? WORLD : a.world;
     ptx::grid_dependency_wait();
@@ -93,11 +101,7 @@ __global__ void __launch_bounds__(kLocalThreads) local_kernel(const __grid_const
                 load_unit<Tin, E>(x[0], a.send[owner], e0 - in_off);
 #pragma unroll
                 for (int q = 0; q < kMaxW; ++q)
-                    if (q < W) {
-#pragma unroll
-                        for (int i = 0; i < NIN; ++i)
-                            ptx::st_v4(static_cast<char*>(a.recv[q]) + e0 * sizeof(Tout) + i * 16, x[0][i]);
-                    }
+                    if (q < W) store_vectors<WIDE>(a.recv[q], e0 * sizeof(Tout), x[0]);
             } else {
                 float f[E];
 #pragma unroll
@@ -113,12 +117,15 @@ __global__ void __launch_bounds__(kLocalThreads) local_kernel(const __grid_const
                     }
 #pragma unroll
                 for (int i = 0; i < E; ++i) f[i] = epi(f[i]);
+                uint4 y[NOUT];
+#pragma unroll
+                for (int i = 0; i < NOUT; ++i) y[i] = pack16<Tout>(f + i * VOUT);
                 if constexpr (KIND == LocalKind::ReduceScatter) {
-                    store_unit<Tout, E>(a.recv[owner], e0 - out_off, f);
+                    store_vectors<WIDE>(a.recv[owner], (e0 - out_off) * sizeof(Tout), y);
                 } else {
 #pragma unroll
                     for (int q = 0; q < kMaxW; ++q)
-                        if (q < W) store_unit<Tout, E>(a.recv[q], e0, f);
+                        if (q < W) store_vectors<WIDE>(a.recv[q], e0 * sizeof(Tout), y);
                 }
             }
         }
@@ -325,15 +332,22 @@ __global__ void __launch_bounds__(kLocalThreads) __maxnreg__(norm_regs(WORLD, NV
     local_trace_end(a);
 }
 
-template <typename Tin, typename Tout, LocalKind KIND>
+template <typename Tin, typename Tout, LocalKind KIND, bool WIDE = false>
 const void* pick_world(int world) {
     switch (world) {
-        case 1: return (const void*)local_kernel<Tin, Tout, 1, KIND>;
-        case 2: return (const void*)local_kernel<Tin, Tout, 2, KIND>;
-        case 4: return (const void*)local_kernel<Tin, Tout, 4, KIND>;
-        case 8: return (const void*)local_kernel<Tin, Tout, 8, KIND>;
-        default: return (const void*)local_kernel<Tin, Tout, 0, KIND>;
+        case 1: return (const void*)local_kernel<Tin, Tout, 1, KIND, WIDE>;
+        case 2: return (const void*)local_kernel<Tin, Tout, 2, KIND, WIDE>;
+        case 4: return (const void*)local_kernel<Tin, Tout, 4, KIND, WIDE>;
+        case 8: return (const void*)local_kernel<Tin, Tout, 8, KIND, WIDE>;
+        default: return (const void*)local_kernel<Tin, Tout, 0, KIND, WIDE>;
     }
+}
+template <typename Tin, typename Tout>
+const void* pick_mixed(int world, bool wide) {
+    if constexpr (sizeof(Tout) > sizeof(Tin)) {
+        if (wide) return pick_world<Tin, Tout, LocalKind::Sum, true>(world);
+    }
+    return pick_world<Tin, Tout, LocalKind::Sum>(world);
 }
 template <typename T>
 const void* pick_host(int world) {
@@ -401,16 +415,16 @@ const void* pick_norm(int world, const LocalNormShape& s) {
 
 }  // namespace
 
-const void* LocalKernelFor(Dtype in, Dtype out, int world, LocalKind kind) {
+const void* LocalKernelFor(Dtype in, Dtype out, int world, LocalKind kind, bool wide) {
     using bf16 = __nv_bfloat16;
     if (kind == LocalKind::ReduceScatter) return in == out ? pick_same<LocalKind::ReduceScatter>(in, world) : nullptr;
     if (kind == LocalKind::AllGather) return in == out ? pick_same<LocalKind::AllGather>(in, world) : nullptr;
     constexpr LocalKind S = LocalKind::Sum;
     if (in == out) return pick_same<S>(in, world);
-    if (in == Dtype::FP32 && out == Dtype::BF16) return pick_world<float, bf16, S>(world);
-    if (in == Dtype::FP32 && out == Dtype::FP16) return pick_world<float, __half, S>(world);
-    if (in == Dtype::BF16 && out == Dtype::FP32) return pick_world<bf16, float, S>(world);
-    if (in == Dtype::FP16 && out == Dtype::FP32) return pick_world<__half, float, S>(world);
+    if (in == Dtype::FP32 && out == Dtype::BF16) return pick_mixed<float, bf16>(world, wide);
+    if (in == Dtype::FP32 && out == Dtype::FP16) return pick_mixed<float, __half>(world, wide);
+    if (in == Dtype::BF16 && out == Dtype::FP32) return pick_mixed<bf16, float>(world, wide);
+    if (in == Dtype::FP16 && out == Dtype::FP32) return pick_mixed<__half, float>(world, wide);
     return nullptr;
 }
 

@@ -73,8 +73,9 @@ inline LocalNormShape LocalNormShapeFor(uint64_t rows, uint32_t vec_per_row, int
     return s;
 }
 
-// nullptr when the combination is not built.
-const void* LocalKernelFor(Dtype in, Dtype out, int world, LocalKind kind);
+// nullptr when the combination is not built.  `wide`: every buffer starts on a 32-byte
+// boundary (sums to a type of twice the width store 32 bytes at a time).
+const void* LocalKernelFor(Dtype in, Dtype out, int world, LocalKind kind, bool wide);
 // Sum of buffers in host memory that the GPU can address; any number of CTAs.
 const void* LocalHostKernelFor(Dtype dt, int world);
 const void* LocalNormKernelFor(Dtype dt, int world, const LocalNormShape& shape);

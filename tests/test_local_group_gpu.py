@@ -52,6 +52,22 @@ def test_sum(comm, src, dst, n):
         assert comm.last_call()["flags"] & ONE_LAUNCH and all(torch.equal(x.double(), want) for x in xs)
 
 
+@pytest.mark.parametrize("src,dst", [(BF16, F32), (F16, F32), (F32, BF16), (F32, F16)])
+@pytest.mark.parametrize("n", [8, 15, 4096, 4103, 400003, 3000001])
+def test_sum_to_another_width_on_and_off_32_byte_boundaries(comm, src, dst, n):
+    """Units of 32 bytes are stored in one access where every buffer allows it; one rank's input or output starts 16 bytes behind such a boundary."""
+    size = lambda t: torch.empty(0, dtype=t).element_size()  # noqa: E731
+    for in_off, out_off in ((0, 0), (16 // size(src), 0), (0, 16 // size(dst))):
+        xs = [whole((n,), src, n + r, in_off if r == 0 else 0) for r in range(comm.world)]
+        ys = [whole((n + 8,), dst, 1, out_off if r == comm.world - 1 else 0) for r in range(comm.world)]
+        tails = [y[n:].clone() for y in ys]
+        comm.all_reduce(xs, [y[:n] for y in ys], scale=0.5)
+        assert comm.last_call()["flags"] & ONE_LAUNCH
+        want = total(xs) * 0.5
+        for y, tail in zip(ys, tails):
+            assert torch.equal(y[:n].double(), want) and torch.equal(y[n:], tail)
+
+
 @pytest.mark.parametrize("dtype", [F32, BF16])
 @pytest.mark.parametrize("n", [1, 16, 17, 129, 8192, 65535, 65537])
 def test_halves(comm, dtype, n):
