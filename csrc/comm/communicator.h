@@ -163,6 +163,10 @@ class Communicator {
     // Every rank in one ordinary launch on one GPU (kernels/local_group.cu).
     bool CanRunInOneLaunch(const void* const* send, void* const* recv, uint64_t send_bytes, uint64_t recv_bytes,
                            uint64_t shard_bytes, Dtype in, Dtype out, const OpOptions& opt, uint32_t extra_flags) const;
+    bool RowsFitRowKernels(uint64_t count, Dtype in, Dtype out, const OpOptions& opt) const;
+    // False: the call is not one for it; nothing was launched.
+    bool NormInOneLaunch(const void* const* send, void* const* recv, uint64_t count, Dtype dt, const OpOptions& opt,
+                         const cudaStream_t* streams, Result* r);
     Result LaunchLocal(const Plan& plan, const void* const* send, void* const* recv, uint64_t count, Dtype in, Dtype out,
                        const OpOptions& opt, const cudaStream_t* streams);
     Result EnsureSmemAttr(const void* fn, uint32_t smem_bytes);

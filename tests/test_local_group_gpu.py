@@ -197,6 +197,45 @@ def test_norm_beyond_the_one_shot_staging(comm, dtype, hidden, off):
         assert torch.equal(pre[r].float(), sum(x.float() for x in xs) + res[r].float())
 
 
+@pytest.mark.parametrize("dtype,hidden", [(BF16, 4096), (F16, 1000), (F32, 8192)])
+def test_norm_far_beyond_the_one_shot_staging(comm, dtype, hidden):
+    """One launch; two passes (one launch and one per rank) for calls whose outputs lie on one another, on inputs or off a boundary.  Whole-number
+    inputs: the sums are the same in both, the norms differ by their roundings."""
+    if comm.world == 1:
+        pytest.skip("a group of one stages nothing")
+    W, size, rtol = comm.world, torch.empty(0, dtype=dtype).element_size(), {F32: 2e-6, F16: 2.0 ** -10, BF16: 2.0 ** -7}[dtype]
+    rows = (comm.layout()["flash_cap"] + (1 << 20)) // (hidden * size) + 1
+    xs, res = [whole((rows, hidden), dtype, r) for r in range(W)], [whole((rows, hidden), dtype, 50 + r) for r in range(W)]
+    ws = [whole((hidden,), dtype, 90 + r) for r in range(W)]
+    s = sum(x.float() for x in xs)
+
+    def check(ys, pre, launches, residual=res):
+        for r in range(W):
+            row = s + (residual[r].float() if residual else 0)
+            if pre:
+                assert torch.equal(pre[r].float(), row)
+            ref = row * torch.rsqrt(row.double().pow(2).mean(-1, keepdim=True) + 1e-5) * ws[r].double()
+            torch.testing.assert_close(ys[r].double(), ref, rtol=rtol, atol=1e-6)
+        assert comm.launches - before == launches
+
+    before, pre = comm.launches, [torch.empty_like(x) for x in xs]
+    check(comm.all_reduce_rmsnorm(xs, ws, res, eps=1e-5, residual_out=pre), pre, 1)
+    assert comm.last_call()["kernel"] == "local_norm"
+    before = comm.launches
+    check(comm.all_reduce_rmsnorm(xs, ws, None, eps=1e-5), None, 1, None)
+    keep, before = [r.clone() for r in res], comm.launches
+    check(comm.all_reduce_rmsnorm(xs, ws, keep, eps=1e-5, residual_out=keep), keep, 1)
+    # Two passes: in place; one tensor for every rank's rows; a weight off a 16-byte boundary; a geometry of the caller's.
+    own, before = [x.clone() for x in xs], comm.launches
+    check(comm.all_reduce_rmsnorm(own, ws, res, eps=1e-5, out=own), None, 1 + W)
+    one, before = torch.empty_like(xs[0]), comm.launches
+    check(comm.all_reduce_rmsnorm(xs, ws, res[:1] * W, eps=1e-5, residual_out=[one] * W), [one] * W, 1 + W, res[:1] * W)
+    ws, before = [whole((hidden,), dtype, 90 + r, 1) for r in range(W)], comm.launches
+    check(comm.all_reduce_rmsnorm(xs, ws, res, eps=1e-5, residual_out=pre), pre, 1 + W)
+    before = comm.launches
+    check(comm.all_reduce_rmsnorm(xs, ws, res, eps=1e-5, residual_out=pre, mode="stream"), pre, 1 + W)
+
+
 @pytest.mark.parametrize("odd", ["x", "weight", "residual", "out", "residual_out"])
 @pytest.mark.parametrize("mode", ["auto", "flash"])
 def test_norm_refuses_tensors_off_a_16_byte_boundary(comm, odd, mode):
