@@ -395,8 +395,8 @@ namespace {
 constexpr uint32_t kFlagSleepNs = 1500, kFlagNearNs = 400, kLineSleepNs = 40;
 
 // A unit of work is a row for G ranks (unit u: row u / ngroups, ranks from (u % ngroups) * G); a thread holds NV 16-byte
-// vectors of the row.  SPLIT: more than one K split; LINES: the sums come as flag-in-data lines; SLIM: of the instances that serve one
-// rank, the one that leaves room for a second CTA beside the GEMM.
+// vectors of the row.  SPLIT: more than one K split; LINES: the sums come as flag-in-data lines; SLIM: of two instances for
+// the same, the one that takes fewer registers.
 //
 // Bound by memory once enough is in flight, and before that by the chain of a unit: residuals and sums, two barriers, weights, stores.
 // So a unit waits for memory as seldom as it can (the sums of a complete tile are asked for with the residuals, the weights of all its
@@ -457,7 +457,7 @@ __global__ void __launch_bounds__(kLocalLinearNormThreads) __maxnreg__(LocalLine
     // When a step asks for its weights (plain loads: the rows of an SM share them in L1).  One by one behind the stores and the barrier
     // each rank's is a latency of its own, so: 0 with the residuals, 1 ahead of the stores, 2 all at once behind the barrier, 3 one by
     // one where registers are short and there are enough rows to hide it.
-    constexpr int kWeights = G == 1 ? 0 : NV * G == 2 ? 1 : NV == 1 || SPLIT ? 2 : 3;
+    constexpr int kWeights = G == 1 ? 0 : NV * G == 2 ? 1 : NV == 2 && !SPLIT && SLIM ? 3 : 2;
     uint4 w1[NV][G];
     auto load_weight = [&](int g, int j, uint32_t q) { w1[j][g] = ptx::ld_v4(static_cast<const char*>(a.weight[q]) + at[j]); };
     const uint32_t most = a.world - 1;  // a group beyond the last rank computes that one again and stores nothing
@@ -689,6 +689,7 @@ const void* LocalLinearNormKernel(uint32_t N, int ranks_per_cta, bool split, boo
         return slim ? (const void*)local_linear_norm_kernel<1, 1, true, true, true> : (const void*)local_linear_norm_kernel<1, 1, true, true, false>;
     }
     if (ranks_per_cta == 4) return pick_linear_norm<1, 4>(split);
+    if (ranks_per_cta == 2 && wide && !split && !slim) return (const void*)local_linear_norm_kernel<2, 2, false, false, false>;
     if (ranks_per_cta == 2) return wide ? pick_linear_norm<2, 2>(split) : pick_linear_norm<1, 2>(split);
     return wide ? pick_linear_norm<2, 1>(split) : pick_linear_norm<1, 1>(split);
 }

@@ -63,11 +63,12 @@ struct LocalLinearNormArgs {
 
 // Registers per thread of the row kernel.  Up to 72, two CTAs of 256 threads fit beside the GEMM's, so that up to two units per SM are there,
 // with their residuals, when the sums come; CTAs that start when the GEMM's have left are 2.5 us later (8 ranks, 32 x 1792 x 4096 31.0
-// with 128 registers, 26.9 with 72).  `slim` is about the instances that serve one rank: the other one asks for the lines of four K splits
-// at a time.  Two vectors of two ranks and several splits do not fit 72 (spills: 50 -> 55 us).
+// with 128 registers, 26.9 with 72).  `slim`, where there are two instances: one rank, the other one asks for the lines of four K
+// splits at a time; two ranks, two vectors, one split: the other one, with three CTAs per SM instead of four, asks for the weights at once.
+// Two vectors of two ranks and several splits do not fit 72 (spills: 50 -> 55 us).
 constexpr int LocalLinearNormRegs(int vectors, int ranks_per_cta, bool split, bool slim) {
     if (ranks_per_cta == 1) return slim ? 72 : vectors == 1 ? 104 : 144;
-    if (ranks_per_cta == 2) return !split ? 64 : vectors == 1 ? 72 : 96;
+    if (ranks_per_cta == 2) return !split ? (vectors == 1 || slim ? 64 : 72) : vectors == 1 ? 72 : 96;
     return !split ? 72 : 96;
 }
 

@@ -362,9 +362,9 @@ bool CanRunLocal(Communicator& comm, const FusedLinearDesc* descs, uint32_t T, u
 // CTAs of the row kernel on an SM with the GEMM gone.  Asked for once: registers are shared out to the SM's four quarters by warps, which
 // no formula of threads and registers says.
 uint32_t LocalLinearNormPlaces(uint32_t N, int ranks_per_cta, bool split, bool lines, bool slim) {
-    static std::atomic<int> known[4][3][2][kLocalLinearNormThreads / 32 + 1];
+    static std::atomic<int> known[5][3][2][kLocalLinearNormThreads / 32 + 1];
     const int threads = LocalLinearNormThreads(N);
-    std::atomic<int>& k = known[ranks_per_cta == 1 && slim ? 3 : ranks_per_cta / 2][lines ? 2 : split ? 1 : 0][LocalLinearNormVectors(N) - 1][threads / 32];
+    std::atomic<int>& k = known[slim && ranks_per_cta < 4 ? 3 + ranks_per_cta / 2 : ranks_per_cta / 2][lines ? 2 : split ? 1 : 0][LocalLinearNormVectors(N) - 1][threads / 32];
     int n = k.load(std::memory_order_relaxed);
     if (n == 0) {
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, LocalLinearNormKernel(N, ranks_per_cta, split, lines, slim), threads, 0) != cudaSuccess) (void)cudaGetLastError();
@@ -453,8 +453,8 @@ Result LaunchLocal(Communicator& comm, const DriverApi* drv, const FusedLinearDe
     auto units_of = [&](int gr) { return static_cast<uint32_t>(T * ((W + gr - 1) / gr)); };
     // Few CTAs have the SMs' registers to themselves, and then ask for the lines of four splits at a time (slim / not: 2 ranks, 8 x 2048 x
     // 4096 10.2 / 9.5; 8 ranks, 8 x 1792 x 4096 24.3 / 24.9, 24 x 512 x 1024 7.2 / 6.9, 30 x 1024 x 2048 11.7 / 13.6).
-    const bool slim = narrow ? units_of(1) * threads > 256 * sms : units_of(1) > 32;
-    auto places_of = [&](int gr) { return sms * LocalLinearNormPlaces(N, gr, split, lines, slim); };
+    bool slim = narrow ? units_of(1) * threads > 256 * sms : units_of(1) > 32;
+    auto places_of = [&](int gr, bool slim) { return sms * LocalLinearNormPlaces(N, gr, split, lines, slim); };
     // Ranks that a CTA serves, each CTA adding the splits again: one while that needs no more than two CTAs of 256 threads per SM and four
     // of any size (one / two / four ranks, us: 8 ranks, 40 x 256 x 512 7.1 / 8.4 / 8.4, 60 x 512 x 1024 9.7 / 10.2 / 10.3; 4 ranks, 76 x 1024 x
     // 2048 10.9 / 10.5 / 12.3; 2 ranks, 1000 x 256 x 128 13.2 / 9.7).  Above, two for wide rows (four, which spill: 8 ranks, 2048 x 512 x 4096
@@ -464,8 +464,11 @@ Result LaunchLocal(Communicator& comm, const DriverApi* drv, const FusedLinearDe
     // 2048 21.2 / 21.8).
     int group = 1;
     if (!few && !(narrow && units_of(1) <= 4 * sms && units_of(1) * threads <= 512 * sms))
-        group = !narrow || (W & 3) == 1 || (W & 3) == 2 || 2 * units_of(2) <= places_of(2) ? 2 : 4;
-    const uint32_t ngroups = (W + group - 1) / group, units = units_of(group), places = places_of(group);
+        group = !narrow || (W & 3) == 1 || (W & 3) == 2 || 2 * units_of(2) <= places_of(2, true) ? 2 : 4;
+    // Four CTAs per SM with the weights one by one while they take all units at once, else three that ask for them together (four / three:
+    // 2 ranks, N = 4096, K = 2048: T = 512 24.6 / 25.9, T = 700 30.1 / 29.4; 1000 x 512 x 3072 25.8 / 24.8; 4 ranks, 1000 x 512 x 4096 41.1 / 38.0).
+    if (group == 2) slim = units_of(2) <= places_of(2, true);
+    const uint32_t ngroups = (W + group - 1) / group, units = units_of(group), places = places_of(group, slim);
     n.by_groups = static_cast<uint32_t>(((1ull << 32) + ngroups - 1) / ngroups);
     const void* const fn2 = LocalLinearNormKernel(N, group, split, lines, slim);
     const cudaStream_t s = streams && streams[0] ? streams[0] : comm.default_stream(0);

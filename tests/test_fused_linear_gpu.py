@@ -193,7 +193,7 @@ def test_ranks_on_one_gpu_add_in_the_gemm(world, T, K, N):
 @pytest.mark.parametrize("world,T,K,N", [(8, 3, 64, 2304), (8, 33, 128, 4096), (4, 40, 64, 640), (4, 36, 256, 384), (2, 100, 256, 3968),
                                          (4, 75, 128, 1024), (3, 120, 64, 768), (2, 300, 64, 512), (5, 130, 64, 1280), (3, 260, 64, 2048),
                                          (7, 200, 128, 1152), (8, 161, 64, 1664), (4, 1025, 64, 1152), (6, 100, 64, 2176), (7, 60, 512, 2176),
-                                         (8, 150, 256, 3200)])
+                                         (8, 150, 256, 3200), (4, 400, 64, 3200), (3, 450, 64, 2304)])
 def test_rows_of_ranks_on_one_gpu(world, T, K, N):
     """Whole-number inputs as above: residuals bit by bit, the norm to one rounding.  Two calls, the second with other inputs."""
     g = torch.Generator(device="cuda").manual_seed(T * N + world)
