@@ -451,9 +451,11 @@ Result LaunchLocal(Communicator& comm, const DriverApi* drv, const FusedLinearDe
     const bool split = g.s.nsplit > 1;
     const bool narrow = LocalLinearNormVectors(N) == 1;
     auto units_of = [&](int gr) { return static_cast<uint32_t>(T * ((W + gr - 1) / gr)); };
-    // Few CTAs have the SMs' registers to themselves, and then ask for the lines of four splits at a time (slim / not: 2 ranks, 8 x 2048 x
-    // 4096 10.2 / 9.5; 8 ranks, 8 x 1792 x 4096 24.3 / 24.9, 24 x 512 x 1024 7.2 / 6.9, 30 x 1024 x 2048 11.7 / 13.6).
-    bool slim = narrow ? units_of(1) * threads > 256 * sms : units_of(1) > 32;
+    // Lines of one rank: while a CTA has its share of an SM beside the GEMM to itself, it may ask for the lines of four splits at a time instead
+    // of one or two, which pays with many splits and few rows (slim / not: 2 ranks, 8 x 2048 x 4096, 4 splits 10.2 / 9.5; 4 ranks, 10 x
+    // 1024 x 3072, 6 splits 9.1 / 8.5, 32 x 512 x 2304, 8 splits 9.5 / 7.9; 8 ranks, 8 x 1792 x 4096, 4 splits 24.3 / 24.9; 2 ranks, 64 x 2048 x
+    // 3328, 5 splits 10.2 / 10.5).  Narrow rows: 8 ranks, 24 x 512 x 1024 7.2 / 6.9, 30 x 1024 x 2048 11.7 / 13.6.
+    bool slim = units_of(1) * threads > 256 * sms || (!narrow && units_of(1) > (g.s.nsplit > 5 ? sms : 32u));
     auto places_of = [&](int gr, bool slim) { return sms * LocalLinearNormPlaces(N, gr, split, lines, slim); };
     // Ranks that a CTA serves, each CTA adding the splits again: one while that needs no more than two CTAs of 256 threads per SM and four
     // of any size (one / two / four ranks, us: 8 ranks, 40 x 256 x 512 7.1 / 8.4 / 8.4, 60 x 512 x 1024 9.7 / 10.2 / 10.3; 4 ranks, 76 x 1024 x
