@@ -74,7 +74,7 @@ __global__ void validate_sum_kernel(const Tout* out, uint64_t n, uint64_t index_
 
 // In-place residual add + RMSNorm over rows of `hidden` elements, one CTA per row.
 // Used when a message is too large for the one-shot kernel that fuses this step: the all-reduce
-// runs first, then this kernel normalises the local result.
+// runs first, then this kernel normalises the local result.  (Ranks that share one GPU have local_group.cu, except for what that does not take.)
 // Bound by HBM (three or four row images in and out).  A thread keeps its NV vectors of the row in registers
 // between the sum of squares and the store, so the row is read once; 16-byte accesses.
 template <typename T, int NV>
