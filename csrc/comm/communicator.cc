@@ -575,8 +575,6 @@ bool Communicator::NormInOneLaunch(const void* const* send, void* const* recv, u
                 (i != j && (overlap(recv[i], bytes, recv[j], bytes) || overlap(ro, bytes, other, bytes))))
                 return false;
         }
-        // (There the sum would be in the residual's place before the residual is read.)
-        if (opt.residual && overlap(opt.residual[i], bytes, recv[i], bytes)) return false;
     }
     Plan plan;
     std::string why;
@@ -723,6 +721,58 @@ Result Communicator::Collective(const void* const* send, void* const* recv, uint
     return Launch(plan, in, out, opt.epilogue, args, streams);
 }
 
+namespace {
+
+// Sum first, norm afterwards: a residual under a rank's output would be gone, and one under another rank's updated residual changed,
+// before it is read.  Those are read from copies in stream-ordered memory, taken ahead of the sum.  (A rank's residual updated in
+// place needs none: each thread reads what it overwrites.)
+class ResidualCopies {
+  public:
+    ResidualCopies(void* const* recv, const OpOptions& opt, int n, uint64_t bytes) : recv_(recv), opt_(opt), n_(n), bytes_(bytes) {}
+    ~ResidualCopies() {
+        for (int i = 0; i < n_; ++i)
+            if (copy_[i]) cudaFreeAsync(copy_[i], stream_[i]);
+    }
+    ResidualCopies(const ResidualCopies&) = delete;
+    ResidualCopies& operator=(const ResidualCopies&) = delete;
+
+    bool Needed(int i) const {
+        const void* const res = opt_.residual ? opt_.residual[i] : nullptr;
+        if (!res || !recv_) return false;
+        for (int j = 0; j < n_; ++j) {
+            const void* const ro = opt_.residual_out ? opt_.residual_out[j] : nullptr;
+            if (Overlap(res, recv_[j]) || (Overlap(res, ro) && !(i == j && res == ro))) return true;
+        }
+        return false;
+    }
+    cudaError_t Take(int i, cudaStream_t s) {
+        cudaError_t e = cudaMallocAsync(&copy_[i], bytes_, s);
+        if (e == cudaSuccess) {
+            stream_[i] = s;
+            e = cudaMemcpyAsync(copy_[i], opt_.residual[i], bytes_, cudaMemcpyDeviceToDevice, s);
+        } else {
+            copy_[i] = nullptr;
+        }
+        if (e != cudaSuccess) (void)cudaGetLastError();
+        return e;
+    }
+    const void* Of(int i) const { return copy_[i] ? copy_[i] : opt_.residual ? opt_.residual[i] : nullptr; }
+
+  private:
+    bool Overlap(const void* a, const void* b) const {
+        const char *p = static_cast<const char*>(a), *q = static_cast<const char*>(b);
+        return q && p < q + bytes_ && q < p + bytes_;
+    }
+    void* const* recv_;
+    const OpOptions& opt_;
+    const int n_;
+    const uint64_t bytes_;
+    void* copy_[kMaxRanks] = {};
+    cudaStream_t stream_[kMaxRanks] = {};
+};
+
+}  // namespace
+
 Result Communicator::AllReduce(const void* const* send, void* const* recv, uint64_t count, Dtype in, Dtype out,
                                const OpOptions& opt, const cudaStream_t* streams) {
     YALI_NVTX_RANGE("yali::AllReduce");
@@ -738,15 +788,23 @@ Result Communicator::AllReduce(const void* const* send, void* const* recv, uint6
         OpOptions plain = opt;
         plain.epilogue = kEpiIdentity;
         if (plain.mode == KernelMode::Flash) plain.mode = KernelMode::Auto;
+        auto stream_of = [&](int i) {
+            if (emulated_) i = 0;
+            return streams && streams[i] ? streams[i] : local_[i].stream;
+        };
+        ResidualCopies kept(recv, opt, nlocal(), count * DtypeSize(in));
+        for (int i = 0; i < nlocal(); ++i) {
+            if (!kept.Needed(i)) continue;
+            if (nlocal() > 1) cudaSetDevice(local_[i].device);
+            const cudaError_t e = kept.Take(i, stream_of(i));
+            if (e != cudaSuccess) return Fail(Result::CudaError, std::string("copy of a residual that an output lies on: ") + cudaGetErrorString(e));
+        }
         r = Collective(send, recv, count, in, out, plain, streams, 0);
         if (r != Result::Success) return r;
         for (int i = 0; i < nlocal(); ++i) {
             if (nlocal() > 1) cudaSetDevice(local_[i].device);
-            cudaStream_t s = streams && streams[i] ? streams[i] : local_[i].stream;
-            if (emulated_) s = streams && streams[0] ? streams[0] : local_[0].stream;
-            cudaError_t e = ResidualRmsNormInPlace(recv[i], opt.residual ? opt.residual[i] : nullptr,
-                                                   opt.residual_out ? opt.residual_out[i] : nullptr, opt.weight[i],
-                                                   count / opt.hidden, static_cast<uint32_t>(opt.hidden), opt.eps, out, s);
+            cudaError_t e = ResidualRmsNormInPlace(recv[i], kept.Of(i), opt.residual_out ? opt.residual_out[i] : nullptr, opt.weight[i],
+                                                   count / opt.hidden, static_cast<uint32_t>(opt.hidden), opt.eps, out, stream_of(i));
             if (e != cudaSuccess) return Fail(Result::CudaError, std::string("rmsnorm kernel: ") + cudaGetErrorString(e));
             last_.launches += 1;
         }

@@ -236,6 +236,41 @@ def test_norm_far_beyond_the_one_shot_staging(comm, dtype, hidden):
     check(comm.all_reduce_rmsnorm(xs, ws, res, eps=1e-5, residual_out=pre, mode="stream"), pre, 1 + W)
 
 
+@pytest.mark.parametrize("hidden,off,mode", [(4096, 0, "auto"), (4096, 0, "stream"), (1001, 0, "auto"), (1024, 1, "auto")])
+@pytest.mark.parametrize("extra", [-1, 1, 1 << 20])
+def test_norm_of_residuals_that_outputs_lie_on(comm, hidden, off, mode, extra):
+    """The residual is the one that the call was given, in one launch and in two passes: a rank's rows go to its own residual; to the next rank's;
+    one tensor is every rank's residual and its update.  `extra`: bytes above the one-shot kernel's staging."""
+    W = comm.world
+    if W == 1 and extra > 0:
+        pytest.skip("a group of one stages nothing")
+    if extra < 0 and (hidden % 8 or off or mode != "auto"):
+        pytest.skip("below the staging these are refused, or the multi-GPU kernel's")
+    staging = comm.layout()["flash_cap"] if W > 1 else 4 << 20
+    rows = (staging + extra) // (2 * hidden) + (extra > 0)
+    xs = [whole((rows, hidden), BF16, r) for r in range(W)]
+    res, ws = [whole((rows, hidden), BF16, 50 + r) for r in range(W)], [whole((hidden,), BF16, 90 + r, off) for r in range(W)]
+    s = sum(x.float() for x in xs)
+
+    def check(ys, residual):
+        for r in range(W):
+            row = s + residual[r].float()
+            ref = row * torch.rsqrt(row.pow(2).mean(-1, keepdim=True) + 1e-5) * ws[r].float()
+            torch.testing.assert_close(ys[r].float(), ref, rtol=2.0 ** -7, atol=1e-6)
+
+    own = [r.clone() for r in res]
+    pre = [torch.empty_like(r) for r in res]
+    check(comm.all_reduce_rmsnorm(xs, ws, own, eps=1e-5, out=own, residual_out=pre, mode=mode), res)
+    assert all(torch.equal(p.float(), s + r.float()) for p, r in zip(pre, res))
+    if extra < 0 or W == 1:
+        return
+    own = [r.clone() for r in res]
+    check(comm.all_reduce_rmsnorm(xs, ws, own, eps=1e-5, out=own[1:] + own[:1], mode=mode), res)
+    one = res[0].clone()
+    check(comm.all_reduce_rmsnorm(xs, ws, [one] * W, eps=1e-5, residual_out=[one] * W, mode=mode), res[:1] * W)
+    assert torch.equal(one.float(), s + res[0].float())
+
+
 @pytest.mark.parametrize("odd", ["x", "weight", "residual", "out", "residual_out"])
 @pytest.mark.parametrize("mode", ["auto", "flash"])
 def test_norm_refuses_tensors_off_a_16_byte_boundary(comm, odd, mode):
