@@ -126,7 +126,8 @@ __global__ void __launch_bounds__(512) residual_rmsnorm_kernel(T* x, const T* re
 }
 
 // The same element by element: rows that are no whole number of 16-byte vectors, are longer than 2048 of
-// them, or start on an address that is aligned to the element only.
+// them, or start on an address that is aligned to the element only.  A row is read twice, so nothing is stored before the second time:
+// the residual may be updated in place.
 template <typename T>
 __global__ void residual_rmsnorm_elems_kernel(T* x, const T* residual, T* residual_out, const T* weight, uint64_t rows,
                                               uint32_t hidden, float eps) {
@@ -138,7 +139,6 @@ __global__ void residual_rmsnorm_elems_kernel(T* x, const T* residual, T* residu
         for (uint32_t c = tid; c < hidden; c += nt) {
             float v = to_f32<T>(xr[c]);
             if (residual) v += to_f32<T>(residual[row * hidden + c]);
-            if (residual_out) residual_out[row * hidden + c] = from_f32<T>(v);
             ss += v * v;
         }
         for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
@@ -151,6 +151,7 @@ __global__ void residual_rmsnorm_elems_kernel(T* x, const T* residual, T* residu
         for (uint32_t c = tid; c < hidden; c += nt) {
             float v = to_f32<T>(xr[c]);
             if (residual) v += to_f32<T>(residual[row * hidden + c]);
+            if (residual_out) residual_out[row * hidden + c] = from_f32<T>(v);
             xr[c] = from_f32<T>(v * inv * to_f32<T>(weight[c]));
         }
     }

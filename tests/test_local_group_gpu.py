@@ -239,8 +239,8 @@ def test_norm_far_beyond_the_one_shot_staging(comm, dtype, hidden):
 @pytest.mark.parametrize("hidden,off,mode", [(4096, 0, "auto"), (4096, 0, "stream"), (1001, 0, "auto"), (1024, 1, "auto")])
 @pytest.mark.parametrize("extra", [-1, 1, 1 << 20])
 def test_norm_of_residuals_that_outputs_lie_on(comm, hidden, off, mode, extra):
-    """The residual is the one that the call was given, in one launch and in two passes: a rank's rows go to its own residual; to the next rank's;
-    one tensor is every rank's residual and its update.  `extra`: bytes above the one-shot kernel's staging."""
+    """The residual is the one that the call was given, in one launch and in two passes: a rank's rows go to its own residual; the residual is
+    updated in place; rows go to the next rank's residual; one tensor is every rank's residual and its update.  `extra`: bytes above the one-shot kernel's staging."""
     W = comm.world
     if W == 1 and extra > 0:
         pytest.skip("a group of one stages nothing")
@@ -264,6 +264,9 @@ def test_norm_of_residuals_that_outputs_lie_on(comm, hidden, off, mode, extra):
     assert all(torch.equal(p.float(), s + r.float()) for p, r in zip(pre, res))
     if extra < 0 or W == 1:
         return
+    own = [r.clone() for r in res]
+    check(comm.all_reduce_rmsnorm(xs, ws, own, eps=1e-5, residual_out=own, mode=mode), res)
+    assert all(torch.equal(o.float(), s + r.float()) for o, r in zip(own, res))
     own = [r.clone() for r in res]
     check(comm.all_reduce_rmsnorm(xs, ws, own, eps=1e-5, out=own[1:] + own[:1], mode=mode), res)
     one = res[0].clone()
