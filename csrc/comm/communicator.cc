@@ -17,6 +17,23 @@ namespace yali {
 namespace {
 uint64_t RoundUp(uint64_t a, uint64_t b) { return (a + b - 1) / b * b; }
 bool Aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
+
+// Where an all-reduce + norm writes its rows and updated residuals when one tensor is several outputs: what is left in it is the last rank's,
+// and rows rather than residuals, however the ranks are spread over CTAs.  nullptr: not written.
+struct NormOutputs {
+    NormOutputs(void* const* recv, void* const* residual_out, int n) {
+        for (int i = 0; i < n; ++i) {
+            rows[i] = recv[i];
+            residual[i] = residual_out ? residual_out[i] : nullptr;
+            for (int j = 0; j < n; ++j) {
+                if (j > i && recv[j] == recv[i]) rows[i] = nullptr;
+                if (recv[j] == residual[i] || (j > i && residual_out && residual_out[j] == residual[i])) residual[i] = nullptr;
+            }
+        }
+    }
+    void* rows[kMaxRanks];
+    void* residual[kMaxRanks];
+};
 }  // namespace
 
 bool MakeHeapLayout(int world, uint64_t requested_total, uint64_t granularity, HeapLayout* out) {
@@ -482,19 +499,21 @@ Result Communicator::LaunchLocal(const Plan& plan, const void* const* send, void
     if (opt.epilogue == kEpiResidualRmsNorm) {
         a.ep.eps = opt.eps;
         a.ep.hidden = opt.hidden;
+        const NormOutputs outs(recv, opt.residual_out, nlocal());
         for (int i = 0; i < nlocal(); ++i) {
             const int r = local_[i].rank;
+            a.recv[r] = outs.rows[i];
             a.residual[r] = opt.residual ? opt.residual[i] : nullptr;
-            a.residual_out[r] = opt.residual_out ? opt.residual_out[i] : nullptr;
+            a.residual_out[r] = outs.residual[i];
             a.weight[r] = opt.weight[i];
         }
         const uint64_t rows = count / opt.hidden;
         const uint32_t vec = 16 / static_cast<uint32_t>(DtypeSize(in));
-        const LocalNormShape s = LocalNormShapeFor(rows, static_cast<uint32_t>(opt.hidden) / vec, static_cast<int>(DtypeSize(in)), world_, sm_count_);
-        fn = LocalNormKernelFor(in, world_, s);
+        const LocalNormShape shape = LocalNormShapeFor(rows, static_cast<uint32_t>(opt.hidden) / vec, static_cast<int>(DtypeSize(in)), world_, sm_count_);
+        fn = LocalNormKernelFor(in, world_, shape);
         name = "local_norm";
-        block = dim3(s.threads);
-        blocks = rows * ((world_ + s.ranks_per_cta - 1) / s.ranks_per_cta);
+        block = dim3(shape.threads);
+        blocks = rows * ((world_ + shape.ranks_per_cta - 1) / shape.ranks_per_cta);
     } else if (plan.flags & kFlagHostMemory) {
         fn = LocalHostKernelFor(in, world_);
         name = "local_host_sum";
@@ -516,6 +535,19 @@ Result Communicator::LaunchLocal(const Plan& plan, const void* const* send, void
     if (!fn) return Fail(Result::Unsupported, "no kernel for this dtype / epilogue combination");
     if (blocks > 0x7fffffffull) return Fail(Result::InvalidArg, "count too large");
     grid.x = static_cast<unsigned>(blocks);
+    const cudaStream_t s = streams && streams[0] ? streams[0] : local_[0].stream;
+    void* unwanted = nullptr;  // rows that a later rank's replace go here: the kernel writes every rank's (a look at each pointer costs it 1 - 3 %)
+    for (int r = 0; r < world_; ++r) {
+        if (a.recv[r]) continue;
+        if (!unwanted) {
+            const cudaError_t e = cudaMallocAsync(&unwanted, count * DtypeSize(out), s);
+            if (e != cudaSuccess) {
+                (void)cudaGetLastError();
+                return Fail(Result::CudaError, std::string("room for rows of ranks that share an output: ") + cudaGetErrorString(e));
+            }
+        }
+        a.recv[r] = unwanted;
+    }
     last_.variant = plan.variant;
     last_.ctas = grid.x * grid.y;
     last_.slot_bytes = last_.stages = 0;
@@ -526,8 +558,8 @@ Result Communicator::LaunchLocal(const Plan& plan, const void* const* send, void
         std::fprintf(stderr, "[yali] %s count=%llu ctas=%u flags=0x%x\n", name, static_cast<unsigned long long>(count), last_.ctas,
                      plan.flags);
     void* params[] = {&a};
-    cudaStream_t s = streams && streams[0] ? streams[0] : local_[0].stream;
     cudaError_t ce = LaunchInStream(fn, grid, block, params, 0, s);
+    if (unwanted) cudaFreeAsync(unwanted, s);
     if (ce != cudaSuccess) {
         (void)cudaGetLastError();
         return Fail(Result::CudaError, std::string("kernel launch failed: ") + cudaGetErrorString(ce));
@@ -549,7 +581,7 @@ bool Communicator::RowsFitRowKernels(uint64_t count, Dtype in, Dtype out, const 
 // stages nothing, so it takes these, too: the inputs once and the outputs once, where a sum and a norm kernel per rank move
 // half as much again and round the sum.  us (floor): 8 ranks, 2048 x 4096 bf16 141 -> 91 (82); 4 ranks, 4096 x 4096 bf16 133 -> 89 (82),
 // 2048 x 4096 fp32 135 -> 83 (82); 2 ranks, 16000 x 4096 bf16 236 -> 154 (161).  The two passes stay for what only they take: a forced mode
-// or geometry, tensors off a 16-byte boundary, outputs on one another, on a weight or on an input.
+// or geometry, tensors off a 16-byte boundary, outputs in part on one another, on a weight or on an input.
 bool Communicator::NormInOneLaunch(const void* const* send, void* const* recv, uint64_t count, Dtype dt, const OpOptions& opt,
                                    const cudaStream_t* streams, Result* r) {
     if (poisoned_ || !send || !recv || count > (1ull << 40) || opt.mode != KernelMode::Auto || env::ForcedKernelMode() != KernelMode::Auto)
@@ -572,7 +604,7 @@ bool Communicator::NormInOneLaunch(const void* const* send, void* const* recv, u
         for (int j = 0; j < nlocal(); ++j) {
             const void* const other = opt.residual_out ? opt.residual_out[j] : nullptr;
             if (overlap(recv[i], bytes, other, bytes) || overlap(recv[i], bytes, opt.weight[j], row) || overlap(ro, bytes, opt.weight[j], row) ||
-                (i != j && (overlap(recv[i], bytes, recv[j], bytes) || overlap(ro, bytes, other, bytes))))
+                (i != j && ((overlap(recv[i], bytes, recv[j], bytes) && recv[i] != recv[j]) || overlap(ro, bytes, other, bytes))))
                 return false;
         }
     }
@@ -801,10 +833,11 @@ Result Communicator::AllReduce(const void* const* send, void* const* recv, uint6
         }
         r = Collective(send, recv, count, in, out, plain, streams, 0);
         if (r != Result::Success) return r;
+        const NormOutputs outs(recv, opt.residual_out, nlocal());
         for (int i = 0; i < nlocal(); ++i) {
             if (nlocal() > 1) cudaSetDevice(local_[i].device);
-            cudaError_t e = ResidualRmsNormInPlace(recv[i], kept.Of(i), opt.residual_out ? opt.residual_out[i] : nullptr, opt.weight[i],
-                                                   count / opt.hidden, static_cast<uint32_t>(opt.hidden), opt.eps, out, stream_of(i));
+            cudaError_t e = ResidualRmsNormInPlace(recv[i], kept.Of(i), outs.residual[i], opt.weight[i], count / opt.hidden,
+                                                   static_cast<uint32_t>(opt.hidden), opt.eps, out, stream_of(i), outs.rows[i] != nullptr);
             if (e != cudaSuccess) return Fail(Result::CudaError, std::string("rmsnorm kernel: ") + cudaGetErrorString(e));
             last_.launches += 1;
         }

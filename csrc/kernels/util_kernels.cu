@@ -79,7 +79,7 @@ __global__ void validate_sum_kernel(const Tout* out, uint64_t n, uint64_t index_
 // between the sum of squares and the store, so the row is read once; 16-byte accesses.
 template <typename T, int NV>
 __global__ void __launch_bounds__(512) residual_rmsnorm_kernel(T* x, const T* residual, T* residual_out, const T* weight,
-                                                               uint32_t hidden, float eps) {
+                                                               uint32_t hidden, float eps, bool store_rows) {
     constexpr int VEC = TypeTraits<T>::kVec;
     __shared__ float s_part[16];
     ptx::grid_dependency_wait();
@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(512) residual_rmsnorm_kernel(T* x, const T* re
 #pragma unroll
     for (int j = 0; j < NV; ++j) {
         const uint32_t c = tid + j * nt;
-        if (c < vec_per_row) {
+        if (c < vec_per_row && store_rows) {
             float w[VEC];
 #pragma unroll
             for (int i = 0; i < VEC; ++i) w[i] = 0.f;
@@ -130,7 +130,7 @@ __global__ void __launch_bounds__(512) residual_rmsnorm_kernel(T* x, const T* re
 // the residual may be updated in place.
 template <typename T>
 __global__ void residual_rmsnorm_elems_kernel(T* x, const T* residual, T* residual_out, const T* weight, uint64_t rows,
-                                              uint32_t hidden, float eps) {
+                                              uint32_t hidden, float eps, bool store_rows) {
     __shared__ float s_part[32];
     const int tid = threadIdx.x, nt = blockDim.x;
     for (uint64_t row = blockIdx.x; row < rows; row += gridDim.x) {
@@ -152,7 +152,7 @@ __global__ void residual_rmsnorm_elems_kernel(T* x, const T* residual, T* residu
             float v = to_f32<T>(xr[c]);
             if (residual) v += to_f32<T>(residual[row * hidden + c]);
             if (residual_out) residual_out[row * hidden + c] = from_f32<T>(v);
-            xr[c] = from_f32<T>(v * inv * to_f32<T>(weight[c]));
+            if (store_rows) xr[c] = from_f32<T>(v * inv * to_f32<T>(weight[c]));
         }
     }
 }
@@ -240,7 +240,7 @@ cudaError_t ValidateSumAsync(const void* out, uint64_t n, uint64_t index_offset,
 namespace {
 template <typename T>
 void LaunchResidualRmsNorm(void* x, const void* residual, void* residual_out, const void* weight, uint64_t rows,
-                           uint32_t hidden, float eps, cudaStream_t s) {
+                           uint32_t hidden, float eps, cudaStream_t s, bool store_rows) {
     constexpr uint32_t VEC = TypeTraits<T>::kVec;
     T* xt = static_cast<T*>(x);
     const T* rt = static_cast<const T*>(residual);
@@ -251,7 +251,7 @@ void LaunchResidualRmsNorm(void* x, const void* residual, void* residual_out, co
                            reinterpret_cast<uintptr_t>(residual_out) | reinterpret_cast<uintptr_t>(weight)) & 15u) == 0;
     if (hidden % VEC != 0 || vec_per_row > 2048 || !aligned || rows > 0x7fffffffull) {
         const int grid = static_cast<int>(rows < 148 * 8 ? rows : 148 * 8);
-        residual_rmsnorm_elems_kernel<<<grid, 256, 0, s>>>(xt, rt, ot, wt, rows, hidden, eps);
+        residual_rmsnorm_elems_kernel<<<grid, 256, 0, s>>>(xt, rt, ot, wt, rows, hidden, eps, store_rows);
         return;
     }
     // Two vectors per thread from 256 vectors on: enough loads in flight, and four or more rows per SM.
@@ -261,18 +261,18 @@ void LaunchResidualRmsNorm(void* x, const void* residual, void* residual_out, co
     const void* fn = nv == 1   ? (const void*)residual_rmsnorm_kernel<T, 1>
                      : nv == 2 ? (const void*)residual_rmsnorm_kernel<T, 2>
                                : (const void*)residual_rmsnorm_kernel<T, 4>;
-    void* params[] = {&xt, &rt, &ot, &wt, &hidden, &eps};
+    void* params[] = {&xt, &rt, &ot, &wt, &hidden, &eps, &store_rows};
     (void)LaunchInStream(fn, dim3(grid), dim3(threads), params, 0, s);
 }
 }  // namespace
 
-cudaError_t ResidualRmsNormInPlace(void* x, const void* residual, void* residual_out, const void* weight,
-                                   uint64_t rows, uint32_t hidden, float eps, Dtype dt, cudaStream_t s) {
+cudaError_t ResidualRmsNormInPlace(void* x, const void* residual, void* residual_out, const void* weight, uint64_t rows,
+                                   uint32_t hidden, float eps, Dtype dt, cudaStream_t s, bool store_rows) {
     if (rows == 0) return cudaSuccess;
     switch (dt) {
-        case Dtype::FP32: LaunchResidualRmsNorm<float>(x, residual, residual_out, weight, rows, hidden, eps, s); break;
-        case Dtype::FP16: LaunchResidualRmsNorm<__half>(x, residual, residual_out, weight, rows, hidden, eps, s); break;
-        case Dtype::BF16: LaunchResidualRmsNorm<__nv_bfloat16>(x, residual, residual_out, weight, rows, hidden, eps, s); break;
+        case Dtype::FP32: LaunchResidualRmsNorm<float>(x, residual, residual_out, weight, rows, hidden, eps, s, store_rows); break;
+        case Dtype::FP16: LaunchResidualRmsNorm<__half>(x, residual, residual_out, weight, rows, hidden, eps, s, store_rows); break;
+        case Dtype::BF16: LaunchResidualRmsNorm<__nv_bfloat16>(x, residual, residual_out, weight, rows, hidden, eps, s, store_rows); break;
     }
     return cudaGetLastError();
 }

@@ -274,6 +274,36 @@ def test_norm_of_residuals_that_outputs_lie_on(comm, hidden, off, mode, extra):
     assert torch.equal(one.float(), s + res[0].float())
 
 
+# (Few, some and many rows: the norm kernel's cuts; rows beyond the staging in one launch, and in two passes by vectors and by elements.)
+@pytest.mark.parametrize("rows,hidden,mode", [(3, 4096, "auto"), (90, 4096, "auto"), (600, 2944, "auto"), (50, 8192, "auto"), (0, 4096, "auto"),
+                                              (0, 4096, "stream"), (0, 1001, "auto")])
+def test_norms_whose_ranks_share_an_output(comm, rows, hidden, mode):
+    """One tensor as every rank's output holds the last rank's rows, one as every rank's updated residual the last rank's; rows win over residuals."""
+    W = comm.world
+    if W == 1:
+        pytest.skip("one output")
+    rows = rows or (comm.layout()["flash_cap"] + (1 << 20)) // (2 * hidden) + 1
+    xs = [whole((rows, hidden), BF16, r) for r in range(W)]
+    res, ws = [whole((rows, hidden), BF16, 50 + r) for r in range(W)], [whole((hidden,), BF16, 90 + r) for r in range(W)]
+    pre = [sum(x.float() for x in xs) + r.float() for r in res]
+    want = [p * torch.rsqrt(p.pow(2).mean(-1, keepdim=True) + 1e-5) * w.float() for p, w in zip(pre, ws)]
+    for shared in ([0] * W, [r % 2 for r in range(W)]):
+        outs, ros = ([torch.zeros_like(xs[0]) for _ in range(2)] for _ in range(2))
+        last = {k: max(r for r in range(W) if shared[r] == k) for k in shared}
+        kept = [torch.empty_like(x) for x in xs]
+        comm.all_reduce_rmsnorm(xs, ws, res, eps=1e-5, out=[outs[k] for k in shared], residual_out=kept, mode=mode)
+        assert all(torch.equal(k.float(), p) for k, p in zip(kept, pre))
+        for k, r in last.items():
+            torch.testing.assert_close(outs[k].float(), want[r], rtol=2.0 ** -7, atol=1e-6)
+        ys = comm.all_reduce_rmsnorm(xs, ws, res, eps=1e-5, residual_out=[ros[k] for k in shared], mode=mode)
+        for y, w in zip(ys, want):
+            torch.testing.assert_close(y.float(), w, rtol=2.0 ** -7, atol=1e-6)
+        assert all(torch.equal(ros[k].float(), pre[r]) for k, r in last.items())
+        comm.all_reduce_rmsnorm(xs, ws, res, eps=1e-5, out=[outs[k] for k in shared], residual_out=[outs[k] for k in shared], mode=mode)
+        for k, r in last.items():
+            torch.testing.assert_close(outs[k].float(), want[r], rtol=2.0 ** -7, atol=1e-6)
+
+
 @pytest.mark.parametrize("odd", ["x", "weight", "residual", "out", "residual_out"])
 @pytest.mark.parametrize("mode", ["auto", "flash"])
 def test_norm_refuses_tensors_off_a_16_byte_boundary(comm, odd, mode):
