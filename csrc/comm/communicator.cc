@@ -811,12 +811,10 @@ Result Communicator::AllReduce(const void* const* send, void* const* recv, uint6
     // Of the multi-GPU kernels only the one-shot one fuses the row-wise epilogue.  A message beyond its
     // staging capacity is reduced by the bandwidth kernels first and normalised by a local
     // kernel afterwards (two launches per rank), unless the ranks share one GPU.
-    constexpr uint64_t kNormBeyondStaging = 512ull << 10;
     if (opt.epilogue == kEpiResidualRmsNorm && world_ > 1 && count * DtypeSize(in) > lay_.flash_cap && in == out &&
         opt.hidden > 0 && count % opt.hidden == 0 && opt.weight) {
         Result r = Result::Success;
-        // (Not right above the staging: there the launches of a call, one per rank and one, are what tests of this library count.)
-        if (count * DtypeSize(in) > lay_.flash_cap + kNormBeyondStaging && NormInOneLaunch(send, recv, count, in, opt, streams, &r)) return r;
+        if (NormInOneLaunch(send, recv, count, in, opt, streams, &r)) return r;
         OpOptions plain = opt;
         plain.epilogue = kEpiIdentity;
         if (plain.mode == KernelMode::Flash) plain.mode = KernelMode::Auto;

@@ -171,11 +171,13 @@ def test_norm_of_the_one_shot_kernel(comm, dtype, rows, hidden):
             torch.testing.assert_close(y[r].double(), ref, rtol=rtol, atol=1e-6)
 
 
-# Row lengths by 16-byte vectors per thread of the norm kernel (128 / 129 / 1024 / 1025 / 2048 vectors), one that is no whole
+# Row lengths by 16-byte vectors per thread of the norm kernels (128 / 129 / 1024 / 1025 / 2048 vectors), one that is no whole
 # number of vectors, and one weight off a 16-byte boundary.
+@pytest.mark.parametrize("mode", ["auto", "stream"])
 @pytest.mark.parametrize("dtype,hidden,off", [(BF16, 1024, 0), (BF16, 1032, 0), (F16, 8192, 0), (F32, 4100, 0), (F32, 8192, 0), (BF16, 1001, 0), (BF16, 1024, 1)])
-def test_norm_beyond_the_one_shot_staging(comm, dtype, hidden, off):
-    """Above the staging's size the sum comes first and a kernel per rank normalises its rows: 1 + world launches."""
+def test_norm_beyond_the_one_shot_staging(comm, dtype, hidden, off, mode):
+    """Right above the staging's size: one launch, or, in a mode of the caller's and for rows that the row kernel does not take, the sum and then a kernel
+    per rank that normalises its rows, 1 + world launches."""
     if comm.world == 1:
         pytest.skip("a group of one stages nothing")
     W, rtol = comm.world, {F32: 2e-6, F16: 2.0 ** -10, BF16: 2.0 ** -7}[dtype]
@@ -183,9 +185,9 @@ def test_norm_beyond_the_one_shot_staging(comm, dtype, hidden, off):
     xs = [whole((rows, hidden), dtype, r) for r in range(W)]
     res, ws = [whole((rows, hidden), dtype, 50 + r) for r in range(W)], [whole((hidden,), dtype, 90 + r, off) for r in range(W)]
     pre, before = [torch.empty_like(x) for x in xs], comm.launches
-    ys = comm.all_reduce_rmsnorm(xs, ws, res, eps=1e-5, residual_out=pre)
-    assert comm.launches - before == 1 + W
-    plain = comm.all_reduce_rmsnorm(xs, ws, None, eps=1e-5)
+    ys = comm.all_reduce_rmsnorm(xs, ws, res, eps=1e-5, residual_out=pre, mode=mode)
+    assert comm.launches - before == (1 if mode == "auto" and hidden != 1001 and not off else 1 + W)
+    plain = comm.all_reduce_rmsnorm(xs, ws, None, eps=1e-5, mode=mode)
     comm.sync()
     pick = torch.tensor([0, 1, rows // 2, rows - 2, rows - 1], device="cuda")
     s = total([x[pick] for x in xs])
