@@ -477,6 +477,11 @@ bool Communicator::CanRunInOneLaunch(const void* const* send, void* const* recv,
     return true;
 }
 
+LocalNormShape Communicator::NormShape(uint64_t count, Dtype dt, const OpOptions& opt) const {
+    const uint32_t vec = 16 / static_cast<uint32_t>(DtypeSize(dt));
+    return LocalNormShapeFor(count / opt.hidden, static_cast<uint32_t>(opt.hidden) / vec, static_cast<int>(DtypeSize(dt)), world_, sm_count_);
+}
+
 Result Communicator::LaunchLocal(const Plan& plan, const void* const* send, void* const* recv, uint64_t count, Dtype in,
                                  Dtype out, const OpOptions& opt, const cudaStream_t* streams) {
     LocalArgs a;
@@ -508,12 +513,11 @@ Result Communicator::LaunchLocal(const Plan& plan, const void* const* send, void
             a.weight[r] = opt.weight[i];
         }
         const uint64_t rows = count / opt.hidden;
-        const uint32_t vec = 16 / static_cast<uint32_t>(DtypeSize(in));
-        const LocalNormShape shape = LocalNormShapeFor(rows, static_cast<uint32_t>(opt.hidden) / vec, static_cast<int>(DtypeSize(in)), world_, sm_count_);
+        const LocalNormShape shape = NormShape(count, in, opt);
         fn = LocalNormKernelFor(in, world_, shape);
         name = "local_norm";
         block = dim3(shape.threads);
-        blocks = rows * ((world_ + shape.ranks_per_cta - 1) / shape.ranks_per_cta);
+        blocks = LocalNormCtas(rows, world_, shape);
     } else if (plan.flags & kFlagHostMemory) {
         fn = LocalHostKernelFor(in, world_);
         name = "local_host_sum";
@@ -533,7 +537,7 @@ Result Communicator::LaunchLocal(const Plan& plan, const void* const* send, void
         if (rs || ag) grid.y = static_cast<unsigned>(world_);
     }
     if (!fn) return Fail(Result::Unsupported, "no kernel for this dtype / epilogue combination");
-    if (blocks > 0x7fffffffull) return Fail(Result::InvalidArg, "count too large");
+    if (blocks > kMostLocalCtas) return Fail(Result::InvalidArg, "count too large");
     grid.x = static_cast<unsigned>(blocks);
     const cudaStream_t s = streams && streams[0] ? streams[0] : local_[0].stream;
     void* unwanted = nullptr;  // rows that a later rank's replace go here: the kernel writes every rank's (a look at each pointer costs it 1 - 3 %)
@@ -581,7 +585,7 @@ bool Communicator::RowsFitRowKernels(uint64_t count, Dtype in, Dtype out, const 
 // stages nothing, so it takes these, too: the inputs once and the outputs once, where a sum and a norm kernel per rank move
 // half as much again and round the sum.  us (floor): 8 ranks, 2048 x 4096 bf16 141 -> 91 (82); 4 ranks, 4096 x 4096 bf16 133 -> 89 (82),
 // 2048 x 4096 fp32 135 -> 83 (82); 2 ranks, 16000 x 4096 bf16 236 -> 154 (161).  The two passes stay for what only they take: a forced mode
-// or geometry, tensors off a 16-byte boundary, outputs in part on one another, on a weight or on an input.
+// or geometry, tensors off a 16-byte boundary, outputs in part on one another, on a weight or on an input, and more rows than a grid has CTAs.
 bool Communicator::NormInOneLaunch(const void* const* send, void* const* recv, uint64_t count, Dtype dt, const OpOptions& opt,
                                    const cudaStream_t* streams, Result* r) {
     if (poisoned_ || !send || !recv || count > (1ull << 40) || opt.mode != KernelMode::Auto || env::ForcedKernelMode() != KernelMode::Auto)
@@ -593,7 +597,9 @@ bool Communicator::NormInOneLaunch(const void* const* send, void* const* recv, u
     for (int i = 0; i < nlocal(); ++i)
         if (!send[i] || !recv[i] || !opt.weight[i] || !Aligned16(send[i]) || !Aligned16(recv[i])) return false;
     const uint64_t bytes = count * DtypeSize(dt);
-    if (!RowsFitRowKernels(count, dt, dt, opt) || !CanRunInOneLaunch(send, recv, bytes, bytes, 0, dt, dt, opt, 0)) return false;
+    if (!RowsFitRowKernels(count, dt, dt, opt) || LocalNormCtas(count / opt.hidden, world_, NormShape(count, dt, opt)) > kMostLocalCtas ||
+        !CanRunInOneLaunch(send, recv, bytes, bytes, 0, dt, dt, opt, 0))
+        return false;
     auto overlap = [](const void* a, uint64_t an, const void* b, uint64_t bn) {
         const char *p = static_cast<const char*>(a), *q = static_cast<const char*>(b);
         return p && q && p < q + bn && q < p + an;

@@ -28,6 +28,8 @@
 
 namespace yali {
 
+struct LocalNormShape;  // kernels/local_group.h
+
 struct CommOptions {
     uint64_t heap_bytes = 0;     // 0: YALI_HEAP_BYTES or the default for the world size
     bool want_multicast = true;  // try to set up NVLS
@@ -163,6 +165,7 @@ class Communicator {
     // Every rank in one ordinary launch on one GPU (kernels/local_group.cu).
     bool CanRunInOneLaunch(const void* const* send, void* const* recv, uint64_t send_bytes, uint64_t recv_bytes,
                            uint64_t shard_bytes, Dtype in, Dtype out, const OpOptions& opt, uint32_t extra_flags) const;
+    LocalNormShape NormShape(uint64_t count, Dtype dt, const OpOptions& opt) const;
     bool RowsFitRowKernels(uint64_t count, Dtype in, Dtype out, const OpOptions& opt) const;
     // False: the call is not one for it; nothing was launched.
     bool NormInOneLaunch(const void* const* send, void* const* recv, uint64_t count, Dtype dt, const OpOptions& opt,

@@ -73,6 +73,12 @@ inline LocalNormShape LocalNormShapeFor(uint64_t rows, uint32_t vec_per_row, int
     return s;
 }
 
+// CTAs: one per row and group of ranks.  A launch takes up to kMostLocalCtas.
+constexpr uint64_t kMostLocalCtas = 0x7fffffff;
+inline uint64_t LocalNormCtas(uint64_t rows, int world, const LocalNormShape& s) {
+    return rows * ((world + s.ranks_per_cta - 1) / s.ranks_per_cta);
+}
+
 // nullptr when the combination is not built.  `wide`: every buffer starts on a 32-byte
 // boundary (sums to a type of twice the width store 32 bytes at a time).
 const void* LocalKernelFor(Dtype in, Dtype out, int world, LocalKind kind, bool wide);

@@ -276,6 +276,26 @@ def test_norm_of_residuals_that_outputs_lie_on(comm, hidden, off, mode, extra):
     assert torch.equal(one.float(), s + res[0].float())
 
 
+def test_norm_of_more_rows_than_a_grid_has_ctas():
+    """2^29 + 1 rows of one vector for eight ranks: more CTAs than a launch takes, so the sum comes first.  Input and output are one tensor for all ranks."""
+    if torch.cuda.mem_get_info()[0] < 24 << 30:
+        pytest.skip("needs 16 GiB")
+    n, W = 1 << 29, 8
+    tile = whole((8192, 8), BF16, 1)
+    x, y, w = torch.empty((n + 1, 8), dtype=BF16, device="cuda"), torch.empty((n + 1, 8), dtype=BF16, device="cuda"), whole((8,), BF16, 2)
+    x[:n].view(-1, 8192, 8).copy_(tile)
+    x[n] = tile[5]
+    with yali.Comm.emulated(W, device=0) as c:
+        c.all_reduce_rmsnorm([x] * W, [w] * W, None, eps=1e-5, out=[y] * W)
+        assert c.last_call()["kernel"] == "local_sum"
+        c.sync()
+    row = W * tile.float()
+    want = row * torch.rsqrt(row.pow(2).mean(-1, keepdim=True) + 1e-5) * w.float()
+    for first in (0, n // 2, n - 8192):
+        torch.testing.assert_close(y[first:first + 8192].float(), want, rtol=2.0 ** -7, atol=1e-6)
+    torch.testing.assert_close(y[n].float(), want[5], rtol=2.0 ** -7, atol=1e-6)
+
+
 # (Few, some and many rows: the norm kernel's cuts; rows beyond the staging in one launch, and in two passes by vectors and by elements.)
 @pytest.mark.parametrize("rows,hidden,mode", [(3, 4096, "auto"), (90, 4096, "auto"), (600, 2944, "auto"), (50, 8192, "auto"), (0, 4096, "auto"),
                                               (0, 4096, "stream"), (0, 1001, "auto")])
