@@ -173,6 +173,11 @@ void yali_c_local_gemm_shape(uint32_t T, uint32_t N, uint32_t kb_total, uint64_t
     const uint32_t v[4] = {s.tiles, s.tokens, s.nsplit, s.kper};
     std::memcpy(out, v, sizeof(v));
 }
+uint32_t yali_c_fused_row_places(int device, uint32_t N, int ranks_per_cta, int split, int lines, int slim) {
+    uint32_t n = 0;
+    if (N < 1 || N > 16u * kLocalLinearNormThreads || (ranks_per_cta != 1 && ranks_per_cta != 2 && ranks_per_cta != 4)) return 0;
+    return FusedLinearRowPlaces(device, N, ranks_per_cta, split != 0, lines != 0, slim != 0, &n) == cudaSuccess ? n : 0;
+}
 uint32_t yali_c_fused_linear_oneshot_max_rows(int world) { return FusedLinearOneShotMaxRows(world); }
 uint32_t yali_c_fused_tile_split(uint32_t T, uint32_t N, uint32_t K, int world, uint32_t resident_ctas, uint64_t gemm_cap,
                                  uint32_t want) {

@@ -81,11 +81,12 @@ void yali_c_oracle_residual_rmsnorm(const double* sum, const float* residual, co
 /* Fused linear layer: rows and 128 x 256 tiles per owner (arrays of `world`), default one-shot limit and multicast form;
  * how the tile form cuts T rows for `pairs` pairs of CTAs per rank (out: span, domains, tiles, tokens, group) and its
  * i-th item on a rank (out: tile, first row, rows, column tile, split); token tiles and K splits of the form for ranks
- * on one GPU (out: tiles, tokens, nsplit, kper). */
+ * on one GPU (out: tiles, tokens, nsplit, kper); CTAs of its row kernel per SM of `device`, the current one (0: it cannot be told). */
 void yali_c_fused_tiling(uint32_t T, uint32_t N, int world, int oneshot, uint32_t ksplit, uint32_t pairs, uint32_t* out);
 void yali_c_fused_item(const uint32_t* tiling, uint32_t T, uint32_t rank, uint32_t i, uint32_t col_tiles, uint32_t ks_shift,
                        uint32_t* out);
 void yali_c_local_gemm_shape(uint32_t T, uint32_t N, uint32_t kb_total, uint64_t room, uint32_t pairs, int lines, uint32_t* out);
+uint32_t yali_c_fused_row_places(int device, uint32_t N, int ranks_per_cta, int split, int lines, int slim);
 /* K splits per 256-column tile of the few-token fused layer (want = 0: the measured rule). */
 uint32_t yali_c_fused_tile_split(uint32_t T, uint32_t N, uint32_t K, int world, uint32_t resident_ctas, uint64_t gemm_cap,
                                  uint32_t want);

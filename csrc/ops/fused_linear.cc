@@ -360,21 +360,6 @@ bool CanRunLocal(Communicator& comm, const FusedLinearDesc* descs, uint32_t T, u
     return true;
 }
 
-// CTAs of the row kernel on an SM with the GEMM gone.  Asked for once: registers are shared out to the SM's four quarters by warps, which
-// no formula of threads and registers says.
-uint32_t LocalLinearNormPlaces(uint32_t N, int ranks_per_cta, bool split, bool lines, bool slim) {
-    static std::atomic<int> known[5][3][2][kLocalLinearNormThreads / 32 + 1];
-    const int threads = LocalLinearNormThreads(N);
-    std::atomic<int>& k = known[slim && ranks_per_cta < 4 ? 3 + ranks_per_cta / 2 : ranks_per_cta / 2][lines ? 2 : split ? 1 : 0][LocalLinearNormVectors(N) - 1][threads / 32];
-    int n = k.load(std::memory_order_relaxed);
-    if (n == 0) {
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, LocalLinearNormKernel(N, ranks_per_cta, split, lines, slim), threads, 0) != cudaSuccess) (void)cudaGetLastError();
-        n = std::max(n, 1);
-        k.store(n, std::memory_order_relaxed);
-    }
-    return static_cast<uint32_t>(n);
-}
-
 Result LaunchLocal(Communicator& comm, const DriverApi* drv, const FusedLinearDesc* descs, uint32_t T, uint32_t N,
                    uint32_t K, const FusedLinearOptions& opt, const cudaStream_t* streams) {
     auto fail = [&](Result r, const std::string& what) {
@@ -457,7 +442,13 @@ Result LaunchLocal(Communicator& comm, const DriverApi* drv, const FusedLinearDe
     // 1024 x 3072, 6 splits 9.1 / 8.5, 32 x 512 x 2304, 8 splits 9.5 / 7.9; 8 ranks, 8 x 1792 x 4096, 4 splits 24.3 / 24.9; 2 ranks, 64 x 2048 x
     // 3328, 5 splits 10.2 / 10.5).  Narrow rows: 8 ranks, 24 x 512 x 1024 7.2 / 6.9, 30 x 1024 x 2048 11.7 / 13.6.
     bool slim = units_of(1) * threads > 256 * sms || (!narrow && units_of(1) > (g.s.nsplit > 5 ? sms : 32u));
-    auto places_of = [&](int gr, bool slim) { return sms * LocalLinearNormPlaces(N, gr, split, lines, slim); };
+    cudaError_t asked = cudaSuccess;
+    auto places_of = [&](int gr, bool slim) {
+        uint32_t n = 1;
+        const cudaError_t e = FusedLinearRowPlaces(comm.device_of(0), N, gr, split, lines, slim, &n);
+        if (e != cudaSuccess) asked = e;
+        return sms * n;
+    };
     // Ranks that a CTA serves, each CTA adding the splits again: one while that needs no more than two CTAs of 256 threads per SM and four
     // of any size (one / two / four ranks, us: 8 ranks, 40 x 256 x 512 7.1 / 8.4 / 8.4, 60 x 512 x 1024 9.7 / 10.2 / 10.3; 4 ranks, 76 x 1024 x
     // 2048 10.9 / 10.5 / 12.3; 2 ranks, 1000 x 256 x 128 13.2 / 9.7).  Above, two for wide rows (four, which spill: 8 ranks, 2048 x 512 x 4096
@@ -472,6 +463,7 @@ Result LaunchLocal(Communicator& comm, const DriverApi* drv, const FusedLinearDe
     // 2 ranks, N = 4096, K = 2048: T = 512 24.6 / 25.9, T = 700 30.1 / 29.4; 1000 x 512 x 3072 25.8 / 24.8; 4 ranks, 1000 x 512 x 4096 41.1 / 38.0).
     if (group == 2) slim = units_of(2) <= places_of(2, true);
     const uint32_t ngroups = (W + group - 1) / group, units = units_of(group), places = places_of(group, slim);
+    if (asked != cudaSuccess) return fail(Result::CudaError, std::string("fused linear: ") + cudaGetErrorString(asked));
     n.by_groups = static_cast<uint32_t>(((1ull << 32) + ngroups - 1) / ngroups);
     const void* const fn2 = LocalLinearNormKernel(N, group, split, lines, slim);
     const cudaStream_t s = streams && streams[0] ? streams[0] : comm.default_stream(0);
@@ -489,6 +481,27 @@ Result LaunchLocal(Communicator& comm, const DriverApi* drv, const FusedLinearDe
 }
 
 }  // namespace
+
+cudaError_t FusedLinearRowPlaces(int device, uint32_t N, int ranks_per_cta, bool split, bool lines, bool slim, uint32_t* places) {
+    constexpr int kDevices = 32;  // beyond: asked for on every call
+    static std::atomic<int> known[kDevices][5][3][2][kLocalLinearNormThreads / 32 + 1];
+    const int threads = LocalLinearNormThreads(N);
+    std::atomic<int>* const k = device < 0 || device >= kDevices ? nullptr
+                                : &known[device][slim && ranks_per_cta < 4 ? 3 + ranks_per_cta / 2 : ranks_per_cta / 2]
+                                        [lines ? 2 : split ? 1 : 0][LocalLinearNormVectors(N) - 1][threads / 32];
+    int n = k ? k->load(std::memory_order_relaxed) : 0;
+    if (n == 0) {
+        const cudaError_t e =
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, LocalLinearNormKernel(N, ranks_per_cta, split, lines, slim), threads, 0);
+        if (e != cudaSuccess || n < 1) {
+            (void)cudaGetLastError();
+            return e != cudaSuccess ? e : cudaErrorLaunchOutOfResources;
+        }
+        if (k) k->store(n, std::memory_order_relaxed);
+    }
+    *places = static_cast<uint32_t>(n);
+    return cudaSuccess;
+}
 
 Result FusedLinearAllReduceRmsNorm(Communicator& comm, const FusedLinearDesc* descs, uint32_t T, uint32_t N,
                                    uint32_t K, const FusedLinearOptions& opt, const cudaStream_t* streams) {

@@ -42,6 +42,11 @@ struct FusedLinearOptions {
 Result FusedLinearAllReduceRmsNorm(Communicator& comm, const FusedLinearDesc* descs, uint32_t T, uint32_t N,
                                    uint32_t K, const FusedLinearOptions& opt, const cudaStream_t* streams);
 
+// Ranks on one GPU: CTAs of the row kernel that share an SM of `device` (the current one) with the GEMM gone.  Asked for once per device and
+// instance, an answer that failed not kept: registers are shared out to the SM's four quarters by warps, which no formula of threads and
+// registers says.
+cudaError_t FusedLinearRowPlaces(int device, uint32_t N, int ranks_per_cta, bool split, bool lines, bool slim, uint32_t* places);
+
 // Largest T the few-token form takes for rows of N elements (limited by its landing zone and by
 // the two TMEM lane quarters its epilogue reads); 0 when it cannot run.
 uint32_t FusedLinearDecodeMaxRows(const HeapLayout& lay, uint32_t N, int world);

@@ -9,6 +9,7 @@ import json
 
 import numpy as np
 import pytest
+import torch
 
 from yali_b200 import _native
 from yali_b200._native import Plan, PlanCaps
@@ -119,6 +120,15 @@ def test_few_token_form_splits_k_to_eight_sources(native_lib):
         kblocks, ntn = K // 64, -(-N // 256)
         kper = -(-kblocks // ks)
         assert ks in (1, 2, 4, 8) and T * N * 4 * ks <= cap and ntn * ks <= 148 and (ks - 1) * kper < kblocks
+
+
+def test_ctas_of_the_row_kernel_are_told_by_the_device(native_lib):
+    """Without a device there is no answer, the second time neither: a query that failed is an error of the call, not one CTA per SM from then on."""
+    f, there = native_lib.yali_c_fused_row_places, torch.cuda.is_available()
+    for N, ranks, split, lines, slim in [(4096, 2, 1, 0, 1), (4096, 2, 0, 0, 0), (4096, 1, 1, 1, 1), (512, 4, 0, 0, 1), (128, 1, 1, 0, 0)]:
+        first = f(0, N, ranks, split, lines, slim)
+        assert (1 <= first <= 32 if there else first == 0) and f(0, N, ranks, split, lines, slim) == first
+        assert f(1000, N, ranks, split, lines, slim) == first  # beyond the table of devices
 
 
 def test_one_shot_tile_form_splits_k(native_lib):

@@ -96,6 +96,7 @@ def _declare(lib: ctypes.CDLL) -> None:
         "yali_c_fused_tiling": (None, [u32, u32, i32, i32, u32, u32, vp]),
         "yali_c_fused_item": (None, [vp, u32, u32, u32, u32, u32, vp]),
         "yali_c_local_gemm_shape": (None, [u32, u32, u32, u64, u32, i32, vp]),
+        "yali_c_fused_row_places": (u32, [i32, u32, i32, i32, i32, i32]),
         "yali_c_fused_decode_split": (u32, [u32, u32, u32, i32, u32, u64, u32]),
         "yali_c_fused_decode_tile": (u32, [u32, u32, u32]),
         "yali_c_fused_tile_split": (u32, [u32, u32, u32, i32, u32, u64, u32]),
