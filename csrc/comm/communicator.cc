@@ -527,9 +527,9 @@ Result Communicator::LaunchLocal(const Plan& plan, const void* const* send, void
     } else {
         const bool rs = plan.flags & kFlagReduceScatterOnly, ag = plan.flags & kFlagAllGatherOnly;
         name = rs ? "local_reduce_scatter" : ag ? "local_all_gather" : "local_sum";
-        bool wide = DtypeSize(out) > DtypeSize(in);
-        for (int i = 0; i < nlocal() && wide; ++i)
-            wide = ((reinterpret_cast<uintptr_t>(send[i]) | reinterpret_cast<uintptr_t>(recv[i])) & 31u) == 0;
+        bool wide = DtypeSize(out) > DtypeSize(in) && (plan.flags & kFlagVecOk);  // (Inputs are loaded 16 bytes at a time either way.)
+        for (int i = 0; i < nlocal() && wide; ++i) wide = (reinterpret_cast<uintptr_t>(recv[i]) & 31u) == 0;
+        if (wide) a.flags |= kFlagWideStores;
         fn = LocalKernelFor(in, out, world_, rs ? LocalKind::ReduceScatter : ag ? LocalKind::AllGather : LocalKind::Sum, wide);
         const uint64_t unit = 16 / std::min(DtypeSize(in), DtypeSize(out));
         const uint64_t span = rs || ag ? std::min(plan.shard_elems, count) : count;
@@ -555,7 +555,7 @@ Result Communicator::LaunchLocal(const Plan& plan, const void* const* send, void
     last_.variant = plan.variant;
     last_.ctas = grid.x * grid.y;
     last_.slot_bytes = last_.stages = 0;
-    last_.flags = plan.flags;
+    last_.flags = a.flags;
     last_.kernel = name;
     static const int debug_level = env::DebugLevel();
     if (debug_level > 1)

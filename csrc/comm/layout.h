@@ -180,6 +180,7 @@ enum CollFlags : uint32_t {
     kFlagPullOneShot = 1u << 8, // pipelined kernel: every rank pulls and sums the whole message (no pushes)
     kFlagHostMemory = 1u << 10,  // with kFlagOneLaunch: the buffers are page-locked host memory
     kFlagOneLaunch = 1u << 9,   // all ranks share one GPU and one launch: no exchange (kernels/local_group.cu)
+    kFlagWideStores = 1u << 11,  // with kFlagOneLaunch: a sum to a wider type that stores 32 bytes at a time
 };
 
 // All ranks of an emulated communicator in one launch (ranks = blockIdx.y).

@@ -79,7 +79,7 @@ inline uint64_t LocalNormCtas(uint64_t rows, int world, const LocalNormShape& s)
     return rows * ((world + s.ranks_per_cta - 1) / s.ranks_per_cta);
 }
 
-// nullptr when the combination is not built.  `wide`: every buffer starts on a 32-byte
+// nullptr when the combination is not built.  `wide`: every output starts on a 32-byte
 // boundary (sums to a type of twice the width store 32 bytes at a time).
 const void* LocalKernelFor(Dtype in, Dtype out, int world, LocalKind kind, bool wide);
 // Sum of buffers in host memory that the GPU can address; any number of CTAs.

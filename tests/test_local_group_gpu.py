@@ -14,7 +14,7 @@ import yali_b200 as yali
 
 pytestmark = pytest.mark.gpu
 
-ONE_LAUNCH = 1 << 9
+ONE_LAUNCH, WIDE_STORES = 1 << 9, 1 << 11
 F32, F16, BF16 = torch.float32, torch.float16, torch.bfloat16
 
 
@@ -55,14 +55,15 @@ def test_sum(comm, src, dst, n):
 @pytest.mark.parametrize("src,dst", [(BF16, F32), (F16, F32), (F32, BF16), (F32, F16)])
 @pytest.mark.parametrize("n", [8, 15, 4096, 4103, 400003, 3000001])
 def test_sum_to_another_width_on_and_off_32_byte_boundaries(comm, src, dst, n):
-    """Units of 32 bytes are stored in one access where every buffer allows it; one rank's input or output starts 16 bytes behind such a boundary."""
+    """Units of 32 bytes are stored in one access where every output allows it; one rank's input or output starts 16 bytes behind such a boundary."""
     size = lambda t: torch.empty(0, dtype=t).element_size()  # noqa: E731
     for in_off, out_off in ((0, 0), (16 // size(src), 0), (0, 16 // size(dst))):
         xs = [whole((n,), src, n + r, in_off if r == 0 else 0) for r in range(comm.world)]
         ys = [whole((n + 8,), dst, 1, out_off if r == comm.world - 1 else 0) for r in range(comm.world)]
         tails = [y[n:].clone() for y in ys]
         comm.all_reduce(xs, [y[:n] for y in ys], scale=0.5)
-        assert comm.last_call()["flags"] & ONE_LAUNCH
+        flags = comm.last_call()["flags"]
+        assert flags & ONE_LAUNCH and bool(flags & WIDE_STORES) == (dst == F32 and out_off == 0)
         want = total(xs) * 0.5
         for y, tail in zip(ys, tails):
             assert torch.equal(y[:n].double(), want) and torch.equal(y[n:], tail)
