@@ -390,8 +390,9 @@ namespace {
 // Pauses between two looks at a flag and at a line.  Polling costs the GEMM more than a late look costs the row: with 50 ns
 // and all lines asked for on every look, us: 2 ranks, K = 2048: T = 8 10.0 -> 9.8, T = 64 17.3 -> 14.6, T = 128 18.3 -> 16.5
 // (flags, 3000 ns level, 600 ns 16.8); 4 ranks, K = 1792, T = 100 20.4 -> 18.5 (3000 ns 20.5, 1000 ns 19.1).  Lines: 0 to 100 ns
-// are level.  Once one flag of a tile is set, the others are not far: 8 ranks, 678 x 640 x 1664 31.0 -> 29.3 us, 688 x 1792 x 2816
-// 67.5 -> 65.5 (100 and 400 ns are level).
+// are level.  Once one of a warp's flags is set, the others are not far: kFlagNearNs from then on against 1500 ns always / 400 ns always, us: 2 ranks,
+// 182 x 832 x 3072 10.6 / 10.8 / 11.4, 96 x 2048 x 2048 10.5 / 10.6 / 11.3, 300 x 2048 x 4096 19.7 / 20.4 / 19.9; 4 ranks, 1500 x 640 x 1536 26.1
+// / 26.6 / 26.3; 8 ranks, 678 x 640 x 1664 28.9 / 29.4 / 29.1, 418 x 704 x 1152 18.7 / 18.7 / 19.5; of 25 sizes 1.2 % and 1.6 % in the mean.
 constexpr uint32_t kFlagSleepNs = 1500, kFlagNearNs = 400, kLineSleepNs = 40;
 
 // A unit of work is a row for G ranks (unit u: row u / ngroups, ranks from (u % ngroups) * G); a thread holds NV 16-byte
@@ -505,16 +506,17 @@ __global__ void __launch_bounds__(kLocalLinearNormThreads) __maxnreg__(LocalLine
             // The flags of this row's token tile, a few per thread.
             while (row >= tile_end) tile_end += a.s.tokens, ++tile;
             const uint32_t first = kLocalGemmFlagOff + (tile - 1) * nsplit * flags_per_split;
-            // (There are no more flags than threads: at most eight splits of one flag per 128 columns.)
+            static_assert(kLocalGemmMaxSplit * VEC * NV <= kLocalGemmUnitCols, "a thread waits for one flag: a split's columns / kLocalGemmUnitCols");
             bool there = tid >= nsplit * flags_per_split || late;
+            const uint32_t mine = __ballot_sync(0xffffffffu, !there);  // lanes that have a flag
             for (uint32_t polls = 1;; ++polls) {
                 uint32_t seen = 0;
                 if (!there) there = ptx::seq_reached(seen = ptx::ld_acquire_gpu(flag_word(cv, 0, first + tid)), epoch);
                 const uint32_t waiting = __ballot_sync(0xffffffffu, !there);
                 if (waiting == 0) break;
-                // This CTA shares the SM with the GEMM, and hundreds of them poll; but once the first unit of the tile is there, the
+                // This CTA shares the SM with the GEMM, and hundreds of them poll; but once the first of a warp's units is there, the
                 // last one is not far.
-                if (polls > 2) ptx::nanosleep(waiting == 0xffffffffu ? kFlagSleepNs : kFlagNearNs);
+                if (polls > 2) ptx::nanosleep(waiting == mine ? kFlagSleepNs : kFlagNearNs);
                 if ((polls & 7u) == 0 && __any_sync(0xffffffffu, ptx::globaltimer() > deadline)) {
                     if (!there) report_timeout(cv, kSiteGemmPartials, 0, blockIdx.x, epoch, seen);
                     late = true;
