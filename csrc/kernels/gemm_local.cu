@@ -413,7 +413,7 @@ constexpr uint32_t kFlagSleepNs = 1500, kFlagNearNs = 400, kLineSleepNs = 40;
 // 2 ranks: 188 x 1024 x 2944 13.5 / 11.9, 2048 x 2048 x 4096 level.  Of the 16 us that the rows of 8 x 300 x 4096 take behind the GEMM
 // for 59 MB, 2 go by before the first row is complete and 3 while the last CTAs finish.
 template <int NV, int G, bool SPLIT, bool LINES, bool SLIM>
-__global__ void __launch_bounds__(kLocalLinearNormThreads) __maxnreg__(LocalLinearNormRegs(NV, G, SPLIT, SLIM))
+__global__ void __maxnreg__(LocalLinearNormRegs(NV, G, SPLIT, SLIM))
     local_linear_norm_kernel(const __grid_constant__ LocalLinearNormArgs a) {
     constexpr int VEC = 8, kMostWarps = kLocalLinearNormThreads / 32;
     __shared__ __align__(16) float s_red[G][kMostWarps];

@@ -211,12 +211,12 @@ __global__ void __launch_bounds__(kLocalHostThreads) local_host_kernel(const __g
     local_trace_end(a);
 }
 
-// Registers per thread of the norm kernel.  What counts is the warps that share an SM: 2 ranks, 2048 x 4096 bf16 22.9 us with 40
-// registers, 23.4 with 64.
-constexpr int norm_regs(int world, int nv, int g, bool late, int elem_bytes) {
-    if (world == 1) return nv == 1 ? 32 : (nv == 2 ? 48 : 96) - (elem_bytes == 4 ? nv * 8 - 8 : 0);
-    if (nv == 1) return late ? 40 : 64;
-    return nv == 2 ? 64 : g == 1 && world < 5 ? 96 : 128;
+// CTAs of 512 threads of the norm kernel that share an SM, which caps their registers at 32, 40, 64 or 128.  What counts is the warps that share an
+// SM: 2 ranks, 2048 x 4096 bf16 22.9 us with 40 registers, 23.4 with 64; 2 ranks, 1024 x 8192 fp32 43.2 with 64, 47.7 with the 72 that it
+// takes by itself.
+constexpr int norm_ctas(int world, int nv, bool late, int elem_bytes) {
+    if (nv == 1) return world == 1 ? 4 : late ? 3 : 2;
+    return nv == 2 || (world == 2 && late && elem_bytes == 4) ? 2 : 1;
 }
 
 // Sum + residual + RMSNorm of one row for the ranks [g * G, g * G + G) of the group; CTA b handles row
@@ -233,7 +233,7 @@ constexpr int norm_regs(int world, int nv, int g, bool late, int elem_bytes) {
 // 2 ranks: 64 x 8192 4.1 / 2.9, 2000 x 8192 44.6 / 41.7 (40.2), 2048 x 4096 22.9 / 22.8 (20.6); 3 ranks, 1500 x 4096 45 / 27.4 (22.6); one rank,
 // 8192 x 8192 83.6 / 82.2 (82.2); fp32, 8 ranks, 250 x 8192 71.8 / 49.6 (40.2).
 template <typename T, int WORLD, int NV, int G, bool LATE>
-__global__ void __launch_bounds__(kLocalThreads) __maxnreg__(norm_regs(WORLD, NV, G, LATE, sizeof(T))) local_norm_kernel(const __grid_constant__ LocalArgs a) {
+__global__ void __launch_bounds__(kLocalThreads, norm_ctas(WORLD, NV, LATE, sizeof(T))) local_norm_kernel(const __grid_constant__ LocalArgs a) {
     constexpr int VEC = TypeTraits<T>::kVec, kMostWarps = kLocalThreads / 32;
     constexpr uint32_t W = WORLD;
     __shared__ __align__(16) float s_red[G][kMostWarps];
@@ -259,16 +259,27 @@ __global__ void __launch_bounds__(kLocalThreads) __maxnreg__(norm_regs(WORLD, NV
 
     uint4 res[NV][G], wgt[NV][LATE ? 1 : G];
     float f[NV][VEC];
-#pragma unroll
-    for (int j = 0; j < NV; ++j) {
-        uint4 x[W];
-#pragma unroll
-        for (int q = 0; q < WORLD; ++q) x[q] = ptx::ld_cg_v4(static_cast<const char*>(a.send[q]) + row_off + at[j]);
+    auto load_residuals = [&](int j) {
 #pragma unroll
         for (int g = 0; g < G; ++g) {
             const char* const r = q0 + g < W ? static_cast<const char*>(a.residual[q0 + g]) : nullptr;
             res[j][g] = r ? ptx::ld_cg_v4(r + row_off + at[j]) : make_uint4(0, 0, 0, 0);
         }
+    };
+    // Residuals ahead of all inputs or with the inputs of their vector: how many loads the compiler leaves in flight under its cap depends on it (us,
+    // ahead / with: fp32, 3 ranks 300 x 8192 23.2 / 26.1, 5 ranks 40 x 8192 8.1 / 8.6, 7 ranks 60 x 4096 8.1 / 10.3; but 6 ranks 300 x 8192 46.7 / 44.0,
+    // 8 ranks 120 x 4096 15.9 / 15.5, bf16 500 x 8192 49.8 / 48.3).
+    constexpr bool kResidualsFirst = sizeof(T) == 4 && WORLD > 1 && (WORLD & 1);
+    if constexpr (kResidualsFirst) {
+#pragma unroll
+        for (int j = 0; j < NV; ++j) load_residuals(j);
+    }
+#pragma unroll
+    for (int j = 0; j < NV; ++j) {
+        uint4 x[W];
+#pragma unroll
+        for (int q = 0; q < WORLD; ++q) x[q] = ptx::ld_cg_v4(static_cast<const char*>(a.send[q]) + row_off + at[j]);
+        if constexpr (!kResidualsFirst) load_residuals(j);
         unpack16<T>(f[j], x[0]);
 #pragma unroll
         for (int q = 1; q < WORLD; ++q) accumulate<T>(f[j], x[q]);

@@ -1,6 +1,7 @@
 """Tooling without a GPU: statistics, report generation from sweep lines, nccl-tests log parsing, NVLink status
 parsing, the launcher, and the baseline validator's version check."""
 import json
+import re
 import subprocess
 import sys
 from pathlib import Path
@@ -208,3 +209,10 @@ def test_fused_layer_output_buffer_is_cached_per_shape():
     y4 = comm.fused_linear_rmsnorm(x, w, g)
     assert impl.allocs == 3 and tuple(y4.shape) == (6, 16)
     comm.close()
+
+
+def test_kernels_cap_their_registers_in_one_way():
+    """CUDA's guide: __launch_bounds__ and __maxnreg__ cannot be applied to the same kernel."""
+    for path in sorted((ROOT / "csrc").rglob("*.cu")):
+        for head in re.findall(r"__global__[^{;]*", path.read_text()):
+            assert not ("__launch_bounds__" in head and "__maxnreg__" in head), (path.name, head.split("(")[0])
