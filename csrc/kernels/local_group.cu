@@ -382,8 +382,9 @@ const void* pick_same(Dtype dt, int world) {
 // The instances that LocalNormShapeFor asks for; nullptr for others.
 template <typename T, int WORLD, int NV, int G>
 const void* pick_norm_late(bool late) {
-    constexpr bool kEarly = NV == 1 || G == 1 || (sizeof(T) == 4 && WORLD == 2 && NV == 2);
-    constexpr bool kLate = WORLD > 1 && (NV == 1 ? G == 2 && WORLD != 4 : NV == 2 ? G == 2 : G == (WORLD == 2 ? 1 : 2));
+    constexpr bool kPairEarly = sizeof(T) == 4 && WORLD == 2 && NV == 2;
+    constexpr bool kEarly = NV == 1 || G == 1 || kPairEarly;
+    constexpr bool kLate = WORLD > 1 && (NV == 1 ? G == 2 && WORLD != 4 : NV == 2 ? G == 2 && !kPairEarly : G == (WORLD == 2 ? 1 : 2));
     if constexpr (kLate) {
         if (late) return (const void*)local_norm_kernel<T, WORLD, NV, G, true>;
     }
