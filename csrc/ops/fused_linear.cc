@@ -437,11 +437,14 @@ Result LaunchLocal(Communicator& comm, const DriverApi* drv, const FusedLinearDe
     const bool split = g.s.nsplit > 1;
     const bool narrow = LocalLinearNormVectors(N) == 1;
     auto units_of = [&](int gr) { return static_cast<uint32_t>(T * ((W + gr - 1) / gr)); };
-    // Lines of one rank: while a CTA has its share of an SM beside the GEMM to itself, it may ask for the lines of four splits at a time instead
-    // of one or two, which pays with many splits and few rows (slim / not: 2 ranks, 8 x 2048 x 4096, 4 splits 10.2 / 9.5; 4 ranks, 10 x
-    // 1024 x 3072, 6 splits 9.1 / 8.5, 32 x 512 x 2304, 8 splits 9.5 / 7.9; 8 ranks, 8 x 1792 x 4096, 4 splits 24.3 / 24.9; 2 ranks, 64 x 2048 x
-    // 3328, 5 splits 10.2 / 10.5).  Narrow rows: 8 ranks, 24 x 512 x 1024 7.2 / 6.9, 30 x 1024 x 2048 11.7 / 13.6.
-    bool slim = units_of(1) * threads > 256 * sms || (!narrow && units_of(1) > (g.s.nsplit > 5 ? sms : 32u));
+    // Lines of one rank: the instance that is not slim asks for the lines of four splits at a time instead of one or two, in registers that leave
+    // no room for a second CTA beside the GEMM's.  Wide rows: with six to eight splits that pays while every SM has one unit and a few have a second one
+    // (slim / not, us: 8 ranks, 17 x 256 x 2176, 136 units 9.4 / 7.8; 6 ranks, 26 x 1792 x 2432, 156 units 15.5 / 14.2, 28 x 768 x 2816, 168 units 10.8 /
+    // 12.4; 8 ranks, 35 x 1536 x 3072, 280 units 20.0 / 23.7), with fewer while there are few threads per SM (2 ranks, 40 x 512 x 2176, 86 threads 7.1 /
+    // 6.7; 4 ranks, 12 x 1024 x 3328, 73 10.1 / 9.3; 4 ranks, 17 x 1536 x 3584, 103 12.2 / 12.9; 2 ranks, 64 x 1024 x 3328, 194 9.7 / 10.4; 5 ranks, 30 x 1280 x
+    // 3200, 227 12.1 / 15.7).  Of 129 sizes the worst loses 7 %, the mean 0.3 %.  Narrow rows: 8 ranks, 24 x 512 x 1024 7.2 / 6.9, 30 x 1024 x 2048 11.7 /
+    // 13.6.
+    bool slim = narrow ? units_of(1) * threads > 256 * sms : g.s.nsplit > 5 ? units_of(1) > sms + sms / 18 : units_of(1) * threads > 100 * sms;
     cudaError_t asked = cudaSuccess;
     auto places_of = [&](int gr, bool slim) {
         uint32_t n = 1;
