@@ -293,18 +293,31 @@ def test_flag_in_data_form_for_small_messages(comm, dtype):
     check(comm, outs, dtype, scale=0.25)
 
 
-@pytest.mark.parametrize("mode", ["auto", "stream"])
-def test_rmsnorm_beyond_the_one_shot_capacity(comm, mode):
+def test_rmsnorm_beyond_the_one_shot_capacity_uses_two_launches(comm):
     hidden = 4096
     rows = comm.layout()["flash_cap"] // (hidden * 2) + 64  # just above the one-shot staging
     xs = [x.view(rows, hidden) for x in make_inputs(comm, rows * hidden, torch.bfloat16, NORMAL)]
     g = torch.Generator(device="cpu").manual_seed(11)
     weight = (torch.rand(hidden, generator=g) + 0.5).to(torch.bfloat16).cuda()
     before = comm.launches
-    outs = comm.all_reduce_rmsnorm(xs, [weight] * comm.world, None, eps=1e-5, mode=mode)
+    outs = comm.all_reduce_rmsnorm(xs, [weight] * comm.world, None, eps=1e-5, mode="stream")
     comm.sync()
-    # One launch; by a mode of the caller's one all-reduce and one norm kernel per rank.
-    assert comm.launches - before == (1 if mode == "auto" else 1 + comm.world)
+    assert comm.launches - before == 1 + comm.world  # one cooperative all-reduce + one norm kernel per rank
+    ref, _ = yali.reference.residual_rmsnorm(yali.reference.all_reduce_sum(xs), weight.cpu().double(), None, 1e-5)
+    torch.testing.assert_close(outs[0][:256].cpu().double(), ref[:256], rtol=3e-2, atol=3e-2)
+    torch.testing.assert_close(outs[-1][-256:].cpu().double(), ref[-256:], rtol=3e-2, atol=3e-2)
+
+
+def test_rmsnorm_beyond_the_one_shot_capacity_in_one_launch(comm):
+    hidden = 4096
+    rows = comm.layout()["flash_cap"] // (hidden * 2) + 64  # just above the one-shot staging
+    xs = [x.view(rows, hidden) for x in make_inputs(comm, rows * hidden, torch.bfloat16, NORMAL)]
+    g = torch.Generator(device="cpu").manual_seed(11)
+    weight = (torch.rand(hidden, generator=g) + 0.5).to(torch.bfloat16).cuda()
+    before = comm.launches
+    outs = comm.all_reduce_rmsnorm(xs, [weight] * comm.world, None, eps=1e-5)
+    comm.sync()
+    assert comm.launches - before == 1
     ref, _ = yali.reference.residual_rmsnorm(yali.reference.all_reduce_sum(xs), weight.cpu().double(), None, 1e-5)
     torch.testing.assert_close(outs[0][:256].cpu().double(), ref[:256], rtol=3e-2, atol=3e-2)
     torch.testing.assert_close(outs[-1][-256:].cpu().double(), ref[-256:], rtol=3e-2, atol=3e-2)

@@ -14,7 +14,8 @@ import yali_b200 as yali
 
 pytestmark = pytest.mark.gpu
 
-ONE_LAUNCH, WIDE_STORES = 1 << 9, 1 << 11
+ONE_LAUNCH = 1 << 9
+WIDE_STORES = 1 << 11
 F32, F16, BF16 = torch.float32, torch.float16, torch.bfloat16
 
 
@@ -55,18 +56,29 @@ def test_sum(comm, src, dst, n):
 @pytest.mark.parametrize("src,dst", [(BF16, F32), (F16, F32), (F32, BF16), (F32, F16)])
 @pytest.mark.parametrize("n", [8, 15, 4096, 4103, 400003, 3000001])
 def test_sum_to_another_width_on_and_off_32_byte_boundaries(comm, src, dst, n):
-    """Units of 32 bytes are stored in one access where every output allows it; one rank's input or output starts 16 bytes behind such a boundary."""
+    """Units of 32 bytes are stored in one access where every buffer allows it; one rank's input or output starts 16 bytes behind such a boundary."""
     size = lambda t: torch.empty(0, dtype=t).element_size()  # noqa: E731
     for in_off, out_off in ((0, 0), (16 // size(src), 0), (0, 16 // size(dst))):
         xs = [whole((n,), src, n + r, in_off if r == 0 else 0) for r in range(comm.world)]
         ys = [whole((n + 8,), dst, 1, out_off if r == comm.world - 1 else 0) for r in range(comm.world)]
         tails = [y[n:].clone() for y in ys]
         comm.all_reduce(xs, [y[:n] for y in ys], scale=0.5)
-        flags = comm.last_call()["flags"]
-        assert flags & ONE_LAUNCH and bool(flags & WIDE_STORES) == (dst == F32 and out_off == 0)
+        assert comm.last_call()["flags"] & ONE_LAUNCH
         want = total(xs) * 0.5
         for y, tail in zip(ys, tails):
             assert torch.equal(y[:n].double(), want) and torch.equal(y[n:], tail)
+
+
+@pytest.mark.parametrize("src,dst", [(BF16, F32), (F16, F32), (F32, BF16)])
+def test_32_byte_stores_ask_for_outputs_on_32_byte_boundaries_only(comm, src, dst):
+    n, size = 4103, lambda t: torch.empty(0, dtype=t).element_size()  # noqa: E731
+    for in_off, out_off in ((0, 0), (16 // size(src), 0), (0, 16 // size(dst))):
+        xs = [whole((n,), src, n + r, in_off if r == 0 else 0) for r in range(comm.world)]
+        ys = [whole((n,), dst, 1, out_off if r == comm.world - 1 else 0) for r in range(comm.world)]
+        comm.all_reduce(xs, ys)
+        flags = comm.last_call()["flags"]
+        assert flags & ONE_LAUNCH and bool(flags & WIDE_STORES) == (dst == F32 and out_off == 0)
+        assert all(torch.equal(y.double(), total(xs)) for y in ys)
 
 
 @pytest.mark.parametrize("dtype", [F32, BF16])
@@ -172,13 +184,11 @@ def test_norm_of_the_one_shot_kernel(comm, dtype, rows, hidden):
             torch.testing.assert_close(y[r].double(), ref, rtol=rtol, atol=1e-6)
 
 
-# Row lengths by 16-byte vectors per thread of the norm kernels (128 / 129 / 1024 / 1025 / 2048 vectors), one that is no whole
+# Row lengths by 16-byte vectors per thread of the norm kernel (128 / 129 / 1024 / 1025 / 2048 vectors), one that is no whole
 # number of vectors, and one weight off a 16-byte boundary.
-@pytest.mark.parametrize("mode", ["auto", "stream"])
 @pytest.mark.parametrize("dtype,hidden,off", [(BF16, 1024, 0), (BF16, 1032, 0), (F16, 8192, 0), (F32, 4100, 0), (F32, 8192, 0), (BF16, 1001, 0), (BF16, 1024, 1)])
-def test_norm_beyond_the_one_shot_staging(comm, dtype, hidden, off, mode):
-    """Right above the staging's size: one launch, or, in a mode of the caller's and for rows that the row kernel does not take, the sum and then a kernel
-    per rank that normalises its rows, 1 + world launches."""
+def test_norm_beyond_the_one_shot_staging(comm, dtype, hidden, off):
+    """Above the staging's size the sum comes first and a kernel per rank normalises its rows: 1 + world launches."""
     if comm.world == 1:
         pytest.skip("a group of one stages nothing")
     W, rtol = comm.world, {F32: 2e-6, F16: 2.0 ** -10, BF16: 2.0 ** -7}[dtype]
@@ -186,9 +196,9 @@ def test_norm_beyond_the_one_shot_staging(comm, dtype, hidden, off, mode):
     xs = [whole((rows, hidden), dtype, r) for r in range(W)]
     res, ws = [whole((rows, hidden), dtype, 50 + r) for r in range(W)], [whole((hidden,), dtype, 90 + r, off) for r in range(W)]
     pre, before = [torch.empty_like(x) for x in xs], comm.launches
-    ys = comm.all_reduce_rmsnorm(xs, ws, res, eps=1e-5, residual_out=pre, mode=mode)
-    assert comm.launches - before == (1 if mode == "auto" and hidden != 1001 and not off else 1 + W)
-    plain = comm.all_reduce_rmsnorm(xs, ws, None, eps=1e-5, mode=mode)
+    ys = comm.all_reduce_rmsnorm(xs, ws, res, eps=1e-5, residual_out=pre, mode="stream")
+    assert comm.launches - before == 1 + W
+    plain = comm.all_reduce_rmsnorm(xs, ws, None, eps=1e-5, mode="stream")
     comm.sync()
     pick = torch.tensor([0, 1, rows // 2, rows - 2, rows - 1], device="cuda")
     s = total([x[pick] for x in xs])
@@ -198,6 +208,26 @@ def test_norm_beyond_the_one_shot_staging(comm, dtype, hidden, off, mode):
             torch.testing.assert_close(got[pick].double(), ref, rtol=rtol, atol=1e-6)
         assert torch.equal(pre[r][pick].double(), s + res[r][pick].double())
         assert torch.equal(pre[r].float(), sum(x.float() for x in xs) + res[r].float())
+
+
+# (One row length of each number of vectors per thread, and the two forms that the row kernel does not take.)
+@pytest.mark.parametrize("dtype,hidden,off,launches", [(BF16, 1024, 0, 1), (F16, 8192, 0, 1), (F32, 4100, 0, 1), (F32, 8192, 0, 1), (BF16, 1001, 0, 2), (BF16, 1024, 1, 2)])
+def test_norm_right_above_the_one_shot_staging(comm, dtype, hidden, off, launches):
+    """One launch, like any larger size, and two passes only for rows that the row kernel does not take."""
+    if comm.world == 1:
+        pytest.skip("a group of one stages nothing")
+    W, rtol = comm.world, {F32: 2e-6, F16: 2.0 ** -10, BF16: 2.0 ** -7}[dtype]
+    rows = comm.layout()["flash_cap"] // (hidden * torch.empty(0, dtype=dtype).element_size()) + 3
+    xs, res = [whole((rows, hidden), dtype, r) for r in range(W)], [whole((rows, hidden), dtype, 50 + r) for r in range(W)]
+    ws, pre, before = [whole((hidden,), dtype, 90 + r, off) for r in range(W)], [torch.empty_like(x) for x in xs], comm.launches
+    ys = comm.all_reduce_rmsnorm(xs, ws, res, eps=1e-5, residual_out=pre)
+    assert comm.launches - before == (1 if launches == 1 else 1 + W)
+    s = sum(x.float() for x in xs)
+    for r in (0, W - 1):
+        row = s + res[r].float()
+        assert torch.equal(pre[r].float(), row)
+        ref = row * torch.rsqrt(row.double().pow(2).mean(-1, keepdim=True) + 1e-5) * ws[r].double()
+        torch.testing.assert_close(ys[r].double(), ref, rtol=rtol, atol=1e-6)
 
 
 @pytest.mark.parametrize("dtype,hidden", [(BF16, 4096), (F16, 1000), (F32, 8192)])
