@@ -357,6 +357,38 @@ def test_norms_whose_ranks_share_an_output(comm, rows, hidden, mode):
             torch.testing.assert_close(outs[k].float(), want[r], rtol=2.0 ** -7, atol=1e-6)
 
 
+@pytest.mark.parametrize("mode", ["auto", "stream"])
+def test_norms_that_take_memory_for_a_call_replay_from_a_graph(comm, mode):
+    """An output on the rank's own residual (in two passes read from a copy) and one output for every rank, captured in one graph and replayed."""
+    W, hidden = comm.world, 4096
+    if W == 1:
+        pytest.skip("one output, and a group of one stages nothing")
+    rows = (comm.layout()["flash_cap"] + (1 << 20)) // (2 * hidden) + 1
+    xs = [whole((rows, hidden), BF16, r) for r in range(W)]
+    res, ws = [whole((rows, hidden), BF16, 50 + r) for r in range(W)], [whole((hidden,), BF16, 90 + r) for r in range(W)]
+    pre = [sum(x.float() for x in xs) + r.float() for r in res]
+    want = [p * torch.rsqrt(p.pow(2).mean(-1, keepdim=True) + 1e-5) * w.float() for p, w in zip(pre, ws)]
+    own, one = [r.clone() for r in res], torch.empty_like(res[0])
+
+    def calls():
+        comm.all_reduce_rmsnorm(xs, ws, own, eps=1e-5, out=own, mode=mode)
+        comm.all_reduce_rmsnorm(xs, ws, res, eps=1e-5, out=[one] * W, mode=mode)
+
+    calls()
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        calls()
+    for _ in range(2):
+        for o, r in zip(own, res):
+            o.copy_(r)
+        one.zero_()
+        graph.replay()
+        torch.cuda.synchronize()
+        for y, w in zip(own + [one], want + want[-1:]):
+            torch.testing.assert_close(y.float(), w, rtol=2.0 ** -7, atol=1e-6)
+
+
 @pytest.mark.parametrize("odd", ["x", "weight", "residual", "out", "residual_out"])
 @pytest.mark.parametrize("mode", ["auto", "flash"])
 def test_norm_refuses_tensors_off_a_16_byte_boundary(comm, odd, mode):
