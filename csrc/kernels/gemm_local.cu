@@ -411,7 +411,8 @@ constexpr uint32_t kFlagSleepNs = 1500, kFlagNearNs = 400, kLineSleepNs = 40;
 // 1500 x 512 x 2304 68.9 / 53.4, 678 x 640 x 1664 33.4 / 29.0, 688 x 1792 x 2816 72.9 / 65.4, 300 x 1792 x 4096 51.0 / 49.0, 32 x 1792 x 4096
 // 31.0 / 26.9, 21 x 384 x 3328 11.9 / 9.4; 4 ranks: 300 x 512 x 1024 14.7 / 10.4, 512 x 2048 x 4096 41.7 / 40.2, 60 x 256 x 3072 10.5 / 8.4;
 // 2 ranks: 188 x 1024 x 2944 13.5 / 11.9, 2048 x 2048 x 4096 level.  Of the 16 us that the rows of 8 x 300 x 4096 take behind the GEMM
-// for 59 MB, 2 go by before the first row is complete and 3 while the last CTAs finish.
+// for 59 MB, 2 go by before the first row is complete and 3 while the last CTAs finish (1200 units on 296 places, two CTAs of 96 registers per SM:
+// 16 units are left for a fifth round).
 template <int NV, int G, bool SPLIT, bool LINES, bool SLIM>
 __global__ void __maxnreg__(LocalLinearNormRegs(NV, G, SPLIT, SLIM))
     local_linear_norm_kernel(const __grid_constant__ LocalLinearNormArgs a) {

@@ -213,7 +213,10 @@ __global__ void __launch_bounds__(kLocalHostThreads) local_host_kernel(const __g
 
 // CTAs of 512 threads of the norm kernel that share an SM, which caps their registers at 32, 40, 64 or 128.  What counts is the warps that share an
 // SM: 2 ranks, 2048 x 4096 bf16 22.9 us with 40 registers, 23.4 with 64; 2 ranks, 1024 x 8192 fp32 43.2 with 64, 47.7 with the 72 that it
-// takes by itself.
+// takes by itself.  13 instances spill 4 to 12 bytes under it: four ranks per CTA in bf16 and fp16, and three of seven ranks behind the barrier.
+// One CTA per SM less and no spills cost more (us, as it is / without): 8 ranks, 256 x 4096 bf16 14.2 / 17.9, 180 x 4096 11.3 / 13.3; 4 ranks, 256 x 4096
+// bf16 7.9 / 9.7, 300 x 4096 fp16 10.6 / 12.0, but 512 x 2944 11.6 / 11.2; 5 ranks, 300 x 4096 fp16 level; 7 ranks, 1000 x 4096 bf16 45.6 / 51.1,
+// 300 x 8192 fp16 29.2 / 36.8.
 constexpr int norm_ctas(int world, int nv, bool late, int elem_bytes) {
     if (nv == 1) return world == 1 ? 4 : late ? 3 : 2;
     return nv == 2 || (world == 2 && late && elem_bytes == 4) ? 2 : 1;
